@@ -1171,6 +1171,156 @@ pgk_status launch_bonded_hf(pgk_ctx* c, const HfDev& h) {
     return PGK_OK;
 }
 
+// The same terms straight into the heat flux's region sums (FluxDev): a
+// pair's calvirihf share is fact (f_i . v_i - f_j . v_j).  Every thread keeps
+// its own column of sums in shared memory (no atomics inside the block), one
+// (potential, virial) pair per region; a block's terms are of one type.
+// FP64 latency of one term per thread bounds it; one launch for all types.
+struct FluxTerms {
+    int n[5], b0[6];                 // terms and first block of bonds, angles, torsions, RB torsions, 1-4 pairs
+    const int2* bond; const double2* bond_p;
+    const int4* angl; const double2* angl_p;
+    const int4* tors; const double4* tors_p;
+    const int4* rb; const double* rb_c;
+    const int2* p14; const double2* p14_f;
+};
+#define FLUX_BT 64
+
+__device__ __forceinline__ void flux_pair(const FluxDev& f, const double* z, const uint4* b, const int* mol,
+                                          const double* v, double Lz, int p, int q, const double* fp,
+                                          const double* fq, double nbc, double* sv) {
+    if (mol[p] < 0 && mol[p] == mol[q]) return;                  // both molecule-based, same molecule
+    const double rz = z[p] - z[q], az = fabs(rz);
+    if (az * (1.0 / Lz) >= 0.5) return;
+    const double* vp = v + 3 * p;
+    const double* vq = v + 3 * q;
+    const double s = nbc * (fp[0] * vp[0] + fp[1] * vp[1] + fp[2] * vp[2] -
+                            (fq[0] * vq[0] + fq[1] * vq[1] + fq[2] * vq[2]));
+    const unsigned all = f.h.nreg >= 32 ? 0xffffffffu : (1u << f.h.nreg) - 1u;
+    unsigned t = ~((b[p].x & b[q].x) | (b[p].y & b[q].y)) & all;
+    while (t) {
+        const int r = __ffs(t) - 1;
+        t &= t - 1;
+        double frag;
+        if (hf_frag(z[p], z[q], f.h.z1[r], f.h.z2[r], az, frag)) sv[2 * FLUX_BT * r] += rz >= 0.0 ? s * frag : -s * frag;
+    }
+}
+
+__global__ void __launch_bounds__(FLUX_BT) k_bonded_flux(const double* __restrict__ pos, const double* __restrict__ chrg,
+                                                         const int* __restrict__ typ, int ntyp,
+                                                         const double2* __restrict__ lj64, FluxTerms t, FluxDev f,
+                                                         const DynState* __restrict__ dyn, unsigned* status) {
+    extern __shared__ double fsm[];                      // [nreg][potential, virial][FLUX_BT]
+    const int nreg = f.h.nreg;
+    for (int q = threadIdx.x; q < 2 * nreg * FLUX_BT; q += FLUX_BT) fsm[q] = 0.0;
+    __syncthreads();
+    double* sp = fsm + threadIdx.x;
+    double* sv = sp + FLUX_BT;
+    int ty = 0;
+    while (ty < 4 && (int)blockIdx.x >= t.b0[ty + 1]) ++ty;
+    const double Lz = dyn->box[2];
+    const int step = (t.b0[ty + 1] - t.b0[ty]) * FLUX_BT;
+    for (int k = ((int)blockIdx.x - t.b0[ty]) * FLUX_BT + threadIdx.x; k < t.n[ty]; k += step) {
+        int at[4] = {0, 0, 0, 0}, na = 2;
+        double F[4][3], rd[3], e = 0.0, share = 0.5;
+        bool on = true;
+        if (ty == 0) {
+            at[0] = t.bond[k].x; at[1] = t.bond[k].y;
+            on = eval_bond<double>(pos, at[0], at[1], t.bond_p[k], dyn, F[0], rd, e);
+        } else if (ty == 1) {
+            at[0] = t.angl[k].x; at[1] = t.angl[k].y; at[2] = t.angl[k].z;
+            na = 3; share = 1.0 / 3.0;
+            double G[3][3];
+            on = eval_angl<double>(pos, at[0], at[1], at[2], t.angl_p[k], dyn, G, e);
+            if (on)
+#pragma unroll
+                for (int q = 0; q < 9; ++q) F[q / 3][q % 3] = G[q / 3][q % 3];
+        } else if (ty == 2) {
+            at[0] = t.tors[k].x; at[1] = t.tors[k].y; at[2] = t.tors[k].z; at[3] = t.tors[k].w;
+            na = 4; share = 0.25;
+            eval_tors<double, false>(pos, at[0], at[1], at[2], at[3], t.tors_p[k], nullptr, dyn, F, e, status);
+        } else if (ty == 3) {
+            at[0] = t.rb[k].x; at[1] = t.rb[k].y; at[2] = t.rb[k].z; at[3] = t.rb[k].w;
+            na = 4; share = 0.25;
+            eval_tors<double, true>(pos, at[0], at[1], at[2], at[3], make_double4(0, 0, 0, 0), t.rb_c + 6 * (size_t)k,
+                                    dyn, F, e, status);
+        } else {
+            at[0] = t.p14[k].x; at[1] = t.p14[k].y;
+            double de, dv;
+            eval_14<double>(pos, at[0], at[1], chrg[at[0]] * chrg[at[1]], lj64[typ[at[0]] * ntyp + typ[at[1]]],
+                            t.p14_f[k], dyn, F[0], rd, de, dv);
+            e = de + dv;
+        }
+        if (!on) continue;
+        if (na == 2)
+            for (int d = 0; d < 3; ++d) F[1][d] = -F[0][d];
+        double z[4], v[12];
+        uint4 b[4];
+        int mol[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (q >= na) break;
+            const int i = at[q];
+            z[q] = hf_z(f.h, pos, i, Lz);
+            b[q] = flux_bits(f.h, z[q], Lz);
+            mol[q] = f.h.hftyp[i] == PGK_HFTYP_MOLE ? ~f.h.mol_of[i] : 0;     // negative: molecule-based
+            v[3 * q] = f.vel[3 * i]; v[3 * q + 1] = f.vel[3 * i + 1]; v[3 * q + 2] = f.vel[3 * i + 2];
+            const double tr = share * e * flux_vz(f, i);
+            unsigned in = b[q].z;
+            while (in) {
+                const int r = __ffs(in) - 1;
+                in &= in - 1;
+                sp[2 * FLUX_BT * r] += tr;
+            }
+        }
+        if (na == 3) {                                   // calangl_hf.F90: (i,j), (j,k), (k,i)
+            flux_pair(f, z, b, mol, v, Lz, 0, 1, F[0], F[1], share, sv);
+            flux_pair(f, z, b, mol, v, Lz, 1, 2, F[1], F[2], share, sv);
+            flux_pair(f, z, b, mol, v, Lz, 2, 0, F[2], F[0], share, sv);
+        } else {
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int q = p + 1; q < 4; ++q)
+                    if (q < na) flux_pair(f, z, b, mol, v, Lz, p, q, F[p], F[q], share, sv);
+        }
+    }
+    __syncthreads();
+    const int cat = ty < 2 ? ty : (ty < 4 ? PGK_HF_TO : PGK_HF_14);
+    double* acc = f.acc + (size_t)(blockIdx.x % FLUX_COPIES) * nreg * FLUX_COLS;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = w; q < 2 * nreg; q += FLUX_BT / 32) {
+        const double s = warp_sum(fsm[q * FLUX_BT + lane] + fsm[q * FLUX_BT + 32 + lane]);
+        if (lane == 0 && s != 0.0) atomicAdd(acc + (q >> 1) * FLUX_COLS + ((q & 1) ? 9 : 1) + cat, s);
+    }
+}
+
+pgk_status launch_bonded_flux(pgk_ctx* c, const FluxDev& f) {
+    auto on = [](int mts) { return mts == PGK_MTS_LONG || mts == PGK_MTS_SHORT; };
+    FluxTerms t;
+    t.n[0] = on(c->prm.mts_bond) ? c->nbond : 0;
+    t.n[1] = on(c->prm.mts_angl) ? c->nangl : 0;
+    t.n[2] = on(c->prm.mts_tors) ? c->ntors : 0;
+    t.n[3] = on(c->prm.mts_torsrb) ? c->ntorsrb : 0;
+    t.n[4] = on(c->prm.mts_vdw14) && c->prm.mts_vdw14 == c->prm.mts_elc14 ? c->n14 : 0;
+    t.bond = c->bond_ij; t.bond_p = c->bond_p; t.angl = c->angl_ijk; t.angl_p = c->angl_p;
+    t.tors = c->tors_ijkl; t.tors_p = c->tors_p; t.rb = c->rb_ijkl; t.rb_c = c->rb_c;
+    t.p14 = c->p14_ij; t.p14_f = c->p14_f;
+    int nb = 0;
+    for (int q = 0; q < 5; ++q) {
+        t.b0[q] = nb;
+        nb += std::min((t.n[q] + FLUX_BT - 1) / FLUX_BT, 8 * c->nsm);
+    }
+    t.b0[5] = nb;
+    if (nb == 0) return PGK_OK;
+    const size_t sm = sizeof(double) * 2 * f.h.nreg * FLUX_BT;
+    PGK_CUDA(c, smem_limit(k_bonded_flux, sm));
+    k_bonded_flux<<<nb, FLUX_BT, sm, c->st>>>(c->pos, c->chrg, c->typ, c->ntyp, c->lj64, t, f, c->dyn, c->status);
+    PGK_LAUNCHED(c);
+    PGK_CUDA(c, cudaGetLastError());
+    return PGK_OK;
+}
+
 // One MTS group's bonded terms (mask bits: 0 bond, 1 angle, 2 periodic
 // torsion, 3 RB torsion, 4 1-4 pairs, 5 excluded-pair Ewald correction): the
 // block kernel for the near terms, the per-type kernels for the far ones.

@@ -1,19 +1,19 @@
 // k_heatf.cu -- heat flux of the -DHF build and the region Langevin thermostat.
 //
-//   calcom.F90                  molecule centres of mass (k_calcom)
+//   calcom.F90                  molecule centres of mass, velocities (k_calcom)
 //   ewaldr_hf.F90:213-520       per-atom pair potentials and the calvirihf
 //                               virial of every list pair (k_hf_pair)
 //   cal*_hf.F90                 bonded parts (k_bonded.cu, launch_bonded_hf)
 //   calheatf.F90:365-1466       region sums of the kinetic, potential and
-//                               virial transport terms (k_heatf_part/_final)
+//                               virial transport terms (k_flux_*)
 //   langevin_regist.F90         region of each atom (k_lt_regist)
 //   langevin_region.F90         half steps with random and friction terms
 //                               (k_langevin)
 //
 // The per-atom arrays stay on the device in original atom order:
 // pot[8][N] and the z column of the per-atom virial W[8][nreg][3][N]
-// (category-major, so calheatf reads them coalesced).  Heat-flux steps only
-// (heatfinterval); the ordinary force kernels are unchanged on those steps.
+// (category-major).  They are written for the last heat-flux evaluation of a
+// call; the records come from region sums formed term by term (k_flux_*).
 //
 // k_hf_pair walks the same 8-atom cluster rows as the pair kernel: one warp
 // per cluster, one lane per (cluster, j) entry, a loop over the cluster atoms
@@ -31,13 +31,8 @@
 #include "pgk_hf.cuh"
 
 // ---- calcom.F90 / molecule velocities of calheatf.F90:556-607 -------------------
-__global__ void k_calcom(const double* __restrict__ x, const double* __restrict__ mass,
-                         const int* __restrict__ mol_idx, const int* __restrict__ mol_list, int nmole,
-                         const DynState* __restrict__ dyn, int wrap, double* __restrict__ out) {
-    int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= nmole) return;
-    int b = mol_idx[m], e = mol_idx[m + 1];
-    double c[3];
+__device__ __forceinline__ void mole_mean(const double* __restrict__ x, const double* __restrict__ mass,
+                                          const int* __restrict__ mol_list, int b, int e, double* c) {
     if (e - b == 1) {
         int i = mol_list[b];
         c[0] = x[3 * i]; c[1] = x[3 * i + 1]; c[2] = x[3 * i + 2];
@@ -53,7 +48,21 @@ __global__ void k_calcom(const double* __restrict__ x, const double* __restrict_
         double inv = 1.0 / ms;
         c[0] = c[0] * inv; c[1] = c[1] * inv; c[2] = c[2] * inv;
     }
-    for (int d = 0; d < 3; ++d) out[3 * m + d] = wrap ? hf_wrap1(c[d], dyn->box[d]) : c[d];
+}
+// vel null: the centres only
+__global__ void k_calcom(const double* __restrict__ pos, const double* __restrict__ vel,
+                          const double* __restrict__ mass, const int* __restrict__ mol_idx,
+                          const int* __restrict__ mol_list, int nmole, const DynState* __restrict__ dyn,
+                          double* __restrict__ com, double* __restrict__ cvel) {
+    int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= nmole) return;
+    const int b = mol_idx[m], e = mol_idx[m + 1];
+    double c[3];
+    mole_mean(pos, mass, mol_list, b, e, c);
+    for (int d = 0; d < 3; ++d) com[3 * m + d] = hf_wrap1(c[d], dyn->box[d]);
+    if (!vel) return;
+    mole_mean(vel, mass, mol_list, b, e, c);
+    for (int d = 0; d < 3; ++d) cvel[3 * m + d] = c[d];
 }
 
 // heat-flux z and molecule tag of every sorted slot (bit 31: molecule-based)
@@ -78,14 +87,16 @@ struct HfPairArgs {
 // zj) * frag / 2 per region); the cluster atom's share goes to its shared-
 // memory accumulators wi[nreg][3], j's share to the global array (stride N).
 // (pair categories ELIN, LJIN, ELC, VDW = PGK_HF_ELIN + 0..3)
+// first: the cluster atom has the lower atom index, as the reference's i (an
+// atom exactly on a plane makes hf_frag depend on the order).
 template <typename T>
 __device__ __forceinline__ void hf_pair_regions(T* wi, double* wj, size_t N, int nreg, const HfDev& h, double zi,
-                                                double zj, double rz, double az, T fx, T fy, T fz) {
+                                                double zj, bool first, double rz, double az, T fx, T fy, T fz) {
     const double zlo = fmin(zi, zj), zhi = fmax(zi, zj);
     for (int r = 0; r < nreg; ++r) {
         if (zhi < h.z1[r] || zlo > h.z2[r]) continue;
         double frag;
-        if (!hf_frag(zi, zj, h.z1[r], h.z2[r], az, frag)) continue;
+        if (!hf_frag(first ? zi : zj, first ? zj : zi, h.z1[r], h.z2[r], az, frag)) continue;
         const T fact = (T)(rz >= 0.0 ? frag * 0.5 : -frag * 0.5);
         const T vx = fx * fact, vy = fy * fact, vz = fz * fact;
         atomicAdd(wi + 3 * r + 0, vx);
@@ -154,6 +165,7 @@ __global__ void __launch_bounds__(128) k_hf_pair(const int4* __restrict__ xq, co
                 const double zi = a.zs[s];
                 const double rz = zi - zj, az = fabs(rz);
                 const bool vir = !((mi < 0) && (mj < 0) && same) && az * invLz < 0.5;
+                const bool first = a.perm[s] < oj;
                 T* w = acc + ii * per;
                 const bool coul = MIXED ? (r2 <= rr2) : (sqrt((double)r2) <= a.rrcut);
                 if (coul) {                           // ewaldr_hf.F90:336-371, bare 1/r
@@ -164,7 +176,7 @@ __global__ void __launch_bounds__(128) k_hf_pair(const int4* __restrict__ xq, co
                     atomicAdd(w + cat, (T)0.5 * phi);
                     atomicAdd(h.pot + (PGK_HF_ELIN + cat) * N + oj, (double)((T)0.5 * phi));
                     if (vir) hf_pair_regions<T>(w + 4 + cat * 3 * nreg, h.W + (size_t)(PGK_HF_ELIN + cat) * nreg * 3 * N + oj,
-                                                N, nreg, h, zi, zj, rz, az, ft * dx, ft * dy, ft * dz);
+                                                N, nreg, h, zi, zj, first, rz, az, ft * dx, ft * dy, ft * dz);
                 }
                 if (r2 <= rl2) {                      // ewaldr_hf.F90:376-470
                     T R2, E;
@@ -177,7 +189,7 @@ __global__ void __launch_bounds__(128) k_hf_pair(const int4* __restrict__ xq, co
                     atomicAdd(w + cat, (T)0.5 * phi);
                     atomicAdd(h.pot + (PGK_HF_ELIN + cat) * N + oj, (double)((T)0.5 * phi));
                     if (vir) hf_pair_regions<T>(w + 4 + cat * 3 * nreg, h.W + (size_t)(PGK_HF_ELIN + cat) * nreg * 3 * N + oj,
-                                                N, nreg, h, zi, zj, rz, az, ft * dx, ft * dy, ft * dz);
+                                                N, nreg, h, zi, zj, first, rz, az, ft * dx, ft * dy, ft * dz);
                 }
             }
         }
@@ -200,57 +212,357 @@ __global__ void __launch_bounds__(128) k_hf_pair(const int4* __restrict__ xq, co
 }
 
 // ---- calheatf.F90, volume-based, z components --------------------------------
-// per block: [nreg][17] partial sums (kinetic, 8 potential, 8 virial terms)
-__global__ void __launch_bounds__(256) k_heatf_part(const double* __restrict__ pos, const double* __restrict__ vel,
-                                                    const double* __restrict__ mass, const double* __restrict__ molevel,
-                                                    HfDev h, const DynState* __restrict__ dyn,
-                                                    double* __restrict__ part) {
-    extern __shared__ double hs[];
-    const int nreg = h.nreg, nv = nreg * 17;
-    for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = 0.0;
+// A record needs the region sums only, and they are linear in the terms
+// (FluxDev), so they are formed pair by pair and bonded term by bonded term
+// from the velocities; the per-atom arrays (190 MB for 43,200 atoms and 23
+// regions, FP64 atomics per pair, category, region and axis) are written for
+// the evaluation that pgk_get_hf_atm can read, not for every record.
+
+// Per atom: heat-flux z, molecule tag, velocities and region bits into the
+// sorted slots (iperm; null: no pair list), kinetic transport into the sums.
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ pos, const double* __restrict__ mass,
+                                                    const int* __restrict__ iperm, FluxDev f,
+                                                    const DynState* __restrict__ dyn, double* __restrict__ zs,
+                                                    int* __restrict__ ms, void* __restrict__ vs,
+                                                    uint4* __restrict__ bs) {
+    __shared__ double sk[PGK_HF_MAX_REGIONS];
+    const int nreg = f.h.nreg;
+    if (threadIdx.x < PGK_HF_MAX_REGIONS) sk[threadIdx.x] = 0.0;
     __syncthreads();
-    const size_t N = (size_t)h.natom;
-    const double Lz = dyn->box[2];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < h.natom; i += gridDim.x * blockDim.x) {
-        const double vx = vel[3 * i], vy = vel[3 * i + 1], vz = vel[3 * i + 2];
-        double pz, pvz;
-        if (h.hftyp[i] == PGK_HFTYP_MOLE) { pz = h.molecom[3 * h.mol_of[i] + 2]; pvz = molevel[3 * h.mol_of[i] + 2]; }
-        else { pz = pos[3 * i + 2]; pvz = vz; }
-        pz = hf_wrap1(pz, Lz);
-        const double kin = 0.5 * mass[i] * (vx * vx + vy * vy + vz * vz);
-        for (int r = 0; r < nreg; ++r) {
-            double* o = hs + r * 17;
-            if (h.z1[r] <= pz && pz <= h.z2[r]) {
-                atomicAdd(o, kin * pvz);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double kz = 0.0;
+    unsigned in = 0u;
+    if (i < f.h.natom) {
+        const double vx = f.vel[3 * i], vy = f.vel[3 * i + 1], vz = f.vel[3 * i + 2];
+        const double z = hf_z(f.h, pos, i, dyn->box[2]), pvz = flux_vz(f, i);
+        const uint4 m = flux_bits(f.h, z, dyn->box[2]);
+        in = m.z;
+        kz = 0.5 * mass[i] * (vx * vx + vy * vy + vz * vz) * pvz;
+        if (iperm) {
+            const int s = iperm[i];
+            zs[s] = z;
+            ms[s] = f.h.mol_of[i] | (f.h.hftyp[i] == PGK_HFTYP_MOLE ? (int)0x80000000 : 0);
+            bs[s] = m;
+            if (MIXED) ((float4*)vs)[s] = make_float4((float)vx, (float)vy, (float)vz, (float)pvz);
+            else ((double4*)vs)[s] = make_double4(vx, vy, vz, pvz);
+        }
+    }
+    unsigned any = __reduce_or_sync(0xffffffffu, in);
+    while (any) {
+        const int r = __ffs(any) - 1;
+        any &= any - 1;
+        const double s = warp_sum((in >> r) & 1u ? kz : 0.0);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sk[r], s);
+    }
+    __syncthreads();
+    double* acc = f.acc + (size_t)(blockIdx.x % FLUX_COPIES) * nreg * FLUX_COLS;
+    if (threadIdx.x < nreg && sk[threadIdx.x] != 0.0) atomicAdd(acc + threadIdx.x * FLUX_COLS, sk[threadIdx.x]);
+}
+
+// Pair part of the region sums over the cluster rows (the book rows, or the
+// pruned rows while they are current): one warp per (cluster, row segment),
+// one lane per entry, a loop over the entry's mask bits.  A pair's share of
+// region r is s (C_r(z_i) - C_r(z_j)) / 2 with s = f_ij . (v_i + v_j) and
+// C_r(z) = z clamped to the slab -- the plane-crossing cases of calvirihf as
+// one difference; C_r(z_j) is formed once per entry, C_r(z_i) once per
+// cluster.  The regions that a row can touch (bits of FluxDev: 3-4 of 23 for
+// 10 A slabs and a 12 A cutoff) are taken KW at a time, so that all sums stay
+// in registers; a row that touches more walks again for the next KW.  Pairs
+// inside one molecule and atoms exactly on a plane (hf_frag's own cases) take
+// a slower branch with shared-memory sums.
+// Pair arithmetic is T (FP32 in mixed precision, the reciprocal root refined
+// by one Newton step), all region sums are FP64.
+// Bound by issue (about 60 FP32 and 12 FP64 instructions per pair) at 16 warps
+// per SM.  Measured: 43,200-atom slab, 23 regions, mixed: 0.327 ms per
+// evaluation against 4.86 ms for the per-atom arrays and 0.52 ms for summing
+// them; 8,232-atom water box, one region: 0.042 ms against 1.27 + 0.24 ms.
+// Rows are cut into segments until 16 warps per SM have work (small boxes).
+struct FluxPairArgs {
+    const int* rows; const int* cnt; int ccap; int ncl; int nseg;
+    const int* typ_s; const int* perm; int ntyp;
+    const double* zs; const int* ms; const void* vs; const uint4* bs;
+    double rr2, rl2, rmax2;
+};
+
+template <bool MIXED> struct FluxT { typedef float T; typedef float4 V; };
+template <> struct FluxT<false> { typedef double T; typedef double4 V; };
+
+__device__ __forceinline__ float flux_rinv(float r2) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
+    return y * fmaf(-0.5f * r2 * y, y, 1.5f);
+}
+__device__ __forceinline__ double flux_rinv(double r2) { return rsqrt(r2); }
+
+template <bool MIXED, int KW>
+__global__ void __launch_bounds__(128, MIXED ? 4 : 3)
+k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPairArgs a,
+            const float2* __restrict__ lj32, const double2* __restrict__ lj64, FluxDev f,
+            const DynState* __restrict__ dyn) {
+    typedef typename FluxT<MIXED>::T T;
+    typedef typename FluxT<MIXED>::V V;
+    __shared__ double sb[8 * PGK_HF_MAX_REGIONS];        // [nreg][pot 4 | virial 4], categories ELIN..VDW
+    __shared__ double sz1[PGK_HF_MAX_REGIONS], sz2[PGK_HF_MAX_REGIONS];
+    __shared__ int4 sxq[4][8];
+    __shared__ double4 sx64[MIXED ? 1 : 4][8];
+    __shared__ V sv[4][8];
+    __shared__ double szi[4][8], sC[4][8][KW];
+    __shared__ uint4 sbi[4][8];
+    __shared__ int smi[4][8], sti[4][8];
+    const int nreg = f.h.nreg;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = threadIdx.x; q < 8 * nreg; q += blockDim.x) sb[q] = 0.0;
+    if (threadIdx.x < nreg) { sz1[threadIdx.x] = f.h.z1[threadIdx.x]; sz2[threadIdx.x] = f.h.z2[threadIdx.x]; }
+    __syncthreads();
+    const unsigned all = nreg >= 32 ? 0xffffffffu : (1u << nreg) - 1u;
+    const double L0 = dyn->box[0], L1 = dyn->box[1], Lz = dyn->box[2];
+    const double B0 = 1.0 / L0, B1 = 1.0 / L1, B2 = 1.0 / Lz;
+    const T sx = (T)(L0 * (1.0 / 4294967296.0)), sy = (T)(L1 * (1.0 / 4294967296.0)), sz = (T)(Lz * (1.0 / 4294967296.0));
+    const T rr2 = (T)a.rr2, rl2 = (T)a.rl2, rmax2 = (T)a.rmax2;
+    const V* __restrict__ vs = (const V*)a.vs;
+    const long long nunit = (long long)a.ncl * a.nseg;
+    for (long long u = blockIdx.x * 4 + w; u < nunit; u += gridDim.x * 4) {
+        const int cl = (int)(u / a.nseg), seg = (int)(u - (long long)cl * a.nseg);
+        const int cnt = a.cnt[cl];
+        const int chunk = ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
+        const int k_lo = seg * chunk, k_hi = min(cnt, k_lo + chunk);
+        if (k_lo >= k_hi) continue;                       // warp-uniform
+        const int* __restrict__ row = a.rows + (size_t)cl * a.ccap;
+        __syncwarp();
+        if (lane < 8) {
+            const int s = 8 * cl + lane;
+            if (MIXED) sxq[w][lane] = xq[s]; else sx64[MIXED ? 0 : w][lane] = xq64[s];
+            sv[w][lane] = vs[s];
+            szi[w][lane] = a.zs[s];
+            sbi[w][lane] = a.bs[s];
+            smi[w][lane] = a.ms[s];
+            sti[w][lane] = a.typ_s[s] * a.ntyp;
+        }
+        __syncwarp();
+        // regions that a pair of this row segment can touch, or its atoms lie in
+        unsigned todo = all;
+        if (nreg > KW) {
+            unsigned t = 0u;
+            for (int k = k_lo + lane; k < k_hi; k += 32) {
+                const unsigned e = (unsigned)row[k];
+                const uint4 bj = a.bs[e & 0xFFFFFFu];
+                t |= bj.z;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) atomicAdd(o + 1 + c, h.pot[c * N + i] * pvz);
+                for (int ii = 0; ii < 8; ++ii)
+                    if ((e >> (24 + ii)) & 1u) {
+                        const uint4 bi = sbi[w][ii];
+                        t |= bi.z | ~((bi.x & bj.x) | (bi.y & bj.y));
+                    }
+            }
+            todo = __reduce_or_sync(0xffffffffu, t) & all;
+        }
+        while (todo) {
+            int rk[KW];
+            unsigned win = 0u;
+#pragma unroll
+            for (int k = 0; k < KW; ++k) {
+                rk[k] = todo ? __ffs(todo) - 1 : -1;
+                if (todo) { win |= 1u << rk[k]; todo &= todo - 1; }
+            }
+            __syncwarp();
+            if (lane < 8) {
+#pragma unroll
+                for (int k = 0; k < KW; ++k) {
+                    const double z = szi[w][lane];
+                    const int r = max(rk[k], 0);
+                    const uint4 b = sbi[w][lane];
+                    sC[w][lane][k] = (b.x >> r) & 1u ? sz1[r] : ((b.y >> r) & 1u ? sz2[r] : z);
+                }
+            }
+            __syncwarp();
+            double vc[KW], vl[KW], pc[KW], pl[KW];
+            T pic[8], pil[8];
+#pragma unroll
+            for (int k = 0; k < KW; ++k) { vc[k] = 0.0; vl[k] = 0.0; pc[k] = 0.0; pl[k] = 0.0; }
+#pragma unroll
+            for (int ii = 0; ii < 8; ++ii) { pic[ii] = (T)0; pil[ii] = (T)0; }
+            for (int k = k_lo + lane; k < k_hi; k += 32) {
+                const unsigned e = (unsigned)row[k];
+                const int j = (int)(e & 0xFFFFFFu);
+                const unsigned m = e >> 24;
+                const double zj = a.zs[j];
+                const int mj = a.ms[j], tj = a.typ_s[j];
+                const uint4 bj = a.bs[j];
+                const V vj = vs[j];
+                int4 qj = make_int4(0, 0, 0, 0);
+                double4 pj = make_double4(0, 0, 0, 0);
+                if (MIXED) qj = xq[j]; else pj = xq64[j];
+                double Cj[KW];
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    const int r = max(rk[q], 0);
+                    Cj[q] = (bj.x >> r) & 1u ? sz1[r] : ((bj.y >> r) & 1u ? sz2[r] : zj);
+                }
+                T pjc = (T)0, pjl = (T)0;
+#pragma unroll
+                for (int ii = 0; ii < 8; ++ii) {
+                    if (!((m >> ii) & 1u)) continue;
+                    T dx, dy, dz, qq;
+                    if (MIXED) {
+                        const int4 qi = sxq[w][ii];
+                        dx = (T)(qi.x - qj.x) * sx; dy = (T)(qi.y - qj.y) * sy; dz = (T)(qi.z - qj.z) * sz;
+                        qq = (T)(__int_as_float(qi.w) * __int_as_float(qj.w));
+                    } else {
+                        const double4 pi = sx64[MIXED ? 0 : w][ii];
+                        const double wx = pi.x - pj.x, wy = pi.y - pj.y, wz = pi.z - pj.z;
+                        dx = (T)(wx - L0 * round(wx * B0));
+                        dy = (T)(wy - L1 * round(wy * B1));
+                        dz = (T)(wz - Lz * round(wz * B2));
+                        qq = (T)(pi.w * pj.w);
+                    }
+                    const T r2 = dx * dx + dy * dy + dz * dz;
+                    if (r2 > rmax2) continue;
+                    const T rinv = flux_rinv(r2), rinv2 = rinv * rinv;
+                    const T phc = r2 <= rr2 ? qq * rinv : (T)0;          // ewaldr_hf.F90:336-371, bare 1/r
+                    T phl = (T)0, ftl = (T)0;
+                    if (r2 <= rl2) {                                     // ewaldr_hf.F90:376-470
+                        T R2, E;
+                        if (MIXED) { const float2 lp = lj32[sti[w][ii] + tj]; R2 = lp.x; E = lp.y; }
+                        else { const double2 lp = lj64[sti[w][ii] + tj]; R2 = lp.x; E = lp.y; }
+                        const T t2 = rinv2 * R2, t6 = t2 * t2 * t2, t12 = t6 * t6;
+                        phl = E * (t12 - (T)2 * t6);
+                        ftl = (T)12 * E * (t12 - t6) * rinv2;
+                    }
+                    const V vi = sv[w][ii];
+                    const T fv = dx * (vi.x + vj.x) + dy * (vi.y + vj.y) + dz * (vi.z + vj.z);
+                    const int mi = smi[w][ii];
+                    const bool same = (mi & 0x7fffffff) == (mj & 0x7fffffff);
+                    const uint4 bi = sbi[w][ii];
+                    const double zi = szi[w][ii];
+                    const double az = fabs(zi - zj);
+                    const bool vir = !((mi < 0) && (mj < 0) && same) && az * B2 < 0.5;
+                    double sc = vir ? 0.5 * (double)(phc * rinv2 * fv) : 0.0;
+                    double sl = vir ? 0.5 * (double)(ftl * fv) : 0.0;
+                    if (same || ((bi.w | bj.w) & win)) {
+                        const int cc = same ? 0 : 2, lc = same ? 1 : 3;
+                        // the lower atom index first: the reference's i
+                        const bool first = a.perm[8 * cl + ii] < a.perm[j];
+                        const double za = first ? zi : zj, zb = first ? zj : zi;
+#pragma unroll
+                        for (int q = 0; q < KW; ++q) {
+                            const int r = rk[q];
+                            if (r < 0) continue;
+                            double* o = sb + 8 * r;
+                            if (same) {
+                                const double tv = 0.5 * (((bi.z >> r) & 1u ? (double)vi.w : 0.0) +
+                                                         ((bj.z >> r) & 1u ? (double)vj.w : 0.0));
+                                if (tv != 0.0) { atomicAdd(o + cc, (double)phc * tv); atomicAdd(o + lc, (double)phl * tv); }
+                            }
+                            double frag;
+                            if (vir && !(((bi.x & bj.x) | (bi.y & bj.y)) >> r & 1u) &&
+                                hf_frag(za, zb, sz1[r], sz2[r], az, frag)) {
+                                const double d = zi - zj >= 0.0 ? frag : -frag;
+                                atomicAdd(o + 4 + cc, sc * d);
+                                atomicAdd(o + 4 + lc, sl * d);
+                            }
+                        }
+                        sc = 0.0;
+                        sl = 0.0;
+                    }
+                    if (!same) { pic[ii] += phc; pil[ii] += phl; pjc += phc; pjl += phl; }
+#pragma unroll
+                    for (int q = 0; q < KW; ++q) {
+                        const double D = sC[w][ii][q] - Cj[q];
+                        vc[q] = fma(sc, D, vc[q]);
+                        vl[q] = fma(sl, D, vl[q]);
+                    }
+                }
+                const double hz = 0.5 * (double)vj.w;
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    const double t = rk[q] >= 0 && (bj.z >> rk[q]) & 1u ? hz : 0.0;
+                    pc[q] = fma((double)pjc, t, pc[q]);
+                    pl[q] = fma((double)pjl, t, pl[q]);
+                }
+            }
+            // cluster atoms' transport shares, then the warp's sums
+#pragma unroll
+            for (int ii = 0; ii < 8; ++ii) {
+                const double hz = 0.5 * (double)sv[w][ii].w;
+                const unsigned in = sbi[w][ii].z;
+#pragma unroll
+                for (int q = 0; q < KW; ++q)
+                    if (rk[q] >= 0 && (in >> rk[q]) & 1u) {
+                        pc[q] = fma((double)pic[ii], hz, pc[q]);
+                        pl[q] = fma((double)pil[ii], hz, pl[q]);
+                    }
             }
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const double* w = h.W + ((size_t)c * nreg + r) * 3 * N;
-                const double t = w[i] * vx + w[N + i] * vy + w[2 * N + i] * vz;
-                if (t != 0.0) atomicAdd(o + 9 + c, t);
+            for (int q = 0; q < KW; ++q) {
+                if (rk[q] < 0) continue;                   // warp-uniform
+                const double s0 = warp_sum(pc[q]), s1 = warp_sum(pl[q]), s2 = warp_sum(vc[q]), s3 = warp_sum(vl[q]);
+                if (lane < 4) {
+                    const double s = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
+                    const int col = lane == 0 ? 2 : lane == 1 ? 3 : lane == 2 ? 6 : 7;
+                    if (s != 0.0) atomicAdd(sb + 8 * rk[q] + col, s);
+                }
             }
         }
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < nv; q += blockDim.x) part[(size_t)blockIdx.x * nv + q] = hs[q];
+    double* acc = f.acc + (size_t)(blockIdx.x % FLUX_COPIES) * nreg * FLUX_COLS;
+    for (int q = threadIdx.x; q < 8 * nreg; q += blockDim.x) {
+        const int r = q >> 3, c = q & 7;
+        if (sb[q] != 0.0) atomicAdd(acc + r * FLUX_COLS + (c < 4 ? 1 : 9 - 4) + PGK_HF_ELIN + c, sb[q]);
+    }
 }
 
-// fixed-order sum of the block partials, volume normalisation, hftot
-__global__ void k_heatf_final(const double* __restrict__ part, int nblk, int nreg, HfDev h,
-                              const DynState* __restrict__ dyn, double* __restrict__ rec) {
-    const int r = threadIdx.x;
-    if (r >= nreg) return;
-    double s[17];
-    for (int c = 0; c < 17; ++c) s[c] = 0.0;
-    for (int b = 0; b < nblk; ++b)
-        for (int c = 0; c < 17; ++c) s[c] += part[((size_t)b * nreg + r) * 17 + c];
-    const double area_inv = (1.0 / dyn->box[0]) * (1.0 / dyn->box[1]);
-    const double vol_inv = area_inv / (h.z2[r] - h.z1[r]);
-    double tot = 0.0;
-    for (int c = 0; c < 17; ++c) { s[c] = s[c] * vol_inv; tot += s[c]; rec[r * PGK_HF_NCOL + c] = s[c]; }
-    rec[r * PGK_HF_NCOL + 17] = tot;
+// Per-atom reciprocal terms (pgk_set_hf_kspace): the energy is transported in
+// the atom's region, the (a, z) column of the tensor counts in region 1.
+__global__ void __launch_bounds__(256) k_flux_kspace(const double* __restrict__ pos, const double* __restrict__ pot,
+                                                     const double* __restrict__ vir, FluxDev f,
+                                                     const DynState* __restrict__ dyn) {
+    __shared__ double sp[PGK_HF_MAX_REGIONS + 1];
+    const int nreg = f.h.nreg;
+    if (threadIdx.x <= PGK_HF_MAX_REGIONS) sp[threadIdx.x] = 0.0;
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double p = 0.0, v = 0.0;
+    unsigned in = 0u;
+    if (i < f.h.natom) {
+        in = flux_bits(f.h, hf_z(f.h, pos, i, dyn->box[2]), dyn->box[2]).z;
+        p = pot[i] * flux_vz(f, i);
+        const double* t = vir + (size_t)9 * i + 6;
+        v = t[0] * f.vel[3 * i] + t[1] * f.vel[3 * i + 1] + t[2] * f.vel[3 * i + 2];
+    }
+    unsigned any = __reduce_or_sync(0xffffffffu, in);
+    while (any) {
+        const int r = __ffs(any) - 1;
+        any &= any - 1;
+        const double s = warp_sum((in >> r) & 1u ? p : 0.0);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sp[r], s);
+    }
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&sp[PGK_HF_MAX_REGIONS], v);
+    __syncthreads();
+    double* acc = f.acc + (size_t)(blockIdx.x % FLUX_COPIES) * nreg * FLUX_COLS;
+    if (threadIdx.x < nreg && sp[threadIdx.x] != 0.0)
+        atomicAdd(acc + threadIdx.x * FLUX_COLS + 1 + PGK_HF_ELC, sp[threadIdx.x]);
+    if (threadIdx.x == 0) atomicAdd(acc + 9 + PGK_HF_ELC, sp[PGK_HF_MAX_REGIONS]);
+}
+
+// volume normalisation and hftot; leaves the sums zero (one warp per region)
+__global__ void k_flux_final(FluxDev f, const DynState* __restrict__ dyn, double* __restrict__ rec) {
+    const int r = blockIdx.x, c = threadIdx.x;
+    double s = 0.0;
+    if (c < FLUX_COLS) {
+        for (int k = 0; k < FLUX_COPIES; ++k) {
+            double* p = f.acc + ((size_t)k * f.h.nreg + r) * FLUX_COLS + c;
+            s += *p;
+            *p = 0.0;
+        }
+        const double area_inv = (1.0 / dyn->box[0]) * (1.0 / dyn->box[1]);
+        s *= area_inv / (f.h.z2[r] - f.h.z1[r]);
+        rec[r * PGK_HF_NCOL + c] = s;
+    }
+    const double tot = warp_sum(s);
+    if (c == 0) rec[r * PGK_HF_NCOL + 17] = tot;
 }
 
 // ---- region Langevin thermostat ----------------------------------------------
@@ -419,15 +731,15 @@ pgk_status hf_setup(pgk_ctx* c, const pgk_hfparams* p) {
         return PGK_OK;
     };
     const int nreg = c->hfp.nhfregion;
-    c->hf_nblk = 2 * c->nsm;
     if ((s = realloc(&c->molecom, (size_t)3 * std::max(1, c->nmole))) ||
         (s = realloc(&c->molevel, (size_t)3 * std::max(1, c->nmole))) ||
         (s = realloc(&c->hf_pot, (size_t)8 * n)) || (s = realloc(&c->hf_W, (size_t)8 * nreg * 3 * n)) ||
-        (s = realloc(&c->hf_part, (size_t)c->hf_nblk * nreg * 17)) ||
+        (s = realloc(&c->hf_acc, (size_t)FLUX_COPIES * nreg * FLUX_COLS)) ||
         (s = realloc(&c->hf_rec, (size_t)std::max(1, nreg) * PGK_HF_NCOL)) ||   // one record
         (s = realloc(&c->lt_frand, (size_t)3 * n)) || (s = realloc(&c->lt_dekin, PGK_LT_MAX_REGIONS)))
         return s;
     c->hf_rec_cap = 1;
+    c->hf_k_terms = nullptr;
     if (c->lt_reg) pgk_dfree(c, c->lt_reg);
     c->lt_reg = nullptr;
     PGK_CUDA(c, pgk_dmalloc(c, &c->lt_reg, sizeof(int) * n));
@@ -440,10 +752,19 @@ pgk_status hf_setup(pgk_ctx* c, const pgk_hfparams* p) {
 
 static pgk_status ensure_hf_slots(pgk_ctx* c) {
     if (c->hf_slots_cap >= c->npad_cap) return PGK_OK;
-    pgk_dfree(c, c->hf_zs); pgk_dfree(c, c->hf_ms);
-    c->hf_zs = nullptr; c->hf_ms = nullptr;
+    pgk_dfree(c, c->hf_zs); pgk_dfree(c, c->hf_ms); pgk_dfree(c, c->hf_vs); pgk_dfree(c, c->hf_bs);
+    c->hf_zs = nullptr; c->hf_ms = nullptr; c->hf_vs = nullptr; c->hf_bs = nullptr;
+    c->hf_slots_cap = 0;
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_zs, sizeof(double) * c->npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_ms, sizeof(int) * c->npad_cap));
+    const size_t vb = (c->mixed() ? sizeof(float4) : sizeof(double4)) * (size_t)c->npad_cap;
+    PGK_CUDA(c, pgk_dmalloc(c, &c->hf_vs, vb));
+    PGK_CUDA(c, pgk_dmalloc(c, &c->hf_bs, sizeof(uint4) * c->npad_cap));
+    // padding slots take part in no pair, but a cluster stages them
+    PGK_CUDA(c, cudaMemsetAsync(c->hf_zs, 0, sizeof(double) * c->npad_cap, c->st));
+    PGK_CUDA(c, cudaMemsetAsync(c->hf_ms, 0, sizeof(int) * c->npad_cap, c->st));
+    PGK_CUDA(c, cudaMemsetAsync(c->hf_vs, 0, vb, c->st));
+    PGK_CUDA(c, cudaMemsetAsync(c->hf_bs, 0, sizeof(uint4) * c->npad_cap, c->st));
     c->hf_slots_cap = c->npad_cap;
     return PGK_OK;
 }
@@ -464,23 +785,35 @@ __global__ void k_hf_kspace_add(const double* __restrict__ pot, const double* __
         hf_W[((size_t)PGK_HF_ELC * nreg * 3 + a) * n + i] += vir[(size_t)9 * i + a + 6];
 }
 
-pgk_status launch_hf_kspace(pgk_ctx* c) {
+// the per-atom reciprocal terms at the current positions (energies [N] |
+// tensors [9N]; null: the option is off), evaluated once per heat-flux step
+static pgk_status hf_kspace_terms(pgk_ctx* c, const double** pot) {
+    *pot = nullptr;
     const int n = c->natom;
-    const double* pot = nullptr;
-    if (c->hf_kspace == PGK_HF_KSPACE_SPME) {
-        pgk_status s = launch_spme_hf_atm(c);
-        if (s) return s;
-        pot = c->hfk_out;
-    } else if (c->hf_kspace == PGK_HF_KSPACE_EWK) {
-        if (!c->hf_ewk_fresh) {       // not yet evaluated at these positions by the force evaluation
-            int nw = 0;
-            pgk_status s = launch_ewk_hf(c, c->hf_kmax, &nw);
+    if (!c->hf_k_terms) {
+        if (c->hf_kspace == PGK_HF_KSPACE_SPME) {
+            pgk_status s = launch_spme_hf_atm(c);
             if (s) return s;
+            c->hf_k_terms = c->hfk_out;
+        } else if (c->hf_kspace == PGK_HF_KSPACE_EWK) {
+            if (!c->hf_ewk_fresh) {   // not yet evaluated at these positions by the force evaluation
+                int nw = 0;
+                pgk_status s = launch_ewk_hf(c, c->hf_kmax, &nw);
+                if (s) return s;
+            }
+            c->hf_k_terms = c->ewk_out + 3 * (size_t)n;
         }
-        pot = c->ewk_out + 3 * (size_t)n;
+        c->hf_ewk_fresh = false;
     }
-    c->hf_ewk_fresh = false;
-    if (!pot) return PGK_OK;
+    *pot = c->hf_k_terms;
+    return PGK_OK;
+}
+
+static pgk_status launch_hf_kspace(pgk_ctx* c) {
+    const int n = c->natom;
+    const double* pot;
+    pgk_status s = hf_kspace_terms(c, &pot);
+    if (s || !pot) return s;
     k_hf_kspace_add<<<(n + 255) / 256, 256, 0, c->st>>>(pot, pot + n, n, c->hfp.nhfregion, c->hf_pot, c->hf_W);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
@@ -492,8 +825,8 @@ pgk_status launch_hf_atm(pgk_ctx* c) {
     pgk_status s;
     const int n = c->natom, nreg = c->hfp.nhfregion;
     if (c->nmole > 0) {
-        k_calcom<<<(c->nmole + 127) / 128, 128, 0, c->st>>>(c->pos, c->mass, c->mol_idx, c->mol_list, c->nmole,
-                                                             c->dyn, 1, c->molecom);
+        k_calcom<<<(c->nmole + 127) / 128, 128, 0, c->st>>>(c->pos, nullptr, c->mass, c->mol_idx, c->mol_list, c->nmole,
+                                                             c->dyn, c->molecom, nullptr);
         PGK_LAUNCHED(c);
     }
     PGK_CUDA(c, cudaMemsetAsync(c->hf_pot, 0, sizeof(double) * 8 * n, c->st));
@@ -531,19 +864,65 @@ pgk_status launch_hf_atm(pgk_ctx* c) {
     return launch_hf_kspace(c);
 }
 
-// calheatf with the current velocities: one record of nreg * 18 at dst (device)
-pgk_status launch_heatf(pgk_ctx* c, double* dst) {
-    const int nreg = c->hfp.nhfregion;
+// one region: one accumulator set; more: four a walk (most rows touch 3-4)
+template <bool MIXED>
+static void flux_pair_launch(pgk_ctx* c, FluxPairArgs& a, const FluxDev& f) {
+    // about 16 warps per SM, in row segments where the clusters alone are fewer
+    const int want = c->nsm * 16;
+    a.nseg = std::max(1, std::min(8, want / std::max(a.ncl, 1)));
+    const long long units = (long long)a.ncl * a.nseg;
+    const int blocks = (int)std::max(1LL, std::min((units + 3) / 4, (long long)c->nsm * 16));
+    if (f.h.nreg == 1)
+        k_flux_pair<MIXED, 1><<<blocks, 128, 0, c->st>>>(c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
+    else
+        k_flux_pair<MIXED, 4><<<blocks, 128, 0, c->st>>>(c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
+    PGK_LAUNCHED(c);
+}
+
+pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
+    const int nreg = c->hfp.nhfregion, n = c->natom;
+    pgk_status s;
+    FluxDev f;
+    f.h = hf_dev(c);
+    f.vel = c->vel; f.molevel = c->molevel; f.acc = c->hf_acc;
     if (c->nmole > 0) {
-        k_calcom<<<(c->nmole + 127) / 128, 128, 0, c->st>>>(c->vel, c->mass, c->mol_idx, c->mol_list, c->nmole,
-                                                             c->dyn, 0, c->molevel);
+        k_calcom<<<(c->nmole + 127) / 128, 128, 0, c->st>>>(c->pos, c->vel, c->mass, c->mol_idx, c->mol_list, c->nmole,
+                                                             c->dyn, c->molecom, c->molevel);
         PGK_LAUNCHED(c);
     }
-    HfDev h = hf_dev(c);
-    size_t sm = sizeof(double) * nreg * 17;
-    k_heatf_part<<<c->hf_nblk, 256, sm, c->st>>>(c->pos, c->vel, c->mass, c->molevel, h, c->dyn, c->hf_part);
-    k_heatf_final<<<1, 32, 0, c->st>>>(c->hf_part, c->hf_nblk, nreg, h, c->dyn, dst);
-    c->launches += 2;
+    const bool pair_on = (c->prm.mts_vdw == PGK_MTS_LONG || c->prm.mts_vdw == PGK_MTS_SHORT) && c->ncl > 0;
+    if (pair_on && (s = ensure_hf_slots(c))) return s;
+    const int* ip = pair_on ? c->iperm : nullptr;
+    if (c->mixed())
+        k_flux_atoms<true><<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->mass, ip, f, c->dyn, c->hf_zs, c->hf_ms,
+                                                               c->hf_vs, c->hf_bs);
+    else
+        k_flux_atoms<false><<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->mass, ip, f, c->dyn, c->hf_zs, c->hf_ms,
+                                                                c->hf_vs, c->hf_bs);
+    PGK_LAUNCHED(c);
+    if (pair_on) {
+        FluxPairArgs a;
+        const bool pr = pruned && c->mixed() && c->prune_buffer > 0.f;
+        a.rows = pr ? c->plist : c->clist; a.cnt = pr ? c->pcnt : c->ccnt;
+        a.ccap = c->ccap; a.ncl = c->ncl;
+        a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
+        a.zs = c->hf_zs; a.ms = c->hf_ms; a.vs = c->hf_vs; a.bs = c->hf_bs;
+        a.rr2 = c->prm.rrcut * c->prm.rrcut;
+        a.rl2 = c->prm.rcut * c->prm.rcut;
+        a.rmax2 = std::max(a.rr2, a.rl2);
+        if (c->mixed()) flux_pair_launch<true>(c, a, f);
+        else flux_pair_launch<false>(c, a, f);
+    }
+    if ((s = launch_bonded_flux(c, f))) return s;
+    const double* pot;
+    if ((s = hf_kspace_terms(c, &pot))) return s;
+    c->hf_k_terms = nullptr;
+    if (pot) {
+        k_flux_kspace<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, pot, pot + n, f, c->dyn);
+        PGK_LAUNCHED(c);
+    }
+    k_flux_final<<<nreg, 32, 0, c->st>>>(f, c->dyn, dst);
+    PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
 }

@@ -762,8 +762,8 @@ pgk_status pgk_free(pgk_ctx* c) {
                     c->plan[0].tw, c->plan[1].tw, c->plan[2].tw, c->fout, c->cg_span, c->cg_fit, c->blk_a0, c->blk_nloc, c->blk_t, c->blk_soff,
                     c->blk_ip, c->blk_incp, c->blk_inc, c->brec[0], c->brec[1], c->brec[2], c->brec[3], c->brec[4],
                     c->brec[5], c->btab[0], c->btab[1], c->btab[2], c->btab[3], c->btab[4], c->btab[5],
-                    c->mol_of, c->hftyp, c->molecom, c->molevel, c->hf_pot, c->hf_W, c->hf_part, c->hf_rec, c->hf_zs,
-                    c->hf_ms, c->lt_mole, c->lt_reg, c->lt_frand, c->lt_dekin, c->hasup, c->out_rec,
+                    c->mol_of, c->hftyp, c->molecom, c->molevel, c->hf_pot, c->hf_W, c->hf_acc, c->hf_rec, c->hf_zs,
+                    c->hf_ms, c->hf_vs, c->hf_bs, c->lt_mole, c->lt_reg, c->lt_frand, c->lt_dekin, c->hasup, c->out_rec,
                     c->ewk_nv, c->ewk_tab, c->ewk_part, c->ewk_coef, c->ewk_red, c->ewk_out, c->ewk_seg,
                     c->mor_atoms, c->mor_par, c->mor_rows, c->mor_cnt, c->mor_cell, c->mor_csort, c->mor_ccnt,
                     c->mor_cstart, c->mor_cfill, c->mor_ctr, c->hfk_q, c->hfk_g, c->hfk_out, c->hfk_tw[0],
@@ -1035,7 +1035,7 @@ void* pgk_stream(const pgk_ctx* c) { return c ? (void*)c->st : nullptr; }
 
 // ---- stage drivers ---------------------------------------------------------------
 static pgk_status md_step_body(pgk_ctx* c, int kind, int64_t step, const pgk_mdparams* md, bool ene, bool vir,
-                               bool tens, bool hfs, bool lt, bool ke_ready);
+                               bool tens, bool hfs, bool hfa, bool lt, bool ke_ready);
 
 // kind: 0 NVE (moldyn.F90), 1 NHC (moldyn_nhc.F90), 2 MTK (moldyn_mtk.F90),
 // 3 NVE + region Langevin + heat flux (moldyn_hf.F90); hf records go to the
@@ -1060,8 +1060,12 @@ static pgk_status run_md(pgk_ctx* c, int kind, int64_t ini, int64_t end, const p
     // accumulators (the previous step of this run ended with them), so the
     // step's first chain half reuses them instead of summing again
     bool ke_ready = false;
+    // per-atom heat-flux arrays: pgk_get_hf_atm reads the last evaluation, so
+    // only the run's last heat-flux step writes them
+    int64_t last_hf = end;
+    if (hfdrv && hfi > 1) last_hf -= ((end - 1) % hfi + hfi) % hfi;
     auto step_body = [&](int64_t st, bool e_, bool v_, bool t_, bool h_, bool l_) {
-        return md_step_body(c, kind, st, md, e_, v_, t_, h_, l_, ke_ready);
+        return md_step_body(c, kind, st, md, e_, v_, t_, h_, h_ && st == last_hf, l_, ke_ready);
     };
     pgk_status s;
 #define RUN(x) do { if ((s = (x)) != PGK_OK) return s; } while (0)
@@ -1149,7 +1153,9 @@ static pgk_status run_md(pgk_ctx* c, int kind, int64_t ini, int64_t end, const p
         if (step > 0) {
             if (lt) { RUN(launch_lt_regist(c)); RUN(launch_langevin(c, md->dt_long_cal, step, false)); }
             if (hfs) {
-                if (nr < c->hf_rec_cap) RUN(launch_heatf(c, c->hf_rec + nr * per));
+                if (nr < c->hf_rec_cap) RUN(launch_heatf(c, c->hf_rec + nr * per, true));
+                c->hf_ewk_fresh = false;
+                c->hf_k_terms = nullptr;
                 ++nr;
             }
         }
@@ -1179,7 +1185,7 @@ static pgk_status run_md(pgk_ctx* c, int kind, int64_t ini, int64_t end, const p
 // one MD step (step > 0) of run_md: the thermostat / barostat half steps and
 // the XO-RESPA loop with its force evaluations
 static pgk_status md_step_body(pgk_ctx* c, int kind, int64_t step, const pgk_mdparams* md, bool ene, bool vir,
-                               bool tens, bool hfs, bool lt, bool ke_ready) {
+                               bool tens, bool hfs, bool hfa, bool lt, bool ke_ready) {
     const double dts = md->dt_long_cal / (double)md->nstep_short;
     const bool rattle = md->ifrattle && (c->ncgroup > 0 || c->nr3 > 0 || c->nstar > 0);
     const bool mtk = kind == 2;
@@ -1209,7 +1215,7 @@ static pgk_status md_step_body(pgk_ctx* c, int kind, int64_t step, const pgk_mdp
         if (!c->short_empty) RUN(force_group(c, PGK_MTS_SHORT, ene || vir, vir, tens));
         if (last) {
             RUN(force_group(c, PGK_MTS_LONG, ene || vir, vir, tens));
-            if (hfs) RUN(launch_hf_atm(c));
+            if (hfa) RUN(launch_hf_atm(c));
         }
         c->hf_ewk_now = false;
         RUN(launch_kick_drift(c, kshort | KD_SHORT_FIRST | (last ? KD_LONG : 0)));
@@ -1327,7 +1333,7 @@ pgk_status pgk_calheatf(pgk_ctx* c, double* hf) {
     if (!c->hf_set || c->hfp.nhfregion < 1) return pgk_fail(c, PGK_E_INVALID, "no heat-flux regions set");
     pgk_status s;
     if (!c->list_valid && (s = launch_mklist(c))) return s;
-    if ((s = launch_pack(c)) || (s = launch_hf_atm(c)) || (s = launch_heatf(c, c->hf_rec))) return s;
+    if ((s = launch_pack(c)) || (s = launch_hf_atm(c)) || (s = launch_heatf(c, c->hf_rec, false))) return s;
     PGK_CUDA(c, cudaMemcpyAsync(hf, c->hf_rec, sizeof(double) * c->hfp.nhfregion * PGK_HF_NCOL,
                                 cudaMemcpyDeviceToHost, c->st));
     PGK_CUDA(c, cudaStreamSynchronize(c->st));

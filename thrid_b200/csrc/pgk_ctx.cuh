@@ -215,12 +215,13 @@ struct pgk_ctx {
     double* molevel = nullptr;    // [3*nmole]
     double* hf_pot = nullptr;     // [8][N]
     double* hf_W = nullptr;       // [8][nreg][3][N]
-    double* hf_part = nullptr;    // [hf_nblk][nreg][17] calheatf block partials
+    double* hf_acc = nullptr;     // [FLUX_COPIES][nreg][17] region sums (zero between evaluations)
     double* hf_rec = nullptr;     // device heat-flux records
     long long hf_rec_cap = 1;     // records hf_rec holds
-    int hf_nblk = 0;
     double* hf_zs = nullptr;      // [npad_cap] heat-flux z of each sorted slot
     int* hf_ms = nullptr;         // [npad_cap] molecule tag of each sorted slot
+    void* hf_vs = nullptr;        // [npad_cap] (v, transport v_z) of each sorted slot (float4 / double4)
+    uint4* hf_bs = nullptr;       // [npad_cap] region bits of each sorted slot (flux_bits)
     int hf_slots_cap = 0;
     int* lt_mole = nullptr;       // [nmole] register by centre of mass
     int* lt_reg = nullptr;        // [N] Langevin region (-1: none)
@@ -248,6 +249,7 @@ struct pgk_ctx {
     int hf_kspace = 0;            // PGK_HF_KSPACE_* (pgk_set_hf_kspace)
     int hf_kmax = 0;              // waves of the standard-Ewald option
     bool hf_ewk_now = false;      // this force evaluation is the heat-flux step's (standard-Ewald option)
+    const double* hf_k_terms = nullptr;   // per-atom reciprocal terms already formed for this heat-flux evaluation
     bool hf_ewk_fresh = false;    // ewk_out holds ewaldkp_hf at the current positions
 
     // ---- CUDA graphs of captured MD steps (key: driver kind and step flags);
@@ -339,12 +341,15 @@ pgk_status export_morlist(pgk_ctx* c, int32_t* nmorselist, int32_t* mor_index, i
 struct HfDev;
 pgk_status hf_setup(pgk_ctx* c, const pgk_hfparams* p);
 pgk_status launch_hf_atm(pgk_ctx* c);
-pgk_status launch_heatf(pgk_ctx* c, double* dst);
+// record of the region sums at dst (device); pruned: the pruned pair rows are
+// current (the pair kernel ran at these positions)
+pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned);
 pgk_status launch_lt_regist(pgk_ctx* c);
-pgk_status launch_hf_kspace(pgk_ctx* c);           // per-atom reciprocal terms (pgk_set_hf_kspace)
 pgk_status launch_ewk_force(pgk_ctx* c, int group); // ewaldkp_hf force in place of SPME (k_ewald.cu)
 pgk_status launch_langevin(pgk_ctx* c, double dt, long long step, bool former);
 pgk_status launch_bonded_hf(pgk_ctx* c, const HfDev& h);   // k_bonded.cu
+struct FluxDev;
+pgk_status launch_bonded_flux(pgk_ctx* c, const FluxDev& f);
 
 // ---- launchers (k_ewald.cu, ewaldkp_hf) ----
 // one evaluation at the current positions into c->ewk_out (device); nwave out.

@@ -69,6 +69,41 @@ __device__ __forceinline__ void hf_calviri(const HfDev& h, const double* __restr
     }
 }
 
+// ---- region sums of one heat-flux evaluation (calheatf.F90) -------------------
+// J of a region is linear in the per-atom arrays, and those are sums over
+// terms: sum_i viri_i . v_i = sum over pairs of fact (f_i . v_i - f_j . v_j),
+// so the sums form term by term from the velocities, without the arrays.
+// acc: FLUX_COPIES copies of [nreg][17] sums (kinetic, 8 potential, 8 virial
+// terms); a block adds its totals to copy blockIdx % FLUX_COPIES.
+#define FLUX_COPIES 16
+#define FLUX_COLS 17
+struct FluxDev {
+    HfDev h;                 // regions and per-atom typing (pot, W unused)
+    const double* vel;
+    const double* molevel;   // [3*nmole] molecule velocities
+    double* acc;
+};
+
+// bits r of a z: below slab r, above it, inside it (transport term, z wrapped
+// once more as calheatf.F90 does), exactly on one of its planes
+__device__ __forceinline__ uint4 flux_bits(const HfDev& h, double z, double Lz) {
+    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+    const double pz = hf_wrap1(z, Lz);
+    for (int r = 0; r < h.nreg; ++r) {
+        const unsigned b = 1u << r;
+        if (z < h.z1[r]) m.x |= b;
+        if (z > h.z2[r]) m.y |= b;
+        if (h.z1[r] <= pz && pz <= h.z2[r]) m.z |= b;
+        if (z == h.z1[r] || z == h.z2[r]) m.w |= b;
+    }
+    return m;
+}
+
+// heat-flux transport velocity of atom i
+__device__ __forceinline__ double flux_vz(const FluxDev& f, int i) {
+    return f.h.hftyp[i] == PGK_HFTYP_MOLE ? f.molevel[3 * f.h.mol_of[i] + 2] : f.vel[3 * i + 2];
+}
+
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC 2011): counter (atom, step
 // lo, step hi, draw), key = seed; two draws give four uniforms on (0, 1]
 // with 53 random bits each.

@@ -265,7 +265,7 @@ pgk_status pgk_server_submit(pgk_server* sv, const pgk_request* r, int64_t* id) 
         if (r->hf->lt_mole_based) j->ltmole.assign(r->hf->lt_mole_based, r->hf->lt_mole_based + r->sys->nmole);
     }
     j->bytes = pgk_estimate_bytes(r->sys, r->prm);
-    if (j->has_hf) j->bytes += (int64_t)8 * r->sys->natom * (8 + 8 * 3 * j->hf.nhfregion + 4);
+    if (j->has_hf) j->bytes += (int64_t)8 * r->sys->natom * (8 + 8 * 3 * j->hf.nhfregion + 12);
     {
         std::lock_guard<std::mutex> lk(sv->mu);
         j->id = sv->next_id++;
