@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
 // Rows are cut into segments until 16 warps per SM have work (small boxes).
 struct FluxPairArgs {
     const int* rows; const int* cnt; int ccap; int ncl; int nseg;
+    int pruned;                  // rows, cnt: nseg segments of ccap entries per cluster, else whole rows
     const int* typ_s; const int* perm; int ntyp;
     const double* zs; const int* ms; const void* vs; const uint4* bs;
     double rr2, rl2, rmax2;
@@ -324,11 +325,11 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
     const long long nunit = (long long)a.ncl * a.nseg;
     for (long long u = blockIdx.x * 4 + w; u < nunit; u += gridDim.x * 4) {
         const int cl = (int)(u / a.nseg), seg = (int)(u - (long long)cl * a.nseg);
-        const int cnt = a.cnt[cl];
-        const int chunk = ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
-        const int k_lo = seg * chunk, k_hi = min(cnt, k_lo + chunk);
+        const int cnt = a.cnt[a.pruned ? u : cl];
+        const int chunk = a.pruned ? cnt : ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
+        const int k_lo = a.pruned ? 0 : seg * chunk, k_hi = min(cnt, k_lo + chunk);
         if (k_lo >= k_hi) continue;                       // warp-uniform
-        const int* __restrict__ row = a.rows + (size_t)cl * a.ccap;
+        const int* __restrict__ row = a.rows + (size_t)(a.pruned ? u : cl) * a.ccap;
         __syncwarp();
         if (lane < 8) {
             const int s = 8 * cl + lane;
@@ -869,7 +870,7 @@ template <bool MIXED>
 static void flux_pair_launch(pgk_ctx* c, FluxPairArgs& a, const FluxDev& f) {
     // about 16 warps per SM, in row segments where the clusters alone are fewer
     const int want = c->nsm * 16;
-    a.nseg = std::max(1, std::min(8, want / std::max(a.ncl, 1)));
+    a.nseg = a.pruned ? c->pseg : std::max(1, std::min(8, want / std::max(a.ncl, 1)));
     const long long units = (long long)a.ncl * a.nseg;
     const int blocks = (int)std::max(1LL, std::min((units + 3) / 4, (long long)c->nsm * 16));
     if (f.h.nreg == 1)
@@ -902,9 +903,9 @@ pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
     PGK_LAUNCHED(c);
     if (pair_on) {
         FluxPairArgs a;
-        const bool pr = pruned && c->mixed() && c->prune_buffer > 0.f;
-        a.rows = pr ? c->plist : c->clist; a.cnt = pr ? c->pcnt : c->ccnt;
-        a.ccap = c->ccap; a.ncl = c->ncl;
+        a.pruned = pruned && c->prune_buffer > 0.f;
+        a.rows = a.pruned ? c->plist : c->clist; a.cnt = a.pruned ? c->pcnt : c->ccnt;
+        a.ccap = a.pruned ? c->pcap : c->ccap; a.ncl = c->ncl;
         a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
         a.zs = c->hf_zs; a.ms = c->hf_ms; a.vs = c->hf_vs; a.bs = c->hf_bs;
         a.rr2 = c->prm.rrcut * c->prm.rrcut;

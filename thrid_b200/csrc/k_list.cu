@@ -7,10 +7,10 @@
 // each cell's segment is padded with dummy slots (perm = -1) to a multiple of
 // 8, so every 8-slot CLUSTER lies inside one cell.
 //
-// List.  For every i-cluster the row holds each atom slot t that is a
-// partner of at least one of the cluster's atoms s with t > s, as
+// List.  For every i-cluster the row holds each atom slot t of a cluster that
+// it owns (owns) that is a partner of at least one of its atoms, as
 // (mask << 24 | t): bit b of the mask says that (8*cluster + b, t) is a list
-// pair.  Every pair is therefore stored once, in the row of its lower slot.
+// pair.  Every pair is stored once.
 // Membership is the reference test pair for pair: exact FP64
 // r^2 < rcut_book^2 (no FMA, Fortran dnint minimum image) minus the mkexcl
 // exclusions; pgk_get_nblist() writes the pairs back in the reference CSR
@@ -140,22 +140,50 @@ __global__ void k_cell_sort(int* __restrict__ perm, const int* __restrict__ star
     for (int k = threadIdx.x; k < n; k += blockDim.x) perm[b + k] = v[k] & ((1 << SUBKEY_SHIFT) - 1);
 }
 
+// Sorted copies of the build: FP64 positions, types, FP32 positions wrapped
+// into the box (the screening tests) and, per cluster, the centre and half
+// widths of its bounding box (minimum image relative to its first atom).
+// Eight consecutive lanes hold one cluster.
 __global__ void k_sorted_gather(const int* __restrict__ perm, int npad, const double* __restrict__ pos,
-                                const int* __restrict__ typ, int* __restrict__ iperm, double* __restrict__ pos_s,
-                                int* __restrict__ typ_s) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= npad) return;
-    int i = perm[s];
-    if (i < 0) {
-        pos_s[3 * s + 0] = 0.0; pos_s[3 * s + 1] = 0.0; pos_s[3 * s + 2] = 0.0;
-        typ_s[s] = 0;
-        return;
+                                const int* __restrict__ typ, const DynState* __restrict__ dyn,
+                                int* __restrict__ iperm, double* __restrict__ pos_s, int* __restrict__ typ_s,
+                                float4* __restrict__ pf, float4* __restrict__ cbox) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = s < npad ? perm[s] : -1;
+    double x[3] = {0.0, 0.0, 0.0};
+    int ty = 0;
+    if (i >= 0) {
+        iperm[i] = s;
+        ty = typ[i];
+        for (int d = 0; d < 3; ++d) x[d] = pos[3 * (size_t)i + d];
     }
-    iperm[i] = s;
-    pos_s[3 * s + 0] = pos[3 * i + 0];
-    pos_s[3 * s + 1] = pos[3 * i + 1];
-    pos_s[3 * s + 2] = pos[3 * i + 2];
-    typ_s[s] = typ[i];
+    float w[3], lo[3], hi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double L = dyn->box[d];
+        const double xw = x[d] - L * floor(x[d] / L);
+        w[d] = (float)xw;
+        // extent relative to the cluster's first atom (slots of a cluster are real from the front)
+        const double x0 = __shfl_sync(0xffffffffu, xw, threadIdx.x & 24);
+        double r = xw - x0;
+        r -= L * rint(r / L);
+        lo[d] = i >= 0 ? (float)r : 0.f;
+        hi[d] = lo[d];
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+    }
+    if (s >= npad) return;
+    for (int d = 0; d < 3; ++d) pos_s[3 * (size_t)s + d] = x[d];
+    typ_s[s] = ty;
+    pf[s] = make_float4(w[0], w[1], w[2], __int_as_float(i));
+    if ((s & 7) == 0) {
+        cbox[s >> 2] = make_float4(w[0] + 0.5f * (lo[0] + hi[0]), w[1] + 0.5f * (lo[1] + hi[1]),
+                                   w[2] + 0.5f * (lo[2] + hi[2]), 0.f);
+        cbox[(s >> 2) + 1] = make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
+    }
 }
 
 __device__ __forceinline__ bool is_excluded(const int* __restrict__ exs_idx, const int* __restrict__ exs_list,
@@ -169,233 +197,343 @@ __device__ __forceinline__ bool is_excluded(const int* __restrict__ exs_idx, con
     return false;
 }
 
-// one warp per i-cluster: scan the distinct neighbour cells of the cluster's
-// cell, candidates t above the cluster's first slot only (each pair is stored
-// in its lower slot's row).  A candidate farther than rcut_book (+ margin)
-// from the bounding box of the cluster's atoms is skipped; otherwise all 8
-// cluster atoms get the exact reference test (FP64, exclusions) and the entry
-// (mask << 24 | t) is appended when any bit is set.
-// nlistnball (the reference's row count, one sentinel per empty row) is the
-// number of pairs plus the atoms i < n-1 without a partner of higher index;
-// hasup[i] = 1 marks the atoms that have one.
-__global__ void __launch_bounds__(256) k_build_clist(
-        const double* __restrict__ pos_s, const int* __restrict__ perm, const int* __restrict__ cell_of,
-        const int* __restrict__ cell_start, const int* __restrict__ cell_cnt, const int* __restrict__ exs_idx,
-        const int* __restrict__ exs_list, const int2* __restrict__ exs_rng, int n, int ncl, int ccap, int sort_rows,
-        double sqcut, double rbox, float sqlo, float sqhi,
-        const DynState* __restrict__ dyn, int* __restrict__ clist, int* __restrict__ ccnt,
-        unsigned char* __restrict__ hasup, unsigned long long* __restrict__ counters, unsigned* __restrict__ status) {
-    __shared__ double spi[8][3 * 8];
-    __shared__ int sio[8][8];
-    __shared__ int2 srng[8][8];
-    const int wib = threadIdx.x >> 5;
-    const int cl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (cl >= ncl) return;
-    const int s0 = 8 * cl;
-    if (lane < 8) {
-        int io = perm[s0 + lane];
-        sio[wib][lane] = io;
-        srng[wib][lane] = io >= 0 ? exs_rng[io] : make_int2(INT_MAX, -1);
-        spi[wib][3 * lane] = pos_s[3 * (s0 + lane)];
-        spi[wib][3 * lane + 1] = pos_s[3 * (s0 + lane) + 1];
-        spi[wib][3 * lane + 2] = pos_s[3 * (s0 + lane) + 2];
-    }
-    __syncwarp();
-    const double L[3] = {dyn->box[0], dyn->box[1], dyn->box[2]};
-    const double B[3] = {1.0 / L[0], 1.0 / L[1], 1.0 / L[2]};
+// A pair of clusters I != J is kept in the row of the lower one when I + J is
+// odd and of the higher one when it is even: every cluster then owns about
+// half of its neighbours.  (All pairs in the lower cluster's row made the rows
+// of the first cell layers about twice, those of the last a third of the mean,
+// and the pair kernel's blocks as uneven.)
+__device__ __forceinline__ bool owns(int I, int J) { return ((I + J) & 1) ? I < J : I > J; }
+
+// nearest integer of a moderate x (adding 1.5 2^23 rounds to one)
+__device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
+
+// One block of four warps per i-cluster:
+//  1. bounding boxes: the clusters J of the distinct neighbour cells that the
+//     cluster owns (owns) and whose box comes within rcut_book (a warp takes
+//     every fourth cell, a lane a cluster);
+//  2. the eight atoms of each such J against the eight cluster atoms in FP32
+//     (two cluster atoms per packed operation); FRAME boxes (at least four
+//     cells a side) use coordinates relative to the cluster's centre, others
+//     the image of every pair.  r^2 below sqlo (above sqhi) is inside
+//     (outside) rcut_book whatever the rounding; between the two the
+//     reference's exact FP64 test decides.  Exclusions are looked up when j's
+//     block of atom indices is one of the cluster's excluded partners;
+//  3. the entries (mask << 24 | t) grouped by mask by a stable counting sort
+//     (bins of mask_bin), each warp ranking a quarter of the candidates, and
+//     written to the row: 32 consecutive entries then mostly share their mask
+//     bits, which keeps the pair kernel's warps uniform.
+// Every step keeps the candidates' order, so a build of the same positions
+// gives the same rows.  nlistnball (the reference's row count, one sentinel
+// per empty row) is the number of pairs plus the atoms i < n-1 without a
+// partner of higher index; hasup[slot] = 1 marks the atoms that have one.
+// Bound by issue and the latency of the candidate loads (fetched one iteration
+// ahead).  Measured: 200,004 atoms 1.78 ms (one warp per cluster, a
+// bounding-box test per atom, FP64-to-FP32 conversions per pair) -> 0.82;
+// 12,000 atoms 0.311 -> 0.093; 1,536 atoms 0.104 -> 0.030 ms.
+#define CL_JCAP (MAX_CELL_ATOMS / 8)   // clusters that a warp can queue
+#define CL_CCAP 2048         // candidates sorted at a time (multiple of 128)
+#define CL_EXCAP 32          // excluded partners of an atom staged in shared memory (longer lists: global)
+struct ClistArgs {
+    const float4* pf; const float4* cbox; const double* pos_s;
+    const int* cell_of; const int* cell_start; const int* cell_cnt;
+    const int* exs_idx; const int* exs_list; const int2* exs_rng;
+    int ncl, ccap;
+    double sqcut;
+    float rbox, sqlo, sqhi;
+    int* clist; int* ccnt; unsigned char* hasup; unsigned long long* counters; unsigned* status;
+};
+
+template <bool FRAME>
+__global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState* __restrict__ dyn) {
+    __shared__ int sJ[4][CL_JCAP];
+    __shared__ unsigned cand[CL_CCAP];
+    __shared__ int hist[4][256];
+    __shared__ int soff[5], sne[4], swarp[4], smaxj;
+    __shared__ float4 sxy[4], sz[4];               // cluster atoms 2p, 2p+1: (x0, x1, y0, y1), (z0, z1, -, -)
+    __shared__ int sio[8];
+    __shared__ int2 srng[8];
+    __shared__ int2 scell[27];
+    __shared__ unsigned sbloom[64];
+    __shared__ unsigned char sbin[256];            // mask_bin of every mask
+    __shared__ int sexc[8][CL_EXCAP], snex[8];     // excluded partners of the cluster atoms
+    __shared__ double sbox[6];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int cl = blockIdx.x, s0 = 8 * cl;
+    const float L0 = (float)dyn->box[0], L1 = (float)dyn->box[1], L2 = (float)dyn->box[2];
+    const float B0 = 1.f / L0, B1 = 1.f / L1, B2 = 1.f / L2;
     const int nc0 = dyn->ncell[0], nc1 = dyn->ncell[1], nc2 = dyn->ncell[2];
-    // bounding box of the real cluster atoms, minimum image relative to atom 0
-    double ctr[3], hw[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        double lo = 0.0, hi = 0.0;
-        const double x0 = spi[wib][d];
-        for (int ii = 1; ii < 8; ++ii) {
-            if (sio[wib][ii] < 0) continue;
-            double r = spi[wib][3 * ii + d] - x0;
-            r -= L[d] * rint(r * B[d]);
-            lo = fmin(lo, r); hi = fmax(hi, r);
+    const float4 ctr = a.cbox[2 * cl], hw = a.cbox[2 * cl + 1];
+    if (tid < 8) {
+        const float4 p = a.pf[s0 + tid];
+        const int io = __float_as_int(p.w);
+        sio[tid] = io;
+        srng[tid] = io >= 0 ? a.exs_rng[io] : make_int2(INT_MAX, -1);
+        float x = p.x, y = p.y, z = p.z;
+        if (FRAME) {
+            x -= ctr.x; y -= ctr.y; z -= ctr.z;
+            x = fmaf(-L0, rnd_int(x * B0), x); y = fmaf(-L1, rnd_int(y * B1), y); z = fmaf(-L2, rnd_int(z * B2), z);
         }
-        ctr[d] = x0 + 0.5 * (lo + hi);
-        hw[d] = 0.5 * (hi - lo);
+        ((float*)&sxy[tid >> 1])[tid & 1] = x;
+        ((float*)&sxy[tid >> 1])[2 + (tid & 1)] = y;
+        ((float*)&sz[tid >> 1])[tid & 1] = z;
     }
-    const double rb2 = rbox * rbox;
-    // FP32 copies for the screening tests: a pair whose FP32 squared distance
-    // is below sqlo (above sqhi) is inside (outside) rcut_book whatever the
-    // rounding; only pairs between the two take the exact FP64 test
-    const float Lf[3] = {(float)L[0], (float)L[1], (float)L[2]};
-    const float Bf[3] = {(float)B[0], (float)B[1], (float)B[2]};
-    const float ctrf[3] = {(float)ctr[0], (float)ctr[1], (float)ctr[2]};
-    const float hwf[3] = {(float)hw[0], (float)hw[1], (float)hw[2]};
-    const float rb2f = (float)rb2 * 1.0001f + 1.0e-3f;
-    const int key = cell_of[sio[wib][0]];
+    if (tid == 0) smaxj = 1;
+    if (tid >= 64) sbloom[tid - 64] = 0u;
+    if (tid >= 32 && tid < 35) { sbox[tid - 32] = dyn->box[tid - 32]; sbox[tid - 29] = 1.0 / dyn->box[tid - 32]; }
+    sbin[tid] = (unsigned char)mask_bin(tid);
+    sbin[tid + 128] = (unsigned char)mask_bin(tid + 128);
+    __syncthreads();
+    const int key = a.cell_of[sio[0]];
     const int cx = key % nc0, cy = (key / nc0) % nc1, cz = key / (nc0 * nc1);
     const int nz = nc2 >= 3 ? 3 : nc2, ny = nc1 >= 3 ? 3 : nc1, nx = nc0 >= 3 ? 3 : nc0;
-    int count = 0;
-    unsigned long long npair = 0;
-    unsigned up = 0;                                   // bit ii: cluster atom ii has a higher-index partner
-    int* row = clist + (size_t)cl * ccap;
-    // Candidates that pass the bounding-box test queue up (in scan order) and
-    // are tested against the 8 cluster atoms 32 at a time, so the exact tests
-    // run on full warps.  Entries come out in the same order as a direct scan.
-    __shared__ int squeue[8][32 + 4 * 32];
-    int* queue = squeue[wib];
-    int qn = 0;
-    auto test_batch = [&](int t) {          // t < 0: idle lane
-        unsigned mask = 0;
-        if (t >= 0) {
-            const double xj = pos_s[3 * t], yj = pos_s[3 * t + 1], zj = pos_s[3 * t + 2];
-            const float pjf[3] = {(float)xj, (float)yj, (float)zj};
-            const int jo = perm[t];
-            bool jlow = false;
+    const int ncel = nx * ny * nz;
+    if (tid < ncel) {             // the distinct neighbour cells' clusters
+        const int c = tid % nx, b = (tid / nx) % ny, e = tid / (nx * ny);
+        const int x = nc0 >= 3 ? (cx + c - 1 + nc0) % nc0 : c;
+        const int y = nc1 >= 3 ? (cy + b - 1 + nc1) % nc1 : b;
+        const int z = nc2 >= 3 ? (cz + e - 1 + nc2) % nc2 : e;
+        const int cell = x + nc0 * (y + nc1 * z);
+        const int J0 = a.cell_start[cell] >> 3, nj = (a.cell_cnt[cell] + 7) >> 3;
+        scell[tid] = make_int2(J0, J0 + nj);
+        atomicMax(&smaxj, nj);
+    }
+    {                             // 16 threads a cluster atom
+        const int ii = tid >> 4, io = sio[ii];
+        int b = 0, n = 0;
+        if (io >= 0) { b = a.exs_idx[io]; n = a.exs_idx[io + 1] - b; }
+        for (int q = tid & 15; q < min(n, CL_EXCAP); q += 16) sexc[ii][q] = a.exs_list[b + q];
+        if ((tid & 15) == 0) snex[ii] = n;
+    }
+    // filter of the excluded partners: blocks of 16 atom indices, hashed
+    if (tid >= 32 && tid < 40) {
+        const int2 rg = srng[tid - 32];
+        if (rg.y >= rg.x) {
+            const int b0 = rg.x >> 4, b1 = rg.y >> 4;
+            if (b1 - b0 >= 256) for (int q = 0; q < 64; ++q) sbloom[q] = 0xffffffffu;
+            else for (int q = b0; q <= b1; ++q) atomicOr(&sbloom[(q >> 5) & 63], 1u << (q & 31));
+        }
+    }
+    unsigned vmask = 0;                                  // real cluster atoms
 #pragma unroll
-            for (int ii = 0; ii < 8; ++ii) {
-                const int io = sio[wib][ii];
-                if (io < 0 || t <= s0 + ii) continue;
-                float q2 = 0.f;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    float r = (float)spi[wib][3 * ii + d] - pjf[d];
-                    r -= Lf[d] * rintf(r * Bf[d]);
-                    q2 = fmaf(r, r, q2);
+    for (int ii = 0; ii < 8; ++ii) vmask |= sio[ii] >= 0 ? 1u << ii : 0u;
+    __syncthreads();
+    if (smaxj > CL_JCAP) {       // a cell beyond MAX_CELL_ATOMS: k_cell_scan has set the status, the host stops
+        if (tid == 0) a.ccnt[cl] = 0;
+        return;
+    }
+    const int batch = 4 * max(1, CL_JCAP / smaxj);       // cells of one round of step 1
+    const float rb2 = a.rbox * a.rbox;
+    int* __restrict__ row = a.clist + (size_t)cl * a.ccap;
+    const float mid = 0.5f * (a.sqlo + a.sqhi), band = 0.5f * (a.sqhi - a.sqlo) * 1.0001f;
+    int npair = 0;
+    unsigned up = 0;
+    int count = 0;                                       // row entries so far (uniform)
+    for (int q0 = 0; q0 < ncel; q0 += batch) {
+        // 1: owned clusters near the bounding box
+        int nj = 0;
+        for (int q = q0 + w; q < min(ncel, q0 + batch); q += 4) {
+            const int J1 = scell[q].y;
+            for (int jb = scell[q].x; jb < J1; jb += 32) {
+                const int J = jb + lane;
+                bool ok = J < J1 && (J == cl || owns(cl, J));
+                if (ok) {
+                    const float4 c = a.cbox[2 * J], h = a.cbox[2 * J + 1];
+                    float dx = c.x - ctr.x, dy = c.y - ctr.y, dz = c.z - ctr.z;
+                    dx = fmaf(-L0, rnd_int(dx * B0), dx);
+                    dy = fmaf(-L1, rnd_int(dy * B1), dy);
+                    dz = fmaf(-L2, rnd_int(dz * B2), dz);
+                    const float ex = fmaxf(fabsf(dx) - hw.x - h.x, 0.f), ey = fmaxf(fabsf(dy) - hw.y - h.y, 0.f);
+                    const float ez = fmaxf(fabsf(dz) - hw.z - h.z, 0.f);
+                    ok = ex * ex + ey * ey + ez * ez <= rb2;
                 }
-                if (q2 > sqhi) continue;
-                bool in = q2 < sqlo;
-                if (!in) {       // near rcut_book: the reference's exact FP64 test decides
-                    double r0 = mi_exact(__dsub_rn(spi[wib][3 * ii], xj), L[0], B[0]);
-                    double r1 = mi_exact(__dsub_rn(spi[wib][3 * ii + 1], yj), L[1], B[1]);
-                    double r2 = mi_exact(__dsub_rn(spi[wib][3 * ii + 2], zj), L[2], B[2]);
-                    double dr = __dadd_rn(__dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)), __dmul_rn(r2, r2));
-                    in = dr < sqcut;
-                }
-                const int2 rg = srng[wib][ii];
-                if (in && !(jo >= rg.x && jo <= rg.y && is_excluded(exs_idx, exs_list, io, jo))) {
-                    mask |= 1u << ii;
-                    if (jo > io) up |= 1u << ii;
-                    else jlow = true;
-                }
+                const unsigned b = __ballot_sync(0xffffffffu, ok);
+                if (ok) sJ[w][nj + __popc(b & ((1u << lane) - 1u))] = J;
+                nj += __popc(b);
             }
-            if (jlow) hasup[jo] = 1;
-            npair += (unsigned long long)__popc(mask);
         }
-        const unsigned m = __ballot_sync(0xffffffffu, mask != 0);
-        if (mask) {
-            const int off = count + __popc(m & ((1u << lane) - 1u));
-            if (off < ccap) row[off] = (int)((mask << 24) | (unsigned)t);
+        if (lane == 0) swarp[w] = nj;
+        __syncthreads();
+        if (tid == 0) {
+            int o = 0;
+            for (int q = 0; q < 4; ++q) { soff[q] = o; o += swarp[q]; }
+            soff[4] = o;
         }
-        count += __popc(m);
-    };
-    for (int a = 0; a < nz; ++a) {
-        int z = nc2 >= 3 ? (cz + a - 1 + nc2) % nc2 : a;
-        for (int b = 0; b < ny; ++b) {
-            int y = nc1 >= 3 ? (cy + b - 1 + nc1) % nc1 : b;
-            for (int c = 0; c < nx; ++c) {
-                int x = nc0 >= 3 ? (cx + c - 1 + nc0) % nc0 : c;
-                int cell = x + nc0 * (y + nc1 * z);
-                int t0 = cell_start[cell], t1 = t0 + cell_cnt[cell];
-                if (t1 <= s0 + 1) continue;             // every slot of the cell is below the cluster
-                t0 = max(t0, s0 + 1);
-                for (int tb = t0; tb < t1; tb += 128) {
-                    // four candidates a lane: their positions load together
-                    double px[4][3];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int t = tb + 32 * u + lane;
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) px[u][d] = t < t1 ? pos_s[3 * t + d] : 0.0;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int t = tb + 32 * u + lane;
-                        bool acc = false;
-                        if (t < t1) {
-                            float e2 = 0.f;
-#pragma unroll
-                            for (int d = 0; d < 3; ++d) {
-                                float r = (float)px[u][d] - ctrf[d];
-                                r -= Lf[d] * rintf(r * Bf[d]);
-                                const float ex = fmaxf(fabsf(r) - hwf[d], 0.f);
-                                e2 += ex * ex;
-                            }
-                            acc = e2 <= rb2f;
+        __syncthreads();
+        const int ntot = 8 * soff[4];                    // candidate atoms
+        for (int c0 = 0; c0 < ntot; c0 += CL_CCAP) {
+            const int nc = min(CL_CCAP, ntot - c0);
+            const int part = ((nc + 127) >> 7) << 5;     // a warp's share, a multiple of 32
+            const int lo = w * part, hi = min(nc, lo + part);
+            for (int q = tid; q < 4 * 256; q += 128) (&hist[0][0])[q] = 0;
+            __syncthreads();
+            // 2: masks of this warp's candidates, compacted in order
+            int ne = 0;
+            unsigned known = __reduce_or_sync(0xffffffffu, up);
+            // slot, position and flag of a candidate, loaded one iteration ahead
+            auto fetch = [&](int k, int& t, float4& p, bool& hj) {
+                t = 0;
+                p.w = __int_as_float(-1);
+                hj = true;
+                if (k < hi) {
+                    const int g = (c0 + k) >> 3;
+                    const int q = (g >= soff[1]) + (g >= soff[2]) + (g >= soff[3]);
+                    t = 8 * sJ[q][g - soff[q]] + (k & 7);
+                    p = a.pf[t];
+                    hj = a.hasup[t] != 0;
+                }
+            };
+            int tn;
+            float4 pn;
+            bool hn;
+            fetch(lo + lane, tn, pn, hn);
+            for (int k0 = lo; k0 < hi; k0 += 32) {
+                const int t = tn;
+                const float4 pj = pn;
+                const bool hj = hn;
+                fetch(k0 + 32 + lane, tn, pn, hn);
+                unsigned mask = 0;
+                {
+                    const int jo = __float_as_int(pj.w);
+                    if (jo >= 0) {
+                        float near = 1e30f;              // smallest | r^2 - mid |
+                        float jx = pj.x, jy = pj.y, jz = pj.z;
+                        if (FRAME) {
+                            jx -= ctr.x; jy -= ctr.y; jz -= ctr.z;
+                            jx = fmaf(-L0, rnd_int(jx * B0), jx);
+                            jy = fmaf(-L1, rnd_int(jy * B1), jy);
+                            jz = fmaf(-L2, rnd_int(jz * B2), jz);
                         }
-                        const unsigned ba = __ballot_sync(0xffffffffu, acc);
-                        if (acc) queue[qn + __popc(ba & ((1u << lane) - 1u))] = t;
-                        qn += __popc(ba);
-                    }
-                    __syncwarp();
-                    while (qn >= 32) {
-                        const int tq = queue[lane];
-                        int rest[4];
+                        const float2 nx2 = make_float2(-jx, -jx), ny2 = make_float2(-jy, -jy), nz2 = make_float2(-jz, -jz);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) rest[u] = qn - 32 > 32 * u + lane ? queue[32 + 32 * u + lane] : -1;
-                        __syncwarp();
+                        for (int p = 0; p < 4; ++p) {
+                            const float4 xy = sxy[p], zz = sz[p];
+                            float2 dx = __fadd2_rn(make_float2(xy.x, xy.y), nx2);
+                            float2 dy = __fadd2_rn(make_float2(xy.z, xy.w), ny2);
+                            float2 dz = __fadd2_rn(make_float2(zz.x, zz.y), nz2);
+                            if (!FRAME) {
+                                dx.x = fmaf(-L0, rnd_int(dx.x * B0), dx.x); dx.y = fmaf(-L0, rnd_int(dx.y * B0), dx.y);
+                                dy.x = fmaf(-L1, rnd_int(dy.x * B1), dy.x); dy.y = fmaf(-L1, rnd_int(dy.y * B1), dy.y);
+                                dz.x = fmaf(-L2, rnd_int(dz.x * B2), dz.x); dz.y = fmaf(-L2, rnd_int(dz.y * B2), dz.y);
+                            }
+                            const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                            const float2 off = __fadd2_rn(r2, make_float2(-mid, -mid));
+                            if (off.x < 0.f) mask |= 1u << (2 * p);
+                            if (off.y < 0.f) mask |= 2u << (2 * p);
+                            near = fminf(near, fminf(fabsf(off.x), fabsf(off.y)));
+                        }
+                        unsigned valid = vmask;
+                        if ((t >> 3) == cl) valid &= (1u << (t & 7)) - 1u;   // each pair once: t above the atom
+                        mask &= valid;
+                        if (!(near > band)) {     // near rcut_book: the reference's exact FP64 test decides
+                            const double* pt = a.pos_s + 3 * (size_t)t;
+                            const double x = pt[0], y = pt[1], z = pt[2];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) if (rest[u] >= 0) queue[32 * u + lane] = rest[u];
-                        qn -= 32;
-                        __syncwarp();
-                        test_batch(tq);
+                            for (int ii = 0; ii < 8; ++ii) {
+                                const double* pi = a.pos_s + 3 * (size_t)(s0 + ii);
+                                const double r0 = mi_exact(__dsub_rn(pi[0], x), sbox[0], sbox[3]);
+                                const double r1 = mi_exact(__dsub_rn(pi[1], y), sbox[1], sbox[4]);
+                                const double r2 = mi_exact(__dsub_rn(pi[2], z), sbox[2], sbox[5]);
+                                const double dr = __dadd_rn(__dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)),
+                                                            __dmul_rn(r2, r2));
+                                mask = (mask & ~(1u << ii)) | (dr < a.sqcut ? 1u << ii : 0u);
+                            }
+                            mask &= valid;
+                        }
+                        if (mask && ((sbloom[(jo >> 9) & 63] >> ((jo >> 4) & 31)) & 1u)) {
+                            unsigned m = mask;
+                            while (m) {
+                                const int ii = __ffs(m) - 1;
+                                m &= m - 1;
+                                const int2 rg = srng[ii];
+                                if (jo < rg.x || jo > rg.y) continue;
+                                bool ex = false;
+                                if (snex[ii] <= CL_EXCAP)
+                                    for (int q = 0; q < snex[ii]; ++q) ex = ex || sexc[ii][q] == jo;
+                                else ex = is_excluded(a.exs_idx, a.exs_list, sio[ii], jo);
+                                if (ex) mask &= ~(1u << ii);
+                            }
+                        }
+                        // atoms with a partner of higher index, until all are known
+                        if (mask) {
+                            if (!hj || (mask & ~known)) {
+                                unsigned gt = 0;
+#pragma unroll
+                                for (int ii = 0; ii < 8; ++ii) gt |= (jo > sio[ii] ? 1u : 0u) << ii;
+                                up |= gt & mask;
+                                if (!hj && (mask & ~gt)) a.hasup[t] = 1;
+                            }
+                            npair += __popc(mask);
+                        }
                     }
                 }
+                known |= __reduce_or_sync(0xffffffffu, up);
+                const unsigned b = __ballot_sync(0xffffffffu, mask != 0);
+                if (mask) {
+                    cand[lo + ne + __popc(b & ((1u << lane) - 1u))] = (mask << 24) | (unsigned)t;
+                    atomicAdd(&hist[w][sbin[mask]], 1);
+                }
+                ne += __popc(b);
             }
-        }
-    }
-    if (qn > 0) {
-        const int tq = lane < qn ? queue[lane] : -1;
-        test_batch(tq);
-    }
-    // Group the row's entries by mask (stable counting sort in shared memory,
-    // bins in inverse-Gray-code order of the masks): 32 consecutive entries
-    // then mostly share their mask bits, so the pair kernel's loop over the
-    // mask bits is nearly uniform across the warp.  Entries keep their
-    // candidate (spatial) order inside a mask group; the result is the same on
-    // every build of the same positions.
-    if (sort_rows && count <= ccap) {
-        extern __shared__ int srow_raw[];
-        int* buf = srow_raw + (size_t)wib * (ccap + 256);
-        int* bin = buf + ccap;
-        for (int q = lane; q < 256; q += 32) bin[q] = 0;
-        __syncwarp();
-        for (int k = lane; k < count; k += 32) {
-            const int e = row[k];
-            buf[k] = e;
-            atomicAdd(&bin[mask_bin((unsigned)e >> 24)], 1);
-        }
-        __syncwarp();
-        warp_scan256(bin, lane);                 // exclusive scan of the 256 bins
-        __syncwarp();
-        for (int k0 = 0; k0 < count; k0 += 32) {
-            const int k = k0 + lane;
-            const bool ok = k < count;
-            const int e = ok ? buf[k] : 0;
-            const unsigned key = ok ? mask_bin((unsigned)e >> 24) : 256u + lane;
-            const unsigned grp = __match_any_sync(0xffffffffu, key);
-            const int rank = __popc(grp & ((1u << lane) - 1u));
-            const int base = ok ? bin[key] : 0;
-            __syncwarp();
-            if (ok) {
-                row[base + rank] = e;
-                if (rank == 0) bin[key] = base + __popc(grp);
+            if (lane == 0) sne[w] = ne;
+            __syncthreads();
+            // 3: first position of every (bin, warp), then the ranks
+            int v[2][4], tot = 0;
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) { v[e][q] = hist[q][2 * tid + e]; tot += v[e][q]; }
+            int inc = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
             }
-            __syncwarp();
+            if (lane == 31) swarp[w] = inc;
+            __syncthreads();
+            int run = count + inc - tot;
+            for (int q = 0; q < w; ++q) run += swarp[q];
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) { hist[q][2 * tid + e] = run; run += v[e][q]; }
+            __syncthreads();
+            int* __restrict__ bin = hist[w];
+            for (int k0 = 0; k0 < ne; k0 += 32) {
+                const int k = k0 + lane;
+                const bool ok = k < ne;
+                const unsigned e = ok ? cand[lo + k] : 0u;
+                const unsigned kb = ok ? sbin[e >> 24] : 256u + lane;
+                const unsigned grp = __match_any_sync(0xffffffffu, kb);
+                const int rank = __popc(grp & ((1u << lane) - 1u));
+                const int base = ok ? bin[kb] : 0;
+                __syncwarp();
+                if (ok) {
+                    if (base + rank < a.ccap) row[base + rank] = (int)e;
+                    if (rank == 0) bin[kb] = base + __popc(grp);
+                }
+                __syncwarp();
+            }
+            count += sne[0] + sne[1] + sne[2] + sne[3];
+            __syncthreads();                             // cand, hist, sne are reused
         }
+        __syncthreads();                                 // sJ, soff are reused
     }
     up = __reduce_or_sync(0xffffffffu, up);
     npair = warp_sum(npair);
-    if (lane < 8 && ((up >> lane) & 1u)) hasup[sio[wib][lane]] = 1;
-    if (lane == 0) {
-        ccnt[cl] = min(count, ccap);
-        if (count > ccap) atomicOr(status, ST_LIST_OVERFLOW);
-        atomicMax(&counters[1], (unsigned long long)count);
-        atomicAdd(&counters[0], npair);
+    if (lane < 8 && ((up >> lane) & 1u)) a.hasup[s0 + lane] = 1;
+    if (lane == 0 && npair) atomicAdd(&a.counters[0], (unsigned long long)npair);
+    if (tid == 0) {
+        a.ccnt[cl] = min(count, a.ccap);
+        if (count > a.ccap) atomicOr(a.status, ST_LIST_OVERFLOW);
+        atomicMax(&a.counters[1], (unsigned long long)count);
     }
 }
 
 // atoms i < n-1 without a partner of higher index (one sentinel row each)
-__global__ void k_count_noup(const unsigned char* __restrict__ hasup, int m, unsigned long long* counters) {
+__global__ void k_count_noup(const unsigned char* __restrict__ hasup, const int* __restrict__ iperm, int m,
+                             unsigned long long* counters) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned v = (i < m && !hasup[i]) ? 1u : 0u;
+    unsigned v = (i < m && !hasup[iperm[i]]) ? 1u : 0u;
     unsigned w = __popc(__ballot_sync(0xffffffffu, v));
     if ((threadIdx.x & 31) == 0 && w) atomicAdd(&counters[2], (unsigned long long)w);
 }
@@ -427,7 +565,9 @@ static pgk_status alloc_rows(pgk_ctx* c) {
         c->clist = nullptr;
         return pgk_fail(c, PGK_E_NOMEM, "cluster pair list exceeds device memory");
     }
-    if (c->prune_buffer > 0.f && pgk_dmalloc(c, &c->plist, bytes) != cudaSuccess) {
+    c->pcap = ((c->ccap + c->pseg - 1) / c->pseg + 31) / 32 * 32;
+    const size_t pbytes = sizeof(int) * (size_t)(c->npad_cap / 8) * c->pseg * c->pcap;
+    if (c->prune_buffer > 0.f && pgk_dmalloc(c, &c->plist, pbytes) != cudaSuccess) {
         c->plist = nullptr;
         return pgk_fail(c, PGK_E_NOMEM, "pruned pair list exceeds device memory");
     }
@@ -437,6 +577,8 @@ static pgk_status alloc_rows(pgk_ctx* c) {
 static pgk_status ensure_sorted_capacity(pgk_ctx* c, int npad_cap) {
     if (npad_cap <= c->npad_cap) return PGK_OK;
     pgk_dfree(c, c->perm); pgk_dfree(c, c->pos_s); pgk_dfree(c, c->typ_s); pgk_dfree(c, c->xq); pgk_dfree(c, c->xq64);
+    pgk_dfree(c, c->pf_s); pgk_dfree(c, c->cbox); pgk_dfree(c, c->hasup);
+    c->hasup = nullptr; c->pf_s = nullptr; c->cbox = nullptr;
     pgk_dfree(c, c->ccnt); pgk_dfree(c, c->clist); pgk_dfree(c, c->fsort); pgk_dfree(c, c->plist); pgk_dfree(c, c->pcnt);
     pgk_dfree(c, c->xq_prune);
     c->perm = nullptr; c->pos_s = nullptr; c->typ_s = nullptr; c->xq = nullptr; c->xq64 = nullptr;
@@ -446,17 +588,19 @@ static pgk_status ensure_sorted_capacity(pgk_ctx* c, int npad_cap) {
     PGK_CUDA(c, pgk_dmalloc(c, &c->perm, sizeof(int) * npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->pos_s, sizeof(double) * 3 * npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->typ_s, sizeof(int) * npad_cap));
-    if (c->mixed()) {
-        PGK_CUDA(c, pgk_dmalloc(c, &c->xq, sizeof(int4) * npad_cap));
-        PGK_CUDA(c, pgk_dmalloc(c, &c->fsort, sizeof(long long) * 3 * (size_t)npad_cap));
-        PGK_CUDA(c, cudaMemsetAsync(c->fsort, 0, sizeof(long long) * 3 * (size_t)npad_cap, c->st));
-    }
+    PGK_CUDA(c, pgk_dmalloc(c, &c->pf_s, sizeof(float4) * npad_cap));
+    PGK_CUDA(c, pgk_dmalloc(c, &c->hasup, npad_cap));
+    PGK_CUDA(c, pgk_dmalloc(c, &c->cbox, sizeof(float4) * 2 * ncl));
+    PGK_CUDA(c, pgk_dmalloc(c, &c->fsort, sizeof(long long) * 3 * (size_t)npad_cap));
+    PGK_CUDA(c, cudaMemsetAsync(c->fsort, 0, sizeof(long long) * 3 * (size_t)npad_cap, c->st));
+    if (c->mixed()) PGK_CUDA(c, pgk_dmalloc(c, &c->xq, sizeof(int4) * npad_cap));
     else PGK_CUDA(c, pgk_dmalloc(c, &c->xq64, sizeof(double4) * npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->ccnt, sizeof(int) * ncl));
     if (c->prune_buffer > 0.f) {
-        PGK_CUDA(c, pgk_dmalloc(c, &c->pcnt, sizeof(int) * ncl));
-        PGK_CUDA(c, pgk_dmalloc(c, &c->xq_prune, sizeof(int4) * npad_cap));
-        PGK_CUDA(c, cudaMemsetAsync(c->xq_prune, 0, sizeof(int4) * npad_cap, c->st));
+        const size_t xb = (c->mixed() ? sizeof(int4) : sizeof(double4)) * (size_t)npad_cap;
+        PGK_CUDA(c, pgk_dmalloc(c, &c->pcnt, sizeof(int) * ncl * c->pseg));
+        PGK_CUDA(c, pgk_dmalloc(c, &c->xq_prune, xb));
+        PGK_CUDA(c, cudaMemsetAsync(c->xq_prune, 0, xb, c->st));
     }
     c->npad_cap = npad_cap;
     return alloc_rows(c);
@@ -503,26 +647,30 @@ pgk_status launch_mklist(pgk_ctx* c) {
         PGK_CUDA(c, cudaStreamSynchronize(c->st));
         c->npad = npad;
         c->ncl = npad / 8;
-        k_sorted_gather<<<(npad + 255) / 256, 256, 0, c->st>>>(c->perm, npad, c->pos, c->typ, c->iperm, c->pos_s,
-                                                               c->typ_s);
+        k_sorted_gather<<<(npad + 255) / 256, 256, 0, c->st>>>(c->perm, npad, c->pos, c->typ, c->dyn, c->iperm,
+                                                               c->pos_s, c->typ_s, c->pf_s, c->cbox);
         double sq = c->prm.rcut_book * c->prm.rcut_book;
         // screening margin on r^2: FP32 coordinates (up to twice the box) carry
         // 2^-24 relative error each, a distance component up to 4x that
         const double lmax = std::max(h.box[0], std::max(h.box[1], h.box[2]));
         const double eps_pos = 4.0 * 5.96e-8 * 2.0 * lmax;
         const double scr = std::max(0.01, 2.0 * 2.0 * c->prm.rcut_book * 1.7321 * eps_pos + 1.0e-3);
-        long long threads = (long long)c->ncl * 32;
-        PGK_CUDA(c, cudaMemsetAsync(c->hasup, 0, (size_t)n, c->st));
-        // rows are grouped by mask in shared memory when 8 rows fit (<= 160 KB)
-        const size_t sort_sm = (size_t)8 * (c->ccap + 256) * sizeof(int);
-        const int sort_rows = sort_sm <= 160 * 1024 ? 1 : 0;
-        if (sort_rows) PGK_CUDA(c, smem_limit(k_build_clist, sort_sm));
-        k_build_clist<<<(unsigned)((threads + 255) / 256), 256, sort_rows ? sort_sm : 0, c->st>>>(
-            c->pos_s, c->perm, c->cell_of, c->cell_start, c->cell_cnt, c->exs_idx, c->exs_list, c->exs_rng, n, c->ncl,
-            c->ccap,
-            sort_rows, sq, c->prm.rcut_book + 0.05, (float)(sq * (1.0 - 1.0e-5) - scr),
-            (float)(sq * (1.0 + 1.0e-5) + scr), c->dyn, c->clist, c->ccnt, c->hasup, c->counters, c->status);
-        if (n > 1) k_count_noup<<<(n - 1 + 255) / 256, 256, 0, c->st>>>(c->hasup, n - 1, c->counters);
+        PGK_CUDA(c, cudaMemsetAsync(c->hasup, 0, (size_t)npad, c->st));
+        ClistArgs a;
+        a.pf = c->pf_s; a.cbox = c->cbox; a.pos_s = c->pos_s;
+        a.cell_of = c->cell_of; a.cell_start = c->cell_start; a.cell_cnt = c->cell_cnt;
+        a.exs_idx = c->exs_idx; a.exs_list = c->exs_list; a.exs_rng = c->exs_rng;
+        a.ncl = c->ncl; a.ccap = c->ccap;
+        a.sqcut = sq; a.rbox = (float)(c->prm.rcut_book + 0.05);
+        a.sqlo = (float)(sq * (1.0 - 1.0e-5) - scr); a.sqhi = (float)(sq * (1.0 + 1.0e-5) + scr);
+        a.clist = c->clist; a.ccnt = c->ccnt; a.hasup = c->hasup; a.counters = c->counters; a.status = c->status;
+        // the cluster frame is exact when rcut_book plus half a cell stays below half the box
+        bool frame = true;
+        for (int d = 0; d < 3; ++d)
+            frame = frame && nc[d] >= 4 && c->prm.rcut_book + 0.5 * h.cellsize[d] + 0.1 < 0.5 * h.box[d];
+        if (frame) k_build_clist<true><<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
+        else k_build_clist<false><<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
+        if (n > 1) k_count_noup<<<(n - 1 + 255) / 256, 256, 0, c->st>>>(c->hasup, c->iperm, n - 1, c->counters);
         c->launches += 7;
         PGK_CUDA(c, cudaGetLastError());
         unsigned long long cnt[4];

@@ -3,7 +3,7 @@
 // Work decomposition: one warp per 8-atom i-cluster of the cell-sorted order.
 // The cluster's row holds entries (mask << 24 | j); bit b of the mask says
 // that (cluster atom b, j) is a list pair, and every pair is stored once (in
-// the row of its lower slot).  One gather of j serves up to 8 pairs, and the
+// the row of the cluster that owns it, k_list.cu).  One gather of j serves up to 8 pairs, and the
 // index stream is one 4-byte entry per (cluster, j) instead of one per pair.
 // Each evaluation serves both atoms (Newton's third law): the cluster atoms'
 // forces are register sums closed by warp shuffles, j's force is summed over
@@ -75,43 +75,80 @@ __global__ void k_pack_mixed(const double* __restrict__ pos, const double* __res
 }
 
 __global__ void k_pack_fp64(const double* __restrict__ pos, const double* __restrict__ chrg,
-                            const int* __restrict__ perm, int npad, double4* __restrict__ xq) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= npad) return;
-    int i = perm[s];
-    xq[s] = i < 0 ? make_double4(0, 0, 0, 0) : make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], chrg[i]);
+                            const int* __restrict__ perm, int npad, const DynState* __restrict__ dyn,
+                            double4* __restrict__ xq, const double4* __restrict__ xq_prune,
+                            PruneDev* __restrict__ P) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = s < npad ? perm[s] : -1;
+    double4 v = make_double4(0, 0, 0, 0);
+    if (i >= 0) v = make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], chrg[i]);
+    if (s < npad) xq[s] = v;
+    if (P) {
+        // displacement since the last prune (minimum image, current box), rounded up
+        float dd = 0.f;
+        if (i >= 0) {
+            const double4 o = xq_prune[s];
+            double dx = v.x - o.x, dy = v.y - o.y, dz = v.z - o.z;
+            dx -= dyn->box[0] * rint(dx * dyn->boxinv[0]);
+            dy -= dyn->box[1] * rint(dy * dyn->boxinv[1]);
+            dz -= dyn->box[2] * rint(dz * dyn->boxinv[2]);
+            dd = __double2float_ru(sqrt(dx * dx + dy * dy + dz * dz));
+        }
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(dd));
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(&P->dmax, m);
+    }
 }
 
 pgk_status launch_pack(pgk_ctx* c) {
     int n = c->npad;
     if (n <= 0) return PGK_OK;
+    PruneDev* P = c->prune_buffer > 0.f ? c->prune : nullptr;
     if (c->mixed())
-        k_pack_mixed<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq, c->xq_prune,
-                                                          c->prune_buffer > 0.f ? c->prune : nullptr);
+        k_pack_mixed<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq,
+                                                          (const int4*)c->xq_prune, P);
     else
-        k_pack_fp64<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->xq64);
+        k_pack_fp64<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq64,
+                                                         (const double4*)c->xq_prune, P);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
 }
 
 struct PairArgs {
-    const int* clist; const int* ccnt; int ccap; int ncl;
-    const int* typ_s; const int* perm;
+    const int* clist; const int* ccnt; int ccap; int ncl;     // book rows
+    const int* typ_s;
     int ntyp; int nspl; double h, inv_h;
     double rr2, rl2, rmax2, rrcut;
     // FP32 copies for the mixed kernel, read straight from the parameter
     // bank inside the pair loop (no registers held for them)
     float rr2f, rl2f, inv_hf, hf; int nsplm1;
     float ew_pa, ew_c2a, ew_mk;        // analytic real-space Ewald (EwaldF)
-    void* facc; long long* acc;
-    long long* fsort; int fstride;     // mixed: forces by sorted slot (SoA, stride fstride)
-    // pruned rows (mixed; P null = none): on a prune step (P->do_prune) the
-    // kernel reads the book rows (blist/bcnt), writes each entry's pairs inside
-    // rprune (rp2) compacted into plist/pcnt and the new displacement origin
-    // xq_prune; otherwise it reads plist/pcnt
-    const PruneDev* P; const int* blist; const int* bcnt; int* plist; int* pcnt; int4* xq_prune; float rp2;
+    long long* acc;
+    void* fsort; int fstride;          // forces by sorted slot (SoA, stride fstride; int64 / double)
+    // pruned rows (P null = none): on a prune step (P->do_prune) the kernel
+    // reads the book rows, writes each entry's pairs inside rprune (rp2)
+    // compacted into the pruned rows and the new displacement origin xq_prune;
+    // otherwise it reads the pruned rows
+    const PruneDev* P; int* plist; int* pcnt; void* xq_prune; double rp2; float rp2f;
+    // a cluster's row is taken in pseg segments, a warp each: segment g of a
+    // book row is its g-th part, and what a prune keeps of it goes to the
+    // pruned segment (pcap entries) cl * pseg + g
+    int pseg; int pcap;
 };
+
+// entries of work unit u = cl * pseg + g of the book rows or the pruned rows
+__device__ __forceinline__ const int* pair_rows(const PairArgs& a, int u, bool book, int& cnt) {
+    if (!book) {
+        cnt = __ldg(a.pcnt + u);
+        return a.plist + (size_t)u * a.pcap;
+    }
+    const int cl = u / a.pseg, g = u - cl * a.pseg;
+    const int all = __ldg(a.ccnt + cl);
+    const int part = ((all + a.pseg - 1) / a.pseg + 31) & ~31;
+    const int lo = g * part;
+    cnt = max(0, min(part, all - lo));
+    return a.clist + (size_t)cl * a.ccap + lo;
+}
 
 // ---- real-space Ewald force without a table (mixed precision) -----------------
 // The screened Coulomb force per unit charge product, divided by r,
@@ -243,9 +280,9 @@ __device__ __forceinline__ void pair_term(const float dx, const float dy, const 
 // independent of their order.  The next entry and its j record are loaded
 // before the current entry's pairs are evaluated.
 //
-// Block b owns the contiguous cluster range [b*chunk, (b+1)*chunk); its
-// warps take every 8th cluster of it, so they read overlapping j ranges at
-// the same time (shared L1 lines).  Per-lane energy/virial sums stay in FP32
+// Block b owns a contiguous range of work units (row segments, PairArgs); its
+// warps take every 8th of them, so they read overlapping j ranges at the same
+// time (shared L1 lines).  Per-lane energy/virial sums stay in FP32
 // registers across the block's clusters and are reduced once per block.
 // PRUNE: the body of prune steps (reads the book rows, writes the pruned
 // ones); the other body runs on all other steps (one launch, see k_pair_mixed).
@@ -273,31 +310,32 @@ __device__ __forceinline__ void pair_mixed_body(const int4* __restrict__ xq, con
     const float sy = (float)(dyn->box[1] * (1.0 / 4294967296.0));
     const float sz = (float)(dyn->box[2] * (1.0 / 4294967296.0));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int chunk = (a.ncl + gridDim.x - 1) / gridDim.x;
-    const int c_end = min(a.ncl, (blockIdx.x + 1) * chunk);
+    const int nunit = a.ncl * a.pseg;
+    const int chunk = (nunit + gridDim.x - 1) / gridDim.x;
+    const int u_end = min(nunit, (blockIdx.x + 1) * chunk);
     const int* __restrict__ typ_s = a.typ_s;
-    long long* __restrict__ fs0 = a.fsort;
+    long long* __restrict__ fs0 = (long long*)a.fsort;
     const int fst = a.fstride;
     float ev = 0.f, ee = 0.f;
     float wc[6] = {0, 0, 0, 0, 0, 0}, wl[6] = {0, 0, 0, 0, 0, 0};
 
     const bool prune = PRUNE;
-    const int* __restrict__ rows = prune ? a.blist : a.clist;
-    const int* __restrict__ rcnt = prune ? a.bcnt : a.ccnt;
-    const float rp2 = a.rp2;
+    const bool book = PRUNE || a.P == nullptr;
+    const float rp2 = a.rp2f;
 
-    for (int cl = blockIdx.x * chunk + warp; cl < c_end; cl += wpb) {
+    for (int u = blockIdx.x * chunk + warp; u < u_end; u += wpb) {
+        const int cl = u / a.pseg;
         __syncwarp();
         if (lane < 8) {
             const int4 v = __ldg(xq + 8 * cl + lane);
             si[warp][lane] = v;
             sti[warp][lane] = __ldg(typ_s + 8 * cl + lane) * a.ntyp;
-            if (prune) a.xq_prune[8 * cl + lane] = v;
+            if (prune && u == cl * a.pseg) ((int4*)a.xq_prune)[8 * cl + lane] = v;
         }
         __syncwarp();
-        const int cnt = __ldg(rcnt + cl);
-        const int* __restrict__ row = rows + (size_t)cl * a.ccap;
-        int* __restrict__ prow = a.plist + (size_t)cl * a.ccap;
+        int cnt;
+        const int* __restrict__ row = pair_rows(a, u, book, cnt);
+        int* __restrict__ prow = a.plist + (size_t)u * a.pcap;
         int pcount = 0;
         float f[8][3];
 #pragma unroll
@@ -342,7 +380,7 @@ __device__ __forceinline__ void pair_mixed_body(const int4* __restrict__ xq, con
             }
             e = e1; e1 = e2; pj = pjn; tj = tjn;
         }
-        if (prune && lane == 0) a.pcnt[cl] = pcount;
+        if (prune && lane == 0) a.pcnt[u] = pcount;
 #pragma unroll
         for (int ii = 0; ii < 8; ++ii) {
             const float fx = warp_sum(f[ii][0]), fy = warp_sum(f[ii][1]), fz = warp_sum(f[ii][2]);
@@ -493,10 +531,11 @@ __device__ __forceinline__ void pair_mixed_body_x2(const int4* __restrict__ xq, 
     const float sz = (float)(dyn->box[2] * (1.0 / 4294967296.0));
     const float2 inv_h2 = make_float2(a.inv_hf, a.inv_hf), mh2 = make_float2(-a.hf, -a.hf);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int chunk = (a.ncl + gridDim.x - 1) / gridDim.x;
-    const int c_end = min(a.ncl, (blockIdx.x + 1) * chunk);
+    const int nunit = a.ncl * a.pseg;
+    const int chunk = (nunit + gridDim.x - 1) / gridDim.x;
+    const int u_end = min(nunit, (blockIdx.x + 1) * chunk);
     const int* __restrict__ typ_s = a.typ_s;
-    long long* __restrict__ fs0 = a.fsort;
+    long long* __restrict__ fs0 = (long long*)a.fsort;
     const int fst = a.fstride;
     float2 ev = make_float2(0.f, 0.f), ee = make_float2(0.f, 0.f);
     float wt[6] = {0, 0, 0, 0, 0, 0};                     // TENS: sum F (x) x in the cluster frame
@@ -504,11 +543,11 @@ __device__ __forceinline__ void pair_mixed_body_x2(const int4* __restrict__ xq, 
 #pragma unroll
     for (int k = 0; k < 6; ++k) { wc[k] = make_float2(0.f, 0.f); wl[k] = make_float2(0.f, 0.f); }
 
-    const int* __restrict__ rows = PRUNE ? a.blist : a.clist;
-    const int* __restrict__ rcnt = PRUNE ? a.bcnt : a.ccnt;
-    const float rp2 = a.rp2;
+    const bool book = PRUNE || a.P == nullptr;
+    const float rp2 = a.rp2f;
 
-    for (int cl = blockIdx.x * chunk + warp; cl < c_end; cl += wpb) {
+    for (int u = blockIdx.x * chunk + warp; u < u_end; u += wpb) {
+        const int cl = u / a.pseg;
         __syncwarp();
         const int4 p0 = __ldg(xq + 8 * cl);
         if (lane < 8) {
@@ -520,7 +559,7 @@ __device__ __forceinline__ void pair_mixed_body_x2(const int4* __restrict__ xq, 
             ip[4 + h] = (float)(v.z - p0.z) * sz;
             ip[6 + h] = __int_as_float(v.w);
             ((int*)&stp[warp][lane >> 1])[h] = __ldg(typ_s + 8 * cl + lane) * a.ntyp;
-            if (PRUNE) a.xq_prune[8 * cl + lane] = v;
+            if (PRUNE && u == cl * a.pseg) ((int4*)a.xq_prune)[8 * cl + lane] = v;
         }
         __syncwarp();
         for (int k = lane; k < 4 * a.ntyp; k += 32) {
@@ -529,9 +568,9 @@ __device__ __forceinline__ void pair_mixed_body_x2(const int4* __restrict__ xq, 
             sljc[k] = make_float4(la.x, lb.x, la.y, lb.y);
         }
         __syncwarp();
-        const int cnt = __ldg(rcnt + cl);
-        const int* __restrict__ row = rows + (size_t)cl * a.ccap;
-        int* __restrict__ prow = a.plist + (size_t)cl * a.ccap;
+        int cnt;
+        const int* __restrict__ row = pair_rows(a, u, book, cnt);
+        int* __restrict__ prow = a.plist + (size_t)u * a.pcap;
         int pcount = 0;
         float2 f[4][3];
 #pragma unroll
@@ -594,7 +633,7 @@ __device__ __forceinline__ void pair_mixed_body_x2(const int4* __restrict__ xq, 
             }
             e = e1; e1 = e2; pj = pjn; tj = tjn;
         }
-        if (PRUNE && lane == 0) a.pcnt[cl] = pcount;
+        if (PRUNE && lane == 0) a.pcnt[u] = pcount;
 #pragma unroll
         for (int ii = 0; ii < 8; ++ii) {
             const float2* fp = f[ii >> 1];
@@ -658,104 +697,202 @@ __global__ void __launch_bounds__(pair_threads(FRAME), pair_minb(FRAME)) k_pair_
     }
 }
 
-// ---- pair kernel, FP64 (parity path) ---------------------------------------
-template <bool ENE>
-__global__ void __launch_bounds__(256, 2) k_pair_fp64(const double4* __restrict__ xq, PairArgs a,
-                                                      const double2* __restrict__ lj_g,
-                                                      const double4* __restrict__ spl_g,
-                                                      const DynState* __restrict__ dyn) {
+// ---- pair kernel, FP64 -------------------------------------------------------
+// The same units, rows, prune compaction and modes as the mixed kernel, in
+// double with the reference's spline tables in shared memory.  FRAME boxes
+// (frame_ok) take coordinates relative to the cluster's first atom, one
+// subtraction per axis and pair; other boxes the minimum image per pair, with
+// the rounding as an add and a subtraction of 1.5 2^52 (the images differ
+// from the reference's dnint only at exactly half a box, beyond the cutoff).
+// 1/r comes from one reciprocal square root (rsqrt_d); the spline index is
+// floor(r/h) by a rounded-down add of 2^52.
+// Bound by the FP64 pipe's dependent chains at 16 warps per SM (128 registers).  Measured, 200,004-atom butane rows with
+// tensor: 2.22 ms per evaluation on the book rows with divisions, sqrt and
+// dnint on 16 warps per SM; now 0.75 ms on the pruned rows.
+// 1/sqrt(x) in double: the FP32 approximation (relative error e0 ~ 1e-7) and
+// one third-order step y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 (the series of
+// (1 - e)^(-1/2); the next term is 5/16 e^3 < 1e-20), five FP64 operations.
+// For squared distances in FP32's normal range; within 2 ulp there.
+__device__ __forceinline__ double rsqrt_d(double x) {
+    const double y = (double)rsqrt_ftz((float)x);
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+template <int MODE, bool PRUNE, bool FRAME>
+__device__ __forceinline__ void pair_fp64_body(const double4* __restrict__ xq, const PairArgs& a,
+                                               const double2* __restrict__ lj_g, const double4* __restrict__ spl_g,
+                                               const DynState* __restrict__ dyn) {
+    constexpr bool ENE = MODE == PM_FULL;
+    constexpr bool VIRP = MODE == PM_FULL || (MODE == PM_TENS && !FRAME);   // virial summed per pair
     extern __shared__ double4 smd[];
     double4* sf = smd;
     double4* sp = smd + a.nspl;
-    double2* slj = (double2*)(smd + 2 * a.nspl);
-    __shared__ double4 si[8][8];
-    __shared__ int sti[8][8];
-    for (int k = threadIdx.x; k < a.nspl; k += blockDim.x) { sf[k] = spl_g[k]; sp[k] = spl_g[a.nspl + k]; }
+    double2* slj = (double2*)(smd + (ENE ? 2 : 1) * a.nspl);
+    __shared__ double4 si[4][8];
+    __shared__ int sti[4][8];
+    for (int k = threadIdx.x; k < a.nspl; k += blockDim.x) { sf[k] = spl_g[k]; if (ENE) sp[k] = spl_g[a.nspl + k]; }
     for (int k = threadIdx.x; k < a.ntyp * a.ntyp; k += blockDim.x) slj[k] = lj_g[k];
     __syncthreads();
-    const double L0 = dyn->box[0], L1 = dyn->box[1], L2 = dyn->box[2];
-    const double B0 = 1.0 / L0, B1 = 1.0 / L1, B2 = 1.0 / L2;
+    // box, its inverse and the frame origin from shared memory: registers go to
+    // the force sums (four blocks per SM)
+    __shared__ double sbox[6];
+    __shared__ double4 sp0[4];
+    if (threadIdx.x < 3) {
+        sbox[threadIdx.x] = dyn->box[threadIdx.x];
+        sbox[3 + threadIdx.x] = 1.0 / dyn->box[threadIdx.x];
+    }
+    __syncthreads();
+    const volatile double* L = sbox;
+    const double RND = 6755399441055744.0;             // 1.5 2^52: adding and subtracting it rounds to an integer
+    const double TWO52 = 4503599627370496.0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int chunk = (a.ncl + gridDim.x - 1) / gridDim.x;
-    const int c_end = min(a.ncl, (blockIdx.x + 1) * chunk);
+    const int nunit = a.ncl * a.pseg;
+    const int chunk = (nunit + gridDim.x - 1) / gridDim.x;
+    const int u_end = min(nunit, (blockIdx.x + 1) * chunk);
+    const bool book = PRUNE || a.P == nullptr;
+    double* __restrict__ fs0 = (double*)a.fsort;
+    const int fst = a.fstride;
     double e_vdw = 0, e_elc = 0, vc[6] = {0, 0, 0, 0, 0, 0}, vl[6] = {0, 0, 0, 0, 0, 0};
-    for (int cl = blockIdx.x * chunk + warp; cl < c_end; cl += wpb) {
+    for (int u = blockIdx.x * chunk + warp; u < u_end; u += wpb) {
+        const int cl = u / a.pseg;
+        __syncwarp();
+        auto frame = [&](double4 v) {
+            const volatile double* p0 = (const volatile double*)&sp0[warp];
+            v.x -= p0[0]; v.y -= p0[1]; v.z -= p0[2];
+            v.x = fma(-L[0], rint(v.x * L[3]), v.x);
+            v.y = fma(-L[1], rint(v.y * L[4]), v.y);
+            v.z = fma(-L[2], rint(v.z * L[5]), v.z);
+            return v;
+        };
+        if (FRAME && lane == 0) sp0[warp] = xq[8 * cl];
         __syncwarp();
         if (lane < 8) {
-            si[warp][lane] = xq[8 * cl + lane];
+            const double4 v = xq[8 * cl + lane];
+            si[warp][lane] = FRAME ? frame(v) : v;
             sti[warp][lane] = a.typ_s[8 * cl + lane] * a.ntyp;
+            if (PRUNE && u == cl * a.pseg) ((double4*)a.xq_prune)[8 * cl + lane] = v;
         }
         __syncwarp();
-        const int cnt = a.ccnt[cl];
-        const int* row = a.clist + (size_t)cl * a.ccap;
+        int cnt;
+        const int* __restrict__ row = pair_rows(a, u, book, cnt);
+        int* __restrict__ prow = a.plist + (size_t)u * a.pcap;
+        int pcount = 0;
         double f[8][3];
 #pragma unroll
         for (int ii = 0; ii < 8; ++ii) { f[ii][0] = 0; f[ii][1] = 0; f[ii][2] = 0; }
-        for (int k = lane; k < cnt; k += 32) {
-            const unsigned e = (unsigned)__ldg(row + k);
+        unsigned e = lane < cnt ? (unsigned)__ldg(row + lane) : 0u;
+        for (int k0 = 0; k0 < cnt; k0 += 32) {          // warp-uniform trip count
+            const int kn = k0 + 32 + lane;
+            const unsigned en = kn < cnt ? (unsigned)__ldg(row + kn) : 0u;
             const int j = (int)(e & 0xFFFFFFu);
-            const double4 pj = xq[j];
-            const int tj = a.typ_s[j];
             const unsigned m = e >> 24;
+            double4 pj = xq[j];
+            const int tj = a.typ_s[j];
+            if (FRAME) pj = frame(pj);
             double gx = 0, gy = 0, gz = 0;
+            unsigned nm = 0;
 #pragma unroll
             for (int ii = 0; ii < 8; ++ii) {
                 if (!((m >> ii) & 1u)) continue;
                 const double4 pi = si[warp][ii];
-                double dx = pi.x - pj.x; dx = dx - L0 * round(dx * B0);
-                double dy = pi.y - pj.y; dy = dy - L1 * round(dy * B1);
-                double dz = pi.z - pj.z; dz = dz - L2 * round(dz * B2);
-                const double r2 = dx * dx + dy * dy + dz * dz;
+                double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                if (!FRAME) {
+                    dx = fma(-L[0], __dsub_rn(__dadd_rn(dx * L[3], RND), RND), dx);
+                    dy = fma(-L[1], __dsub_rn(__dadd_rn(dy * L[4], RND), RND), dy);
+                    dz = fma(-L[2], __dsub_rn(__dadd_rn(dz * L[5], RND), RND), dz);
+                }
+                const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                if (PRUNE && !(r2 >= a.rp2)) nm |= 1u << ii;
                 if (r2 > a.rmax2) continue;
-                const double rinv2 = 1.0 / r2;
+                const double rinv = rsqrt_d(r2), rinv2 = rinv * rinv, r = r2 * rinv;
                 double fc = 0, fl = 0;
-                const double r = sqrt(r2);
                 if (r <= a.rrcut) {
                     const double qq = pi.w * pj.w;
-                    const int idx = (int)(r / a.h);
-                    const double d = r - (double)idx * a.h;
+                    const double fb = __dadd_rd(r * a.inv_h, TWO52);
+                    const int idx = (int)min((unsigned)__double2loint(fb), (unsigned)a.nsplm1);
+                    const double d = fma(-__dsub_rn(fb, TWO52), a.h, r);
                     const double4 c = sf[idx];
-                    fc = (c.x + d * (c.y + d * (c.z + d * c.w))) * qq;
+                    fc = fma(d, fma(d, fma(d, c.w, c.z), c.y), c.x) * qq;
                     if (ENE) {
                         const double4 p = sp[idx];
-                        e_elc += (p.x + d * (p.y + d * (p.z + d * p.w))) * qq;
+                        e_elc = fma(fma(d, fma(d, fma(d, p.w, p.z), p.y), p.x), qq, e_elc);
                     }
                 }
                 if (r2 <= a.rl2) {
                     const double2 lp = slj[sti[warp][ii] + tj];
                     const double t2 = rinv2 * lp.x;
-                    const double t6 = t2 * t2 * t2, t12 = t6 * t6;
-                    fl = 12.0 * lp.y * (t12 - t6) * rinv2;
-                    if (ENE) e_vdw += lp.y * (t12 - 2.0 * t6);
+                    const double t6 = t2 * t2 * t2;
+                    fl = 12.0 * lp.y * (t6 * (t6 - 1.0)) * rinv2;
+                    if (ENE) e_vdw = fma(lp.y, t6 * (t6 - 2.0), e_vdw);
                 }
-                const double fx = fc * dx + fl * dx, fy = fc * dy + fl * dy, fz = fc * dz + fl * dz;
+                const double fs = fc + fl;
+                const double fx = fs * dx, fy = fs * dy, fz = fs * dz;
                 f[ii][0] += fx; f[ii][1] += fy; f[ii][2] += fz;
                 gx -= fx; gy -= fy; gz -= fz;
+                if (VIRP) {
+                    const double g = ENE ? fc : fs;
+                    const double ax = g * dx, ay = g * dy, az = g * dz;
+                    vc[0] = fma(ax, dx, vc[0]); vc[1] = fma(ax, dy, vc[1]); vc[2] = fma(ax, dz, vc[2]);
+                    vc[3] = fma(ay, dy, vc[3]); vc[4] = fma(ay, dz, vc[4]); vc[5] = fma(az, dz, vc[5]);
+                }
                 if (ENE) {
-                    vc[0] += fc * dx * dx; vc[1] += fc * dx * dy; vc[2] += fc * dx * dz;
-                    vc[3] += fc * dy * dy; vc[4] += fc * dy * dz; vc[5] += fc * dz * dz;
-                    vl[0] += fl * dx * dx; vl[1] += fl * dx * dy; vl[2] += fl * dx * dz;
-                    vl[3] += fl * dy * dy; vl[4] += fl * dy * dz; vl[5] += fl * dz * dz;
+                    const double bx = fl * dx, by = fl * dy, bz = fl * dz;
+                    vl[0] = fma(bx, dx, vl[0]); vl[1] = fma(bx, dy, vl[1]); vl[2] = fma(bx, dz, vl[2]);
+                    vl[3] = fma(by, dy, vl[3]); vl[4] = fma(by, dz, vl[4]); vl[5] = fma(bz, dz, vl[5]);
                 }
             }
-            force_add<false>(a.facc, a.perm[j], gx, gy, gz);
+            if (m) {
+                if (MODE == PM_TENS && FRAME) {     // j's share of sum F (x) x (frame coordinates)
+                    vc[0] = fma(gx, pj.x, vc[0]); vc[1] = fma(gx, pj.y, vc[1]); vc[2] = fma(gx, pj.z, vc[2]);
+                    vc[3] = fma(gy, pj.y, vc[3]); vc[4] = fma(gy, pj.z, vc[4]); vc[5] = fma(gz, pj.z, vc[5]);
+                }
+                atomicAdd(fs0 + j, gx);
+                atomicAdd(fs0 + j + fst, gy);
+                atomicAdd(fs0 + j + 2 * (size_t)fst, gz);
+            }
+            if (PRUNE) {       // compact the entries that keep a pair inside rprune
+                const unsigned b = __ballot_sync(0xffffffffu, nm != 0);
+                if (nm) prow[pcount + __popc(b & ((1u << lane) - 1u))] = (int)((nm << 24) | (unsigned)j);
+                pcount += __popc(b);
+            }
+            e = en;
         }
+        if (PRUNE && lane == 0) a.pcnt[u] = pcount;
 #pragma unroll
         for (int ii = 0; ii < 8; ++ii) {
             const double fx = warp_sum(f[ii][0]), fy = warp_sum(f[ii][1]), fz = warp_sum(f[ii][2]);
-            if (lane == ii) {
-                const int io = a.perm[8 * cl + ii];
-                if (io >= 0) force_add<false>(a.facc, io, fx, fy, fz);
+            if (lane == ii) {     // padding slots get zero sums (no mask bits)
+                if (MODE == PM_TENS && FRAME) {
+                    const double4 p = si[warp][ii];
+                    vc[0] = fma(fx, p.x, vc[0]); vc[1] = fma(fx, p.y, vc[1]); vc[2] = fma(fx, p.z, vc[2]);
+                    vc[3] = fma(fy, p.y, vc[3]); vc[4] = fma(fy, p.z, vc[4]); vc[5] = fma(fz, p.z, vc[5]);
+                }
+                atomicAdd(fs0 + 8 * cl + ii, fx);
+                atomicAdd(fs0 + 8 * cl + ii + fst, fy);
+                atomicAdd(fs0 + 8 * cl + ii + 2 * (size_t)fst, fz);
             }
         }
     }
-    if (ENE) {
+    if (MODE == PM_FULL) {
         double v[16] = {e_vdw, e_elc, e_elc, vc[0], vc[1], vc[2], vc[3], vc[4], vc[5],
                         vl[0], vl[1], vl[2], vl[3], vl[4], vl[5], vl[0] + vl[3] + vl[5]};
         const int idx[16] = {A_VDW, A_ELC, A_VC, A_VTC + 0, A_VTC + 1, A_VTC + 2, A_VTC + 4, A_VTC + 5, A_VTC + 8,
                              A_VTLJ + 0, A_VTLJ + 1, A_VTLJ + 2, A_VTLJ + 4, A_VTLJ + 5, A_VTLJ + 8, A_VLJ};
         block_acc<16>(v, a.acc, idx, true);
+    } else if (MODE == PM_TENS) {
+        const int idx[6] = {A_VTC + 0, A_VTC + 1, A_VTC + 2, A_VTC + 4, A_VTC + 5, A_VTC + 8};
+        block_acc<6>(vc, a.acc, idx, true);
     }
+}
+
+template <int MODE, bool FRAME>
+__global__ void __launch_bounds__(128, 4) k_pair_fp64(const double4* __restrict__ xq, PairArgs a,
+                                                      const double2* __restrict__ lj_g,
+                                                      const double4* __restrict__ spl_g,
+                                                      const DynState* __restrict__ dyn) {
+    if (a.P != nullptr && a.P->do_prune) pair_fp64_body<MODE, true, FRAME>(xq, a, lj_g, spl_g, dyn);
+    else pair_fp64_body<MODE, false, FRAME>(xq, a, lj_g, spl_g, dyn);
 }
 
 // ---- pruned list -------------------------------------------------------------
@@ -777,28 +914,23 @@ __global__ void k_prune_decide(PruneDev* __restrict__ P, const DynState* __restr
     }
 }
 
-// sorted-slot pair forces -> the group accumulator, leaving the slot buffer
-// zero for the next call
-__device__ __forceinline__ void unsort_slots(int blk, long long* __restrict__ fsort, int fst,
-                                             const int* __restrict__ perm, int npad, long long* __restrict__ facc) {
-    const int s = blk * blockDim.x + threadIdx.x;
+// After a pair evaluation: the sorted-slot forces into the group accumulator,
+// leaving the slot buffer zero for the next call (128 threads a block).
+template <bool MIXED>
+__global__ void __launch_bounds__(128) k_pair_finish(void* __restrict__ fsort, int fst, const int* __restrict__ perm,
+                                                     int npad, void* __restrict__ facc) {
+    typedef typename std::conditional<MIXED, unsigned long long, double>::type T;
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= npad) return;
+    T* f = (T*)fsort;
     const int i = perm[s];
-    const long long vx = fsort[s], vy = fsort[s + fst], vz = fsort[s + 2 * (size_t)fst];
-    if (i >= 0 && (vx | vy | vz)) {     // atomic: other force kernels may run beside it
-        atomicAdd((unsigned long long*)facc + 3 * (size_t)i, (unsigned long long)vx);
-        atomicAdd((unsigned long long*)facc + 3 * (size_t)i + 1, (unsigned long long)vy);
-        atomicAdd((unsigned long long*)facc + 3 * (size_t)i + 2, (unsigned long long)vz);
+    const T vx = f[s], vy = f[s + fst], vz = f[s + 2 * (size_t)fst];
+    if (vx == (T)0 && vy == (T)0 && vz == (T)0) return;
+    if (i >= 0) {     // atomic: other force kernels may run beside it
+        T* o = (T*)facc + 3 * (size_t)i;
+        atomicAdd(o, vx); atomicAdd(o + 1, vy); atomicAdd(o + 2, vz);
     }
-    if (vx | vy | vz) { fsort[s] = 0; fsort[s + fst] = 0; fsort[s + 2 * (size_t)fst] = 0; }
-}
-
-// After a mixed pair evaluation: the sorted-slot forces into the group
-// accumulator (128 threads a block).
-__global__ void __launch_bounds__(128) k_pair_finish(long long* __restrict__ fsort, int fst,
-                                                     const int* __restrict__ perm, int npad,
-                                                     long long* __restrict__ facc) {
-    unsort_slots(blockIdx.x, fsort, fst, perm, npad, facc);
+    f[s] = (T)0; f[s + fst] = (T)0; f[s + 2 * (size_t)fst] = (T)0;
 }
 
 template <int MODE, bool FRAME, bool SC>
@@ -812,7 +944,7 @@ static void pair_mixed_launch2(pgk_ctx* c, const PairArgs& a) {
                 (size_t)((c->ntyp * c->ntyp + 1) & ~1) * sizeof(float2);
     if (FRAME) sm += (size_t)(nt / 32) * 4 * c->ntyp * sizeof(float4);
     long long blocks = (long long)c->nsm * pair_minb(FRAME) * (FRAME ? std::max(c->pair_waves, 1) : 1);
-    const long long need = (c->ncl + nt / 32 - 1) / (nt / 32);
+    const long long need = ((long long)c->ncl * c->pseg + nt / 32 - 1) / (nt / 32);
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     smem_limit(k_pair_mixed<MODE, FRAME, SC>, sm);
@@ -832,6 +964,19 @@ static bool frame_ok(const pgk_ctx* c) {
     return 0.5 * lmin > std::sqrt(3.0) * cs + c->prm.rcut_book + 4.0;
 }
 
+template <int MODE, bool FRAME>
+static void pair_fp64_launch(pgk_ctx* c, const PairArgs& a) {
+    // 128-thread blocks, four per SM, one wave: staging the spline rows (35 KB a
+    // block) costs more than finer chunks gain (200,004 atoms: 0.75 ms with
+    // one wave, 0.80 with two or three; 57,000 atoms: 0.30, 0.31, 0.41 ms)
+    const long long need = ((long long)c->ncl * c->pseg + 3) / 4;
+    const int blocks = (int)std::max(1LL, std::min(need, (long long)c->nsm * 4));
+    const size_t sm = (size_t)(MODE == PM_FULL ? 2 : 1) * c->nspl * sizeof(double4) +
+                      (size_t)c->ntyp * c->ntyp * sizeof(double2);
+    smem_limit(k_pair_fp64<MODE, FRAME>, sm);
+    k_pair_fp64<MODE, FRAME><<<blocks, 128, sm, c->st>>>(c->xq64, a, c->lj64, c->spl64, c->dyn);
+}
+
 template <int MODE>
 static void pair_mixed_launch(pgk_ctx* c, const PairArgs& a) {
     if (frame_ok(c) && !c->no_frame) {
@@ -842,7 +987,7 @@ static void pair_mixed_launch(pgk_ctx* c, const PairArgs& a) {
     }
 }
 
-// After the mixed pair kernel: the sorted-slot forces into the group
+// After the pair kernel: the sorted-slot forces into the group
 // accumulator.  Runs on the context's current stream (the force evaluation
 // may put it beside the SPME chain: the accumulator adds are atomic).  The
 // pruned rows keep the order of the book rows (grouped by their book masks):
@@ -850,9 +995,10 @@ static void pair_mixed_launch(pgk_ctx* c, const PairArgs& a) {
 // prune on the 200k-atom butane rows) than it saved on the steps between
 // prunes.
 pgk_status launch_pair_finish(pgk_ctx* c, int group) {
-    if (c->ncl <= 0 || !c->mixed()) return PGK_OK;
+    if (c->ncl <= 0) return PGK_OK;
     const int nbu = (c->npad + 127) / 128;
-    k_pair_finish<<<nbu, 128, 0, c->st>>>(c->fsort, c->npad_cap, c->perm, c->npad, (long long*)c->facc[group]);
+    if (c->mixed()) k_pair_finish<true><<<nbu, 128, 0, c->st>>>(c->fsort, c->npad_cap, c->perm, c->npad, c->facc[group]);
+    else k_pair_finish<false><<<nbu, 128, 0, c->st>>>(c->fsort, c->npad_cap, c->perm, c->npad, c->facc[group]);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
@@ -863,7 +1009,7 @@ pgk_status launch_pair_finish(pgk_ctx* c, int group) {
 static PairArgs pair_args(pgk_ctx* c, int group) {
     PairArgs a;
     a.clist = c->clist; a.ccnt = c->ccnt; a.ccap = c->ccap; a.ncl = c->ncl;
-    a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp; a.nspl = c->nspl;
+    a.typ_s = c->typ_s; a.ntyp = c->ntyp; a.nspl = c->nspl;
     a.h = c->hspl; a.inv_h = 1.0 / c->hspl;
     a.rrcut = c->prm.rrcut;
     a.rr2 = c->prm.rrcut * c->prm.rrcut;
@@ -877,11 +1023,11 @@ static PairArgs pair_args(pgk_ctx* c, int group) {
         a.ew_c2a = (float)(2.0 * al / std::sqrt(std::acos(-1.0)));
         a.ew_mk = (float)(-al * al * 1.4426950408889634);     // -alpha^2 log2(e)
     }
-    a.facc = c->facc[group];
     a.acc = c->acc + (size_t)group * NACC;
     a.fsort = c->fsort; a.fstride = c->npad_cap;
-    a.P = nullptr; a.blist = nullptr; a.bcnt = nullptr; a.plist = nullptr; a.pcnt = nullptr; a.xq_prune = nullptr;
-    a.rp2 = 0.f;
+    a.P = nullptr; a.plist = nullptr; a.pcnt = nullptr; a.xq_prune = nullptr;
+    a.rp2 = 0.0; a.rp2f = 0.f;
+    a.pseg = c->pseg; a.pcap = c->pcap;
     return a;
 }
 
@@ -957,14 +1103,12 @@ std::string pair_tuning_text() {
 pgk_status launch_pair(pgk_ctx* c, int group, int vmode, bool finish) {
     if (c->ncl <= 0) return PGK_OK;
     PairArgs a = pair_args(c, group);
-    const bool pruned = c->mixed() && c->prune_buffer > 0.f;
-    if (pruned) {
+    if (c->prune_buffer > 0.f) {
         const float rp = (float)std::sqrt(a.rmax2) + c->prune_buffer;
         k_prune_decide<<<1, 32, 0, c->st>>>(c->prune, c->dyn, c->prune_buffer, rp);
         c->launches += 1;
-        a.P = c->prune; a.blist = c->clist; a.bcnt = c->ccnt; a.plist = c->plist; a.pcnt = c->pcnt;
-        a.xq_prune = c->xq_prune; a.rp2 = rp * rp;
-        a.clist = c->plist; a.ccnt = c->pcnt;
+        a.P = c->prune; a.plist = c->plist; a.pcnt = c->pcnt;
+        a.xq_prune = c->xq_prune; a.rp2f = rp * rp; a.rp2 = (double)a.rp2f;
     }
     if (c->rec_pre_pair) {
         PGK_CUDA(c, cudaEventRecord(c->ev_pre_pair, c->st));
@@ -978,17 +1122,11 @@ pgk_status launch_pair(pgk_ctx* c, int group, int vmode, bool finish) {
             default: pair_mixed_launch<PM_FORCE>(c, a); break;
         }
     } else {
-        int blocks = c->nsm * 2;                     // 256-thread blocks, two per SM
-        const long long need = (c->ncl + 7) / 8;
-        if (blocks > need) blocks = (int)need;
-        if (blocks < 1) blocks = 1;
-        size_t sm = (size_t)2 * c->nspl * sizeof(double4) + c->ntyp * c->ntyp * sizeof(double2);
-        if (vmode != PM_FORCE) {
-            smem_limit(k_pair_fp64<true>, sm);
-            k_pair_fp64<true><<<blocks, 256, sm, c->st>>>(c->xq64, a, c->lj64, c->spl64, c->dyn);
-        } else {
-            smem_limit(k_pair_fp64<false>, sm);
-            k_pair_fp64<false><<<blocks, 256, sm, c->st>>>(c->xq64, a, c->lj64, c->spl64, c->dyn);
+        const bool fr = frame_ok(c) && !c->no_frame;
+        switch (vmode) {
+            case PM_FORCE: fr ? pair_fp64_launch<PM_FORCE, true>(c, a) : pair_fp64_launch<PM_FORCE, false>(c, a); break;
+            case PM_TENS: fr ? pair_fp64_launch<PM_TENS, true>(c, a) : pair_fp64_launch<PM_TENS, false>(c, a); break;
+            default: fr ? pair_fp64_launch<PM_FULL, true>(c, a) : pair_fp64_launch<PM_FULL, false>(c, a); break;
         }
         PGK_LAUNCHED(c);
     }
@@ -1013,7 +1151,6 @@ __global__ void k_count_pairs(const double* __restrict__ pos_s, const int* __res
             if (!((e >> (24 + ii)) & 1u)) continue;
             ++bits;
             int s = 8 * cl + ii;
-            if (t <= s) continue;
             double dx = pos_s[3 * s] - pos_s[3 * t]; dx -= L0 * round(dx / L0);
             double dy = pos_s[3 * s + 1] - pos_s[3 * t + 1]; dy -= L1 * round(dy / L1);
             double dz = pos_s[3 * s + 2] - pos_s[3 * t + 2]; dz -= L2 * round(dz / L2);

@@ -683,33 +683,37 @@ pgk_status pgk_init(const pgk_system* s, const pgk_params* p, pgk_ctx** out) {
         double rb = p->rcut_book;
         // partners of an 8-atom cluster: the sphere of radius rcut_book swept
         // over the cluster's extent (~ 2 A), about half of them stored (each
-        // pair once, in its lower slot's row); rows regrow on overflow
+        // pair once); rows regrow on overflow
         double rs = rb + 2.0;
         double expect = (double)n / vol * 4.0 / 3.0 * std::acos(-1.0) * rs * rs * rs;
         int cap = p->max_nbr > 0 ? p->max_nbr : (int)(expect + 128);
         cap = std::min(cap, ((n + 31) / 32) * 32);
         cap = ((cap + 31) / 32) * 32;
         c->ccap = std::max(cap, 32);
-        // pruned list buffer (mixed): PGK_PRUNE_BUFFER overrides the 0.7 A default
+        // row segments of the pair kernel: about 24 warps per SM where the
+        // clusters alone are fewer (1,536 atoms: 192 clusters).  FP64 up to 8 (the
+        // kernel is then 28 us against 144); mixed up to 2: beyond that the SPME
+        // stream is the longer one (1,536 waters 3.48, 3.35, 3.46, 3.54 ms a list
+        // period with 1, 2, 4, 8), and eight replicas served at once pay for the
+        // extra blocks (123, 121, 130, 131 ms)
+        c->pseg = std::max(1, std::min(c->mixed() ? 2 : 8, c->nsm * 24 / ((n + 7) / 8)));
+        // pruned list buffer: PGK_PRUNE_BUFFER overrides the 0.7 A default
         // (200k-atom butane NPT: 0.607 ms per step against 0.609 at 1 A with one
         // wave of pair blocks; 0.587 ms at 0.6, 0.7 and 0.8 A with the autotuned
         // waves); 0 disables pruning, as does a book skin too thin for the buffer
-        if (c->mixed()) {
-            const char* pf = getenv("PGK_PAIR_FRAME");
-            c->no_frame = pf && atoi(pf) == 0;
-            const char* pb = getenv("PGK_PRUNE_BUFFER");
-            const double buf = pb ? atof(pb) : 0.7;
-            const double rmax = std::max(p->rcut, p->rrcut);
-            c->prune_buffer = (buf > 0.0 && rmax + buf < p->rcut_book) ? (float)buf : 0.f;
-            if (pgk_dmalloc(c, &c->prune, sizeof(PruneDev)) ||
-                cudaMemsetAsync(c->prune, 0, sizeof(PruneDev), c->st)) {
-                pgk_free(c);
-                return PGK_E_NOMEM;
-            }
+        const char* pf = getenv("PGK_PAIR_FRAME");
+        c->no_frame = pf && atoi(pf) == 0;
+        const char* pb = getenv("PGK_PRUNE_BUFFER");
+        const double buf = pb ? atof(pb) : 0.7;
+        const double rmax = std::max(p->rcut, p->rrcut);
+        c->prune_buffer = (buf > 0.0 && rmax + buf < p->rcut_book) ? (float)buf : 0.f;
+        if (pgk_dmalloc(c, &c->prune, sizeof(PruneDev)) ||
+            cudaMemsetAsync(c->prune, 0, sizeof(PruneDev), c->st)) {
+            pgk_free(c);
+            return PGK_E_NOMEM;
         }
         if (pgk_dmalloc(c, &c->iperm, n * sizeof(int)) || pgk_dmalloc(c, &c->cell_of, n * sizeof(int)) ||
             pgk_dmalloc(c, &c->subkey, n * sizeof(int)) || pgk_dmalloc(c, &c->counters, 8 * sizeof(unsigned long long)) ||
-            pgk_dmalloc(c, &c->hasup, std::max(n, 1)) ||
             cudaMemsetAsync(c->counters, 0, 8 * sizeof(unsigned long long), c->st)) {
             pgk_free(c);
             return PGK_E_NOMEM;
@@ -757,7 +761,7 @@ pgk_status pgk_free(pgk_ctx* c) {
                     c->dyn, c->chain, c->status, c->lj64, c->lj32, c->spl64, c->spl32, c->exs_idx, c->exs_list, c->exs_rng,
                     c->expair, c->mol_idx, c->mol_list, c->bond_ij, c->bond_p, c->angl_ijk, c->angl_p, c->tors_ijkl,
                     c->tors_p, c->rb_ijkl, c->rb_c, c->p14_ij, c->p14_f, c->cg_idx, c->cg_list, c->c_ij, c->c_d,
-                    c->cell_of, c->subkey, c->cell_cnt, c->cell_start, c->cell_fill, c->perm, c->iperm, c->pos_s, c->clist,
+                    c->cell_of, c->subkey, c->cell_cnt, c->cell_start, c->cell_fill, c->perm, c->iperm, c->pos_s, c->pf_s, c->cbox, c->clist,
                     c->ccnt, c->xq, c->xq64, c->fsort, c->plist, c->pcnt, c->xq_prune, c->prune, c->typ_s, c->counters, c->qacc, c->qc, c->qr, c->bsp,
                     c->plan[0].tw, c->plan[1].tw, c->plan[2].tw, c->fout, c->cg_span, c->cg_fit, c->blk_a0, c->blk_nloc, c->blk_t, c->blk_soff,
                     c->blk_ip, c->blk_incp, c->blk_inc, c->brec[0], c->brec[1], c->brec[2], c->brec[3], c->brec[4],

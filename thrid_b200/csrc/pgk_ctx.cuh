@@ -148,12 +148,17 @@ struct pgk_ctx {
     int* perm = nullptr;          // sorted slot -> original atom, -1 = padding
     int* iperm = nullptr;         // original -> sorted slot
     double* pos_s = nullptr;      // sorted FP64 positions at list time (3*npad)
+    float4* pf_s = nullptr;       // the same wrapped, FP32, with the atom index (list build)
+    float4* cbox = nullptr;       // [ncl][2] bounding box of each cluster: centre, half widths (list build)
     int* clist = nullptr;         // [ncl * ccap] entries (mask << 24) | j-slot
     int* ccnt = nullptr;          // [ncl]
-    // pruned copy of the rows (mixed precision, see PruneDev)
-    int* plist = nullptr;         // [ncl * ccap]
-    int* pcnt = nullptr;          // [ncl]
-    int4* xq_prune = nullptr;     // xq at the last prune
+    // pruned copy of the rows (see PruneDev), in pseg segments of pcap entries
+    // per cluster: the pair kernel's work units (a warp each), so that small
+    // boxes fill the SMs
+    int pseg = 1, pcap = 0;
+    int* plist = nullptr;         // [ncl * pseg * pcap]
+    int* pcnt = nullptr;          // [ncl * pseg]
+    void* xq_prune = nullptr;     // xq (int4) or xq64 (double4) at the last prune
     PruneDev* prune = nullptr;
     float prune_buffer = 0.f;     // A; 0 = no pruning (pair kernel reads the book rows)
     bool no_frame = false;        // PGK_PAIR_FRAME=0: always the per-pair minimum image
@@ -161,12 +166,12 @@ struct pgk_ctx {
     bool pair_tuned = false;
     int ccap = 0;
     int4* xq = nullptr;           // mixed: fixed-point fractional coords + q bits
-    long long* fsort = nullptr;   // mixed: pair forces by sorted slot, [3][npad_cap] int64 fixed point (kept zero between uses)
+    void* fsort = nullptr;        // pair forces by sorted slot, [3][npad_cap] int64 fixed point or double (kept zero between uses)
     double4* xq64 = nullptr;      // fp64: x,y,z,q sorted
     int* typ_s = nullptr;
     unsigned long long* counters = nullptr;   // [0] list pairs, [1] longest cluster row, [2] rows without
                                               //  a higher-index partner; [4..6] count_pairs scratch
-    unsigned char* hasup = nullptr;           // [N] atom has a list partner of higher index
+    unsigned char* hasup = nullptr;           // [npad_cap] a slot's atom has a list partner of higher index
     bool list_valid = false;
     long long list_epoch = 0;     // incremented by every list build (invalidates captured graphs)
 

@@ -215,10 +215,11 @@ int64_t pgk_estimate_bytes(const pgk_system* s, const pgk_params* p) {
     const double rs = p->rcut_book + 2.0;
     double cap = (n / vol * 4.0 / 3.0 * 3.14159265358979 * rs * rs * rs + 128) * 1.25;   // rows regrow with headroom
     if (p->max_nbr > 0) cap = p->max_nbr;
-    const double rows = mixed ? 2.0 : 1.0;                                 // book + pruned rows (mixed)
+    const double rows = 2.0;                                               // book + pruned rows
     double bytes = n * (3 * 24 + 3 * 8 + 4 + 2 * 24 + 12 + 1 + 24)       // state, forces, list keys
-                 + npad * (4 + 24 + 4 + (mixed ? 16 + 24 + 16 : 32))       // sorted copies, slot forces, prune origin
+                 + npad * (4 + 24 + 4 + 20 + (mixed ? 16 + 24 + 16 : 32 + 24 + 32))  // sorted copies, slot forces, prune origin
                  + rows * npad / 8.0 * (cap + 1) * 4                       // cluster rows
+                 + npad / 8.0 * std::min(8.0, 148.0 * 24.0 * 8.0 / n) * 32 * 4   // row segments rounded up
                  + n * 400.0;                                              // bonded terms and incidence
     if (p->ifspme) {
         const double K = (double)p->nfft1 * p->nfft2 * p->nfft3;
