@@ -700,7 +700,7 @@ def single_system_rate(nsteps=100):
 
 
 EWK_WORKLOAD = "water_12288_box49.66_alpha0.32_ewaldkp_hf"
-EWK_FLOPS = {"k_ewk_sfac": 16, "k_ewk_atom": 34}   # FP64 flops per (atom, wave)
+EWK_FLOPS = {"k_ewk_sfac": 6, "k_ewk_atom": 13}    # FP64 flops per (atom, wave): half the waves are evaluated
 EWK_FLOPS_PER_PAIR = sum(EWK_FLOPS.values())
 FP64_NOMINAL_TFLOPS = 37.0   # B200 (HGX) datasheet FP64; no FP64 peak is measured on this pool
 

@@ -235,9 +235,11 @@ struct pgk_ctx {
 
     // ---- standard-Ewald k-space of the bulk heat flux (k_ewald.cu) ----
     int ewk_kmax = 0;             // wave set held in ewk_nv (0: none)
-    int ewk_nwave = 0;            // waves, (0,0,0) first
+    int ewk_nwave = 0;            // waves of the reference's set ((0,0,0) and both halves)
+    int ewk_nquad = 0;            // groups of up to four waves after the waves in ewk_nv
+    std::vector<int> ewk_segw;    // first wave of every segment of the per-atom kernel, end last
     int ewk_nmax[3] = {0, 0, 0};  // largest |n| per axis
-    int4* ewk_nv = nullptr;       // [nwave] (nx, ny, nz, 0)
+    int4* ewk_nv = nullptr;       // half the waves (nx, ny, nz, opens a run) | their groups of four
     double2* ewk_tab = nullptr;   // [rows][N] exp(2 pi i n r_d / L_d), rows = n 0..nmax of x, y, z
     double2* ewk_part = nullptr;  // [nchunk][nwave] structure-factor partial sums (cos, sin)
     double* ewk_coef = nullptr;   // [nwave][EWK_NCOEF] per-wave coefficients
