@@ -18,9 +18,12 @@
 // flags give (coefficients from the chain kernels in DynState).
 template <bool MIXED>
 __global__ void k_kick_drift(double* __restrict__ vel, double* __restrict__ pos, double* __restrict__ old,
-                             const void* __restrict__ fl, const void* __restrict__ fs,
-                             const double* __restrict__ mass, int n, const DynState* __restrict__ dyn, int flags) {
+                             void* __restrict__ fl, const void* __restrict__ fs,
+                             const double* __restrict__ mass, int n, const DynState* __restrict__ dyn, int flags,
+                             long long* __restrict__ acc) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((flags & KD_ZERO) && k < NACC) acc[k] = 0;
     if (k >= 3 * n) return;
     const int d = k % 3;
     double v = vel[k];
@@ -28,6 +31,7 @@ __global__ void k_kick_drift(double* __restrict__ vel, double* __restrict__ pos,
     if (flags & KD_LONG) v = v * dyn->kl_s[d] + (force_get<MIXED>(fl, k) / mass[k / 3]) * dyn->kl_b[d];
     if ((flags & KD_SHORT) && !(flags & KD_SHORT_FIRST)) v = v + dyn->ks_b * (force_get<MIXED>(fs, k) / mass[k / 3]);
     vel[k] = v;
+    if (flags & KD_ZERO) ((long long*)fl)[k] = 0;      // 0 and 0.0 alike
     if (flags & KD_DRIFT) {
         const double x = pos[k];
         if (flags & KD_SAVE) old[k] = x;
@@ -90,6 +94,7 @@ __global__ void k_rattle_pos(double* __restrict__ pos, double* __restrict__ vel,
                              const int2* __restrict__ span, int ngroup, double eps, double dt, int use_rv,
                              const DynState* __restrict__ dyn, unsigned* status,
                              const unsigned char* __restrict__ fit) {
+    pdl_enter();
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroup || (fit && fit[g >> 5])) return;      // staged groups run in k_rattle_warp
     int i1 = gidx[g], i2 = gidx[g + 1];
@@ -159,6 +164,7 @@ __global__ void k_rattle_vel(const double* __restrict__ pos, double* __restrict_
                              const int* __restrict__ gidx, const int* __restrict__ glist, const int2* __restrict__ cij,
                              const double* __restrict__ cd, const int2* __restrict__ span, int ngroup, double eps,
                              unsigned* status, const unsigned char* __restrict__ fit) {
+    pdl_enter();
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroup || (fit && fit[g >> 5])) return;      // staged groups run in k_rattle_warp
     int i1 = gidx[g], i2 = gidx[g + 1];
@@ -381,6 +387,7 @@ __global__ void k_coeffs(DynState* __restrict__ dyn, const ChainDev* __restrict_
 // chain update followed by the step's coefficients (start of an NHC / MTK step)
 __global__ void k_chain_coeffs(ChainDev* __restrict__ chain, const long long* __restrict__ acc, ChainArgs ca,
                                DynState* __restrict__ dyn, CoefArgs cf) {
+    pdl_enter();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     chain_run(chain, acc, ca);
     coeffs_run(dyn, chain, cf);
@@ -401,6 +408,7 @@ __device__ double rkcut_of(const double* box, int n1, int n2, int n3) {
 struct BoxArgs { double dts, rcut, rcut_book; int aniso, nfft1, nfft2, nfft3, update_rk; };
 
 __global__ void k_box(DynState* __restrict__ dyn, ChainDev* __restrict__ chain, BoxArgs a, unsigned* status) {
+    pdl_enter();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     ChainDev& c = *chain;
     double b[3];
@@ -481,6 +489,7 @@ __global__ void __launch_bounds__(256) k_kinetic_end(const double* __restrict__ 
                                                      int n, long long* acc, int dbl, double* part,
                                                      unsigned* done, const DynState* __restrict__ dyn,
                                                      ChainDev* chain, PressArgs pa, ChainArgs ca) {
+    pdl_enter();
     __shared__ double red[8][10];
     __shared__ bool last;
     double v[10] = {0};
@@ -590,12 +599,13 @@ pgk_status launch_zero_group(pgk_ctx* c, int g) {
 pgk_status launch_kick_drift(pgk_ctx* c, int flags) {
     if (!flags) return PGK_OK;
     const int n3 = 3 * c->natom;
-    if (c->mixed())
-        k_kick_drift<true><<<(n3 + 255) / 256, 256, 0, c->st>>>(c->vel, c->pos, c->pos_old, c->facc[0], c->facc[1],
-                                                               c->mass, c->natom, c->dyn, flags);
+    auto* k = c->mixed() ? k_kick_drift<true> : k_kick_drift<false>;
+    if (flags & KD_JOIN)
+        k<<<(n3 + 255) / 256, 256, 0, c->st>>>(c->vel, c->pos, c->pos_old, c->facc[0], c->facc[1], c->mass, c->natom,
+                                               c->dyn, flags, c->acc);
     else
-        k_kick_drift<false><<<(n3 + 255) / 256, 256, 0, c->st>>>(c->vel, c->pos, c->pos_old, c->facc[0], c->facc[1],
-                                                                c->mass, c->natom, c->dyn, flags);
+        launch_pdl(k, (n3 + 255) / 256, 256, 0, c->st, c->vel, c->pos, c->pos_old, c->facc[0], c->facc[1], c->mass,
+                   c->natom, c->dyn, flags, c->acc);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
@@ -631,6 +641,7 @@ __global__ void __launch_bounds__(32 * RATTLE_WARPS) k_rattle_warp(double* __res
                                                                   const DynState* __restrict__ dyn,
                                                                   unsigned* status,
                                                                   const unsigned char* __restrict__ fit) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char rsm_raw[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int gw = (blockIdx.x * RATTLE_WARPS + w) * 32;
@@ -911,6 +922,7 @@ __global__ void __launch_bounds__(64) k_rattle_rigid3(double* __restrict__ pos, 
                                                       const double4* __restrict__ dl, int ngroup, double eps,
                                                       double dt, int use_rv, const DynState* __restrict__ dyn,
                                                       unsigned* status) {
+    pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroup) return;
     double rvi[3] = {1.0, 1.0, 1.0};
@@ -948,6 +960,7 @@ __global__ void __launch_bounds__(64) k_rattle_star(double* __restrict__ pos, do
                                                      const int* __restrict__ sa, const double* __restrict__ sd,
                                                      int4 seg, double eps, double dt, int use_rv,
                                                      const DynState* __restrict__ dyn, unsigned* status) {
+    pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= seg.w) return;
     double rvi[3] = {1.0, 1.0, 1.0};
@@ -962,10 +975,10 @@ static void rattle_star_launch(pgk_ctx* c, bool pos, double eps, double dt, bool
     const int blocks = (c->nstar + 63) / 64;
     const int4 seg = make_int4(c->star_seg[0], c->star_seg[1], c->star_seg[2], c->star_seg[3]);
     if (pos)
-        k_rattle_star<true><<<blocks, 64, 0, c->st>>>(c->pos, c->vel, c->pos_old, c->invmass, c->star_atoms,
+        launch_pdl(k_rattle_star<true>, blocks, 64, 0, c->st, c->pos, c->vel, c->pos_old, c->invmass, c->star_atoms,
                                                        c->star_d, seg, eps, dt, use_rv ? 1 : 0, c->dyn, c->status);
     else
-        k_rattle_star<false><<<blocks, 64, 0, c->st>>>(c->pos, c->vel, nullptr, c->invmass, c->star_atoms,
+        launch_pdl(k_rattle_star<false>, blocks, 64, 0, c->st, c->pos, c->vel, nullptr, c->invmass, c->star_atoms,
                                                         c->star_d, seg, eps, 0.0, 0, c->dyn, c->status);
     PGK_LAUNCHED(c);
 }
@@ -973,10 +986,10 @@ static void rattle_star_launch(pgk_ctx* c, bool pos, double eps, double dt, bool
 static void rattle_rigid3_launch(pgk_ctx* c, bool pos, double eps, double dt, bool use_rv) {
     const int blocks = (c->nr3 + 63) / 64;
     if (pos)
-        k_rattle_rigid3<true><<<blocks, 64, 0, c->st>>>(c->pos, c->vel, c->pos_old, c->invmass, c->r3_atoms,
+        launch_pdl(k_rattle_rigid3<true>, blocks, 64, 0, c->st, c->pos, c->vel, c->pos_old, c->invmass, c->r3_atoms,
                                                          c->r3_d, c->nr3, eps, dt, use_rv ? 1 : 0, c->dyn, c->status);
     else
-        k_rattle_rigid3<false><<<blocks, 64, 0, c->st>>>(c->pos, c->vel, nullptr, c->invmass, c->r3_atoms,
+        launch_pdl(k_rattle_rigid3<false>, blocks, 64, 0, c->st, c->pos, c->vel, nullptr, c->invmass, c->r3_atoms,
                                                           c->r3_d, c->nr3, eps, 0.0, 0, c->dyn, c->status);
     PGK_LAUNCHED(c);
 }
@@ -987,13 +1000,13 @@ static void rattle_warp_launch(pgk_ctx* c, bool pos, double eps, double dt, bool
     const size_t sm = RATTLE_WARPS * sizeof(RattleStage);
     if (pos) {
         smem_limit(k_rattle_warp<true>, sm);
-        k_rattle_warp<true><<<blocks, 32 * RATTLE_WARPS, sm, c->st>>>(c->pos, c->vel, c->pos_old, c->invmass,
+        launch_pdl(k_rattle_warp<true>, blocks, 32 * RATTLE_WARPS, sm, c->st, c->pos, c->vel, c->pos_old, c->invmass,
                                                                      c->cg_idx, c->cg_list, c->c_ij, c->c_d,
                                                                      c->cg_span, c->ncgroup, eps, dt, use_rv ? 1 : 0,
                                                                      c->dyn, c->status, c->cg_fit);
     } else {
         smem_limit(k_rattle_warp<false>, sm);
-        k_rattle_warp<false><<<blocks, 32 * RATTLE_WARPS, sm, c->st>>>(c->pos, c->vel, nullptr, c->invmass,
+        launch_pdl(k_rattle_warp<false>, blocks, 32 * RATTLE_WARPS, sm, c->st, c->pos, c->vel, nullptr, c->invmass,
                                                                       c->cg_idx, c->cg_list, c->c_ij, c->c_d,
                                                                       c->cg_span, c->ncgroup, eps, 0.0, 0, c->dyn,
                                                                       c->status, c->cg_fit);
@@ -1007,7 +1020,7 @@ pgk_status launch_rattle_pos(pgk_ctx* c, double eps, double dt, bool use_rv) {
     if (c->ncgroup == 0) { PGK_CUDA(c, cudaGetLastError()); return PGK_OK; }
     if (c->cg_nfit > 0) rattle_warp_launch(c, true, eps, dt, use_rv);
     if (c->cg_nfit < (c->ncgroup + 31) / 32) {
-        k_rattle_pos<<<(c->ncgroup + 63) / 64, 64, 0, c->st>>>(c->pos, c->vel, c->pos_old, c->invmass, c->cg_idx,
+        launch_pdl(k_rattle_pos, (c->ncgroup + 63) / 64, 64, 0, c->st, c->pos, c->vel, c->pos_old, c->invmass, c->cg_idx,
                                                                c->cg_list, c->c_ij, c->c_d, c->cg_span, c->ncgroup,
                                                                eps, dt, use_rv ? 1 : 0, c->dyn, c->status,
                                                                c->cg_nfit > 0 ? c->cg_fit : nullptr);
@@ -1023,7 +1036,7 @@ pgk_status launch_rattle_vel(pgk_ctx* c, double eps) {
     if (c->ncgroup == 0) { PGK_CUDA(c, cudaGetLastError()); return PGK_OK; }
     if (c->cg_nfit > 0) rattle_warp_launch(c, false, eps, 0.0, false);
     if (c->cg_nfit < (c->ncgroup + 31) / 32) {
-        k_rattle_vel<<<(c->ncgroup + 63) / 64, 64, 0, c->st>>>(c->pos, c->vel, c->invmass, c->cg_idx, c->cg_list,
+        launch_pdl(k_rattle_vel, (c->ncgroup + 63) / 64, 64, 0, c->st, c->pos, c->vel, c->invmass, c->cg_idx, c->cg_list,
                                                                c->c_ij, c->c_d, c->cg_span, c->ncgroup, eps, c->status,
                                                                c->cg_nfit > 0 ? c->cg_fit : nullptr);
         PGK_LAUNCHED(c);
@@ -1063,10 +1076,10 @@ pgk_status launch_kinetic_end(pgk_ctx* c, int mode, int chain_kind, const pgk_md
     int blocks = std::min(c->nsm * 2, (c->natom + 255) / 256);
     if (blocks < 1) blocks = 1;
     if (mode == 2)
-        k_kinetic_end<2><<<blocks, 256, 0, c->st>>>(c->vel, c->mass, c->natom, c->acc, pa.dbl, c->ke_part, c->ke_done,
+        launch_pdl(k_kinetic_end<2>, blocks, 256, 0, c->st, c->vel, c->mass, c->natom, c->acc, pa.dbl, c->ke_part, c->ke_done,
                                                      c->dyn, c->chain, pa, ca);
     else
-        k_kinetic_end<1><<<blocks, 256, 0, c->st>>>(c->vel, c->mass, c->natom, c->acc, pa.dbl, c->ke_part, c->ke_done,
+        launch_pdl(k_kinetic_end<1>, blocks, 256, 0, c->st, c->vel, c->mass, c->natom, c->acc, pa.dbl, c->ke_part, c->ke_done,
                                                      c->dyn, c->chain, pa, ca);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
@@ -1083,7 +1096,7 @@ pgk_status launch_chain_coeffs(pgk_ctx* c, int chain_kind, int coef_kind, const 
     cf.md = md;
     cf.degfree = c->degfree;
     cf.kind = coef_kind;
-    k_chain_coeffs<<<1, 32, 0, c->st>>>(c->chain, c->acc, ca, c->dyn, cf);
+    launch_pdl(k_chain_coeffs, 1, 32, 0, c->st, c->chain, c->acc, ca, c->dyn, cf);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
@@ -1108,7 +1121,7 @@ pgk_status launch_box_update(pgk_ctx* c, int kind, const pgk_mdparams& md, bool 
     a.aniso = (kind == 2 && md.pcont_axis != PGK_PCONT_ISO) ? 1 : 0;
     a.nfft1 = c->prm.nfft1; a.nfft2 = c->prm.nfft2; a.nfft3 = c->prm.nfft3;
     a.update_rk = (with_rkcut || c->prm.mts_ewk == PGK_MTS_SHORT) ? 1 : 0;
-    k_box<<<1, 32, 0, c->st>>>(c->dyn, c->chain, a, c->status);
+    launch_pdl(k_box, 1, 32, 0, c->st, c->dyn, c->chain, a, c->status);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;

@@ -42,9 +42,46 @@ constexpr int pair_minb(bool frame) { return frame ? 5 : 3; }
 constexpr int PAIR_WARPS = 8;                      // shared-memory rows per block (the larger shape)
 
 // ---- pack: sorted (padded) positions for the pair kernel ---------------------
+// decision for this pair evaluation (see PruneDev), by the pack's last block
+__device__ __forceinline__ void prune_decide(PruneDev* __restrict__ P, const DynState* __restrict__ dyn, float buffer,
+                                             float rprune) {
+    const float dmax = __uint_as_float(*(volatile unsigned*)&P->dmax);
+    double bt = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) bt = fmax(bt, fabs(dyn->box[d] / P->box[d] - 1.0));
+    const bool keep = !P->force && (2.0 * (double)dmax + (double)rprune * bt < (double)buffer);   // NaN -> prune
+    P->do_prune = keep ? 0 : 1;
+    if (!keep) {
+        P->dmax = 0u;
+        P->force = 0;
+        for (int d = 0; d < 3; ++d) P->box[d] = dyn->box[d];
+        P->nprune += 1ull;
+    }
+}
+// largest displacement of the block into P->dmax; when a pair evaluation
+// follows (decide), the last block to do so decides (one launch instead of a
+// single-thread kernel behind the pack)
+__device__ __forceinline__ void prune_track(float dd, PruneDev* __restrict__ P, const DynState* __restrict__ dyn,
+                                            float buffer, float rprune, int decide) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(dd));
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(&P->dmax, m);
+    if (!decide) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&P->done, 1u) == gridDim.x - 1u) {
+            __threadfence();
+            P->done = 0u;
+            prune_decide(P, dyn, buffer, rprune);
+        }
+    }
+}
+
 __global__ void k_pack_mixed(const double* __restrict__ pos, const double* __restrict__ chrg,
                              const int* __restrict__ perm, int npad, const DynState* __restrict__ dyn,
-                             int4* __restrict__ xq, const int4* __restrict__ xq_prune, PruneDev* __restrict__ P) {
+                             int4* __restrict__ xq, const int4* __restrict__ xq_prune, PruneDev* __restrict__ P,
+                             float buffer, float rprune, int decide) {
+    pdl_enter();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = s < npad ? perm[s] : -1;
     int4 v = make_int4(0, 0, 0, 0);
@@ -69,15 +106,15 @@ __global__ void k_pack_mixed(const double* __restrict__ pos, const double* __res
             const float dz = (float)(v.z - o.z) * (float)(dyn->box[2] * (1.0 / 4294967296.0));
             dd = sqrtf(dx * dx + dy * dy + dz * dz);
         }
-        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(dd));
-        if ((threadIdx.x & 31) == 0 && m) atomicMax(&P->dmax, m);
+        prune_track(dd, P, dyn, buffer, rprune, decide);
     }
 }
 
 __global__ void k_pack_fp64(const double* __restrict__ pos, const double* __restrict__ chrg,
                             const int* __restrict__ perm, int npad, const DynState* __restrict__ dyn,
                             double4* __restrict__ xq, const double4* __restrict__ xq_prune,
-                            PruneDev* __restrict__ P) {
+                            PruneDev* __restrict__ P, float buffer, float rprune, int decide) {
+    pdl_enter();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = s < npad ? perm[s] : -1;
     double4 v = make_double4(0, 0, 0, 0);
@@ -94,21 +131,26 @@ __global__ void k_pack_fp64(const double* __restrict__ pos, const double* __rest
             dz -= dyn->box[2] * rint(dz * dyn->boxinv[2]);
             dd = __double2float_ru(sqrt(dx * dx + dy * dy + dz * dz));
         }
-        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(dd));
-        if ((threadIdx.x & 31) == 0 && m) atomicMax(&P->dmax, m);
+        prune_track(dd, P, dyn, buffer, rprune, decide);
     }
 }
 
-pgk_status launch_pack(pgk_ctx* c) {
+// the pruned rows hold the pairs inside the larger cutoff plus the buffer
+static float prune_radius(const pgk_ctx* c) {
+    return (float)std::max(c->prm.rrcut, c->prm.rcut) + c->prune_buffer;
+}
+
+pgk_status launch_pack(pgk_ctx* c, bool pair) {
     int n = c->npad;
     if (n <= 0) return PGK_OK;
     PruneDev* P = c->prune_buffer > 0.f ? c->prune : nullptr;
+    const float rp = prune_radius(c);
     if (c->mixed())
-        k_pack_mixed<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq,
-                                                          (const int4*)c->xq_prune, P);
+        launch_pdl(k_pack_mixed, (n + 255) / 256, 256, 0, c->st, c->pos, c->chrg, c->perm, n, c->dyn, c->xq,
+                   (const int4*)c->xq_prune, P, c->prune_buffer, rp, pair ? 1 : 0);
     else
-        k_pack_fp64<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq64,
-                                                         (const double4*)c->xq_prune, P);
+        launch_pdl(k_pack_fp64, (n + 255) / 256, 256, 0, c->st, c->pos, c->chrg, c->perm, n, c->dyn, c->xq64,
+                   (const double4*)c->xq_prune, P, c->prune_buffer, rp, pair ? 1 : 0);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
@@ -679,7 +721,7 @@ __device__ __forceinline__ void pair_mixed_body_x2(const int4* __restrict__ xq, 
     }
 }
 
-// One launch per evaluation: the step kind that k_prune_decide wrote on the
+// One launch per evaluation: the step kind that the pack wrote on the
 // device (prune step or not) selects the body, block-uniformly.  FRAME boxes
 // run the packed body (SC: equal LJ and Coulomb cutoffs).
 template <int MODE, bool FRAME, bool SC>
@@ -687,6 +729,7 @@ __global__ void __launch_bounds__(pair_threads(FRAME), pair_minb(FRAME)) k_pair_
                                                                         const float2* __restrict__ lj_g,
                                                                         const float4* __restrict__ spl_g,
                                                                         const DynState* __restrict__ dyn) {
+    pdl_enter();
     const bool prune = a.P != nullptr && a.P->do_prune;
     if (FRAME) {
         if (prune) pair_mixed_body_x2<MODE, true, SC>(xq, a, lj_g, spl_g, dyn);
@@ -891,34 +934,18 @@ __global__ void __launch_bounds__(128, 4) k_pair_fp64(const double4* __restrict_
                                                       const double2* __restrict__ lj_g,
                                                       const double4* __restrict__ spl_g,
                                                       const DynState* __restrict__ dyn) {
+    pdl_enter();
     if (a.P != nullptr && a.P->do_prune) pair_fp64_body<MODE, true, FRAME>(xq, a, lj_g, spl_g, dyn);
     else pair_fp64_body<MODE, false, FRAME>(xq, a, lj_g, spl_g, dyn);
 }
 
 // ---- pruned list -------------------------------------------------------------
-// decision for this pair evaluation (one thread; see PruneDev)
-__global__ void k_prune_decide(PruneDev* __restrict__ P, const DynState* __restrict__ dyn, float buffer,
-                               float rprune) {
-    if (threadIdx.x || blockIdx.x) return;
-    const float dmax = __uint_as_float(P->dmax);
-    double bt = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) bt = fmax(bt, fabs(dyn->box[d] / P->box[d] - 1.0));
-    const bool keep = !P->force && (2.0 * (double)dmax + (double)rprune * bt < (double)buffer);   // NaN -> prune
-    P->do_prune = keep ? 0 : 1;
-    if (!keep) {
-        P->dmax = 0u;
-        P->force = 0;
-        for (int d = 0; d < 3; ++d) P->box[d] = dyn->box[d];
-        P->nprune += 1ull;
-    }
-}
-
 // After a pair evaluation: the sorted-slot forces into the group accumulator,
 // leaving the slot buffer zero for the next call (128 threads a block).
 template <bool MIXED>
 __global__ void __launch_bounds__(128) k_pair_finish(void* __restrict__ fsort, int fst, const int* __restrict__ perm,
                                                      int npad, void* __restrict__ facc) {
+    pdl_enter();
     typedef typename std::conditional<MIXED, unsigned long long, double>::type T;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= npad) return;
@@ -948,7 +975,7 @@ static void pair_mixed_launch2(pgk_ctx* c, const PairArgs& a) {
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     smem_limit(k_pair_mixed<MODE, FRAME, SC>, sm);
-    k_pair_mixed<MODE, FRAME, SC><<<(int)blocks, nt, sm, c->st>>>(c->xq, a, c->lj32, c->spl32, c->dyn);
+    launch_pdl(k_pair_mixed<MODE, FRAME, SC>, (unsigned)blocks, nt, sm, c->st, c->xq, a, c->lj32, c->spl32, c->dyn);
     PGK_LAUNCHED(c);
 }
 
@@ -974,7 +1001,7 @@ static void pair_fp64_launch(pgk_ctx* c, const PairArgs& a) {
     const size_t sm = (size_t)(MODE == PM_FULL ? 2 : 1) * c->nspl * sizeof(double4) +
                       (size_t)c->ntyp * c->ntyp * sizeof(double2);
     smem_limit(k_pair_fp64<MODE, FRAME>, sm);
-    k_pair_fp64<MODE, FRAME><<<blocks, 128, sm, c->st>>>(c->xq64, a, c->lj64, c->spl64, c->dyn);
+    launch_pdl(k_pair_fp64<MODE, FRAME>, blocks, 128, sm, c->st, c->xq64, a, c->lj64, c->spl64, c->dyn);
 }
 
 template <int MODE>
@@ -997,8 +1024,8 @@ static void pair_mixed_launch(pgk_ctx* c, const PairArgs& a) {
 pgk_status launch_pair_finish(pgk_ctx* c, int group) {
     if (c->ncl <= 0) return PGK_OK;
     const int nbu = (c->npad + 127) / 128;
-    if (c->mixed()) k_pair_finish<true><<<nbu, 128, 0, c->st>>>(c->fsort, c->npad_cap, c->perm, c->npad, c->facc[group]);
-    else k_pair_finish<false><<<nbu, 128, 0, c->st>>>(c->fsort, c->npad_cap, c->perm, c->npad, c->facc[group]);
+    if (c->mixed()) launch_pdl(k_pair_finish<true>, nbu, 128, 0, c->st, c->fsort, c->npad_cap, c->perm, c->npad, c->facc[group]);
+    else launch_pdl(k_pair_finish<false>, nbu, 128, 0, c->st, c->fsort, c->npad_cap, c->perm, c->npad, c->facc[group]);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
@@ -1054,7 +1081,7 @@ pgk_status pair_autotune(pgk_ctx* c) {
     const char* env = getenv("PGK_PAIR_AUTOTUNE");
     if (!env || atoi(env) == 0 || !c->mixed() || c->ncl <= 0 || !frame_ok(c) || c->no_frame) return PGK_OK;
     pgk_status s;
-    if ((s = launch_pack(c))) return s;               // current positions into the sorted slots
+    if ((s = launch_pack(c, false))) return s;        // current positions into the sorted slots
     const PairArgs a = pair_args(c, 0);
     const bool sc = a.rr2f == a.rl2f;
     cudaEvent_t e0, e1;
@@ -1104,9 +1131,7 @@ pgk_status launch_pair(pgk_ctx* c, int group, int vmode, bool finish) {
     if (c->ncl <= 0) return PGK_OK;
     PairArgs a = pair_args(c, group);
     if (c->prune_buffer > 0.f) {
-        const float rp = (float)std::sqrt(a.rmax2) + c->prune_buffer;
-        k_prune_decide<<<1, 32, 0, c->st>>>(c->prune, c->dyn, c->prune_buffer, rp);
-        c->launches += 1;
+        const float rp = prune_radius(c);
         a.P = c->prune; a.plist = c->plist; a.pcnt = c->pcnt;
         a.xq_prune = c->xq_prune; a.rp2f = rp * rp; a.rp2 = (double)a.rp2f;
     }

@@ -113,6 +113,7 @@ template <bool MIXED, int P>
 __global__ void __launch_bounds__(256) k_spread_rows(const double* __restrict__ pos, const double* __restrict__ chrg,
                                                      int n, const DynState* __restrict__ dyn, int K1, int K2, int K3,
                                                      void* __restrict__ qacc, const int* __restrict__ order) {
+    pdl_enter();
     constexpr int G = 32 / P;
     const int lane = threadIdx.x & 31;
     const int g = lane / P, i1 = lane - g * P;
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(256) k_fft(typename C2<T>::t* __restrict__ dat
     T2* bufB = bufA + P * ld;
     T2* tws = bufB + P * ld;              // twiddle table (n entries) staged in shared memory
     for (int k = threadIdx.x; k < n; k += blockDim.x) tws[k] = ((const T2*)plan.tw)[k];
+    pdl_enter();                          // the twiddles are constant
     size_t base;
     size_t stride;
     int yz = 0;
@@ -536,6 +538,7 @@ __global__ void __launch_bounds__(256) k_fft_rx(typename C2<T>::t* __restrict__ 
     T2* tw2 = tws + N;                    // exp(-2 pi i k / K1), k = 0..N
     for (int k = threadIdx.x; k < N; k += blockDim.x) tws[k] = ((const T2*)plan.tw)[k];
     for (int k = threadIdx.x; k <= N; k += blockDim.x) tw2[k] = ((const T2*)tw2g)[k];
+    pdl_enter();                          // the twiddles are constant
     const int line0 = blockIdx.x * P;
     if (FWD) {
         for (int idx = threadIdx.x; idx < P * N; idx += blockDim.x) {
@@ -724,6 +727,7 @@ __global__ void __launch_bounds__(256) k_gather_rows(const double* __restrict__ 
                                                      int n, const DynState* __restrict__ dyn, int K1, int K2, int K3,
                                                      const void* __restrict__ qc, void* facc,
                                                      const int* __restrict__ order) {
+    pdl_enter();
     typedef typename std::conditional<MIXED, float, double>::type T;
     typedef typename C2<T>::t T2;
     constexpr int G = 32 / P;
@@ -903,9 +907,10 @@ template <typename T, int AXIS, int SRC, int NC, bool CONV>
 static void fft_launch(pgk_ctx* c, const FftDev& fd, int grid, int P, size_t sm, int sign, const ConvArgs& ca,
                        int K1) {
     typedef typename C2<T>::t T2;
-    smem_limit(k_fft<T, AXIS, SRC, NC, CONV>, sm);
-    k_fft<T, AXIS, SRC, NC, CONV><<<grid, 256, sm, c->st>>>((T2*)c->qc, SRC == 3 ? c->qr : c->qacc, K1, c->K[1],
-                                                            c->K[2], fd, P, (T)sign, ca, c->dyn);
+    auto* k = k_fft<T, AXIS, SRC, NC, CONV>;
+    smem_limit(k, sm);
+    launch_pdl(k, grid, 256, sm, c->st, (T2*)c->qc, SRC == 3 ? c->qr : c->qacc, K1, c->K[1], c->K[2], fd, P, (T)sign,
+               ca, c->dyn);
 }
 
 // x_ext: x points of the complex grid (0: K1; K1/2 + 1 on the half spectrum of
@@ -959,7 +964,7 @@ static pgk_status fft_rx_pass(pgk_ctx* c) {
 #define PGK_RX(NCV)                                                                                            \
     do {                                                                                                       \
         smem_limit(k_fft_rx<T, SRC, NCV, FWD>, sm);                                                            \
-        k_fft_rx<T, SRC, NCV, FWD><<<grid, 256, sm, c->st>>>((T2*)c->qc, real, c->K[0], nline, fd, c->tw_rx, P); \
+        launch_pdl(k_fft_rx<T, SRC, NCV, FWD>, grid, 256, sm, c->st, (T2*)c->qc, real, c->K[0], nline, fd, c->tw_rx, P); \
     } while (0)
     switch (pl.n) {
         case 16: PGK_RX(16); break;
@@ -1173,8 +1178,8 @@ static void spread_gather(pgk_ctx* c, bool gather, int group) {
         k_spread_rows<MIXED, P><<<(warps + 7) / 8, 256, 0, c->st>>>(c->pos, c->chrg, n, c->dyn, c->K[0], c->K[1],
                                                                     c->K[2], c->qacc, order);
     else
-        k_gather_rows<MIXED, P><<<(warps + 7) / 8, 256, 0, c->st>>>(c->pos, c->chrg, n, c->dyn, c->K[0], c->K[1],
-                                                                    c->K[2], c->qr, c->facc[group], order);
+        launch_pdl(k_gather_rows<MIXED, P>, (warps + 7) / 8, 256, 0, c->st, c->pos, c->chrg, n, c->dyn, c->K[0], c->K[1],
+                   c->K[2], c->qr, c->facc[group], order);
     PGK_LAUNCHED(c);
 }
 
@@ -1194,8 +1199,10 @@ static pgk_status dispatch_sg(pgk_ctx* c, bool gather, int group) {
 }
 
 pgk_status launch_spme(pgk_ctx* c, int group, bool ene, bool vir) {
-    size_t KK = (size_t)c->K[0] * c->K[1] * c->K[2];
-    PGK_CUDA(c, cudaMemsetAsync(c->qacc, 0, KK * 8, c->st));
+    // cleared here, beside the start of the pair kernel (clearing each point
+    // behind the first forward pass's read put the writes on the step's tail:
+    // 200,004 atoms 0.60 -> 0.64 ms)
+    PGK_CUDA(c, cudaMemsetAsync(c->qacc, 0, (size_t)c->K[0] * c->K[1] * c->K[2] * 8, c->st));
     pgk_status s;
     long long* acc = c->acc + (size_t)group * NACC;
     int want = (ene || vir) ? 1 : 0;

@@ -132,10 +132,11 @@ pgk_status read_status(pgk_ctx* c) {
 // the prune decision, so the pair kernel's blocks are dispatched first.
 // Every add into the shared force and energy accumulators is atomic (int64 in
 // mixed precision: exact and independent of the interleaving).
-pgk_status force_group(pgk_ctx* c, int flag, bool ene, bool vir, bool tensor_only = false) {
+// zeroed: the group's accumulators are already zero (KD_ZERO).
+pgk_status force_group(pgk_ctx* c, int flag, bool ene, bool vir, bool tensor_only = false, bool zeroed = false) {
     int g = flag == PGK_MTS_LONG ? 0 : 1;
     pgk_status s;
-    if ((s = launch_zero_group(c, g))) return s;
+    if (!zeroed && (s = launch_zero_group(c, g))) return s;
     const bool pairs = c->prm.mts_vdw == flag;
     if (pairs && !c->list_valid && (s = launch_mklist(c))) return s;
     const int mask = (c->prm.mts_bond == flag ? 1 : 0) | (c->prm.mts_angl == flag ? 2 : 0) |
@@ -164,7 +165,7 @@ pgk_status force_group(pgk_ctx* c, int flag, bool ene, bool vir, bool tensor_onl
     }
     bool bonded_after_pair = false;
     if (pairs) {
-        if ((s = launch_pack(c))) return s;
+        if ((s = launch_pack(c, true))) return s;
         const int vmode = vir ? (tensor_only ? PM_TENS : PM_FULL) : (ene ? PM_ENE : PM_FORCE);
         c->rec_pre_pair = third;
         c->rec_pre_pair_done = false;
@@ -864,7 +865,7 @@ pgk_status pgk_ewaldr(pgk_ctx* c, double* force, pgk_energies* e, pgk_virials* v
     bool want = e || v;
     if ((s = launch_zero_group(c, 0))) return s;
     if (!c->list_valid && (s = launch_mklist(c))) return s;
-    if ((s = launch_pack(c)) || (s = launch_pair(c, 0, want ? PM_FULL : PM_FORCE)) ||
+    if ((s = launch_pack(c, true)) || (s = launch_pair(c, 0, want ? PM_FULL : PM_FORCE)) ||
         (s = launch_intra(c, 0, 32, want)))
         return s;
     if (force && (s = force_to_host(c, 0, force, true))) return s;
@@ -986,7 +987,7 @@ pgk_status pgk_bench_kernel(pgk_ctx* c, int32_t which, int32_t iters, double* ms
     if (!c || iters < 1 || !ms) return PGK_E_INVALID;
     pgk_status s;
     if (!c->list_valid && (s = launch_mklist(c))) return s;
-    if ((s = launch_pack(c))) return s;
+    if ((s = launch_pack(c, which == 0))) return s;
     if (which == 0) {
         long long np = 0, ne = 0;
         if ((s = count_pairs(c, &np, &ne))) return s;
@@ -1021,6 +1022,7 @@ pgk_status pgk_bench_kernel(pgk_ctx* c, int32_t which, int32_t iters, double* ms
         }
     };
     if ((s = launch_zero_group(c, 0)) || (s = one())) return s;    // warm-up launch
+    if (which == 0 && (s = launch_pack(c, true))) return s;        // it may have pruned: time the regular body
     PGK_CUDA(c, cudaEventRecord(e0, c->st));
     for (int k = 0; k < iters; ++k)
         if ((s = one())) return s;
@@ -1212,17 +1214,17 @@ static pgk_status md_step_body(pgk_ctx* c, int kind, int64_t step, const pgk_mdp
         // the standard-Ewald heat-flux option evaluates the reciprocal term of
         // the last short step of a heat-flux step by ewaldkp_hf
         c->hf_ewk_now = hfs && last && c->hf_kspace == PGK_HF_KSPACE_EWK;
-        RUN(launch_kick_drift(c, (is == 1 ? KD_LONG : 0) | kshort | KD_DRIFT | (rattle ? KD_SAVE : 0)));
+        RUN(launch_kick_drift(c, (is == 1 ? KD_LONG | KD_ZERO : 0) | kshort | KD_DRIFT | (rattle ? KD_SAVE : 0)));
         // the box update also refreshes the Ewald k cutoff for the long group's SPME
         if (mtk) RUN(launch_box_update(c, kind, *md, last));
         if (rattle) RUN(launch_rattle_pos(c, md->eps_rattle, dts, mtk));
         if (!c->short_empty) RUN(force_group(c, PGK_MTS_SHORT, ene || vir, vir, tens));
         if (last) {
-            RUN(force_group(c, PGK_MTS_LONG, ene || vir, vir, tens));
+            RUN(force_group(c, PGK_MTS_LONG, ene || vir, vir, tens, true));
             if (hfa) RUN(launch_hf_atm(c));
         }
         c->hf_ewk_now = false;
-        RUN(launch_kick_drift(c, kshort | KD_SHORT_FIRST | (last ? KD_LONG : 0)));
+        RUN(launch_kick_drift(c, kshort | KD_SHORT_FIRST | KD_JOIN | (last ? KD_LONG : 0)));
         if (rattle) RUN(launch_rattle_vel(c, md->eps_rattle));
     }
     if (kind == 1) RUN(launch_kinetic_end(c, 1, chain_kind, *md));      // kinetic sums + nhcint
@@ -1337,7 +1339,7 @@ pgk_status pgk_calheatf(pgk_ctx* c, double* hf) {
     if (!c->hf_set || c->hfp.nhfregion < 1) return pgk_fail(c, PGK_E_INVALID, "no heat-flux regions set");
     pgk_status s;
     if (!c->list_valid && (s = launch_mklist(c))) return s;
-    if ((s = launch_pack(c)) || (s = launch_hf_atm(c)) || (s = launch_heatf(c, c->hf_rec, false))) return s;
+    if ((s = launch_pack(c, false)) || (s = launch_hf_atm(c)) || (s = launch_heatf(c, c->hf_rec, false))) return s;
     PGK_CUDA(c, cudaMemcpyAsync(hf, c->hf_rec, sizeof(double) * c->hfp.nhfregion * PGK_HF_NCOL,
                                 cudaMemcpyDeviceToHost, c->st));
     PGK_CUDA(c, cudaStreamSynchronize(c->st));

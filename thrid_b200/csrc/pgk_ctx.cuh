@@ -292,6 +292,23 @@ cudaError_t smem_limit(const void* kernel, size_t bytes);
 template <typename K>
 inline cudaError_t smem_limit(K* kernel, size_t bytes) { return smem_limit((const void*)kernel, bytes); }
 
+// launch with the programmatic-stream-serialization attribute: only for
+// kernels that call pdl_enter() first, after a kernel of the same stream
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // error helpers
 pgk_status pgk_fail(pgk_ctx* c, pgk_status s, const std::string& msg);
 #define PGK_CUDA(ctx, call)                                                               \
@@ -308,7 +325,8 @@ pgk_status launch_mklist(pgk_ctx* c);
 pgk_status export_nblist(pgk_ctx* c, int32_t* nb_index, int32_t* nb_list, int64_t cap, int64_t* nl);
 
 // ---- launchers (k_nonbond.cu) ----
-pgk_status launch_pack(pgk_ctx* c);
+// pair: a pair evaluation follows (the pack then decides whether it prunes)
+pgk_status launch_pack(pgk_ctx* c, bool pair);
 #define PM_FORCE 0
 #define PM_ENE 1
 #define PM_TENS 2
@@ -374,6 +392,11 @@ pgk_status launch_zero_group(pgk_ctx* c, int group);
 #define KD_DRIFT 4
 #define KD_SAVE 8
 #define KD_SHORT_FIRST 16
+// KD_ZERO clears the long group's force and energy accumulators behind the
+// long kick that reads them last (the next evaluation then skips its clearing);
+// KD_JOIN: the stream has just joined the other two (no dependent launch)
+#define KD_ZERO 32
+#define KD_JOIN 64
 pgk_status launch_kick_drift(pgk_ctx* c, int flags);
 pgk_status launch_chain_coeffs(pgk_ctx* c, int chain_kind, int coef_kind, const pgk_mdparams& md);
 pgk_status launch_rattle_pos(pgk_ctx* c, double eps, double dt, bool use_rvinv);
