@@ -197,97 +197,125 @@ struct ChainArgs {
     int degfree;
     int dbl;
     int kind;          // 1 nhcint, 2 nhcpisoint, 3 nhcpanisoint
+    // formed on the host, so that the serial update holds no division
+    double iq[8], ivm, idf;            // 1/qmass, 1/vmass, 1/degfree
+    double w2[8];                      // yscoeff dt / next / 2
 };
+static ChainArgs chain_args(const pgk_ctx* c, int kind, const pgk_mdparams& md) {
+    ChainArgs a{};
+    a.md = md;
+    a.degfree = c->degfree;
+    a.dbl = c->mixed() ? 0 : 1;
+    a.kind = kind;
+    for (int k = 0; k < 8; ++k) {
+        a.iq[k] = 1.0 / md.qmass[k];
+        a.w2[k] = md.yscoeff[k] * md.dt_long_cal / (double)md.next / 2.0;
+    }
+    a.ivm = 1.0 / md.vmass;
+    a.idf = 1.0 / (double)c->degfree;
+    return a;
+}
+
+// exp of the small arguments of a chain step (rate times a part of the time
+// step): Taylor series to x^9 below 1/16 (next term < 3e-19), summed pairwise
+// (five dependent operations; the update is a serial chain of a dozen of them)
+__device__ __forceinline__ double exp_step(double x) {
+    if (!(fabs(x) < 0.0625)) return exp(x);
+    const double x2 = x * x, x4 = x2 * x2;
+    const double a = fma(x2, fma(x, 1.0 / 6.0, 0.5), 1.0 + x);
+    const double b = fma(x2, fma(x, 1.0 / 5040.0, 1.0 / 720.0), fma(x, 1.0 / 120.0, 1.0 / 24.0));
+    return fma(x4, fma(x4, fma(x, 1.0 / 362880.0, 1.0 / 40320.0), b), a);
+}
 
 // The chain length M is a template parameter (mchain is checked to be 2..8
 // before any launch), so the loops over the chain unroll and the chain's
 // variables stay in registers through the serial update.
 template <int M>
-__device__ __forceinline__ void chain_tail(ChainDev& c, const pgk_mdparams& md, double* glogs, double w4,
+__device__ __forceinline__ void chain_tail(ChainDev& c, const ChainArgs& ca, double* glogs, double w4,
                                            double w8, double gkt, bool down) {
-    const double* q = md.qmass;
+    const double* q = ca.md.qmass;
+    const double* iq = ca.iq;
     if (down) {
-        glogs[M - 1] = (q[M - 2] * c.vlogs[M - 2] * c.vlogs[M - 2] - gkt) / q[M - 1];
+        glogs[M - 1] = (q[M - 2] * c.vlogs[M - 2] * c.vlogs[M - 2] - gkt) * iq[M - 1];
         c.vlogs[M - 1] = c.vlogs[M - 1] + glogs[M - 1] * w4;
 #pragma unroll
         for (int i = M - 2; i >= 1; --i) {
-            glogs[i] = (q[i - 1] * c.vlogs[i - 1] * c.vlogs[i - 1] - gkt) / q[i];
-            double e8 = exp(-1.0 * w8 * c.vlogs[i + 1]);
+            glogs[i] = (q[i - 1] * c.vlogs[i - 1] * c.vlogs[i - 1] - gkt) * iq[i];
+            double e8 = exp_step(-w8 * c.vlogs[i + 1]);
             c.vlogs[i] = c.vlogs[i] * e8 * e8 + w4 * glogs[i] * e8;
         }
     } else {
 #pragma unroll
         for (int i = 1; i <= M - 2; ++i) {
-            glogs[i] = (q[i - 1] * c.vlogs[i - 1] * c.vlogs[i - 1] - gkt) / q[i];
-            double e8 = exp(-1.0 * w8 * c.vlogs[i + 1]);
+            glogs[i] = (q[i - 1] * c.vlogs[i - 1] * c.vlogs[i - 1] - gkt) * iq[i];
+            double e8 = exp_step(-w8 * c.vlogs[i + 1]);
             c.vlogs[i] = c.vlogs[i] * e8 * e8 + w4 * glogs[i] * e8;
         }
-        glogs[M - 1] = (q[M - 2] * c.vlogs[M - 2] * c.vlogs[M - 2] - gkt) / q[M - 1];
+        glogs[M - 1] = (q[M - 2] * c.vlogs[M - 2] * c.vlogs[M - 2] - gkt) * iq[M - 1];
         c.vlogs[M - 1] = c.vlogs[M - 1] + glogs[M - 1] * w4;
     }
 }
 
 template <int M>
-__device__ void chain_run_m(ChainDev* __restrict__ chain, const long long* __restrict__ acc, const ChainArgs& a) {
+__device__ void chain_run_m(ChainDev* chain, const long long* acc, const ChainArgs& a) {
     ChainDev c = *chain;
     const pgk_mdparams& md = a.md;
-    double dt = md.dt_long_cal;
     double kint = acc_get(acc, A_KE, a.dbl != 0);
     double glogs[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     double gkt = md.text;
     if (a.kind == 1) {   // nhcint.F90:8-140
         double gnkt = md.text * (double)a.degfree;
-        glogs[0] = (kint - gnkt) / md.qmass[0];
+        glogs[0] = (kint - gnkt) * a.iq[0];
         for (int inc = 0; inc < md.next; ++inc)
             for (int iy = 0; iy < md.nyosh; ++iy) {
-                double w2 = md.yscoeff[iy] * dt / (double)md.next / 2.0, w4 = w2 / 2.0, w8 = w4 / 2.0;
-                chain_tail<M>(c, md, glogs, w4, w8, gkt, true);
-                double e8 = exp(-1.0 * w8 * c.vlogs[1]);
+                const double w2 = a.w2[iy], w4 = w2 / 2.0, w8 = w4 / 2.0;
+                chain_tail<M>(c, a, glogs, w4, w8, gkt, true);
+                double e8 = exp_step(-w8 * c.vlogs[1]);
                 c.vlogs[0] = c.vlogs[0] * e8 * e8 + w4 * glogs[0] * e8;
 #pragma unroll
                 for (int i = 0; i < M; ++i) c.xlogs[i] = c.xlogs[i] + c.vlogs[i] * w2;
                 c.vlogs[0] = c.vlogs[0] * e8 * e8 + w4 * glogs[0] * e8;
-                chain_tail<M>(c, md, glogs, w4, w8, gkt, false);
+                chain_tail<M>(c, a, glogs, w4, w8, gkt, false);
             }
     } else if (a.kind == 2) {   // nhcpisoint.F90:6-162
         double gn1kt = md.text * (double)(a.degfree + 1);
-        double dnf = 3.0 / (double)a.degfree;
+        const double dnf = 3.0 * a.idf;
         double vol = exp(3.0 * c.xlogv);
-        glogs[0] = (kint + md.vmass * c.vlogv * c.vlogv - gn1kt) / md.qmass[0];
-        double glogv = (dnf * kint + 3.0 * vol * (c.pint - md.pext)) / md.vmass;
+        glogs[0] = (kint + md.vmass * c.vlogv * c.vlogv - gn1kt) * a.iq[0];
+        double glogv = (dnf * kint + 3.0 * vol * (c.pint - md.pext)) * a.ivm;
         for (int inc = 0; inc < md.next; ++inc)
             for (int iy = 0; iy < md.nyosh; ++iy) {
-                double w2 = md.yscoeff[iy] * dt / (double)md.next / 2.0, w4 = w2 / 2.0, w8 = w4 / 2.0;
-                chain_tail<M>(c, md, glogs, w4, w8, gkt, true);
-                double e8 = exp(-1.0 * w8 * c.vlogs[1]);
+                const double w2 = a.w2[iy], w4 = w2 / 2.0, w8 = w4 / 2.0;
+                chain_tail<M>(c, a, glogs, w4, w8, gkt, true);
+                double e8 = exp_step(-w8 * c.vlogs[1]);
                 c.vlogs[0] = c.vlogs[0] * e8 * e8 + w4 * glogs[0] * e8;
-                e8 = exp(-1.0 * w8 * c.vlogs[0]);
+                e8 = exp_step(-w8 * c.vlogs[0]);
                 c.vlogv = c.vlogv * e8 * e8 + w4 * glogv * e8;
 #pragma unroll
                 for (int i = 0; i < M; ++i) c.xlogs[i] = c.xlogs[i] + c.vlogs[i] * w2;
                 c.vlogv = c.vlogv * e8 * e8 + w4 * glogv * e8;
-                glogs[0] = (kint + md.vmass * c.vlogv * c.vlogv - gn1kt) / md.qmass[0];
-                e8 = exp(-1.0 * w8 * c.vlogs[1]);
+                glogs[0] = (kint + md.vmass * c.vlogv * c.vlogv - gn1kt) * a.iq[0];
+                e8 = exp_step(-w8 * c.vlogs[1]);
                 c.vlogs[0] = c.vlogs[0] * e8 * e8 + w4 * glogs[0] * e8;
-                chain_tail<M>(c, md, glogs, w4, w8, gkt, false);
+                chain_tail<M>(c, a, glogs, w4, w8, gkt, false);
             }
     } else {   // nhcpanisoint.F90:8-189
         int dir = md.pcont_axis == PGK_PCONT_ANISO ? 0 : md.pcont_axis - 1;
         double gndfkt = md.text * (double)(a.degfree + (dir == 0 ? 3 : 1));
-        double dnf = 1.0 / (double)a.degfree;
+        const double dnf = a.idf;
         double vol = c.xboxh[0] * c.xboxh[1] * c.xboxh[2];
         double pv[3] = {c.pintt[0], c.pintt[4], c.pintt[8]};
         double vb2 = c.vboxg[0] * c.vboxg[0] + c.vboxg[1] * c.vboxg[1] + c.vboxg[2] * c.vboxg[2];
-        glogs[0] = (kint + md.vmass * vb2 - gndfkt) / md.qmass[0];
+        glogs[0] = (kint + md.vmass * vb2 - gndfkt) * a.iq[0];
         double gb[3];
-        for (int d = 0; d < 3; ++d) gb[d] = (dnf * kint + vol * (pv[d] - md.pext)) / md.vmass;
+        for (int d = 0; d < 3; ++d) gb[d] = (dnf * kint + vol * (pv[d] - md.pext)) * a.ivm;
         for (int inc = 0; inc < md.next; ++inc)
             for (int iy = 0; iy < md.nyosh; ++iy) {
-                double w2 = md.yscoeff[iy] * dt / (double)md.next / 2.0, w4 = w2 / 2.0, w8 = w4 / 2.0;
-                chain_tail<M>(c, md, glogs, w4, w8, gkt, true);
-                double e8 = exp(-1.0 * w8 * c.vlogs[1]);
+                const double w2 = a.w2[iy], w4 = w2 / 2.0, w8 = w4 / 2.0;
+                chain_tail<M>(c, a, glogs, w4, w8, gkt, true);
+                double e8 = exp_step(-w8 * c.vlogs[1]);
                 c.vlogs[0] = c.vlogs[0] * e8 * e8 + w4 * glogs[0] * e8;
-                e8 = exp(-1.0 * w8 * c.vlogs[0]);
+                e8 = exp_step(-w8 * c.vlogs[0]);
                 for (int d = 0; d < 3; ++d)
                     if (dir == 0 || d == dir - 1) c.vboxg[d] = c.vboxg[d] * e8 * e8 + w4 * gb[d] * e8;
 #pragma unroll
@@ -295,16 +323,16 @@ __device__ void chain_run_m(ChainDev* __restrict__ chain, const long long* __res
                 for (int d = 0; d < 3; ++d)
                     if (dir == 0 || d == dir - 1) c.vboxg[d] = c.vboxg[d] * e8 * e8 + w4 * gb[d] * e8;
                 vb2 = c.vboxg[0] * c.vboxg[0] + c.vboxg[1] * c.vboxg[1] + c.vboxg[2] * c.vboxg[2];
-                glogs[0] = (kint + md.vmass * vb2 - gndfkt) / md.qmass[0];
-                e8 = exp(-1.0 * w8 * c.vlogs[1]);
+                glogs[0] = (kint + md.vmass * vb2 - gndfkt) * a.iq[0];
+                e8 = exp_step(-w8 * c.vlogs[1]);
                 c.vlogs[0] = c.vlogs[0] * e8 * e8 + w4 * glogs[0] * e8;
-                chain_tail<M>(c, md, glogs, w4, w8, gkt, false);
+                chain_tail<M>(c, a, glogs, w4, w8, gkt, false);
             }
     }
     *chain = c;
 }
 
-__device__ void chain_run(ChainDev* __restrict__ chain, const long long* __restrict__ acc, const ChainArgs& a) {
+__device__ void chain_run(ChainDev* chain, const long long* acc, const ChainArgs& a) {
     switch (a.md.mchain) {
         case 2: chain_run_m<2>(chain, acc, a); break;
         case 3: chain_run_m<3>(chain, acc, a); break;
@@ -318,79 +346,59 @@ __device__ void chain_run(ChainDev* __restrict__ chain, const long long* __restr
 
 // kick / drift coefficients of the step (moldyn_*.F90 at istep_short == 1)
 // kind: 0 NVE, 1 NHC, 2 MTK
-struct CoefArgs { pgk_mdparams md; int degfree; int kind; };
+struct CoefArgs { pgk_mdparams md; int degfree; int kind; double idf; };   // idf: 1/degfree
 
-__device__ void coeffs_run(DynState* __restrict__ dyn, const ChainDev* __restrict__ chain, const CoefArgs& a) {
+// lanes 0..2 of a warp take one axis each
+__device__ void coeffs_run(DynState* __restrict__ dyn, const ChainDev& c, const CoefArgs& a, int d) {
+    if (d > 2) return;
     const pgk_mdparams& md = a.md;
     const double dtl = md.dt_long_cal, dts = md.dt_long_cal / (double)md.nstep_short;
     const double e2 = 1.0 / 6.0, e4 = e2 / 20.0, e6 = e4 / 42.0, e8 = e6 / 72.0;
-    const ChainDev& c = *chain;
-    dyn->ks_b = 0.5 * dts;
-    for (int d = 0; d < 3; ++d) { dyn->dr_a[d] = 1.0; dyn->dr_b[d] = dts; dyn->rvinv[d] = 1.0; }
-    if (a.kind == 0) {
-        for (int d = 0; d < 3; ++d) { dyn->kl_s[d] = 1.0; dyn->kl_b[d] = 0.5 * dtl; }
-        return;
-    }
-    bool aniso = a.kind == 2 && md.pcont_axis != PGK_PCONT_ISO;
-    if (!aniso) {
-        double vext = c.vlogs[0];
-        if (a.kind == 2) vext = c.vlogs[0] + (1.0 + 3.0 / (double)a.degfree) * c.vlogv;
-        double ec4 = exp(-0.25 * dtl * vext);
-        double a2 = (0.25 * dtl * vext) * (0.25 * dtl * vext);
-        double poly = 1.0 + a2 * (e2 + a2 * (e4 + a2 * (e6 + a2 * e8)));
-        double cf = ec4 * poly;
-        for (int d = 0; d < 3; ++d) { dyn->kl_s[d] = ec4 * ec4; dyn->kl_b[d] = cf * 0.5 * dtl; }
-    } else {
-        int dir = md.pcont_axis == PGK_PCONT_ANISO ? 0 : md.pcont_axis - 1;
-        double vx[3] = {c.vlogs[0], c.vlogs[0], c.vlogs[0]};
-        if (dir == 0) {
-            double tr = c.vboxg[0] + c.vboxg[1] + c.vboxg[2];
-            for (int d = 0; d < 3; ++d) vx[d] = c.vlogs[0] + c.vboxg[d] + 1.0 / (double)a.degfree * tr;
+    auto poly = [&](double a2) { return 1.0 + a2 * (e2 + a2 * (e4 + a2 * (e6 + a2 * e8))); };
+    if (d == 0) dyn->ks_b = 0.5 * dts;
+    double dra = 1.0, drb = dts, rvi = 1.0, kls = 1.0, klb = 0.5 * dtl;
+    if (a.kind != 0) {
+        const bool aniso = a.kind == 2 && md.pcont_axis != PGK_PCONT_ISO;
+        double vx = c.vlogs[0];
+        if (!aniso) {
+            if (a.kind == 2) vx = c.vlogs[0] + (1.0 + 3.0 * a.idf) * c.vlogv;
         } else {
-            vx[dir - 1] = vx[dir - 1] + c.vboxg[dir - 1] + 1.0 / (double)a.degfree * c.vboxg[dir - 1];
+            const int dir = md.pcont_axis == PGK_PCONT_ANISO ? 0 : md.pcont_axis - 1;
+            if (dir == 0) vx = c.vlogs[0] + c.vboxg[d] + a.idf * (c.vboxg[0] + c.vboxg[1] + c.vboxg[2]);
+            else if (d == dir - 1) vx = vx + c.vboxg[d] + a.idf * c.vboxg[d];
         }
-        for (int d = 0; d < 3; ++d) {
-            double ec4 = exp(-0.25 * dtl * vx[d]);
-            double a2 = (0.25 * dtl * vx[d]) * (0.25 * dtl * vx[d]);
-            double poly = 1.0 + a2 * (e2 + a2 * (e4 + a2 * (e6 + a2 * e8)));
-            dyn->kl_s[d] = ec4 * ec4;
-            dyn->kl_b[d] = ec4 * poly * 0.5 * dtl;
-        }
+        const double u = 0.25 * dtl * vx;
+        const double ec4 = exp_step(-u);
+        kls = ec4 * ec4;
+        klb = ec4 * poly(u * u) * 0.5 * dtl;
     }
     if (a.kind == 2) {
-        if (!aniso) {
-            double aa = exp(0.5 * dts * c.vlogv), aa2 = aa * aa;
-            double a2 = (0.5 * dts * c.vlogv) * (0.5 * dts * c.vlogv);
-            double poly = 1.0 + a2 * (e2 + a2 * (e4 + a2 * (e6 + a2 * e8)));
-            for (int d = 0; d < 3; ++d) {
-                dyn->dr_a[d] = aa2;
-                dyn->dr_b[d] = aa * poly * dts;
-                dyn->rvinv[d] = 1.0 / (aa * poly);
-            }
-        } else {
-            for (int d = 0; d < 3; ++d) {
-                double aa = exp(0.5 * dts * c.vboxg[d]);
-                double a2 = (0.5 * dts * c.vboxg[d]) * (0.5 * dts * c.vboxg[d]);
-                double poly = 1.0 + a2 * (e2 + a2 * (e4 + a2 * (e6 + a2 * e8)));
-                dyn->dr_a[d] = aa * aa;
-                dyn->dr_b[d] = aa * poly * dts;
-                dyn->rvinv[d] = 1.0 / (aa * poly);
-            }
-        }
+        const double vr = md.pcont_axis == PGK_PCONT_ISO ? c.vlogv : c.vboxg[d];
+        const double u = 0.5 * dts * vr;
+        const double aa = exp_step(u), ap = aa * poly(u * u);
+        dra = aa * aa;
+        drb = ap * dts;
+        rvi = 1.0 / ap;
     }
+    dyn->kl_s[d] = kls; dyn->kl_b[d] = klb;
+    dyn->dr_a[d] = dra; dyn->dr_b[d] = drb; dyn->rvinv[d] = rvi;
 }
 
 __global__ void k_coeffs(DynState* __restrict__ dyn, const ChainDev* __restrict__ chain, CoefArgs a) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) coeffs_run(dyn, chain, a);
+    if (blockIdx.x == 0) coeffs_run(dyn, *chain, a, threadIdx.x);
 }
 
 // chain update followed by the step's coefficients (start of an NHC / MTK step)
-__global__ void k_chain_coeffs(ChainDev* __restrict__ chain, const long long* __restrict__ acc, ChainArgs ca,
+__global__ void k_chain_coeffs(ChainDev* chain, const long long* acc, ChainArgs ca,
                                DynState* __restrict__ dyn, CoefArgs cf) {
     pdl_enter();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    chain_run(chain, acc, ca);
-    coeffs_run(dyn, chain, cf);
+    __shared__ ChainDev sc;                // the updated chain, for the other lanes
+    if (threadIdx.x == 0) {
+        chain_run(chain, acc, ca);
+        sc = *chain;
+    }
+    __syncwarp();
+    coeffs_run(dyn, sc, cf, threadIdx.x);
 }
 
 // erf_corr_cutoff.F90:28-62 (the reference's min-ish rule kept)
@@ -434,44 +442,46 @@ __global__ void k_box(DynState* __restrict__ dyn, ChainDev* __restrict__ chain, 
 // sums and both groups' virials (+ self and net-charge terms)
 struct PressArgs { double pot_ewc, netchrgsq, alpha; int ifspme, ifnetqcorrp, dbl; };
 
-__device__ void press_run(const long long* __restrict__ acc, const DynState* __restrict__ dyn, ChainDev* chain,
-                          const PressArgs& a) {
+// lanes 0..8 of a warp take one tensor component each, lane 9 the scalar
+__device__ void press_run(const long long* acc, const DynState* dyn, ChainDev* chain,
+                          const PressArgs& a, int lane) {
+    if (lane > 9) return;
     const long long* A = acc;              // kinetic sums live in group 0
     const bool dbl = a.dbl != 0;
-    double K = acc_get(A, A_KE, dbl);
-    double vol = dyn->box[0] * dyn->box[1] * dyn->box[2];
-    double pi = 3.14159265358979323846;
-    double a1 = -pi / (a.alpha * a.alpha * vol);
-    double ewnq = a.ifspme ? 0.5 * a1 * a.netchrgsq : 0.0;
-    double ewc = a.ifspme ? a.pot_ewc : 0.0;
-    double W = ewc + ewnq, Wt[9];
-    for (int k = 0; k < 9; ++k) Wt[k] = 0.0;
+    const double vol = dyn->box[0] * dyn->box[1] * dyn->box[2];
+    const double pi = 3.14159265358979323846;
+    const double a1 = -pi / (a.alpha * a.alpha * vol);
+    const double b3 = (1.0 / dyn->box[0]) * (1.0 / dyn->box[1]) * (1.0 / dyn->box[2]);
+    if (lane == 9) {
+        const double ewnq = a.ifspme ? 0.5 * a1 * a.netchrgsq : 0.0;
+        const double ewc = a.ifspme ? a.pot_ewc : 0.0;
+        double W = ewc + ewnq;
+        for (int g = 0; g < 2; ++g) {
+            const long long* G = acc + (size_t)g * NACC;
+            W += acc_get(G, A_VC, dbl) + acc_get(G, A_VLJ, dbl) + acc_get(G, A_VB, dbl) + acc_get(G, A_VA, dbl) + acc_get(G, A_VT, dbl) + acc_get(G, A_V14, dbl) +
+                 acc_get(G, A_VMOR, dbl);   // calpress.F90:146-151 (pot_viri_mor)
+        }
+        if (a.ifspme) W += a.ifnetqcorrp ? -0.5 * a1 * a.netchrgsq : a1 * a.netchrgsq;   // calforce.F90:1018-1050 (long group)
+        chain->pint = 1.0 / 3.0 * b3 * (acc_get(A, A_KE, dbl) + W);
+        return;
+    }
+    const int k = lane;
+    // coulomb / LJ tensors are stored as their lower triangle
+    const int r = k % 3, cl = k / 3;
+    const int ks = r >= cl ? k : cl + 3 * r;
+    double Wt = 0.0;
     for (int g = 0; g < 2; ++g) {
         const long long* G = acc + (size_t)g * NACC;
-        W += acc_get(G, A_VC, dbl) + acc_get(G, A_VLJ, dbl) + acc_get(G, A_VB, dbl) + acc_get(G, A_VA, dbl) + acc_get(G, A_VT, dbl) + acc_get(G, A_V14, dbl) +
-             acc_get(G, A_VMOR, dbl);   // calpress.F90:146-151 (pot_viri_mor)
-        for (int k = 0; k < 9; ++k) {
-            // coulomb / LJ tensors are stored as their lower triangle
-            int r = k % 3, cl = k / 3;
-            int ks = r >= cl ? k : cl + 3 * r;
-            Wt[k] += acc_get(G, A_VTC + ks, dbl) + acc_get(G, A_VTLJ + ks, dbl) + acc_get(G, A_VTB + k, dbl) + acc_get(G, A_VTA + k, dbl) +
-                     acc_get(G, A_VTT + k, dbl) + acc_get(G, A_VT14 + k, dbl) + acc_get(G, A_VTMOR + k, dbl);
-        }
+        Wt += acc_get(G, A_VTC + ks, dbl) + acc_get(G, A_VTLJ + ks, dbl) + acc_get(G, A_VTB + k, dbl) + acc_get(G, A_VTA + k, dbl) +
+              acc_get(G, A_VTT + k, dbl) + acc_get(G, A_VT14 + k, dbl) + acc_get(G, A_VTMOR + k, dbl);
     }
-    if (a.ifspme && !a.ifnetqcorrp) {      // calforce.F90:1018-1050 (long group)
-        W += a1 * a.netchrgsq;
-        for (int d = 0; d < 3; ++d) Wt[4 * d] += 0.5 * a1 * a.netchrgsq;
-    } else if (a.ifspme) {
-        W -= 0.5 * a1 * a.netchrgsq;
-    }
-    double b3 = (1.0 / dyn->box[0]) * (1.0 / dyn->box[1]) * (1.0 / dyn->box[2]);
-    chain->pint = 1.0 / 3.0 * b3 * (K + W);
-    for (int k = 0; k < 9; ++k) chain->pintt[k] = 1.0 * b3 * (acc_get(A, A_KET + k, dbl) + Wt[k]);
+    if (a.ifspme && !a.ifnetqcorrp && r == cl) Wt += 0.5 * a1 * a.netchrgsq;
+    chain->pintt[k] = 1.0 * b3 * (acc_get(A, A_KET + k, dbl) + Wt);
 }
 
 __global__ void k_press(const long long* __restrict__ acc, const DynState* __restrict__ dyn, ChainDev* chain,
                         PressArgs a) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) press_run(acc, dyn, chain, a);
+    if (blockIdx.x == 0) press_run(acc, dyn, chain, a, threadIdx.x);
 }
 
 // Kinetic sums (calkin: sum m v^2 and the tensor sum m v_a v_b) by a
@@ -561,11 +571,14 @@ __global__ void __launch_bounds__(256) k_kinetic_end(const double* __restrict__ 
         acc[idx[k]] = dbl ? __double_as_longlong(sd) : si;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        *done = 0u;
-        if (MODE == 2) press_run(acc, dyn, chain, pa);
-        if (MODE >= 1) chain_run(chain, acc, ca);
+    if (wp != 0) return;
+    if (lane == 0) *done = 0u;
+    if (MODE == 2) {
+        press_run(acc, dyn, chain, pa, lane);
+        __threadfence_block();             // pint, pintt for lane 0
     }
+    __syncwarp();
+    if (MODE >= 1 && lane == 0) chain_run(chain, acc, ca);
 }
 
 template <bool MIXED>
@@ -1068,11 +1081,7 @@ pgk_status launch_kinetic_end(pgk_ctx* c, int mode, int chain_kind, const pgk_md
     pa.ifspme = c->prm.ifspme;
     pa.ifnetqcorrp = c->prm.ifnetqcorrp;
     pa.dbl = c->mixed() ? 0 : 1;
-    ChainArgs ca;
-    ca.md = md;
-    ca.degfree = c->degfree;
-    ca.dbl = c->mixed() ? 0 : 1;
-    ca.kind = chain_kind;
+    const ChainArgs ca = chain_args(c, chain_kind, md);
     int blocks = std::min(c->nsm * 2, (c->natom + 255) / 256);
     if (blocks < 1) blocks = 1;
     if (mode == 2)
@@ -1087,15 +1096,8 @@ pgk_status launch_kinetic_end(pgk_ctx* c, int mode, int chain_kind, const pgk_md
 }
 
 pgk_status launch_chain_coeffs(pgk_ctx* c, int chain_kind, int coef_kind, const pgk_mdparams& md) {
-    ChainArgs ca;
-    ca.md = md;
-    ca.degfree = c->degfree;
-    ca.dbl = c->mixed() ? 0 : 1;
-    ca.kind = chain_kind;
-    CoefArgs cf;
-    cf.md = md;
-    cf.degfree = c->degfree;
-    cf.kind = coef_kind;
+    const ChainArgs ca = chain_args(c, chain_kind, md);
+    const CoefArgs cf{md, c->degfree, coef_kind, 1.0 / (double)c->degfree};
     launch_pdl(k_chain_coeffs, 1, 32, 0, c->st, c->chain, c->acc, ca, c->dyn, cf);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
@@ -1103,10 +1105,7 @@ pgk_status launch_chain_coeffs(pgk_ctx* c, int chain_kind, int coef_kind, const 
 }
 
 pgk_status launch_coeffs(pgk_ctx* c, int kind, const pgk_mdparams& md, int) {
-    CoefArgs a;
-    a.md = md;
-    a.degfree = c->degfree;
-    a.kind = kind;
+    const CoefArgs a{md, c->degfree, kind, 1.0 / (double)c->degfree};
     k_coeffs<<<1, 32, 0, c->st>>>(c->dyn, c->chain, a);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
