@@ -15,12 +15,9 @@
 // (category-major).  They are written for the last heat-flux evaluation of a
 // call; the records come from region sums formed term by term (k_flux_*).
 //
-// k_hf_pair walks the same 8-atom cluster rows as the pair kernel: one warp
-// per cluster, one lane per (cluster, j) entry, a loop over the cluster atoms
-// whose mask bit is set; every list pair is stored once.  The cluster atom's
-// shares collect in per-warp shared memory and are flushed once per cluster;
-// j's shares go straight to the global arrays.  Both use FP64 atomics, since
-// other warps add j shares to the same atoms.
+// k_hf_pair walks the same 8-atom cluster rows as the pair kernel, twice: lanes
+// own entries and sum the neighbour's shares, then lanes own cluster atoms and
+// sum theirs.
 // Pair arithmetic is FP32 in mixed precision and FP64 otherwise; region
 // geometry and all sums are FP64 in global memory.
 #include <algorithm>
@@ -65,150 +62,19 @@ __global__ void k_calcom(const double* __restrict__ pos, const double* __restric
     for (int d = 0; d < 3; ++d) cvel[3 * m + d] = c[d];
 }
 
-// heat-flux z and molecule tag of every sorted slot (bit 31: molecule-based)
+// heat-flux z, molecule tag (bit 31: molecule-based) and region bits of every
+// sorted slot
 __global__ void k_hf_slots(const int* __restrict__ perm, int npad, const double* __restrict__ pos, HfDev h,
-                           const DynState* __restrict__ dyn, double* __restrict__ zs, int* __restrict__ ms) {
+                           const DynState* __restrict__ dyn, double* __restrict__ zs, int* __restrict__ ms,
+                           uint4* __restrict__ bs) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= npad) return;
     int i = perm[s];
-    if (i < 0) { zs[s] = 0.0; ms[s] = 0x7fffffff; return; }
-    zs[s] = hf_z(h, pos, i, dyn->box[2]);
+    if (i < 0) { zs[s] = 0.0; ms[s] = 0x7fffffff; bs[s] = make_uint4(0u, 0u, 0u, 0u); return; }
+    const double z = hf_z(h, pos, i, dyn->box[2]);
+    zs[s] = z;
+    bs[s] = flux_bits(h, z, dyn->box[2]);
     ms[s] = h.mol_of[i] | (h.hftyp[i] == PGK_HFTYP_MOLE ? (int)0x80000000 : 0);
-}
-
-struct HfPairArgs {
-    const int* clist; const int* ccnt; int ccap; int ncl;
-    const int* typ_s; const int* perm; int ntyp;
-    const double* zs; const int* ms;
-    double rrcut, rr2, rl2, rmax2;
-};
-
-// calvirihf of one list pair: both atoms receive f_ij * fact (fact = sign(zi -
-// zj) * frag / 2 per region); the cluster atom's share goes to its shared-
-// memory accumulators wi[nreg][3], j's share to the global array (stride N).
-// (pair categories ELIN, LJIN, ELC, VDW = PGK_HF_ELIN + 0..3)
-// first: the cluster atom has the lower atom index, as the reference's i (an
-// atom exactly on a plane makes hf_frag depend on the order).
-template <typename T>
-__device__ __forceinline__ void hf_pair_regions(T* wi, double* wj, size_t N, int nreg, const HfDev& h, double zi,
-                                                double zj, bool first, double rz, double az, T fx, T fy, T fz) {
-    const double zlo = fmin(zi, zj), zhi = fmax(zi, zj);
-    for (int r = 0; r < nreg; ++r) {
-        if (zhi < h.z1[r] || zlo > h.z2[r]) continue;
-        double frag;
-        if (!hf_frag(first ? zi : zj, first ? zj : zi, h.z1[r], h.z2[r], az, frag)) continue;
-        const T fact = (T)(rz >= 0.0 ? frag * 0.5 : -frag * 0.5);
-        const T vx = fx * fact, vy = fy * fact, vz = fz * fact;
-        atomicAdd(wi + 3 * r + 0, vx);
-        atomicAdd(wi + 3 * r + 1, vy);
-        atomicAdd(wi + 3 * r + 2, vz);
-        atomicAdd(wj + (3 * r + 0) * N, (double)vx);
-        atomicAdd(wj + (3 * r + 1) * N, (double)vy);
-        atomicAdd(wj + (3 * r + 2) * N, (double)vz);
-    }
-}
-
-template <bool MIXED>
-__global__ void __launch_bounds__(128) k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64,
-                                                 HfPairArgs a, const float2* __restrict__ lj32,
-                                                 const double2* __restrict__ lj64, HfDev h,
-                                                 const DynState* __restrict__ dyn) {
-    typedef typename std::conditional<MIXED, float, double>::type T;
-    extern __shared__ __align__(16) unsigned char hf_sm[];
-    const int nreg = h.nreg;
-    const int per = 4 + 12 * nreg;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T* acc = (T*)hf_sm + (size_t)warp * 8 * per;
-    for (int q = lane; q < 8 * per; q += 32) acc[q] = (T)0;
-    const double Lz = dyn->box[2], invLz = 1.0 / Lz;
-    const double L0 = dyn->box[0], L1 = dyn->box[1];
-    const double B0 = 1.0 / L0, B1 = 1.0 / L1, B2 = 1.0 / Lz;
-    const T sx = (T)(L0 * (1.0 / 4294967296.0)), sy = (T)(L1 * (1.0 / 4294967296.0)), sz = (T)(Lz * (1.0 / 4294967296.0));
-    const T rr2 = (T)a.rr2, rl2 = (T)a.rl2, rmax2 = (T)a.rmax2;
-    const size_t N = (size_t)h.natom;
-    __syncwarp();
-    for (int cl = blockIdx.x * 4 + warp; cl < a.ncl; cl += gridDim.x * 4) {
-        const int cnt = a.ccnt[cl];
-        const int* row = a.clist + (size_t)cl * a.ccap;
-        for (int k = lane; k < cnt; k += 32) {
-            const unsigned e = (unsigned)row[k];
-            const int j = (int)(e & 0xFFFFFFu);
-            const unsigned m = e >> 24;
-            const double zj = a.zs[j];
-            const int mj = a.ms[j];
-            const int tj = a.typ_s[j];
-            const int oj = a.perm[j];
-            int4 qj = make_int4(0, 0, 0, 0);
-            double4 pj = make_double4(0, 0, 0, 0);
-            if (MIXED) qj = xq[j]; else pj = xq64[j];
-            for (int ii = 0; ii < 8; ++ii) {
-                if (!((m >> ii) & 1u)) continue;
-                const int s = 8 * cl + ii;
-                T dx, dy, dz, qq;
-                if (MIXED) {
-                    const int4 qi = xq[s];
-                    dx = (T)(qi.x - qj.x) * sx; dy = (T)(qi.y - qj.y) * sy; dz = (T)(qi.z - qj.z) * sz;
-                    qq = (T)(__int_as_float(qi.w) * __int_as_float(qj.w));
-                } else {
-                    const double4 pi = xq64[s];
-                    double vx = pi.x - pj.x, vy = pi.y - pj.y, vz = pi.z - pj.z;
-                    dx = (T)(vx - L0 * round(vx * B0));
-                    dy = (T)(vy - L1 * round(vy * B1));
-                    dz = (T)(vz - Lz * round(vz * B2));
-                    qq = (T)(pi.w * pj.w);
-                }
-                const T r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 > rmax2) continue;
-                const T rinv2 = (T)1 / r2;
-                const int mi = a.ms[s];
-                const bool same = (mi & 0x7fffffff) == (mj & 0x7fffffff);
-                const double zi = a.zs[s];
-                const double rz = zi - zj, az = fabs(rz);
-                const bool vir = !((mi < 0) && (mj < 0) && same) && az * invLz < 0.5;
-                const bool first = a.perm[s] < oj;
-                T* w = acc + ii * per;
-                const bool coul = MIXED ? (r2 <= rr2) : (sqrt((double)r2) <= a.rrcut);
-                if (coul) {                           // ewaldr_hf.F90:336-371, bare 1/r
-                    const T rinv1 = (T)1 / sqrt(r2);
-                    const T phi = qq * rinv1;
-                    const T ft = phi * rinv2;
-                    const int cat = same ? 0 : 2;
-                    atomicAdd(w + cat, (T)0.5 * phi);
-                    atomicAdd(h.pot + (PGK_HF_ELIN + cat) * N + oj, (double)((T)0.5 * phi));
-                    if (vir) hf_pair_regions<T>(w + 4 + cat * 3 * nreg, h.W + (size_t)(PGK_HF_ELIN + cat) * nreg * 3 * N + oj,
-                                                N, nreg, h, zi, zj, first, rz, az, ft * dx, ft * dy, ft * dz);
-                }
-                if (r2 <= rl2) {                      // ewaldr_hf.F90:376-470
-                    T R2, E;
-                    if (MIXED) { const float2 lp = lj32[a.typ_s[s] * a.ntyp + tj]; R2 = lp.x; E = lp.y; }
-                    else { const double2 lp = lj64[a.typ_s[s] * a.ntyp + tj]; R2 = lp.x; E = lp.y; }
-                    const T t2 = rinv2 * R2, t6 = t2 * t2 * t2, t12 = t6 * t6;
-                    const T phi = E * (t12 - (T)2 * t6);
-                    const T ft = (T)12 * E * (t12 - t6) * rinv2;
-                    const int cat = same ? 1 : 3;
-                    atomicAdd(w + cat, (T)0.5 * phi);
-                    atomicAdd(h.pot + (PGK_HF_ELIN + cat) * N + oj, (double)((T)0.5 * phi));
-                    if (vir) hf_pair_regions<T>(w + 4 + cat * 3 * nreg, h.W + (size_t)(PGK_HF_ELIN + cat) * nreg * 3 * N + oj,
-                                                N, nreg, h, zi, zj, first, rz, az, ft * dx, ft * dy, ft * dz);
-                }
-            }
-        }
-        __syncwarp();
-        for (int q = lane; q < 8 * per; q += 32) {
-            const int ii = q / per, w = q - ii * per;
-            const T v = acc[q];
-            acc[q] = (T)0;
-            const int io = a.perm[8 * cl + ii];
-            if (io < 0 || v == (T)0) continue;
-            if (w < 4) {
-                atomicAdd(h.pot + (size_t)(PGK_HF_ELIN + w) * N + io, (double)v);
-            } else {
-                const int u = w - 4, cat = u / (3 * nreg), rem = u - cat * 3 * nreg;
-                atomicAdd(h.W + ((size_t)(PGK_HF_ELIN + cat) * nreg * 3 + rem) * N + io, (double)v);
-            }
-        }
-        __syncwarp();
-    }
 }
 
 // ---- calheatf.F90, volume-based, z components --------------------------------
@@ -275,15 +141,15 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
 // by one Newton step), all region sums are FP64.
 // Bound by issue (about 60 FP32 and 12 FP64 instructions per pair) at 16 warps
 // per SM.  Measured: 43,200-atom slab, 23 regions, mixed: 0.327 ms per
-// evaluation against 4.86 ms for the per-atom arrays and 0.52 ms for summing
-// them; 8,232-atom water box, one region: 0.042 ms against 1.27 + 0.24 ms.
+// evaluation against 0.79 ms for the per-atom arrays and 0.52 ms for summing
+// them; 8,232-atom water box, one region: 0.042 ms against 0.10 + 0.24 ms.
 // Rows are cut into segments until 16 warps per SM have work (small boxes).
 struct FluxPairArgs {
     const int* rows; const int* cnt; int ccap; int ncl; int nseg;
     int pruned;                  // rows, cnt: nseg segments of ccap entries per cluster, else whole rows
     const int* typ_s; const int* perm; int ntyp;
     const double* zs; const int* ms; const void* vs; const uint4* bs;
-    double rr2, rl2, rmax2;
+    double rrcut, rr2, rl2, rmax2;
 };
 
 template <bool MIXED> struct FluxT { typedef float T; typedef float4 V; };
@@ -295,6 +161,309 @@ __device__ __forceinline__ float flux_rinv(float r2) {
     return y * fmaf(-0.5f * r2 * y, y, 1.5f);
 }
 __device__ __forceinline__ double flux_rinv(double r2) { return rsqrt(r2); }
+
+// One pair's terms of the per-atom arrays (categories Coulomb, LJ): energies
+// and half forces; false beyond both cutoffs.
+template <bool MIXED> struct HfTerm {
+    typename FluxT<MIXED>::T pc, pl, fc[3], fl[3];
+};
+struct HfBox { double L0, L1, L2, B0, B1, B2; };
+template <bool MIXED>
+__device__ __forceinline__ bool hf_term(const int4& qi, const double4& pi, const int4& qj, const double4& pj,
+                                        const FluxPairArgs& a, const HfBox& b, int lj, const float2* lj32,
+                                        const double2* lj64, HfTerm<MIXED>& o) {
+    typedef typename FluxT<MIXED>::T T;
+    T dx, dy, dz, qq;
+    if (MIXED) {
+        dx = (T)(qi.x - qj.x) * (T)(b.L0 * (1.0 / 4294967296.0));
+        dy = (T)(qi.y - qj.y) * (T)(b.L1 * (1.0 / 4294967296.0));
+        dz = (T)(qi.z - qj.z) * (T)(b.L2 * (1.0 / 4294967296.0));
+        qq = (T)(__int_as_float(qi.w) * __int_as_float(qj.w));
+    } else {
+        const double x = pi.x - pj.x, y = pi.y - pj.y, z = pi.z - pj.z;
+        dx = (T)(x - b.L0 * round(x * b.B0));
+        dy = (T)(y - b.L1 * round(y * b.B1));
+        dz = (T)(z - b.L2 * round(z * b.B2));
+        qq = (T)(pi.w * pj.w);
+    }
+    const T r2 = dx * dx + dy * dy + dz * dz;
+    if (r2 > (T)a.rmax2) return false;
+    const T rinv = flux_rinv(r2), rinv2 = rinv * rinv;
+    const bool coul = MIXED ? r2 <= (T)a.rr2 : sqrt((double)r2) <= a.rrcut;
+    const T phc = coul ? qq * rinv : (T)0;               // ewaldr_hf.F90:336-371, bare 1/r
+    T phl = (T)0, ftl = (T)0;
+    if (r2 <= (T)a.rl2) {                                // ewaldr_hf.F90:376-470
+        T R2, E;
+        if (MIXED) { const float2 lp = lj32[lj]; R2 = lp.x; E = lp.y; }
+        else { const double2 lp = lj64[lj]; R2 = lp.x; E = lp.y; }
+        const T t2 = rinv2 * R2, t6 = t2 * t2 * t2, t12 = t6 * t6;
+        phl = E * (t12 - (T)2 * t6);
+        ftl = (T)6 * E * (t12 - t6) * rinv2;
+    }
+    const T ftc = (T)0.5 * phc * rinv2;
+    o.pc = (T)0.5 * phc;
+    o.pl = (T)0.5 * phl;
+    o.fc[0] = ftc * dx; o.fc[1] = ftc * dy; o.fc[2] = ftc * dz;
+    o.fl[0] = ftl * dx; o.fl[1] = ftl * dy; o.fl[2] = ftl * dz;
+    return true;
+}
+
+// Per-atom arrays of the pair categories: both atoms of a pair receive its
+// energy shares and f_ij times the signed length of (zi, zj) inside each
+// region, which is C_i - C_j with C the z clamped to the region (see
+// k_flux_pair).  A warp takes a cluster's row (segment) twice per window of KW
+// regions that the row touches: with one entry per lane, for the shares of the
+// entries' atoms (one FP64 atomic per atom, category, region and axis instead
+// of one per pair), and with 8 cluster atoms x 4 entries, for the cluster
+// atoms', added over the four lanes and flushed once.  Pairs of the class
+// (same molecule / different) that the row has fewer of, and atoms exactly on
+// a plane, add to both atoms directly.
+// Bound by issue (the pair arithmetic is done twice) and by the entries'
+// atomics.  Measured, mixed: 43,200-atom slab, 23 regions 0.79 ms (4.86 ms with
+// one lane's atomics for every pair, into shared memory for the cluster atom
+// and global memory for the entry's); 8,232-atom water box, one region 0.103 ms
+// (1.27 ms).  Three blocks per SM without spills, or six regions a walk, were
+// no faster (call of 14 steps 7.92, 8.04 ms against 7.87).
+template <bool MIXED, int KW>
+__global__ void __launch_bounds__(128, MIXED ? 4 : 3)
+k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPairArgs a,
+          const float2* __restrict__ lj32, const double2* __restrict__ lj64, HfDev h,
+          const DynState* __restrict__ dyn) {
+    __shared__ double sz1[PGK_HF_MAX_REGIONS], sz2[PGK_HF_MAX_REGIONS];
+    __shared__ int4 sxq[4][8];
+    __shared__ double4 sx64[MIXED ? 1 : 4][8];
+    __shared__ double szi[4][8], sC[4][8][KW];
+    __shared__ uint4 sbi[4][8];
+    __shared__ int smi[4][8], sti[4][8], soi[4][8];
+    const int nreg = h.nreg;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x < nreg) { sz1[threadIdx.x] = h.z1[threadIdx.x]; sz2[threadIdx.x] = h.z2[threadIdx.x]; }
+    __syncthreads();
+    const unsigned all = nreg >= 32 ? 0xffffffffu : (1u << nreg) - 1u;
+    HfBox bx;
+    bx.L0 = dyn->box[0]; bx.L1 = dyn->box[1]; bx.L2 = dyn->box[2];
+    bx.B0 = 1.0 / bx.L0; bx.B1 = 1.0 / bx.L1; bx.B2 = 1.0 / bx.L2;
+    const size_t N = (size_t)h.natom;
+    double* const pot0 = h.pot + (size_t)PGK_HF_ELIN * N;
+    double* const W0 = h.W + (size_t)PGK_HF_ELIN * nreg * 3 * N;
+    const long long nunit = (long long)a.ncl * a.nseg;
+    for (long long u = blockIdx.x * 4 + w; u < nunit; u += gridDim.x * 4) {
+        const int cl = (int)(u / a.nseg), seg = (int)(u - (long long)cl * a.nseg);
+        const int cnt = a.cnt[a.pruned ? u : cl];
+        const int chunk = a.pruned ? cnt : ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
+        const int k_lo = a.pruned ? 0 : seg * chunk, k_hi = min(cnt, k_lo + chunk);
+        if (k_lo >= k_hi) continue;                       // warp-uniform
+        const int* __restrict__ row = a.rows + (size_t)(a.pruned ? u : cl) * a.ccap;
+        __syncwarp();
+        if (lane < 8) {
+            const int s = 8 * cl + lane;
+            if (MIXED) sxq[w][lane] = xq[s]; else sx64[MIXED ? 0 : w][lane] = xq64[s];
+            szi[w][lane] = a.zs[s];
+            sbi[w][lane] = a.bs[s];
+            smi[w][lane] = a.ms[s];
+            sti[w][lane] = a.typ_s[s] * a.ntyp;
+            soi[w][lane] = a.perm[s];
+        }
+        __syncwarp();
+        // regions that a pair of this row segment can touch; the larger class
+        unsigned todo = 0u;
+        int nsame = 0, npair = 0;
+        for (int k = k_lo + lane; k < k_hi; k += 32) {
+            const unsigned e = (unsigned)row[k];
+            const uint4 bj = a.bs[e & 0xFFFFFFu];
+            const int mj = a.ms[e & 0xFFFFFFu];
+            npair += __popc(e >> 24);
+#pragma unroll
+            for (int ii = 0; ii < 8; ++ii)
+                if ((e >> (24 + ii)) & 1u) {
+                    const uint4 bi = sbi[w][ii];
+                    todo |= ~((bi.x & bj.x) | (bi.y & bj.y));
+                    nsame += !((smi[w][ii] ^ mj) & 0x7fffffff);
+                }
+        }
+        todo = __reduce_or_sync(0xffffffffu, todo) & all;
+        const bool maj = 2 * __reduce_add_sync(0xffffffffu, nsame) > __reduce_add_sync(0xffffffffu, npair);
+        const int cc = maj ? 0 : 2;                       // PGK_HF_ELIN + cc: Coulomb, + 1: LJ
+        double* const Wc = W0 + (size_t)cc * nreg * 3 * N;
+        const size_t ljo = (size_t)nreg * 3 * N;
+        bool w0 = true;                                   // energies with the first window
+        do {
+            int rk[KW];
+            unsigned win = 0u;
+#pragma unroll
+            for (int q = 0; q < KW; ++q) {
+                rk[q] = todo ? __ffs(todo) - 1 : -1;
+                if (todo) { win |= 1u << rk[q]; todo &= todo - 1; }
+            }
+            __syncwarp();
+            if (lane < 8) {
+                const double z = szi[w][lane];
+                const uint4 b = sbi[w][lane];
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    const int r = max(rk[q], 0);
+                    sC[w][lane][q] = (b.x >> r) & 1u ? sz1[r] : ((b.y >> r) & 1u ? sz2[r] : z);
+                }
+            }
+            __syncwarp();
+            // ---- the entries' atoms: lane = entry
+            for (int k = k_lo + lane; k < k_hi; k += 32) {
+                const unsigned e = (unsigned)row[k];
+                const int j = (int)(e & 0xFFFFFFu);
+                const unsigned m = e >> 24;
+                const double zj = a.zs[j];
+                const int mj = a.ms[j], tj = a.typ_s[j], oj = a.perm[j];
+                const uint4 bj = a.bs[j];
+                int4 qj = make_int4(0, 0, 0, 0);
+                double4 pj = make_double4(0, 0, 0, 0);
+                if (MIXED) qj = xq[j]; else pj = xq64[j];
+                double Cj[KW], ac[KW][3], al[KW][3], pc = 0.0, pl = 0.0;
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    const int r = max(rk[q], 0);
+                    Cj[q] = (bj.x >> r) & 1u ? sz1[r] : ((bj.y >> r) & 1u ? sz2[r] : zj);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) { ac[q][d] = 0.0; al[q][d] = 0.0; }
+                }
+#pragma unroll 1
+                for (unsigned mm = m; mm; mm &= mm - 1) {
+                    const int ii = __ffs(mm) - 1;
+                    HfTerm<MIXED> t;
+                    if (!hf_term<MIXED>(sxq[w][ii], sx64[MIXED ? 0 : w][ii], qj, pj, a, bx, sti[w][ii] + tj, lj32, lj64, t))
+                        continue;
+                    const int mi = smi[w][ii];
+                    const bool same = !((mi ^ mj) & 0x7fffffff);
+                    const uint4 bi = sbi[w][ii];
+                    const double zi = szi[w][ii], az = fabs(zi - zj);
+                    const bool vir = !((mi < 0) && (mj < 0) && same) && az * bx.B2 < 0.5;
+                    if (same != maj || (vir && ((bi.w | bj.w) & win))) {
+                        const int oi = soi[w][ii], c0 = same ? 0 : 2;
+                        if (same != maj && w0) {
+                            double* p = pot0 + (size_t)c0 * N;
+                            atomicAdd(p + oi, (double)t.pc); atomicAdd(p + oj, (double)t.pc);
+                            atomicAdd(p + N + oi, (double)t.pl); atomicAdd(p + N + oj, (double)t.pl);
+                        }
+                        // the lower atom index first: the reference's i
+                        const double za = oi < oj ? zi : zj, zb = oi < oj ? zj : zi;
+#pragma unroll 1
+                        for (unsigned rm = vir ? win & ~((bi.x & bj.x) | (bi.y & bj.y)) : 0u; rm; rm &= rm - 1) {
+                            const int r = __ffs(rm) - 1;
+                            double frag;
+                            if (!hf_frag(za, zb, sz1[r], sz2[r], az, frag)) continue;
+                            const double D = zi - zj >= 0.0 ? frag : -frag;
+                            double* p = W0 + ((size_t)c0 * nreg + r) * 3 * N;
+#pragma unroll
+                            for (int d = 0; d < 3; ++d) {
+                                const double vc = (double)t.fc[d] * D, vl = (double)t.fl[d] * D;
+                                if (vc != 0.0) { atomicAdd(p + d * N + oi, vc); atomicAdd(p + d * N + oj, vc); }
+                                if (vl != 0.0) { atomicAdd(p + ljo + d * N + oi, vl); atomicAdd(p + ljo + d * N + oj, vl); }
+                            }
+                        }
+                        if (same == maj) { pc += (double)t.pc; pl += (double)t.pl; }
+                        continue;
+                    }
+                    pc += (double)t.pc;
+                    pl += (double)t.pl;
+                    if (!vir) continue;
+#pragma unroll
+                    for (int q = 0; q < KW; ++q) {
+                        const double D = sC[w][ii][q] - Cj[q];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            ac[q][d] = fma((double)t.fc[d], D, ac[q][d]);
+                            al[q][d] = fma((double)t.fl[d], D, al[q][d]);
+                        }
+                    }
+                }
+                if (w0) {
+                    double* p = pot0 + (size_t)cc * N + oj;
+                    if (pc != 0.0) atomicAdd(p, pc);
+                    if (pl != 0.0) atomicAdd(p + N, pl);
+                }
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    if (rk[q] < 0) continue;
+                    double* p = Wc + (size_t)rk[q] * 3 * N + oj;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        if (ac[q][d] != 0.0) atomicAdd(p + d * N, ac[q][d]);
+                        if (al[q][d] != 0.0) atomicAdd(p + ljo + d * N, al[q][d]);
+                    }
+                }
+            }
+            // ---- the cluster atoms: lane = 8 atoms x 4 entries
+            {
+                const int ii = lane & 7, sub = lane >> 3;
+                const int4 qi = sxq[w][ii];
+                const double4 pi = sx64[MIXED ? 0 : w][ii];
+                const int mi = smi[w][ii], ti = sti[w][ii];
+                const uint4 bi = sbi[w][ii];
+                const double zi = szi[w][ii];
+                double Ci[KW], ac[KW][3], al[KW][3], pc = 0.0, pl = 0.0;
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    Ci[q] = sC[w][ii][q];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) { ac[q][d] = 0.0; al[q][d] = 0.0; }
+                }
+#pragma unroll 1
+                for (int k = k_lo + sub; k < k_hi; k += 4) {
+                    const unsigned e = (unsigned)row[k];
+                    if (!((e >> (24 + ii)) & 1u)) continue;
+                    const int j = (int)(e & 0xFFFFFFu);
+                    int4 qj = make_int4(0, 0, 0, 0);
+                    double4 pj = make_double4(0, 0, 0, 0);
+                    if (MIXED) qj = xq[j]; else pj = xq64[j];
+                    HfTerm<MIXED> t;
+                    if (!hf_term<MIXED>(qi, pi, qj, pj, a, bx, ti + a.typ_s[j], lj32, lj64, t)) continue;
+                    const int mj = a.ms[j];
+                    const bool same = !((mi ^ mj) & 0x7fffffff);
+                    if (same != maj) continue;
+                    pc += (double)t.pc;
+                    pl += (double)t.pl;
+                    const double zj = a.zs[j];
+                    const uint4 bj = a.bs[j];
+                    if (((mi < 0) && (mj < 0) && same) || fabs(zi - zj) * bx.B2 >= 0.5 || ((bi.w | bj.w) & win)) continue;
+#pragma unroll
+                    for (int q = 0; q < KW; ++q) {
+                        const int r = max(rk[q], 0);
+                        const double D = Ci[q] - ((bj.x >> r) & 1u ? sz1[r] : ((bj.y >> r) & 1u ? sz2[r] : zj));
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            ac[q][d] = fma((double)t.fc[d], D, ac[q][d]);
+                            al[q][d] = fma((double)t.fl[d], D, al[q][d]);
+                        }
+                    }
+                }
+                __syncwarp();
+                const int oi = soi[w][ii];
+                auto four = [](double v) {
+                    v += __shfl_xor_sync(0xffffffffu, v, 8);
+                    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+                };
+                if (w0) {
+                    pc = four(pc);
+                    pl = four(pl);
+                    double* p = pot0 + (size_t)cc * N;
+                    if (sub == 0 && pc != 0.0) atomicAdd(p + oi, pc);
+                    if (sub == 1 && pl != 0.0) atomicAdd(p + N + oi, pl);
+                }
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    if (rk[q] < 0) continue;               // warp-uniform
+                    double* p = Wc + (size_t)rk[q] * 3 * N;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const double vc = four(ac[q][d]), vl = four(al[q][d]);
+                        if (sub == (d & 1) && vc != 0.0) atomicAdd(p + d * N + oi, vc);
+                        if (sub == 2 + (d & 1) && vl != 0.0) atomicAdd(p + ljo + d * N + oi, vl);
+                    }
+                }
+            }
+            w0 = false;
+        } while (todo);
+    }
+}
 
 template <bool MIXED, int KW>
 __global__ void __launch_bounds__(128, MIXED ? 4 : 3)
@@ -821,7 +990,32 @@ static pgk_status launch_hf_kspace(pgk_ctx* c) {
     return PGK_OK;
 }
 
-pgk_status launch_hf_atm(pgk_ctx* c) {
+static bool flux_pair_on(const pgk_ctx* c) {
+    return (c->prm.mts_vdw == PGK_MTS_LONG || c->prm.mts_vdw == PGK_MTS_SHORT) && c->ncl > 0;
+}
+// pruned: this step's pair kernel has left its rows (c->plist)
+static FluxPairArgs flux_pair_args(pgk_ctx* c, bool pruned) {
+    FluxPairArgs a;
+    a.pruned = pruned && c->prune_buffer > 0.f;
+    a.rows = a.pruned ? c->plist : c->clist; a.cnt = a.pruned ? c->pcnt : c->ccnt;
+    a.ccap = a.pruned ? c->pcap : c->ccap; a.ncl = c->ncl;
+    a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
+    a.zs = c->hf_zs; a.ms = c->hf_ms; a.vs = c->hf_vs; a.bs = c->hf_bs;
+    a.rrcut = c->prm.rrcut;
+    a.rr2 = c->prm.rrcut * c->prm.rrcut;
+    a.rl2 = c->prm.rcut * c->prm.rcut;
+    a.rmax2 = std::max(a.rr2, a.rl2);
+    // about 16 warps per SM, in row segments where the clusters alone are fewer
+    a.nseg = a.pruned ? c->pseg : std::max(1, std::min(8, c->nsm * 16 / std::max(a.ncl, 1)));
+    return a;
+}
+static int flux_pair_grid(const pgk_ctx* c, const FluxPairArgs& a) {
+    const long long units = (long long)a.ncl * a.nseg;
+    return (int)std::max(1LL, std::min((units + 3) / 4, (long long)c->nsm * 16));
+}
+
+// pruned: this step's pair kernel has left its rows
+pgk_status launch_hf_atm(pgk_ctx* c, bool pruned) {
     if (!c->hf_set || c->hfp.nhfregion < 1) return pgk_fail(c, PGK_E_INVALID, "no heat-flux regions set");
     pgk_status s;
     const int n = c->natom, nreg = c->hfp.nhfregion;
@@ -833,31 +1027,17 @@ pgk_status launch_hf_atm(pgk_ctx* c) {
     PGK_CUDA(c, cudaMemsetAsync(c->hf_pot, 0, sizeof(double) * 8 * n, c->st));
     PGK_CUDA(c, cudaMemsetAsync(c->hf_W, 0, sizeof(double) * 8 * nreg * 3 * (size_t)n, c->st));
     HfDev h = hf_dev(c);
-    const bool pair_on = c->prm.mts_vdw == PGK_MTS_LONG || c->prm.mts_vdw == PGK_MTS_SHORT;
-    if (pair_on && c->ncl > 0) {
+    if (flux_pair_on(c)) {
         if ((s = ensure_hf_slots(c))) return s;
         k_hf_slots<<<(c->npad + 255) / 256, 256, 0, c->st>>>(c->perm, c->npad, c->pos, h, c->dyn, c->hf_zs,
-                                                              c->hf_ms);
+                                                              c->hf_ms, c->hf_bs);
         PGK_LAUNCHED(c);
-        HfPairArgs a;
-        a.clist = c->clist; a.ccnt = c->ccnt; a.ccap = c->ccap; a.ncl = c->ncl;
-        a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
-        a.zs = c->hf_zs; a.ms = c->hf_ms;
-        a.rrcut = c->prm.rrcut;
-        a.rr2 = c->prm.rrcut * c->prm.rrcut;
-        a.rl2 = c->prm.rcut * c->prm.rcut;
-        a.rmax2 = std::max(a.rr2, a.rl2);
-        const int per = 4 + 12 * nreg;
-        int blocks = std::min((c->ncl + 3) / 4, c->nsm * 8);
-        if (c->mixed()) {
-            size_t sm = (size_t)4 * 8 * per * sizeof(float);
-            smem_limit(k_hf_pair<true>, sm);
-            k_hf_pair<true><<<blocks, 128, sm, c->st>>>(c->xq, nullptr, a, c->lj32, c->lj64, h, c->dyn);
-        } else {
-            size_t sm = (size_t)4 * 8 * per * sizeof(double);
-            smem_limit(k_hf_pair<false>, sm);
-            k_hf_pair<false><<<blocks, 128, sm, c->st>>>(nullptr, c->xq64, a, c->lj32, c->lj64, h, c->dyn);
-        }
+        FluxPairArgs a = flux_pair_args(c, pruned);
+        const int blocks = flux_pair_grid(c, a);
+#define PGK_HFP(M, KW) k_hf_pair<M, KW><<<blocks, 128, 0, c->st>>>(c->xq, c->xq64, a, c->lj32, c->lj64, h, c->dyn)
+        if (c->mixed()) { if (nreg == 1) PGK_HFP(true, 1); else PGK_HFP(true, 4); }
+        else { if (nreg == 1) PGK_HFP(false, 1); else PGK_HFP(false, 4); }
+#undef PGK_HFP
         PGK_LAUNCHED(c);
         PGK_CUDA(c, cudaGetLastError());
     }
@@ -867,12 +1047,8 @@ pgk_status launch_hf_atm(pgk_ctx* c) {
 
 // one region: one accumulator set; more: four a walk (most rows touch 3-4)
 template <bool MIXED>
-static void flux_pair_launch(pgk_ctx* c, FluxPairArgs& a, const FluxDev& f) {
-    // about 16 warps per SM, in row segments where the clusters alone are fewer
-    const int want = c->nsm * 16;
-    a.nseg = a.pruned ? c->pseg : std::max(1, std::min(8, want / std::max(a.ncl, 1)));
-    const long long units = (long long)a.ncl * a.nseg;
-    const int blocks = (int)std::max(1LL, std::min((units + 3) / 4, (long long)c->nsm * 16));
+static void flux_pair_launch(pgk_ctx* c, const FluxPairArgs& a, const FluxDev& f) {
+    const int blocks = flux_pair_grid(c, a);
     if (f.h.nreg == 1)
         k_flux_pair<MIXED, 1><<<blocks, 128, 0, c->st>>>(c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
     else
@@ -891,7 +1067,7 @@ pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
                                                              c->dyn, c->molecom, c->molevel);
         PGK_LAUNCHED(c);
     }
-    const bool pair_on = (c->prm.mts_vdw == PGK_MTS_LONG || c->prm.mts_vdw == PGK_MTS_SHORT) && c->ncl > 0;
+    const bool pair_on = flux_pair_on(c);
     if (pair_on && (s = ensure_hf_slots(c))) return s;
     const int* ip = pair_on ? c->iperm : nullptr;
     if (c->mixed())
@@ -902,15 +1078,7 @@ pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
                                                                 c->hf_vs, c->hf_bs);
     PGK_LAUNCHED(c);
     if (pair_on) {
-        FluxPairArgs a;
-        a.pruned = pruned && c->prune_buffer > 0.f;
-        a.rows = a.pruned ? c->plist : c->clist; a.cnt = a.pruned ? c->pcnt : c->ccnt;
-        a.ccap = a.pruned ? c->pcap : c->ccap; a.ncl = c->ncl;
-        a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
-        a.zs = c->hf_zs; a.ms = c->hf_ms; a.vs = c->hf_vs; a.bs = c->hf_bs;
-        a.rr2 = c->prm.rrcut * c->prm.rrcut;
-        a.rl2 = c->prm.rcut * c->prm.rcut;
-        a.rmax2 = std::max(a.rr2, a.rl2);
+        const FluxPairArgs a = flux_pair_args(c, pruned);
         if (c->mixed()) flux_pair_launch<true>(c, a, f);
         else flux_pair_launch<false>(c, a, f);
     }

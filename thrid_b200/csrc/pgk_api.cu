@@ -1219,12 +1219,11 @@ static pgk_status md_step_body(pgk_ctx* c, int kind, int64_t step, const pgk_mdp
         if (mtk) RUN(launch_box_update(c, kind, *md, last));
         if (rattle) RUN(launch_rattle_pos(c, md->eps_rattle, dts, mtk));
         if (!c->short_empty) RUN(force_group(c, PGK_MTS_SHORT, ene || vir, vir, tens));
-        if (last) {
-            RUN(force_group(c, PGK_MTS_LONG, ene || vir, vir, tens, true));
-            if (hfa) RUN(launch_hf_atm(c));
-        }
+        if (last) RUN(force_group(c, PGK_MTS_LONG, ene || vir, vir, tens, true));
         c->hf_ewk_now = false;
         RUN(launch_kick_drift(c, kshort | KD_SHORT_FIRST | KD_JOIN | (last ? KD_LONG : 0)));
+        // after the join: the pair kernel's pruned rows are complete
+        if (last && hfa) RUN(launch_hf_atm(c, true));
         if (rattle) RUN(launch_rattle_vel(c, md->eps_rattle));
     }
     if (kind == 1) RUN(launch_kinetic_end(c, 1, chain_kind, *md));      // kinetic sums + nhcint
@@ -1339,7 +1338,7 @@ pgk_status pgk_calheatf(pgk_ctx* c, double* hf) {
     if (!c->hf_set || c->hfp.nhfregion < 1) return pgk_fail(c, PGK_E_INVALID, "no heat-flux regions set");
     pgk_status s;
     if (!c->list_valid && (s = launch_mklist(c))) return s;
-    if ((s = launch_pack(c, false)) || (s = launch_hf_atm(c)) || (s = launch_heatf(c, c->hf_rec, false))) return s;
+    if ((s = launch_pack(c, false)) || (s = launch_hf_atm(c, false)) || (s = launch_heatf(c, c->hf_rec, false))) return s;
     PGK_CUDA(c, cudaMemcpyAsync(hf, c->hf_rec, sizeof(double) * c->hfp.nhfregion * PGK_HF_NCOL,
                                 cudaMemcpyDeviceToHost, c->st));
     PGK_CUDA(c, cudaStreamSynchronize(c->st));

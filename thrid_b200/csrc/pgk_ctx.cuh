@@ -365,7 +365,7 @@ pgk_status export_morlist(pgk_ctx* c, int32_t* nmorselist, int32_t* mor_index, i
 // ---- launchers (k_heatf.cu, heat flux + region Langevin) ----
 struct HfDev;
 pgk_status hf_setup(pgk_ctx* c, const pgk_hfparams* p);
-pgk_status launch_hf_atm(pgk_ctx* c);
+pgk_status launch_hf_atm(pgk_ctx* c, bool pruned);
 // record of the region sums at dst (device); pruned: the pruned pair rows are
 // current (the pair kernel ran at these positions)
 pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned);
