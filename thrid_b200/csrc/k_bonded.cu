@@ -1210,6 +1210,7 @@ __global__ void __launch_bounds__(FLUX_BT) k_bonded_flux(const double* __restric
                                                          const int* __restrict__ typ, int ntyp,
                                                          const double2* __restrict__ lj64, FluxTerms t, FluxDev f,
                                                          const DynState* __restrict__ dyn, unsigned* status) {
+    pdl_enter();
     extern __shared__ double fsm[];                      // [nreg][potential, virial][FLUX_BT]
     const int nreg = f.h.nreg;
     for (int q = threadIdx.x; q < 2 * nreg * FLUX_BT; q += FLUX_BT) fsm[q] = 0.0;
@@ -1315,7 +1316,7 @@ pgk_status launch_bonded_flux(pgk_ctx* c, const FluxDev& f) {
     if (nb == 0) return PGK_OK;
     const size_t sm = sizeof(double) * 2 * f.h.nreg * FLUX_BT;
     PGK_CUDA(c, smem_limit(k_bonded_flux, sm));
-    k_bonded_flux<<<nb, FLUX_BT, sm, c->st>>>(c->pos, c->chrg, c->typ, c->ntyp, c->lj64, t, f, c->dyn, c->status);
+    launch_pdl(k_bonded_flux, nb, FLUX_BT, sm, c->st, c->pos, c->chrg, c->typ, c->ntyp, c->lj64, t, f, c->dyn, c->status);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;

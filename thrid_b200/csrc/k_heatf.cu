@@ -51,6 +51,7 @@ __global__ void k_calcom(const double* __restrict__ pos, const double* __restric
                           const double* __restrict__ mass, const int* __restrict__ mol_idx,
                           const int* __restrict__ mol_list, int nmole, const DynState* __restrict__ dyn,
                           double* __restrict__ com, double* __restrict__ cvel) {
+    pdl_enter();
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nmole) return;
     const int b = mol_idx[m], e = mol_idx[m + 1];
@@ -62,19 +63,27 @@ __global__ void k_calcom(const double* __restrict__ pos, const double* __restric
     for (int d = 0; d < 3; ++d) cvel[3 * m + d] = c[d];
 }
 
-// heat-flux z, molecule tag (bit 31: molecule-based) and region bits of every
-// sorted slot
+// molecule tag of a sorted slot: molecule number, and whether the heat-flux z
+// is the molecule's (the sign bit) and lies exactly on a region's plane
+#define HF_MS_ID 0x3fffffff
+#define HF_MS_PLANE 0x40000000
+__device__ __forceinline__ int hf_tag(const HfDev& h, int i, unsigned planes) {
+    return h.mol_of[i] | (planes ? HF_MS_PLANE : 0) | (h.hftyp[i] == PGK_HFTYP_MOLE ? (int)0x80000000 : 0);
+}
+
+// heat-flux z, molecule tag and region bits of every sorted slot
 __global__ void k_hf_slots(const int* __restrict__ perm, int npad, const double* __restrict__ pos, HfDev h,
                            const DynState* __restrict__ dyn, double* __restrict__ zs, int* __restrict__ ms,
                            uint4* __restrict__ bs) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= npad) return;
     int i = perm[s];
-    if (i < 0) { zs[s] = 0.0; ms[s] = 0x7fffffff; bs[s] = make_uint4(0u, 0u, 0u, 0u); return; }
+    if (i < 0) { zs[s] = 0.0; ms[s] = HF_MS_ID; bs[s] = make_uint4(0u, 0u, 0u, 0u); return; }
     const double z = hf_z(h, pos, i, dyn->box[2]);
+    const uint4 b = flux_bits(h, z, dyn->box[2]);
     zs[s] = z;
-    bs[s] = flux_bits(h, z, dyn->box[2]);
-    ms[s] = h.mol_of[i] | (h.hftyp[i] == PGK_HFTYP_MOLE ? (int)0x80000000 : 0);
+    bs[s] = b;
+    ms[s] = hf_tag(h, i, b.w);
 }
 
 // ---- calheatf.F90, volume-based, z components --------------------------------
@@ -92,6 +101,7 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
                                                     const DynState* __restrict__ dyn, double* __restrict__ zs,
                                                     int* __restrict__ ms, void* __restrict__ vs,
                                                     uint4* __restrict__ bs) {
+    pdl_enter();
     __shared__ double sk[PGK_HF_MAX_REGIONS];
     const int nreg = f.h.nreg;
     if (threadIdx.x < PGK_HF_MAX_REGIONS) sk[threadIdx.x] = 0.0;
@@ -108,8 +118,9 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
         if (iperm) {
             const int s = iperm[i];
             zs[s] = z;
-            ms[s] = f.h.mol_of[i] | (f.h.hftyp[i] == PGK_HFTYP_MOLE ? (int)0x80000000 : 0);
+            ms[s] = hf_tag(f.h, i, m.w);
             bs[s] = m;
+            for (int q = 0; q < FLUX_SUMS; ++q) f.sum[(size_t)FLUX_SUMS * s + q] = 0.0;
             if (MIXED) ((float4*)vs)[s] = make_float4((float)vx, (float)vy, (float)vz, (float)pvz);
             else ((double4*)vs)[s] = make_double4(vx, vy, vz, pvz);
         }
@@ -131,18 +142,19 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
 // one lane per entry, a loop over the entry's mask bits.  A pair's share of
 // region r is s (C_r(z_i) - C_r(z_j)) / 2 with s = f_ij . (v_i + v_j) and
 // C_r(z) = z clamped to the slab -- the plane-crossing cases of calvirihf as
-// one difference; C_r(z_j) is formed once per entry, C_r(z_i) once per
-// cluster.  The regions that a row can touch (bits of FluxDev: 3-4 of 23 for
-// 10 A slabs and a 12 A cutoff) are taken KW at a time, so that all sums stay
-// in registers; a row that touches more walks again for the next KW.  Pairs
-// inside one molecule and atoms exactly on a plane (hf_frag's own cases) take
-// a slower branch with shared-memory sums.
+// one difference.  It is linear in s, so the pairs only add s to one atom and
+// take it from the other, next to their energies (FluxDev.sum), and the
+// regions are a sum over the atoms (k_flux_regions).  The cluster atoms' sums
+// stay in registers until the end of the row; an entry's go out once per
+// entry, those of a pair inside one molecule at once (they are a class of
+// their own).  An atom exactly on a plane has hf_frag's own cases: the virial
+// part of its pairs goes to the regions directly.
 // Pair arithmetic is T (FP32 in mixed precision, the reciprocal root refined
-// by one Newton step), all region sums are FP64.
-// Bound by issue (about 60 FP32 and 12 FP64 instructions per pair) at 16 warps
-// per SM.  Measured: 43,200-atom slab, 23 regions, mixed: 0.327 ms per
-// evaluation against 0.79 ms for the per-atom arrays and 0.52 ms for summing
-// them; 8,232-atom water box, one region: 0.042 ms against 0.10 + 0.24 ms.
+// by one Newton step), all sums over atoms and regions are FP64.
+// Bound by issue (about 70 instructions per pair) at 16 warps per SM.
+// Measured, mixed: 43,200-atom slab, 23 regions: 0.159 ms and 0.020 ms for the
+// regions (0.33 ms with the regions inside the pair loop, four a walk); 8,232-
+// atom water box, one region: 0.035 ms, unchanged.
 // Rows are cut into segments until 16 warps per SM have work (small boxes).
 struct FluxPairArgs {
     const int* rows; const int* cnt; int ccap; int ncl; int nseg;
@@ -278,7 +290,7 @@ k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPai
                 if ((e >> (24 + ii)) & 1u) {
                     const uint4 bi = sbi[w][ii];
                     todo |= ~((bi.x & bj.x) | (bi.y & bj.y));
-                    nsame += !((smi[w][ii] ^ mj) & 0x7fffffff);
+                    nsame += !((smi[w][ii] ^ mj) & HF_MS_ID);
                 }
         }
         todo = __reduce_or_sync(0xffffffffu, todo) & all;
@@ -332,7 +344,7 @@ k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPai
                     if (!hf_term<MIXED>(sxq[w][ii], sx64[MIXED ? 0 : w][ii], qj, pj, a, bx, sti[w][ii] + tj, lj32, lj64, t))
                         continue;
                     const int mi = smi[w][ii];
-                    const bool same = !((mi ^ mj) & 0x7fffffff);
+                    const bool same = !((mi ^ mj) & HF_MS_ID);
                     const uint4 bi = sbi[w][ii];
                     const double zi = szi[w][ii], az = fabs(zi - zj);
                     const bool vir = !((mi < 0) && (mj < 0) && same) && az * bx.B2 < 0.5;
@@ -417,7 +429,7 @@ k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPai
                     HfTerm<MIXED> t;
                     if (!hf_term<MIXED>(qi, pi, qj, pj, a, bx, ti + a.typ_s[j], lj32, lj64, t)) continue;
                     const int mj = a.ms[j];
-                    const bool same = !((mi ^ mj) & 0x7fffffff);
+                    const bool same = !((mi ^ mj) & HF_MS_ID);
                     if (same != maj) continue;
                     pc += (double)t.pc;
                     pl += (double)t.pl;
@@ -465,27 +477,20 @@ k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPai
     }
 }
 
-template <bool MIXED, int KW>
+template <bool MIXED>
 __global__ void __launch_bounds__(128, MIXED ? 4 : 3)
 k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPairArgs a,
             const float2* __restrict__ lj32, const double2* __restrict__ lj64, FluxDev f,
             const DynState* __restrict__ dyn) {
+    pdl_enter();
     typedef typename FluxT<MIXED>::T T;
     typedef typename FluxT<MIXED>::V V;
-    __shared__ double sb[8 * PGK_HF_MAX_REGIONS];        // [nreg][pot 4 | virial 4], categories ELIN..VDW
-    __shared__ double sz1[PGK_HF_MAX_REGIONS], sz2[PGK_HF_MAX_REGIONS];
     __shared__ int4 sxq[4][8];
     __shared__ double4 sx64[MIXED ? 1 : 4][8];
     __shared__ V sv[4][8];
-    __shared__ double szi[4][8], sC[4][8][KW];
-    __shared__ uint4 sbi[4][8];
+    __shared__ double szi[4][8];
     __shared__ int smi[4][8], sti[4][8];
-    const int nreg = f.h.nreg;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = threadIdx.x; q < 8 * nreg; q += blockDim.x) sb[q] = 0.0;
-    if (threadIdx.x < nreg) { sz1[threadIdx.x] = f.h.z1[threadIdx.x]; sz2[threadIdx.x] = f.h.z2[threadIdx.x]; }
-    __syncthreads();
-    const unsigned all = nreg >= 32 ? 0xffffffffu : (1u << nreg) - 1u;
     const double L0 = dyn->box[0], L1 = dyn->box[1], Lz = dyn->box[2];
     const double B0 = 1.0 / L0, B1 = 1.0 / L1, B2 = 1.0 / Lz;
     const T sx = (T)(L0 * (1.0 / 4294967296.0)), sy = (T)(L1 * (1.0 / 4294967296.0)), sz = (T)(Lz * (1.0 / 4294967296.0));
@@ -505,181 +510,186 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
             if (MIXED) sxq[w][lane] = xq[s]; else sx64[MIXED ? 0 : w][lane] = xq64[s];
             sv[w][lane] = vs[s];
             szi[w][lane] = a.zs[s];
-            sbi[w][lane] = a.bs[s];
             smi[w][lane] = a.ms[s];
             sti[w][lane] = a.typ_s[s] * a.ntyp;
         }
         __syncwarp();
-        // regions that a pair of this row segment can touch, or its atoms lie in
-        unsigned todo = all;
-        if (nreg > KW) {
-            unsigned t = 0u;
-            for (int k = k_lo + lane; k < k_hi; k += 32) {
-                const unsigned e = (unsigned)row[k];
-                const uint4 bj = a.bs[e & 0xFFFFFFu];
-                t |= bj.z;
+        T pic[8], pil[8];
+        double sic[8], sil[8];
 #pragma unroll
-                for (int ii = 0; ii < 8; ++ii)
-                    if ((e >> (24 + ii)) & 1u) {
-                        const uint4 bi = sbi[w][ii];
-                        t |= bi.z | ~((bi.x & bj.x) | (bi.y & bj.y));
-                    }
-            }
-            todo = __reduce_or_sync(0xffffffffu, t) & all;
-        }
-        while (todo) {
-            int rk[KW];
-            unsigned win = 0u;
+        for (int ii = 0; ii < 8; ++ii) { pic[ii] = (T)0; pil[ii] = (T)0; sic[ii] = 0.0; sil[ii] = 0.0; }
+        for (int k = k_lo + lane; k < k_hi; k += 32) {
+            const unsigned e = (unsigned)row[k];
+            const int j = (int)(e & 0xFFFFFFu);
+            const unsigned m = e >> 24;
+            const double zj = a.zs[j];
+            const int mj = a.ms[j], tj = a.typ_s[j];
+            const V vj = vs[j];
+            int4 qj = make_int4(0, 0, 0, 0);
+            double4 pj = make_double4(0, 0, 0, 0);
+            if (MIXED) qj = xq[j]; else pj = xq64[j];
+            T pjc = (T)0, pjl = (T)0;
+            double sjc = 0.0, sjl = 0.0;
 #pragma unroll
-            for (int k = 0; k < KW; ++k) {
-                rk[k] = todo ? __ffs(todo) - 1 : -1;
-                if (todo) { win |= 1u << rk[k]; todo &= todo - 1; }
-            }
-            __syncwarp();
-            if (lane < 8) {
-#pragma unroll
-                for (int k = 0; k < KW; ++k) {
-                    const double z = szi[w][lane];
-                    const int r = max(rk[k], 0);
-                    const uint4 b = sbi[w][lane];
-                    sC[w][lane][k] = (b.x >> r) & 1u ? sz1[r] : ((b.y >> r) & 1u ? sz2[r] : z);
+            for (int ii = 0; ii < 8; ++ii) {
+                if (!((m >> ii) & 1u)) continue;
+                T dx, dy, dz, qq;
+                if (MIXED) {
+                    const int4 qi = sxq[w][ii];
+                    dx = (T)(qi.x - qj.x) * sx; dy = (T)(qi.y - qj.y) * sy; dz = (T)(qi.z - qj.z) * sz;
+                    qq = (T)(__int_as_float(qi.w) * __int_as_float(qj.w));
+                } else {
+                    const double4 pi = sx64[MIXED ? 0 : w][ii];
+                    const double wx = pi.x - pj.x, wy = pi.y - pj.y, wz = pi.z - pj.z;
+                    dx = (T)(wx - L0 * round(wx * B0));
+                    dy = (T)(wy - L1 * round(wy * B1));
+                    dz = (T)(wz - Lz * round(wz * B2));
+                    qq = (T)(pi.w * pj.w);
                 }
-            }
-            __syncwarp();
-            double vc[KW], vl[KW], pc[KW], pl[KW];
-            T pic[8], pil[8];
-#pragma unroll
-            for (int k = 0; k < KW; ++k) { vc[k] = 0.0; vl[k] = 0.0; pc[k] = 0.0; pl[k] = 0.0; }
-#pragma unroll
-            for (int ii = 0; ii < 8; ++ii) { pic[ii] = (T)0; pil[ii] = (T)0; }
-            for (int k = k_lo + lane; k < k_hi; k += 32) {
-                const unsigned e = (unsigned)row[k];
-                const int j = (int)(e & 0xFFFFFFu);
-                const unsigned m = e >> 24;
-                const double zj = a.zs[j];
-                const int mj = a.ms[j], tj = a.typ_s[j];
-                const uint4 bj = a.bs[j];
-                const V vj = vs[j];
-                int4 qj = make_int4(0, 0, 0, 0);
-                double4 pj = make_double4(0, 0, 0, 0);
-                if (MIXED) qj = xq[j]; else pj = xq64[j];
-                double Cj[KW];
-#pragma unroll
-                for (int q = 0; q < KW; ++q) {
-                    const int r = max(rk[q], 0);
-                    Cj[q] = (bj.x >> r) & 1u ? sz1[r] : ((bj.y >> r) & 1u ? sz2[r] : zj);
+                const T r2 = dx * dx + dy * dy + dz * dz;
+                if (r2 > rmax2) continue;
+                const T rinv = flux_rinv(r2), rinv2 = rinv * rinv;
+                const T phc = r2 <= rr2 ? qq * rinv : (T)0;              // ewaldr_hf.F90:336-371, bare 1/r
+                T phl = (T)0, ftl = (T)0;
+                if (r2 <= rl2) {                                         // ewaldr_hf.F90:376-470
+                    T R2, E;
+                    if (MIXED) { const float2 lp = lj32[sti[w][ii] + tj]; R2 = lp.x; E = lp.y; }
+                    else { const double2 lp = lj64[sti[w][ii] + tj]; R2 = lp.x; E = lp.y; }
+                    const T t2 = rinv2 * R2, t6 = t2 * t2 * t2, t12 = t6 * t6;
+                    phl = E * (t12 - (T)2 * t6);
+                    ftl = (T)12 * E * (t12 - t6) * rinv2;
                 }
-                T pjc = (T)0, pjl = (T)0;
-#pragma unroll
-                for (int ii = 0; ii < 8; ++ii) {
-                    if (!((m >> ii) & 1u)) continue;
-                    T dx, dy, dz, qq;
-                    if (MIXED) {
-                        const int4 qi = sxq[w][ii];
-                        dx = (T)(qi.x - qj.x) * sx; dy = (T)(qi.y - qj.y) * sy; dz = (T)(qi.z - qj.z) * sz;
-                        qq = (T)(__int_as_float(qi.w) * __int_as_float(qj.w));
-                    } else {
-                        const double4 pi = sx64[MIXED ? 0 : w][ii];
-                        const double wx = pi.x - pj.x, wy = pi.y - pj.y, wz = pi.z - pj.z;
-                        dx = (T)(wx - L0 * round(wx * B0));
-                        dy = (T)(wy - L1 * round(wy * B1));
-                        dz = (T)(wz - Lz * round(wz * B2));
-                        qq = (T)(pi.w * pj.w);
-                    }
-                    const T r2 = dx * dx + dy * dy + dz * dz;
-                    if (r2 > rmax2) continue;
-                    const T rinv = flux_rinv(r2), rinv2 = rinv * rinv;
-                    const T phc = r2 <= rr2 ? qq * rinv : (T)0;          // ewaldr_hf.F90:336-371, bare 1/r
-                    T phl = (T)0, ftl = (T)0;
-                    if (r2 <= rl2) {                                     // ewaldr_hf.F90:376-470
-                        T R2, E;
-                        if (MIXED) { const float2 lp = lj32[sti[w][ii] + tj]; R2 = lp.x; E = lp.y; }
-                        else { const double2 lp = lj64[sti[w][ii] + tj]; R2 = lp.x; E = lp.y; }
-                        const T t2 = rinv2 * R2, t6 = t2 * t2 * t2, t12 = t6 * t6;
-                        phl = E * (t12 - (T)2 * t6);
-                        ftl = (T)12 * E * (t12 - t6) * rinv2;
-                    }
-                    const V vi = sv[w][ii];
-                    const T fv = dx * (vi.x + vj.x) + dy * (vi.y + vj.y) + dz * (vi.z + vj.z);
-                    const int mi = smi[w][ii];
-                    const bool same = (mi & 0x7fffffff) == (mj & 0x7fffffff);
-                    const uint4 bi = sbi[w][ii];
-                    const double zi = szi[w][ii];
-                    const double az = fabs(zi - zj);
-                    const bool vir = !((mi < 0) && (mj < 0) && same) && az * B2 < 0.5;
-                    double sc = vir ? 0.5 * (double)(phc * rinv2 * fv) : 0.0;
-                    double sl = vir ? 0.5 * (double)(ftl * fv) : 0.0;
-                    if (same || ((bi.w | bj.w) & win)) {
-                        const int cc = same ? 0 : 2, lc = same ? 1 : 3;
+                const V vi = sv[w][ii];
+                const T fv = dx * (vi.x + vj.x) + dy * (vi.y + vj.y) + dz * (vi.z + vj.z);
+                const int mi = smi[w][ii];
+                const bool same = !((mi ^ mj) & HF_MS_ID);
+                const double zi = szi[w][ii], az = fabs(zi - zj);
+                const bool vir = !((mi < 0) && (mj < 0) && same) && az * B2 < 0.5;
+                double sc = vir ? 0.5 * (double)(phc * rinv2 * fv) : 0.0;
+                double sl = vir ? 0.5 * (double)(ftl * fv) : 0.0;
+                if (same || ((mi | mj) & HF_MS_PLANE)) {
+                    const int s = 8 * cl + ii;
+                    if (vir && ((mi | mj) & HF_MS_PLANE)) {
                         // the lower atom index first: the reference's i
-                        const bool first = a.perm[8 * cl + ii] < a.perm[j];
-                        const double za = first ? zi : zj, zb = first ? zj : zi;
-#pragma unroll
-                        for (int q = 0; q < KW; ++q) {
-                            const int r = rk[q];
-                            if (r < 0) continue;
-                            double* o = sb + 8 * r;
-                            if (same) {
-                                const double tv = 0.5 * (((bi.z >> r) & 1u ? (double)vi.w : 0.0) +
-                                                         ((bj.z >> r) & 1u ? (double)vj.w : 0.0));
-                                if (tv != 0.0) { atomicAdd(o + cc, (double)phc * tv); atomicAdd(o + lc, (double)phl * tv); }
-                            }
+                        const bool first = a.perm[s] < a.perm[j];
+                        const uint4 bi = a.bs[s], bj = a.bs[j];
+                        double* acc = f.acc + (size_t)(blockIdx.x % FLUX_COPIES) * f.h.nreg * FLUX_COLS + 9 +
+                                      PGK_HF_ELIN + (same ? 0 : 2);
+#pragma unroll 1
+                        for (int r = 0; r < f.h.nreg; ++r) {
                             double frag;
-                            if (vir && !(((bi.x & bj.x) | (bi.y & bj.y)) >> r & 1u) &&
-                                hf_frag(za, zb, sz1[r], sz2[r], az, frag)) {
-                                const double d = zi - zj >= 0.0 ? frag : -frag;
-                                atomicAdd(o + 4 + cc, sc * d);
-                                atomicAdd(o + 4 + lc, sl * d);
-                            }
+                            if (((bi.x & bj.x) | (bi.y & bj.y)) >> r & 1u) continue;
+                            if (!hf_frag(first ? zi : zj, first ? zj : zi, f.h.z1[r], f.h.z2[r], az, frag)) continue;
+                            const double d = zi - zj >= 0.0 ? frag : -frag;
+                            atomicAdd(acc + r * FLUX_COLS, sc * d);
+                            atomicAdd(acc + r * FLUX_COLS + 1, sl * d);
                         }
                         sc = 0.0;
                         sl = 0.0;
                     }
-                    if (!same) { pic[ii] += phc; pil[ii] += phl; pjc += phc; pjl += phl; }
-#pragma unroll
-                    for (int q = 0; q < KW; ++q) {
-                        const double D = sC[w][ii][q] - Cj[q];
-                        vc[q] = fma(sc, D, vc[q]);
-                        vl[q] = fma(sl, D, vl[q]);
+                    if (same) {
+                        double* si = f.sum + (size_t)FLUX_SUMS * s;
+                        double* sj = f.sum + (size_t)FLUX_SUMS * j;
+                        atomicAdd(si, (double)phc); atomicAdd(sj, (double)phc);
+                        atomicAdd(si + 1, (double)phl); atomicAdd(sj + 1, (double)phl);
+                        if (sc != 0.0) { atomicAdd(si + 2, sc); atomicAdd(sj + 2, -sc); }
+                        if (sl != 0.0) { atomicAdd(si + 3, sl); atomicAdd(sj + 3, -sl); }
+                        continue;
                     }
                 }
-                const double hz = 0.5 * (double)vj.w;
-#pragma unroll
-                for (int q = 0; q < KW; ++q) {
-                    const double t = rk[q] >= 0 && (bj.z >> rk[q]) & 1u ? hz : 0.0;
-                    pc[q] = fma((double)pjc, t, pc[q]);
-                    pl[q] = fma((double)pjl, t, pl[q]);
-                }
+                pic[ii] += phc; pil[ii] += phl; pjc += phc; pjl += phl;
+                sic[ii] += sc; sil[ii] += sl; sjc += sc; sjl += sl;
             }
-            // cluster atoms' transport shares, then the warp's sums
+            double* sj = f.sum + (size_t)FLUX_SUMS * j + 4;
+            if (pjc != (T)0) atomicAdd(sj, (double)pjc);
+            if (pjl != (T)0) atomicAdd(sj + 1, (double)pjl);
+            if (sjc != 0.0) atomicAdd(sj + 2, -sjc);
+            if (sjl != 0.0) atomicAdd(sj + 3, -sjl);
+        }
+        // the cluster atoms' 32 sums: halves exchanged until lane l holds the
+        // total of value l = 4 atom + sum
+        double v[32];
 #pragma unroll
-            for (int ii = 0; ii < 8; ++ii) {
-                const double hz = 0.5 * (double)sv[w][ii].w;
-                const unsigned in = sbi[w][ii].z;
+        for (int ii = 0; ii < 8; ++ii) {
+            v[4 * ii] = (double)pic[ii]; v[4 * ii + 1] = (double)pil[ii];
+            v[4 * ii + 2] = sic[ii]; v[4 * ii + 3] = sil[ii];
+        }
 #pragma unroll
-                for (int q = 0; q < KW; ++q)
-                    if (rk[q] >= 0 && (in >> rk[q]) & 1u) {
-                        pc[q] = fma((double)pic[ii], hz, pc[q]);
-                        pl[q] = fma((double)pil[ii], hz, pl[q]);
-                    }
-            }
+        for (int h = 16; h > 0; h >>= 1) {
+            const bool up = lane & h;
 #pragma unroll
-            for (int q = 0; q < KW; ++q) {
-                if (rk[q] < 0) continue;                   // warp-uniform
-                const double s0 = warp_sum(pc[q]), s1 = warp_sum(pl[q]), s2 = warp_sum(vc[q]), s3 = warp_sum(vl[q]);
-                if (lane < 4) {
-                    const double s = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
-                    const int col = lane == 0 ? 2 : lane == 1 ? 3 : lane == 2 ? 6 : 7;
-                    if (s != 0.0) atomicAdd(sb + 8 * rk[q] + col, s);
-                }
+            for (int q = 0; q < h; ++q) {
+                const double keep = up ? v[q + h] : v[q], send = up ? v[q] : v[q + h];
+                v[q] = keep + __shfl_xor_sync(0xffffffffu, send, h);
             }
         }
+        if (v[0] != 0.0) atomicAdd(f.sum + (size_t)FLUX_SUMS * (8 * cl + (lane >> 2)) + 4 + (lane & 3), v[0]);
+    }
+}
+
+// Region sums of the atoms' pair sums: a warp takes 32 slots, its lanes one
+// region and every (32 / PR)-th slot each, PR the power of two that holds the
+// regions (C_r(z) - z1_r: the pairs' differences stay).  Each slot's 8 sums are
+// one 64-byte line.
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_flux_regions(const int* __restrict__ perm, int npad,
+                                                      const double* __restrict__ zs, const void* __restrict__ vs_,
+                                                      const uint4* __restrict__ bs, FluxDev f) {
+    pdl_enter();
+    typedef typename FluxT<MIXED>::V V;
+    const V* __restrict__ vs = (const V*)vs_;
+    __shared__ double st[8][32][FLUX_SUMS + 2];
+    __shared__ unsigned si[8][32];
+    __shared__ double sb[8 * PGK_HF_MAX_REGIONS];
+    const int nreg = f.h.nreg, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = threadIdx.x; q < 8 * nreg; q += 256) sb[q] = 0.0;
+    __syncthreads();
+    const int s = blockIdx.x * 256 + threadIdx.x;
+    const bool has = s < npad && perm[s] >= 0;
+    if (has) {
+        st[w][lane][0] = zs[s];
+        st[w][lane][1] = 0.5 * (double)vs[s].w;
+        si[w][lane] = bs[s].z;
+#pragma unroll
+        for (int q = 0; q < FLUX_SUMS; ++q) st[w][lane][2 + q] = f.sum[(size_t)FLUX_SUMS * s + q];
+    }
+    const unsigned has_m = __ballot_sync(0xffffffffu, has);      // the slots of st and si that were written
+    __syncwarp();
+    int pr = 1;
+    while (pr < nreg) pr <<= 1;
+    const int r = lane & (pr - 1), part = lane / pr, nq = 32 / pr;
+    const double z1 = r < nreg ? f.h.z1[r] : 0.0, z2 = r < nreg ? f.h.z2[r] : 0.0;
+    double o[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) o[q] = 0.0;
+    if (r < nreg)
+        for (int k = part; k < 32; k += nq) {
+            if (!((has_m >> k) & 1u)) continue;
+            const double* p = st[w][k];
+            const double D = fmin(fmax(p[0], z1), z2) - z1;
+            const double tv = (si[w][k] >> r) & 1u ? p[1] : 0.0;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {        // pairs inside one molecule, between two
+                o[4 * c] = fma(p[2 + 4 * c], tv, o[4 * c]);
+                o[4 * c + 1] = fma(p[3 + 4 * c], tv, o[4 * c + 1]);
+                o[4 * c + 2] = fma(p[4 + 4 * c], D, o[4 * c + 2]);
+                o[4 * c + 3] = fma(p[5 + 4 * c], D, o[4 * c + 3]);
+            }
+        }
+    __syncwarp();
+    for (int h = pr; h < 32; h <<= 1)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) o[q] += __shfl_xor_sync(0xffffffffu, o[q], h);
+    if (part == 0 && r < nreg) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (o[q] != 0.0) atomicAdd(sb + 8 * r + q, o[q]);
     }
     __syncthreads();
     double* acc = f.acc + (size_t)(blockIdx.x % FLUX_COPIES) * nreg * FLUX_COLS;
-    for (int q = threadIdx.x; q < 8 * nreg; q += blockDim.x) {
-        const int r = q >> 3, c = q & 7;
-        if (sb[q] != 0.0) atomicAdd(acc + r * FLUX_COLS + (c < 4 ? 1 : 9 - 4) + PGK_HF_ELIN + c, sb[q]);
+    for (int q = threadIdx.x; q < 8 * nreg; q += 256) {
+        const int c = (q >> 2) & 1, v = q & 3;                   // class; energies, virials
+        if (sb[q] != 0.0) atomicAdd(acc + (q >> 3) * FLUX_COLS + (v < 2 ? 1 : 9 - 2) + PGK_HF_ELIN + 2 * c + v, sb[q]);
     }
 }
 
@@ -719,6 +729,7 @@ __global__ void __launch_bounds__(256) k_flux_kspace(const double* __restrict__ 
 
 // volume normalisation and hftot; leaves the sums zero (one warp per region)
 __global__ void k_flux_final(FluxDev f, const DynState* __restrict__ dyn, double* __restrict__ rec) {
+    pdl_enter();
     const int r = blockIdx.x, c = threadIdx.x;
     double s = 0.0;
     if (c < FLUX_COLS) {
@@ -922,14 +933,15 @@ pgk_status hf_setup(pgk_ctx* c, const pgk_hfparams* p) {
 
 static pgk_status ensure_hf_slots(pgk_ctx* c) {
     if (c->hf_slots_cap >= c->npad_cap) return PGK_OK;
-    pgk_dfree(c, c->hf_zs); pgk_dfree(c, c->hf_ms); pgk_dfree(c, c->hf_vs); pgk_dfree(c, c->hf_bs);
-    c->hf_zs = nullptr; c->hf_ms = nullptr; c->hf_vs = nullptr; c->hf_bs = nullptr;
+    pgk_dfree(c, c->hf_zs); pgk_dfree(c, c->hf_ms); pgk_dfree(c, c->hf_vs); pgk_dfree(c, c->hf_bs); pgk_dfree(c, c->hf_sum);
+    c->hf_zs = nullptr; c->hf_ms = nullptr; c->hf_vs = nullptr; c->hf_bs = nullptr; c->hf_sum = nullptr;
     c->hf_slots_cap = 0;
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_zs, sizeof(double) * c->npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_ms, sizeof(int) * c->npad_cap));
     const size_t vb = (c->mixed() ? sizeof(float4) : sizeof(double4)) * (size_t)c->npad_cap;
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_vs, vb));
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_bs, sizeof(uint4) * c->npad_cap));
+    PGK_CUDA(c, pgk_dmalloc(c, &c->hf_sum, sizeof(double) * FLUX_SUMS * c->npad_cap));
     // padding slots take part in no pair, but a cluster stages them
     PGK_CUDA(c, cudaMemsetAsync(c->hf_zs, 0, sizeof(double) * c->npad_cap, c->st));
     PGK_CUDA(c, cudaMemsetAsync(c->hf_ms, 0, sizeof(int) * c->npad_cap, c->st));
@@ -1020,8 +1032,8 @@ pgk_status launch_hf_atm(pgk_ctx* c, bool pruned) {
     pgk_status s;
     const int n = c->natom, nreg = c->hfp.nhfregion;
     if (c->nmole > 0) {
-        k_calcom<<<(c->nmole + 127) / 128, 128, 0, c->st>>>(c->pos, nullptr, c->mass, c->mol_idx, c->mol_list, c->nmole,
-                                                             c->dyn, c->molecom, nullptr);
+        launch_pdl(k_calcom, (c->nmole + 127) / 128, 128, 0, c->st, c->pos, (const double*)nullptr, c->mass, c->mol_idx,
+                   c->mol_list, c->nmole, c->dyn, c->molecom, (double*)nullptr);
         PGK_LAUNCHED(c);
     }
     PGK_CUDA(c, cudaMemsetAsync(c->hf_pot, 0, sizeof(double) * 8 * n, c->st));
@@ -1045,14 +1057,12 @@ pgk_status launch_hf_atm(pgk_ctx* c, bool pruned) {
     return launch_hf_kspace(c);
 }
 
-// one region: one accumulator set; more: four a walk (most rows touch 3-4)
 template <bool MIXED>
 static void flux_pair_launch(pgk_ctx* c, const FluxPairArgs& a, const FluxDev& f) {
-    const int blocks = flux_pair_grid(c, a);
-    if (f.h.nreg == 1)
-        k_flux_pair<MIXED, 1><<<blocks, 128, 0, c->st>>>(c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
-    else
-        k_flux_pair<MIXED, 4><<<blocks, 128, 0, c->st>>>(c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
+    launch_pdl(k_flux_pair<MIXED>, flux_pair_grid(c, a), 128, 0, c->st, c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
+    PGK_LAUNCHED(c);
+    launch_pdl(k_flux_regions<MIXED>, (c->npad + 255) / 256, 256, 0, c->st, c->perm, c->npad, c->hf_zs, c->hf_vs, c->hf_bs,
+               f);
     PGK_LAUNCHED(c);
 }
 
@@ -1063,19 +1073,16 @@ pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
     f.h = hf_dev(c);
     f.vel = c->vel; f.molevel = c->molevel; f.acc = c->hf_acc;
     if (c->nmole > 0) {
-        k_calcom<<<(c->nmole + 127) / 128, 128, 0, c->st>>>(c->pos, c->vel, c->mass, c->mol_idx, c->mol_list, c->nmole,
-                                                             c->dyn, c->molecom, c->molevel);
+        launch_pdl(k_calcom, (c->nmole + 127) / 128, 128, 0, c->st, c->pos, c->vel, c->mass, c->mol_idx, c->mol_list,
+                   c->nmole, c->dyn, c->molecom, c->molevel);
         PGK_LAUNCHED(c);
     }
     const bool pair_on = flux_pair_on(c);
     if (pair_on && (s = ensure_hf_slots(c))) return s;
+    f.sum = c->hf_sum;
     const int* ip = pair_on ? c->iperm : nullptr;
-    if (c->mixed())
-        k_flux_atoms<true><<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->mass, ip, f, c->dyn, c->hf_zs, c->hf_ms,
-                                                               c->hf_vs, c->hf_bs);
-    else
-        k_flux_atoms<false><<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, c->mass, ip, f, c->dyn, c->hf_zs, c->hf_ms,
-                                                                c->hf_vs, c->hf_bs);
+    launch_pdl(c->mixed() ? k_flux_atoms<true> : k_flux_atoms<false>, (n + 255) / 256, 256, 0, c->st, c->pos, c->mass, ip,
+               f, c->dyn, c->hf_zs, c->hf_ms, c->hf_vs, c->hf_bs);
     PGK_LAUNCHED(c);
     if (pair_on) {
         const FluxPairArgs a = flux_pair_args(c, pruned);
@@ -1090,7 +1097,7 @@ pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
         k_flux_kspace<<<(n + 255) / 256, 256, 0, c->st>>>(c->pos, pot, pot + n, f, c->dyn);
         PGK_LAUNCHED(c);
     }
-    k_flux_final<<<nreg, 32, 0, c->st>>>(f, c->dyn, dst);
+    launch_pdl(k_flux_final, nreg, 32, 0, c->st, f, c->dyn, dst);
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;

@@ -77,11 +77,14 @@ __device__ __forceinline__ void hf_calviri(const HfDev& h, const double* __restr
 // terms); a block adds its totals to copy blockIdx % FLUX_COPIES.
 #define FLUX_COPIES 16
 #define FLUX_COLS 17
+#define FLUX_SUMS 8
 struct FluxDev {
     HfDev h;                 // regions and per-atom typing (pot, W unused)
     const double* vel;
     const double* molevel;   // [3*nmole] molecule velocities
     double* acc;
+    double* sum;             // [slot][FLUX_SUMS] pair sums of the atoms: (Coulomb, LJ energies, s of
+                             // Coulomb, LJ) x (pairs inside one molecule, between two)
 };
 
 // bits r of a z: below slab r, above it, inside it (transport term, z wrapped
