@@ -165,6 +165,7 @@ template <typename T2, typename T> __device__ __forceinline__ T2 mul_i(T2 a, T s
     T2 r; r.x = -s * a.y; r.y = s * a.x; return r;
 }
 
+#define PLANE_BT 512                      // most threads of a plane's block
 struct FftDev {
     int n, nstage;
     int radix[PGK_MAX_RADIX_STAGES];
@@ -172,18 +173,36 @@ struct FftDev {
 };
 
 template <typename T, typename T2>
+__device__ __forceinline__ void dft4(T2* v, T sg) {
+    T2 a0 = v[0], a1 = v[1], a2 = v[2], a3 = v[3];
+    T2 s02 = cadd(a0, a2), d02 = csub(a0, a2), s13 = cadd(a1, a3), d13 = csub(a1, a3);
+    v[0] = cadd(s02, s13);
+    v[2] = csub(s02, s13);
+    T2 t = mul_i<T2, T>(d13, sg);
+    v[1] = cadd(d02, t);
+    v[3] = csub(d02, t);
+}
+
+template <typename T, typename T2>
 __device__ __forceinline__ void dft_r(T2* v, int R, T sg) {
     if (R == 2) {
         T2 a = v[0], b = v[1];
         v[0] = cadd(a, b); v[1] = csub(a, b);
     } else if (R == 4) {
-        T2 a0 = v[0], a1 = v[1], a2 = v[2], a3 = v[3];
-        T2 s02 = cadd(a0, a2), d02 = csub(a0, a2), s13 = cadd(a1, a3), d13 = csub(a1, a3);
-        v[0] = cadd(s02, s13);
-        v[2] = csub(s02, s13);
-        T2 t = mul_i<T2, T>(d13, sg);
-        v[1] = cadd(d02, t);
-        v[3] = csub(d02, t);
+        dft4<T, T2>(v, sg);
+    } else if (R == 8) {
+        const T s = T(0.70710678118654752440);
+        T2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft4<T, T2>(e, sg);
+        dft4<T, T2>(o, sg);
+        T2 w1, w3;                               // o1 exp(sg i pi / 4), o3 exp(3 sg i pi / 4)
+        w1.x = s * (o[1].x - sg * o[1].y); w1.y = s * (o[1].y + sg * o[1].x);
+        w3.x = -s * (o[3].x + sg * o[3].y); w3.y = s * (sg * o[3].x - o[3].y);
+        const T2 w2 = mul_i<T2, T>(o[2], sg);
+        v[0] = cadd(e[0], o[0]); v[4] = csub(e[0], o[0]);
+        v[1] = cadd(e[1], w1); v[5] = csub(e[1], w1);
+        v[2] = cadd(e[2], w2); v[6] = csub(e[2], w2);
+        v[3] = cadd(e[3], w3); v[7] = csub(e[3], w3);
     } else if (R == 3) {
         const T s60 = T(0.86602540378443864676);
         T2 a0 = v[0], a1 = v[1], a2 = v[2];
@@ -212,9 +231,10 @@ __device__ __forceinline__ void dft_r(T2* v, int R, T sg) {
     }
 }
 
-// radix chain of a length (4s first, then 2, 3, 5), usable at compile time
+// radix chain of a compile-time length (8s where they save a stage, 4s, then
+// 2, 3, 5)
 __host__ __device__ constexpr int pick_radix(int m) {
-    return m % 4 == 0 ? 4 : (m % 2 == 0 ? 2 : (m % 3 == 0 ? 3 : (m % 5 == 0 ? 5 : 0)));
+    return m % 8 == 0 && m != 16 ? 8 : m % 4 == 0 ? 4 : (m % 2 == 0 ? 2 : (m % 3 == 0 ? 3 : (m % 5 == 0 ? 5 : 0)));
 }
 __host__ __device__ constexpr int stage_radix(int n, int s) {
     int m = n;
@@ -232,23 +252,31 @@ __host__ __device__ constexpr int nstages(int n) {
     return c;
 }
 
+// registers of a stage's points (RM of fft_stage)
+__host__ __device__ constexpr int stage_rm(int n, int s) { return s < nstages(n) && stage_radix(n, s) > 5 ? 8 : 5; }
+
 // one Stockham stage on P pencils of length n held in shared memory
-// pencils are stored with pitch ld = n + 1 elements, so that the strided
-// loads and stores of the y and z passes (consecutive threads on consecutive
-// pencils) fall into different shared-memory banks
-template <typename T, typename T2>
+// Pencils are stored with pitch ld = n + 1 elements, and consecutive threads
+// take consecutive pencils at one place j: with n even the stage's strided
+// loads and stores fall into different shared-memory banks, and a twiddle
+// factor is one broadcast.  Measured, 128^3 FP32 convolution in five
+// passes: 97 us with consecutive threads on consecutive j and radix 4, 96 with
+// radix 8, 89 with the pencils first, 84 with both.
+// RM: the largest radix
+template <typename T, typename T2, int RM>
 __device__ __forceinline__ void fft_stage(const T2* __restrict__ src, T2* __restrict__ dst, int P, int n, int R,
                                           int Ns, const T2* __restrict__ tw, T sg) {
     const int ld = n + 1;
     const int nr = n / R;
     const int twstep = n / (Ns * R);
-    for (int w = threadIdx.x; w < P * nr; w += blockDim.x) {
-        int p = w / nr, j = w - p * nr;
+    const int dj = blockDim.x / P, dp = blockDim.x - dj * P;
+    int j = threadIdx.x / P, p = threadIdx.x - j * P;
+    while (j < nr) {
         int k = j % Ns;
-        T2 v[5];
+        T2 v[RM];
         const T2* sp = src + p * ld;
 #pragma unroll
-        for (int r = 0; r < 5; ++r)
+        for (int r = 0; r < RM; ++r)
             if (r < R) {
                 T2 x = sp[j + r * nr];
                 if (r > 0 && k > 0) {
@@ -260,10 +288,13 @@ __device__ __forceinline__ void fft_stage(const T2* __restrict__ src, T2* __rest
             }
         dft_r<T, T2>(v, R, sg);
         int o = (j / Ns) * Ns * R + k;
-        T2* dp = dst + p * ld;
+        T2* dpn = dst + p * ld;
 #pragma unroll
-        for (int r = 0; r < 5; ++r)
-            if (r < R) dp[o + r * Ns] = v[r];
+        for (int r = 0; r < RM; ++r)
+            if (r < R) dpn[o + r * Ns] = v[r];
+        j += dj;
+        p += dp;
+        if (p >= P) { p -= P; ++j; }
     }
 }
 
@@ -275,13 +306,13 @@ struct FftStages {
         if (NC == 0) {
             int Ns = 1;
             for (int s = 0; s < plan.nstage; ++s) {
-                fft_stage<T, T2>(src, dst, P, n, plan.radix[s], Ns, tw, sg);
+                fft_stage<T, T2, 5>(src, dst, P, n, plan.radix[s], Ns, tw, sg);
                 __syncthreads();
                 T2* t = src; src = dst; dst = t;
                 Ns *= plan.radix[s];
             }
         } else if (S < nstages(NC)) {
-            fft_stage<T, T2>(src, dst, P, NC, stage_radix(NC, S), stage_ns(NC, S), tw, sg);
+            fft_stage<T, T2, stage_rm(NC, S)>(src, dst, P, NC, stage_radix(NC, S), stage_ns(NC, S), tw, sg);
             __syncthreads();
             T2* t = src; src = dst; dst = t;
             FftStages<T, T2, NC, (S < 12 ? S + 1 : S)>::run(src, dst, P, n, plan, sg, tw);
@@ -604,6 +635,117 @@ __global__ void __launch_bounds__(256) k_fft_rx(typename C2<T>::t* __restrict__ 
             T* out = (T*)real + (size_t)(line0 + p) * K1 + 2 * m;
             out[0] = z.x;
             out[1] = z.y;
+        }
+    }
+}
+
+// One z plane of the real-to-complex transform: the x lines (as k_fft_rx), then
+// the K1/2 + 1 y pencils, in shared memory (FWD); the y pencils, then the x
+// lines, to the real grid (inverse).  One block per plane: one launch and one
+// pass over the grid instead of two.  The stages and their order are those of
+// the separate passes.
+// Bound by latency at one or two blocks per SM (each stage is a trip through
+// shared memory and a barrier).  Measured, whole convolution, FP32, against five
+// passes: 32^3 21 us (27), 64^3 31 (33), 64 x 64 x 192 41 (58), 128^3 64 (84);
+// FP64 64^3 30 (40).  A step of 1,536 water atoms 49 -> 47 us.
+template <typename T, int SRC, int NX, int NY, bool FWD>
+__global__ void __launch_bounds__(PLANE_BT) k_fft_plane(typename C2<T>::t* __restrict__ data, void* __restrict__ real,
+                                                       int K1, int K2_, FftDev px, FftDev py,
+                                                       const void* __restrict__ tw2g) {
+    typedef typename C2<T>::t T2;
+    extern __shared__ unsigned char smraw[];
+    const int N = NX > 0 ? NX : px.n, K2 = NY > 0 ? NY : K2_;
+    const int K1h = N + 1, ldx = N + 1, ldy = K2 + 1;
+    T2* bufA = (T2*)smraw;
+    T2* bufB = bufA + K1h * ldy;          // K2 lines of pitch ldx fit as well
+    T2* twx = bufB + K1h * ldy;
+    T2* tw2 = twx + N;                    // exp(-2 pi i k / K1), k = 0..N
+    T2* twy = tw2 + N + 1;
+    const int tid = threadIdx.x, bt = blockDim.x;
+    for (int k = tid; k < N; k += bt) twx[k] = ((const T2*)px.tw)[k];
+    for (int k = tid; k <= N; k += bt) tw2[k] = ((const T2*)tw2g)[k];
+    for (int k = tid; k < K2; k += bt) twy[k] = ((const T2*)py.tw)[k];
+    pdl_enter();                          // the twiddles are constant
+    T2* src = bufA;
+    T2* dst = bufB;
+    constexpr int LQ = 8;                 // loads in flight per thread
+    T2* const plane = data + (size_t)blockIdx.x * K2 * K1h;
+    if (FWD) {
+        const size_t off0 = (size_t)blockIdx.x * K2 * K1;
+        for (int i0 = tid; i0 < K2 * N; i0 += LQ * bt) {
+            T2 v[LQ];
+#pragma unroll
+            for (int q = 0; q < LQ; ++q) {
+                const int idx = i0 + q * bt;                 // 2 idx: the pair's place in the plane
+                if (idx >= K2 * N) continue;
+                if (SRC == 1) {
+                    const longlong2 g = *(const longlong2*)((const long long*)real + off0 + 2 * idx);
+                    v[q].x = (T)((double)g.x * PGK_GRID_ISCALE);
+                    v[q].y = (T)((double)g.y * PGK_GRID_ISCALE);
+                } else {
+                    const double2 g = *(const double2*)((const double*)real + off0 + 2 * idx);
+                    v[q].x = (T)g.x;
+                    v[q].y = (T)g.y;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < LQ; ++q) {
+                const int idx = i0 + q * bt;
+                if (idx < K2 * N) { const int l = idx / N; src[l * ldx + idx - l * N] = v[q]; }
+            }
+        }
+        __syncthreads();
+        FftStages<T, T2, NX>::run(src, dst, K2, N, px, T(-1), twx);
+        for (int idx = tid; idx < K2 * K1h; idx += bt) {
+            const int l = idx / K1h, k = idx - l * K1h;
+            const T2 zk = src[l * ldx + (k == N ? 0 : k)];
+            T2 zc = src[l * ldx + (k == 0 ? 0 : N - k)];
+            zc.y = -zc.y;
+            const T2 e = cscale<T2, T>(cadd(zk, zc), T(0.5));
+            const T2 d = csub(zk, zc);
+            T2 o; o.x = T(0.5) * d.y; o.y = T(-0.5) * d.x;        // d / 2i
+            dst[k * ldy + l] = cadd(e, cmul(tw2[k], o));
+        }
+        __syncthreads();
+        { T2* s = src; src = dst; dst = s; }
+        FftStages<T, T2, NY>::run(src, dst, K1h, K2, py, T(-1), twy);
+        for (int idx = tid; idx < K2 * K1h; idx += bt) {
+            const int l = idx / K1h, k = idx - l * K1h;
+            plane[idx] = src[k * ldy + l];
+        }
+    } else {
+        for (int i0 = tid; i0 < K2 * K1h; i0 += LQ * bt) {
+            T2 v[LQ];
+#pragma unroll
+            for (int q = 0; q < LQ; ++q)
+                if (i0 + q * bt < K2 * K1h) v[q] = plane[i0 + q * bt];
+#pragma unroll
+            for (int q = 0; q < LQ; ++q) {
+                const int idx = i0 + q * bt;
+                if (idx < K2 * K1h) { const int l = idx / K1h; src[(idx - l * K1h) * ldy + l] = v[q]; }
+            }
+        }
+        __syncthreads();
+        FftStages<T, T2, NY>::run(src, dst, K1h, K2, py, T(1), twy);
+        for (int idx = tid; idx < K2 * N; idx += bt) {
+            const int l = idx / N, k = idx - l * N;
+            const T2 yk = src[k * ldy + l];
+            T2 yc = src[(N - k) * ldy + l];
+            yc.y = -yc.y;
+            const T2 a = cadd(yk, yc);
+            T2 t = tw2[k];
+            t.y = -t.y;                                           // exp(+2 pi i k / K1)
+            const T2 b = cmul(csub(yk, yc), t);
+            T2 z; z.x = a.x - b.y; z.y = a.y + b.x;               // A + iB
+            dst[l * ldx + k] = z;
+        }
+        __syncthreads();
+        { T2* s = src; src = dst; dst = s; }
+        FftStages<T, T2, NX>::run(src, dst, K2, N, px, T(1), twx);
+        T2* const out = (T2*)((T*)real + (size_t)blockIdx.x * K2 * K1);   // K1 even: pairs are aligned
+        for (int idx = tid; idx < K2 * N; idx += bt) {
+            const int l = idx / N;
+            out[idx] = src[l * ldx + idx - l * N];
         }
     }
 }
@@ -978,6 +1120,49 @@ static pgk_status fft_rx_pass(pgk_ctx* c) {
     return PGK_OK;
 }
 
+// shared memory of a plane's block
+template <typename T>
+static size_t plane_smem(const pgk_ctx* c) {
+    const size_t n = c->K[0] / 2;
+    return (2 * (n + 1) * (c->K[1] + 1) + 2 * n + 1 + c->K[1]) * sizeof(typename C2<T>::t);
+}
+// the planes run in one launch of whole planes: they fit an SM's shared memory
+// and all of them are resident at once (a second wave costs more than the pass
+// it saves: 150^3, FP32, one block per SM, 84 us forward, where the two passes
+// of 144 x 144 x 150 take 23 + 27)
+template <typename T>
+static bool plane_fits(const pgk_ctx* c) {
+    if (!c->r2c) return false;
+    const size_t sm = plane_smem<T>(c), limit = 227 * 1024;
+    return sm <= limit && c->K[2] <= c->nsm * std::max<int>(1, std::min<int>(2048 / PLANE_BT, (int)(limit / (sm + 1024))));
+}
+template <typename T, int SRC, int NX, int NY, bool FWD>
+static void plane_launch(pgk_ctx* c, const FftDev& px, const FftDev& py) {
+    typedef typename C2<T>::t T2;
+    const size_t sm = plane_smem<T>(c);
+    smem_limit(k_fft_plane<T, SRC, NX, NY, FWD>, sm);
+    launch_pdl(k_fft_plane<T, SRC, NX, NY, FWD>, c->K[2], c->fft_p[5], sm, c->st, (T2*)c->qc,
+               FWD ? (void*)c->qacc : (void*)c->qr, c->K[0], c->K[1], px, py, c->tw_rx);
+}
+template <typename T, int SRC, bool FWD>
+static pgk_status fft_plane_pass(pgk_ctx* c) {
+    auto dev = [](const FftPlan& pl) {
+        FftDev d;
+        d.n = pl.n; d.nstage = pl.nstage;
+        for (int s = 0; s < PGK_MAX_RADIX_STAGES; ++s) d.radix[s] = pl.radix[s];
+        d.tw = pl.tw;
+        return d;
+    };
+    const FftDev px = dev(c->plan_rx), py = dev(c->plan[1]);
+    if (px.n == 16 && py.n == 32) plane_launch<T, SRC, 16, 32, FWD>(c, px, py);
+    else if (px.n == 32 && py.n == 64) plane_launch<T, SRC, 32, 64, FWD>(c, px, py);
+    else if (px.n == 64 && py.n == 128) plane_launch<T, SRC, 64, 128, FWD>(c, px, py);
+    else plane_launch<T, SRC, 0, 0, FWD>(c, px, py);
+    PGK_LAUNCHED(c);
+    PGK_CUDA(c, cudaGetLastError());
+    return PGK_OK;
+}
+
 template <typename T>
 static pgk_status fft3(pgk_ctx* c, int sign, bool first) {
     pgk_status s;
@@ -1004,6 +1189,11 @@ static pgk_status fft_convolve(pgk_ctx* c, long long* acc, int want) {
     if (c->r2c) {
         const int xh = c->K[0] / 2 + 1;
         ca.K1f = c->K[0];
+        if (c->fft_p[5] > 0) {
+            s = sizeof(T) == 4 ? fft_plane_pass<T, 1, true>(c) : fft_plane_pass<T, 2, true>(c);
+            if (s || (s = fft_pass<T, 2, 0, true>(c, -1, &ca, xh))) return s;
+            return fft_plane_pass<T, 0, false>(c);
+        }
         if (sizeof(T) == 4) s = fft_rx_pass<T, 1, true>(c);
         else s = fft_rx_pass<T, 2, true>(c);
         if (s) return s;
@@ -1025,8 +1215,9 @@ static pgk_status fft_convolve(pgk_ctx* c, long long* acc, int want) {
 // Pencils per block of each axis pass (and of the z pass with the influence
 // function) decide how many blocks a pass has: many pencils per block suit
 // large grids, few suit the small grids of small replicas, whose SPME chain
-// is latency-bound.  Every pencil is transformed on its own, so the results
-// do not depend on the choice.  Each candidate (powers of two that fit the
+// is latency-bound.  A plane's block of 128 to 512 threads replaces the x and y
+// passes where its measured time is below theirs.  Every pencil is transformed
+// on its own, so the results do not depend on the choice.  Each candidate (powers of two that fit the
 // shared memory) is timed with CUDA events on the context's stream over a
 // few launches on the context's grid; the fastest is kept per (grid shape,
 // precision) for the whole process and listed by pgk_tuning_table.
@@ -1036,7 +1227,7 @@ struct TuneKey {
         return std::tie(k1, k2, k3, fp32) < std::tie(o.k1, o.k2, o.k3, o.fp32);
     }
 };
-struct TuneVal { int p[5]; float us[5]; };
+struct TuneVal { int p[6]; float us[6]; };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneVal> g_tune;
 
@@ -1105,6 +1296,39 @@ static pgk_status tune_rx(pgk_ctx* c, int& best, float& best_us) {
     return PGK_OK;
 }
 
+// threads of a plane's block (the mean of both directions), 0 where the two
+// passes that it stands for are faster or the plane does not fit
+template <typename T>
+static pgk_status tune_plane(pgk_ctx* c, TuneVal& v) {
+    v.p[5] = 0; v.us[5] = 0.f;
+    if (!plane_fits<T>(c)) return PGK_OK;
+    cudaEvent_t e0, e1;
+    PGK_CUDA(c, cudaEventCreate(&e0));
+    PGK_CUDA(c, cudaEventCreate(&e1));
+    float best = v.us[4] + v.us[1];
+    for (int bt = 128; bt <= PLANE_BT; bt *= 2) {
+        c->fft_p[5] = bt;
+        pgk_status s = PGK_OK;
+        for (int r = 0; r < 4 && !s; ++r) {
+            if (r == 1) PGK_CUDA(c, cudaEventRecord(e0, c->st));          // r 0: warm-up (and smem limit)
+            s = sizeof(T) == 4 ? fft_plane_pass<T, 1, true>(c) : fft_plane_pass<T, 2, true>(c);
+            if (!s) s = fft_plane_pass<T, 0, false>(c);
+        }
+        if (s) return s;
+        PGK_CUDA(c, cudaEventRecord(e1, c->st));
+        PGK_CUDA(c, cudaEventSynchronize(e1));
+        float ms = 0.f;
+        PGK_CUDA(c, cudaEventElapsedTime(&ms, e0, e1));
+        const float us = ms * 1e3f / 6.f;
+        if (v.us[5] == 0.f || us < v.us[5]) v.us[5] = us;
+        if (us < best) { best = us; v.p[5] = bt; }
+    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    c->fft_p[5] = v.p[5];
+    return PGK_OK;
+}
+
 template <typename T>
 static pgk_status autotune_fft(pgk_ctx* c, TuneVal& v) {
     pgk_status s;
@@ -1116,16 +1340,20 @@ static pgk_status autotune_fft(pgk_ctx* c, TuneVal& v) {
         return s;
     v.p[4] = 0; v.us[4] = 0.f;
     if (c->r2c && (s = tune_rx<T>(c, v.p[4], v.us[4]))) return s;
-    return PGK_OK;
+    return tune_plane<T>(c, v);
 }
 
 // launch shapes of this context's SPME passes: the process-wide choice for
 // its grid shape, measured now if there is none yet (PGK_AUTOTUNE=0: the
 // fixed defaults).  Runs at context set-up, outside any stream capture.
 pgk_status spme_autotune(pgk_ctx* c) {
-    for (int q = 0; q < 5; ++q) c->fft_p[q] = 0;
+    for (int q = 0; q < 6; ++q) c->fft_p[q] = 0;
+    if (!c->prm.ifspme) return PGK_OK;
     const char* env = getenv("PGK_AUTOTUNE");
-    if ((env && atoi(env) == 0) || !c->prm.ifspme) return PGK_OK;
+    if (env && atoi(env) == 0) {
+        if (c->mixed() ? plane_fits<float>(c) : plane_fits<double>(c)) c->fft_p[5] = PLANE_BT;
+        return PGK_OK;
+    }
     const TuneKey key{c->K[0], c->K[1], c->K[2], (c->mixed() ? 1 : 0) | (c->r2c ? 2 : 0)};
     std::lock_guard<std::mutex> lk(g_tune_mu);     // contexts of one grid shape share one measurement
     auto it = g_tune.find(key);
@@ -1139,7 +1367,7 @@ pgk_status spme_autotune(pgk_ctx* c) {
         PGK_CUDA(c, cudaStreamSynchronize(c->st));
         it = g_tune.emplace(key, v).first;
     }
-    for (int q = 0; q < 5; ++q) c->fft_p[q] = it->second.p[q];
+    for (int q = 0; q < 6; ++q) c->fft_p[q] = it->second.p[q];
     return PGK_OK;
 }
 
@@ -1149,8 +1377,10 @@ extern "C" int64_t pgk_tuning_table(char* buf, int64_t cap) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         for (auto& kv : g_tune) {
             char line[256];
-            char rx[64] = "";
-            if (kv.first.fp32 & 2) snprintf(rx, sizeof(rx), " real-x %d (%.1f us)", kv.second.p[4], kv.second.us[4]);
+            char rx[96] = "";
+            if (kv.first.fp32 & 2)
+                snprintf(rx, sizeof(rx), " real-x %d (%.1f us) plane threads %d (%.1f us)", kv.second.p[4],
+                         kv.second.us[4], kv.second.p[5], kv.second.us[5]);
             snprintf(line, sizeof(line),
                      "spme %dx%dx%d %s: pencils per block x %d (%.1f us) y %d (%.1f us) z %d (%.1f us) "
                      "z+influence %d (%.1f us)%s\n",

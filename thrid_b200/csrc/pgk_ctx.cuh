@@ -189,7 +189,9 @@ struct pgk_ctx {
     bool r2c = false;
     FftPlan plan_rx;
     void* tw_rx = nullptr;
-    int fft_p[5] = {0, 0, 0, 0, 0};  // pencils per block: x, y, z, z+influence, real x (0: default)
+    // pencils per block: x, y, z, z+influence, real x (0: default); threads of a
+    // plane's block (0: x and y in passes of their own)
+    int fft_p[6] = {0, 0, 0, 0, 0, 0};
 
     // ---- Morse pairs (k_morse.cu): own list (radius rcut_bookmor) and kernel ----
     int nmor = 0;                 // Morse atoms (0: no Morse pairs or Morse switched off)
