@@ -172,38 +172,20 @@ struct FftDev {
     const void* tw;
 };
 
-template <typename T, typename T2>
-__device__ __forceinline__ void dft4(T2* v, T sg) {
-    T2 a0 = v[0], a1 = v[1], a2 = v[2], a3 = v[3];
-    T2 s02 = cadd(a0, a2), d02 = csub(a0, a2), s13 = cadd(a1, a3), d13 = csub(a1, a3);
-    v[0] = cadd(s02, s13);
-    v[2] = csub(s02, s13);
-    T2 t = mul_i<T2, T>(d13, sg);
-    v[1] = cadd(d02, t);
-    v[3] = csub(d02, t);
-}
-
-template <typename T, typename T2>
-__device__ __forceinline__ void dft_r(T2* v, int R, T sg) {
-    if (R == 2) {
+template <typename T, typename T2, int R>
+__device__ __forceinline__ void dft_r(T2 (&v)[R], T sg) {
+    if constexpr (R == 2) {
         T2 a = v[0], b = v[1];
         v[0] = cadd(a, b); v[1] = csub(a, b);
-    } else if (R == 4) {
-        dft4<T, T2>(v, sg);
-    } else if (R == 8) {
-        const T s = T(0.70710678118654752440);
-        T2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-        dft4<T, T2>(e, sg);
-        dft4<T, T2>(o, sg);
-        T2 w1, w3;                               // o1 exp(sg i pi / 4), o3 exp(3 sg i pi / 4)
-        w1.x = s * (o[1].x - sg * o[1].y); w1.y = s * (o[1].y + sg * o[1].x);
-        w3.x = -s * (o[3].x + sg * o[3].y); w3.y = s * (sg * o[3].x - o[3].y);
-        const T2 w2 = mul_i<T2, T>(o[2], sg);
-        v[0] = cadd(e[0], o[0]); v[4] = csub(e[0], o[0]);
-        v[1] = cadd(e[1], w1); v[5] = csub(e[1], w1);
-        v[2] = cadd(e[2], w2); v[6] = csub(e[2], w2);
-        v[3] = cadd(e[3], w3); v[7] = csub(e[3], w3);
-    } else if (R == 3) {
+    } else if constexpr (R == 4) {
+        T2 a0 = v[0], a1 = v[1], a2 = v[2], a3 = v[3];
+        T2 s02 = cadd(a0, a2), d02 = csub(a0, a2), s13 = cadd(a1, a3), d13 = csub(a1, a3);
+        v[0] = cadd(s02, s13);
+        v[2] = csub(s02, s13);
+        T2 t = mul_i<T2, T>(d13, sg);
+        v[1] = cadd(d02, t);
+        v[3] = csub(d02, t);
+    } else if constexpr (R == 3) {
         const T s60 = T(0.86602540378443864676);
         T2 a0 = v[0], a1 = v[1], a2 = v[2];
         T2 t1 = cadd(a1, a2);
@@ -212,7 +194,7 @@ __device__ __forceinline__ void dft_r(T2* v, int R, T sg) {
         v[0] = cadd(a0, t1);
         v[1] = cadd(t2, t3);
         v[2] = csub(t2, t3);
-    } else if (R == 5) {
+    } else if constexpr (R == 5) {
         const T c72 = T(0.30901699437494742410), s72 = T(0.95105651629515357212);
         const T c144 = T(-0.80901699437494742410), s144 = T(0.58778525229247312917);
         T2 a0 = v[0];
@@ -231,10 +213,13 @@ __device__ __forceinline__ void dft_r(T2* v, int R, T sg) {
     }
 }
 
-// radix chain of a compile-time length (8s where they save a stage, 4s, then
-// 2, 3, 5)
+// radix chain of a length (4s, then 2, 3, 5), the same at compile time and in
+// factor(): the passes and the planes, compiled or not, then round alike, and
+// the launch shape that a timing picks does not change the results.  (Radix 8
+// in some lengths' compiled forms broke that, for 64 us instead of 68 of a
+// 128^3 FP32 convolution and nothing at 64^3 and below.)
 __host__ __device__ constexpr int pick_radix(int m) {
-    return m % 8 == 0 && m != 16 ? 8 : m % 4 == 0 ? 4 : (m % 2 == 0 ? 2 : (m % 3 == 0 ? 3 : (m % 5 == 0 ? 5 : 0)));
+    return m % 4 == 0 ? 4 : (m % 2 == 0 ? 2 : (m % 3 == 0 ? 3 : (m % 5 == 0 ? 5 : 0)));
 }
 __host__ __device__ constexpr int stage_radix(int n, int s) {
     int m = n;
@@ -252,20 +237,16 @@ __host__ __device__ constexpr int nstages(int n) {
     return c;
 }
 
-// registers of a stage's points (RM of fft_stage)
-__host__ __device__ constexpr int stage_rm(int n, int s) { return s < nstages(n) && stage_radix(n, s) > 5 ? 8 : 5; }
-
 // one Stockham stage on P pencils of length n held in shared memory
 // Pencils are stored with pitch ld = n + 1 elements, and consecutive threads
 // take consecutive pencils at one place j: with n even the stage's strided
 // loads and stores fall into different shared-memory banks, and a twiddle
 // factor is one broadcast.  Measured, 128^3 FP32 convolution in five
-// passes: 97 us with consecutive threads on consecutive j and radix 4, 96 with
-// radix 8, 89 with the pencils first, 84 with both.
-// RM: the largest radix
-template <typename T, typename T2, int RM>
-__device__ __forceinline__ void fft_stage(const T2* __restrict__ src, T2* __restrict__ dst, int P, int n, int R,
-                                          int Ns, const T2* __restrict__ tw, T sg) {
+// passes: 97 us with consecutive threads on consecutive j, 89 with the pencils
+// first.  R is a constant in every caller, so that the points stay in registers.
+template <typename T, typename T2, int R>
+__device__ __forceinline__ void fft_stage(const T2* __restrict__ src, T2* __restrict__ dst, int P, int n, int Ns,
+                                          const T2* __restrict__ tw, T sg) {
     const int ld = n + 1;
     const int nr = n / R;
     const int twstep = n / (Ns * R);
@@ -273,25 +254,23 @@ __device__ __forceinline__ void fft_stage(const T2* __restrict__ src, T2* __rest
     int j = threadIdx.x / P, p = threadIdx.x - j * P;
     while (j < nr) {
         int k = j % Ns;
-        T2 v[RM];
+        T2 v[R];
         const T2* sp = src + p * ld;
 #pragma unroll
-        for (int r = 0; r < RM; ++r)
-            if (r < R) {
-                T2 x = sp[j + r * nr];
-                if (r > 0 && k > 0) {
-                    T2 t = tw[r * k * twstep];
-                    if (sg > 0) t.y = -t.y;
-                    x = cmul(x, t);
-                }
-                v[r] = x;
+        for (int r = 0; r < R; ++r) {
+            T2 x = sp[j + r * nr];
+            if (r > 0 && k > 0) {
+                T2 t = tw[r * k * twstep];
+                if (sg > 0) t.y = -t.y;
+                x = cmul(x, t);
             }
-        dft_r<T, T2>(v, R, sg);
+            v[r] = x;
+        }
+        dft_r<T, T2, R>(v, sg);
         int o = (j / Ns) * Ns * R + k;
         T2* dpn = dst + p * ld;
 #pragma unroll
-        for (int r = 0; r < RM; ++r)
-            if (r < R) dpn[o + r * Ns] = v[r];
+        for (int r = 0; r < R; ++r) dpn[o + r * Ns] = v[r];
         j += dj;
         p += dp;
         if (p >= P) { p -= P; ++j; }
@@ -303,16 +282,21 @@ template <typename T, typename T2, int NC, int S = 0>
 struct FftStages {
     static __device__ __forceinline__ void run(T2*& src, T2*& dst, int P, int n, const FftDev& plan, T sg,
                                                const T2* tw) {
-        if (NC == 0) {
+        if constexpr (NC == 0) {
             int Ns = 1;
             for (int s = 0; s < plan.nstage; ++s) {
-                fft_stage<T, T2, 5>(src, dst, P, n, plan.radix[s], Ns, tw, sg);
+                switch (plan.radix[s]) {             // block-uniform
+                    case 4: fft_stage<T, T2, 4>(src, dst, P, n, Ns, tw, sg); break;
+                    case 2: fft_stage<T, T2, 2>(src, dst, P, n, Ns, tw, sg); break;
+                    case 3: fft_stage<T, T2, 3>(src, dst, P, n, Ns, tw, sg); break;
+                    default: fft_stage<T, T2, 5>(src, dst, P, n, Ns, tw, sg); break;
+                }
                 __syncthreads();
                 T2* t = src; src = dst; dst = t;
                 Ns *= plan.radix[s];
             }
-        } else if (S < nstages(NC)) {
-            fft_stage<T, T2, stage_rm(NC, S)>(src, dst, P, NC, stage_radix(NC, S), stage_ns(NC, S), tw, sg);
+        } else if constexpr (S < nstages(NC)) {
+            fft_stage<T, T2, stage_radix(NC, S)>(src, dst, P, NC, stage_ns(NC, S), tw, sg);
             __syncthreads();
             T2* t = src; src = dst; dst = t;
             FftStages<T, T2, NC, (S < 12 ? S + 1 : S)>::run(src, dst, P, n, plan, sg, tw);
@@ -418,8 +402,8 @@ __device__ __forceinline__ float conv_point_f(int k1, int k2, int k3, int K1, in
 //      and backward z transform in one pass over the grid.
 template <typename T, int AXIS, int SRC, int NC, bool CONV>
 __global__ void __launch_bounds__(256) k_fft(typename C2<T>::t* __restrict__ data, const void* __restrict__ acc,
-                                             int K1, int K2, int K3, FftDev plan, int P, T sg, ConvArgs ca,
-                                             const DynState* __restrict__ dyn) {
+                                             int K1, int K2, int K3, const __grid_constant__ FftDev plan, int P,
+                                             T sg, ConvArgs ca, const DynState* __restrict__ dyn) {
     typedef typename C2<T>::t T2;
     extern __shared__ unsigned char smraw[];
     T2* bufA = (T2*)smraw;
@@ -556,7 +540,7 @@ __global__ void __launch_bounds__(256) k_fft(typename C2<T>::t* __restrict__ dat
 // fixed-point accumulation grid, 2 = double accumulation grid.
 template <typename T, int SRC, int NC, bool FWD>
 __global__ void __launch_bounds__(256) k_fft_rx(typename C2<T>::t* __restrict__ data, void* __restrict__ real,
-                                                int K1, int nline, FftDev plan, const void* __restrict__ tw2g,
+                                                int K1, int nline, const __grid_constant__ FftDev plan, const void* __restrict__ tw2g,
                                                 int P) {
     typedef typename C2<T>::t T2;
     extern __shared__ unsigned char smraw[];
@@ -645,12 +629,16 @@ __global__ void __launch_bounds__(256) k_fft_rx(typename C2<T>::t* __restrict__ 
 // pass over the grid instead of two.  The stages and their order are those of
 // the separate passes.
 // Bound by latency at one or two blocks per SM (each stage is a trip through
-// shared memory and a barrier).  Measured, whole convolution, FP32, against five
-// passes: 32^3 21 us (27), 64^3 31 (33), 64 x 64 x 192 41 (58), 128^3 64 (84);
-// FP64 64^3 30 (40).  A step of 1,536 water atoms 49 -> 47 us.
+// shared memory and a barrier).  Measured, whole convolution, FP32, default
+// shapes, against five passes: 32^3 20 us (36), 48^3 33 (49), 64^3 30 (48),
+// 64 x 48 x 64 30 (46), 64 x 64 x 192 43 (60), 128^3 68 (88); FP64 64^3 32 (40),
+// 128^3 does not fit.  With each axis compiled by itself a plane of two unlike
+// lengths costs what its axes do (64 x 48 x 64 37 us with one generic form for
+// both).
 template <typename T, int SRC, int NX, int NY, bool FWD>
 __global__ void __launch_bounds__(PLANE_BT) k_fft_plane(typename C2<T>::t* __restrict__ data, void* __restrict__ real,
-                                                       int K1, int K2_, FftDev px, FftDev py,
+                                                       int K1, int K2_, const __grid_constant__ FftDev px,
+                                                       const __grid_constant__ FftDev py,
                                                        const void* __restrict__ tw2g) {
     typedef typename C2<T>::t T2;
     extern __shared__ unsigned char smraw[];
@@ -946,8 +934,7 @@ static bool factor(int n, FftPlan& pl) {
     pl.n = n; pl.nstage = 0;
     int m = n;
     while (m > 1) {
-        int r = 0;
-        for (int c : {4, 2, 3, 5}) if (m % c == 0) { r = c; break; }
+        const int r = pick_radix(m);
         if (r == 0 || pl.nstage >= PGK_MAX_RADIX_STAGES) return false;
         pl.radix[pl.nstage++] = r;
         m /= r;
@@ -1144,6 +1131,17 @@ static void plane_launch(pgk_ctx* c, const FftDev& px, const FftDev& py) {
     launch_pdl(k_fft_plane<T, SRC, NX, NY, FWD>, c->K[2], c->fft_p[5], sm, c->st, (T2*)c->qc,
                FWD ? (void*)c->qacc : (void*)c->qr, c->K[0], c->K[1], px, py, c->tw_rx);
 }
+template <typename T, int SRC, int NX, bool FWD>
+static void plane_launch_y(pgk_ctx* c, const FftDev& px, const FftDev& py) {
+    switch (py.n) {
+        case 32: plane_launch<T, SRC, NX, 32, FWD>(c, px, py); break;
+        case 64: plane_launch<T, SRC, NX, 64, FWD>(c, px, py); break;
+        case 128: plane_launch<T, SRC, NX, 128, FWD>(c, px, py); break;
+        case 192: plane_launch<T, SRC, NX, 192, FWD>(c, px, py); break;
+        default: plane_launch<T, SRC, NX, 0, FWD>(c, px, py); break;
+    }
+}
+// SRC: the forward pass's grid (1 int64, 2 double), 0 for the inverse
 template <typename T, int SRC, bool FWD>
 static pgk_status fft_plane_pass(pgk_ctx* c) {
     auto dev = [](const FftPlan& pl) {
@@ -1154,10 +1152,13 @@ static pgk_status fft_plane_pass(pgk_ctx* c) {
         return d;
     };
     const FftDev px = dev(c->plan_rx), py = dev(c->plan[1]);
-    if (px.n == 16 && py.n == 32) plane_launch<T, SRC, 16, 32, FWD>(c, px, py);
-    else if (px.n == 32 && py.n == 64) plane_launch<T, SRC, 32, 64, FWD>(c, px, py);
-    else if (px.n == 64 && py.n == 128) plane_launch<T, SRC, 64, 128, FWD>(c, px, py);
-    else plane_launch<T, SRC, 0, 0, FWD>(c, px, py);
+    // each axis by itself: the lengths that the separate passes compile
+    switch (px.n) {
+        case 16: plane_launch_y<T, SRC, 16, FWD>(c, px, py); break;
+        case 32: plane_launch_y<T, SRC, 32, FWD>(c, px, py); break;
+        case 64: plane_launch_y<T, SRC, 64, FWD>(c, px, py); break;
+        default: plane_launch_y<T, SRC, 0, FWD>(c, px, py); break;
+    }
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;
@@ -1190,7 +1191,7 @@ static pgk_status fft_convolve(pgk_ctx* c, long long* acc, int want) {
         const int xh = c->K[0] / 2 + 1;
         ca.K1f = c->K[0];
         if (c->fft_p[5] > 0) {
-            s = sizeof(T) == 4 ? fft_plane_pass<T, 1, true>(c) : fft_plane_pass<T, 2, true>(c);
+            s = fft_plane_pass<T, sizeof(T) == 4 ? 1 : 2, true>(c);
             if (s || (s = fft_pass<T, 2, 0, true>(c, -1, &ca, xh))) return s;
             return fft_plane_pass<T, 0, false>(c);
         }
@@ -1217,7 +1218,8 @@ static pgk_status fft_convolve(pgk_ctx* c, long long* acc, int want) {
 // large grids, few suit the small grids of small replicas, whose SPME chain
 // is latency-bound.  A plane's block of 128 to 512 threads replaces the x and y
 // passes where its measured time is below theirs.  Every pencil is transformed
-// on its own, so the results do not depend on the choice.  Each candidate (powers of two that fit the
+// on its own by the same radix chain in every form (pick_radix), so the results
+// do not depend on the choice.  Each candidate (powers of two that fit the
 // shared memory) is timed with CUDA events on the context's stream over a
 // few launches on the context's grid; the fastest is kept per (grid shape,
 // precision) for the whole process and listed by pgk_tuning_table.
@@ -1311,7 +1313,7 @@ static pgk_status tune_plane(pgk_ctx* c, TuneVal& v) {
         pgk_status s = PGK_OK;
         for (int r = 0; r < 4 && !s; ++r) {
             if (r == 1) PGK_CUDA(c, cudaEventRecord(e0, c->st));          // r 0: warm-up (and smem limit)
-            s = sizeof(T) == 4 ? fft_plane_pass<T, 1, true>(c) : fft_plane_pass<T, 2, true>(c);
+            s = fft_plane_pass<T, sizeof(T) == 4 ? 1 : 2, true>(c);
             if (!s) s = fft_plane_pass<T, 0, false>(c);
         }
         if (s) return s;
@@ -1349,9 +1351,12 @@ static pgk_status autotune_fft(pgk_ctx* c, TuneVal& v) {
 pgk_status spme_autotune(pgk_ctx* c) {
     for (int q = 0; q < 6; ++q) c->fft_p[q] = 0;
     if (!c->prm.ifspme) return PGK_OK;
+    const bool fits = c->mixed() ? plane_fits<float>(c) : plane_fits<double>(c);
     const char* env = getenv("PGK_AUTOTUNE");
+    const char* pe = getenv("PGK_FFT_PLANE");      // 0: separate passes; 1: planes where they fit; unset: the faster
+    const int force = pe ? (atoi(pe) != 0 && fits ? PLANE_BT : 0) : -1;
     if (env && atoi(env) == 0) {
-        if (c->mixed() ? plane_fits<float>(c) : plane_fits<double>(c)) c->fft_p[5] = PLANE_BT;
+        c->fft_p[5] = force >= 0 ? force : (fits ? PLANE_BT : 0);
         return PGK_OK;
     }
     const TuneKey key{c->K[0], c->K[1], c->K[2], (c->mixed() ? 1 : 0) | (c->r2c ? 2 : 0)};
@@ -1368,6 +1373,7 @@ pgk_status spme_autotune(pgk_ctx* c) {
         it = g_tune.emplace(key, v).first;
     }
     for (int q = 0; q < 6; ++q) c->fft_p[q] = it->second.p[q];
+    if (force >= 0) c->fft_p[5] = force;
     return PGK_OK;
 }
 
