@@ -490,7 +490,9 @@ pgk_status pgk_bench_kernel(pgk_ctx* ctx, int32_t which, int32_t iters, double* 
  * keeps its state resident in its own context and non-blocking CUDA stream;
  * one host worker per slot runs it (captured step graphs), so the replicas'
  * kernels overlap on the device.  In mixed precision a replica's results are
- * bit-identical to a run of it alone (integer force sums, private buffers).
+ * bit-identical to a run of it alone in a server (integer force sums, private
+ * buffers, one order of the sums in a row); a context of its own may round
+ * differently.
  * The server copies every input at submit. */
 typedef struct pgk_server pgk_server;
 typedef struct pgk_request {

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
 // Rows are cut into segments until 16 warps per SM have work (small boxes).
 struct FluxPairArgs {
     const int* rows; const int* cnt; int ccap; int ncl; int nseg;
-    int pruned;                  // rows, cnt: nseg segments of ccap entries per cluster, else whole rows
+    int cut;                     // rows, cnt: nseg segments of ccap entries per cluster, else whole rows
     const int* typ_s; const int* perm; int ntyp;
     const double* zs; const int* ms; const void* vs; const uint4* bs;
     double rrcut, rr2, rl2, rmax2;
@@ -261,11 +261,11 @@ k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPai
     const long long nunit = (long long)a.ncl * a.nseg;
     for (long long u = blockIdx.x * 4 + w; u < nunit; u += gridDim.x * 4) {
         const int cl = (int)(u / a.nseg), seg = (int)(u - (long long)cl * a.nseg);
-        const int cnt = a.cnt[a.pruned ? u : cl];
-        const int chunk = a.pruned ? cnt : ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
-        const int k_lo = a.pruned ? 0 : seg * chunk, k_hi = min(cnt, k_lo + chunk);
+        const int cnt = a.cnt[a.cut ? u : cl];
+        const int chunk = a.cut ? cnt : ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
+        const int k_lo = a.cut ? 0 : seg * chunk, k_hi = min(cnt, k_lo + chunk);
         if (k_lo >= k_hi) continue;                       // warp-uniform
-        const int* __restrict__ row = a.rows + (size_t)(a.pruned ? u : cl) * a.ccap;
+        const int* __restrict__ row = a.rows + (size_t)(a.cut ? u : cl) * a.ccap;
         __syncwarp();
         if (lane < 8) {
             const int s = 8 * cl + lane;
@@ -499,11 +499,11 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
     const long long nunit = (long long)a.ncl * a.nseg;
     for (long long u = blockIdx.x * 4 + w; u < nunit; u += gridDim.x * 4) {
         const int cl = (int)(u / a.nseg), seg = (int)(u - (long long)cl * a.nseg);
-        const int cnt = a.cnt[a.pruned ? u : cl];
-        const int chunk = a.pruned ? cnt : ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
-        const int k_lo = a.pruned ? 0 : seg * chunk, k_hi = min(cnt, k_lo + chunk);
+        const int cnt = a.cnt[a.cut ? u : cl];
+        const int chunk = a.cut ? cnt : ((cnt + a.nseg - 1) / a.nseg + 31) & ~31;
+        const int k_lo = a.cut ? 0 : seg * chunk, k_hi = min(cnt, k_lo + chunk);
         if (k_lo >= k_hi) continue;                       // warp-uniform
-        const int* __restrict__ row = a.rows + (size_t)(a.pruned ? u : cl) * a.ccap;
+        const int* __restrict__ row = a.rows + (size_t)(a.cut ? u : cl) * a.ccap;
         __syncwarp();
         if (lane < 8) {
             const int s = 8 * cl + lane;
@@ -926,6 +926,7 @@ pgk_status hf_setup(pgk_ctx* c, const pgk_hfparams* p) {
     PGK_CUDA(c, pgk_dmalloc(c, &c->lt_reg, sizeof(int) * n));
     PGK_CUDA(c, cudaMemsetAsync(c->lt_reg, 0xff, sizeof(int) * n, c->st));
     c->hf_set = true;
+    if (nreg > 0 && (s = keep_plain_order(c))) return s;
     if (c->hfp.nlangeregion > 0 && (s = launch_lt_regist(c))) return s;
     PGK_CUDA(c, cudaStreamSynchronize(c->st));
     return PGK_OK;
@@ -1008,9 +1009,10 @@ static bool flux_pair_on(const pgk_ctx* c) {
 // pruned: this step's pair kernel has left its rows (c->plist)
 static FluxPairArgs flux_pair_args(pgk_ctx* c, bool pruned) {
     FluxPairArgs a;
-    a.pruned = pruned && c->prune_buffer > 0.f;
-    a.rows = a.pruned ? c->plist : c->clist; a.cnt = a.pruned ? c->pcnt : c->ccnt;
-    a.ccap = a.pruned ? c->pcap : c->ccap; a.ncl = c->ncl;
+    pruned = pruned && c->prune_buffer > 0.f;
+    a.cut = pruned && c->pseg > 1;
+    a.rows = pruned ? c->plist : c->clist; a.cnt = pruned ? c->pcnt : c->ccnt;
+    a.ccap = pruned ? c->pcap : c->ccap; a.ncl = c->ncl;
     a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
     a.zs = c->hf_zs; a.ms = c->hf_ms; a.vs = c->hf_vs; a.bs = c->hf_bs;
     a.rrcut = c->prm.rrcut;
@@ -1018,7 +1020,7 @@ static FluxPairArgs flux_pair_args(pgk_ctx* c, bool pruned) {
     a.rl2 = c->prm.rcut * c->prm.rcut;
     a.rmax2 = std::max(a.rr2, a.rl2);
     // about 16 warps per SM, in row segments where the clusters alone are fewer
-    a.nseg = a.pruned ? c->pseg : std::max(1, std::min(8, c->nsm * 16 / std::max(a.ncl, 1)));
+    a.nseg = a.cut ? c->pseg : std::max(1, std::min(8, c->nsm * 16 / std::max(a.ncl, 1)));
     return a;
 }
 static int flux_pair_grid(const pgk_ctx* c, const FluxPairArgs& a) {

@@ -927,7 +927,109 @@ __device__ __forceinline__ void rattle_group(const int (&at)[G::NA], const doubl
     if (!finished) atomicOr(status, POS ? ST_RATTLE_NOCONV : ST_RATTLEV_NOCONV);
 }
 
-template <bool POS>
+// The same sweeps in the reference's plain form, every term formed where it is
+// used (k_rattle_warp's arithmetic in registers): for contexts whose positions
+// must not move by a rounding (pgk_ctx::plain_order).  512 waters 18.0 + 12.6 us.
+template <bool POS, class G>
+__device__ __forceinline__ void rattle_group_plain(const int (&at)[G::NA], const double (&dd)[G::K],
+                                                   double* __restrict__ pos, double* __restrict__ vel,
+                                                   const double* __restrict__ old, const double* __restrict__ invm,
+                                                   double eps, double dt, const double (&rvi)[3], unsigned* status) {
+    constexpr int NA = G::NA, K = G::K;
+    double X[NA][3], V[NA][3], O[NA][3], IM[NA], RC[K];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        IM[a] = invm[at[a]];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            X[a][d] = pos[3 * (size_t)at[a] + d];
+            V[a][d] = vel[3 * (size_t)at[a] + d];
+            O[a][d] = POS ? old[3 * (size_t)at[a] + d] : 0.0;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < K; ++q) RC[q] = POS ? 1.0 / dd[q] : 1.0 / (dd[q] * (IM[G::i(q)] + IM[G::j(q)]));
+    bool finished = false;
+    if (POS) {
+        for (int it = 0; it < 300 && !finished; ++it) {
+            finished = true;
+#pragma unroll
+            for (int q = 0; q < K; ++q) {
+                const int ib = G::i(q), jb = G::j(q);
+                const double d2 = dd[q];
+                const double R0 = X[ib][0] - X[jb][0], R1 = X[ib][1] - X[jb][1], R2 = X[ib][2] - X[jb][2];
+                const double Rsq = R0 * R0 + R1 * R1 + R2 * R2;
+                const double delta = fabs(Rsq - d2) * RC[q];      // |r^2 - d^2| / d^2
+                if (delta < eps) continue;
+                finished = false;
+                const double O0 = O[ib][0] - O[jb][0], O1 = O[ib][1] - O[jb][1], O2 = O[ib][2] - O[jb][2];
+                const double RR = R0 * O0 + R1 * O1 + R2 * O2;
+                const double mi = IM[ib], mj = IM[jb];
+                const double gij = (Rsq - d2) / (2.0 * RR * (mi + mj) * dt);
+                const double F[3] = {gij * O0, gij * O1, gij * O2};
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    X[ib][d] = X[ib][d] - mi * F[d] * dt;
+                    X[jb][d] = X[jb][d] + mj * F[d] * dt;
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const double Fv = F[d] * rvi[d];
+                    V[ib][d] = V[ib][d] - mi * Fv;
+                    V[jb][d] = V[jb][d] + mj * Fv;
+                }
+            }
+        }
+    } else {
+        const double eps2 = eps * eps;
+        for (int it = 0; it < 300 && !finished; ++it) {
+            finished = true;
+#pragma unroll
+            for (int q = 0; q < K; ++q) {
+                const int ib = G::i(q), jb = G::j(q);
+                double R[3], W[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    R[d] = X[ib][d] - X[jb][d];
+                    W[d] = V[ib][d] - V[jb][d];
+                }
+                const double RV = R[0] * W[0] + R[1] * W[1] + R[2] * W[2];
+                const double R2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
+                const double V2 = W[0] * W[0] + W[1] * W[1] + W[2] * W[2];
+                if (RV * RV * V2 < eps2 * R2) continue;     // (RV^2 / R^2) V^2 < eps^2, R^2 > 0
+                finished = false;
+                const double mi = IM[ib], mj = IM[jb];
+                const double kij = RV * RC[q];              // RV / (d^2 (1/m_i + 1/m_j))
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const double KR = kij * R[d];
+                    V[ib][d] = V[ib][d] - mi * KR;
+                    V[jb][d] = V[jb][d] + mj * KR;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (POS) pos[3 * (size_t)at[a] + d] = X[a][d];
+            vel[3 * (size_t)at[a] + d] = V[a][d];
+        }
+    if (!finished) atomicOr(status, POS ? ST_RATTLE_NOCONV : ST_RATTLEV_NOCONV);
+}
+
+// PLAIN: rattle_group_plain
+template <bool POS, bool PLAIN, class G>
+__device__ __forceinline__ void rattle_group_as(const int (&at)[G::NA], const double (&dd)[G::K],
+                                                double* __restrict__ pos, double* __restrict__ vel,
+                                                const double* __restrict__ old, const double* __restrict__ invm,
+                                                double eps, double dt, const double (&rvi)[3], unsigned* status) {
+    if (PLAIN) rattle_group_plain<POS, G>(at, dd, pos, vel, old, invm, eps, dt, rvi, status);
+    else rattle_group<POS, G>(at, dd, pos, vel, old, invm, eps, dt, rvi, status);
+}
+
+template <bool POS, bool PLAIN>
 __global__ void __launch_bounds__(64) k_rattle_rigid3(double* __restrict__ pos, double* __restrict__ vel,
                                                       const double* __restrict__ old,
                                                       const double* __restrict__ invm,
@@ -944,10 +1046,10 @@ __global__ void __launch_bounds__(64) k_rattle_rigid3(double* __restrict__ pos, 
     const double4 D = dl[g];
     const int at[3] = {A.x, A.y, A.z};
     const double dd[3] = {D.x * D.x, D.y * D.y, D.z * D.z};
-    rattle_group<POS, RattleRigid3>(at, dd, pos, vel, old, invm, eps, dt, rvi, status);
+    rattle_group_as<POS, PLAIN, RattleRigid3>(at, dd, pos, vel, old, invm, eps, dt, rvi, status);
 }
 
-template <bool POS, int K>
+template <bool POS, bool PLAIN, int K>
 __device__ __forceinline__ void rattle_star_group(int g, double* __restrict__ pos, double* __restrict__ vel,
                                                   const double* __restrict__ old, const double* __restrict__ invm,
                                                   const int* __restrict__ sa, const double* __restrict__ sd,
@@ -962,12 +1064,12 @@ __device__ __forceinline__ void rattle_star_group(int g, double* __restrict__ po
         const double dij = sd[4 * (size_t)g + q];
         dd[q] = dij * dij;
     }
-    rattle_group<POS, RattleStar<K>>(at, dd, pos, vel, old, invm, eps, dt, rvi, status);
+    rattle_group_as<POS, PLAIN, RattleStar<K>>(at, dd, pos, vel, old, invm, eps, dt, rvi, status);
 }
 
 // seg: first group with K = 3, 2, 1 and the group count (groups sorted by K
 // from 4 down, so a warp's groups mostly share K)
-template <bool POS>
+template <bool POS, bool PLAIN>
 __global__ void __launch_bounds__(64) k_rattle_star(double* __restrict__ pos, double* __restrict__ vel,
                                                      const double* __restrict__ old, const double* __restrict__ invm,
                                                      const int* __restrict__ sa, const double* __restrict__ sd,
@@ -978,32 +1080,28 @@ __global__ void __launch_bounds__(64) k_rattle_star(double* __restrict__ pos, do
     if (g >= seg.w) return;
     double rvi[3] = {1.0, 1.0, 1.0};
     if (POS && use_rv) { rvi[0] = dyn->rvinv[0]; rvi[1] = dyn->rvinv[1]; rvi[2] = dyn->rvinv[2]; }
-    if (g < seg.x) rattle_star_group<POS, 4>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
-    else if (g < seg.y) rattle_star_group<POS, 3>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
-    else if (g < seg.z) rattle_star_group<POS, 2>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
-    else rattle_star_group<POS, 1>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
+    if (g < seg.x) rattle_star_group<POS, PLAIN, 4>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
+    else if (g < seg.y) rattle_star_group<POS, PLAIN, 3>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
+    else if (g < seg.z) rattle_star_group<POS, PLAIN, 2>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
+    else rattle_star_group<POS, PLAIN, 1>(g, pos, vel, old, invm, sa, sd, eps, dt, rvi, status);
 }
 
 static void rattle_star_launch(pgk_ctx* c, bool pos, double eps, double dt, bool use_rv) {
     const int blocks = (c->nstar + 63) / 64;
     const int4 seg = make_int4(c->star_seg[0], c->star_seg[1], c->star_seg[2], c->star_seg[3]);
-    if (pos)
-        launch_pdl(k_rattle_star<true>, blocks, 64, 0, c->st, c->pos, c->vel, c->pos_old, c->invmass, c->star_atoms,
-                                                       c->star_d, seg, eps, dt, use_rv ? 1 : 0, c->dyn, c->status);
-    else
-        launch_pdl(k_rattle_star<false>, blocks, 64, 0, c->st, c->pos, c->vel, nullptr, c->invmass, c->star_atoms,
-                                                        c->star_d, seg, eps, 0.0, 0, c->dyn, c->status);
+    auto* k = c->plain_order ? (pos ? k_rattle_star<true, true> : k_rattle_star<false, true>)
+                            : (pos ? k_rattle_star<true, false> : k_rattle_star<false, false>);
+    launch_pdl(k, blocks, 64, 0, c->st, c->pos, c->vel, pos ? c->pos_old : nullptr, c->invmass, c->star_atoms, c->star_d,
+               seg, eps, pos ? dt : 0.0, pos && use_rv ? 1 : 0, c->dyn, c->status);
     PGK_LAUNCHED(c);
 }
 
 static void rattle_rigid3_launch(pgk_ctx* c, bool pos, double eps, double dt, bool use_rv) {
     const int blocks = (c->nr3 + 63) / 64;
-    if (pos)
-        launch_pdl(k_rattle_rigid3<true>, blocks, 64, 0, c->st, c->pos, c->vel, c->pos_old, c->invmass, c->r3_atoms,
-                                                         c->r3_d, c->nr3, eps, dt, use_rv ? 1 : 0, c->dyn, c->status);
-    else
-        launch_pdl(k_rattle_rigid3<false>, blocks, 64, 0, c->st, c->pos, c->vel, nullptr, c->invmass, c->r3_atoms,
-                                                          c->r3_d, c->nr3, eps, 0.0, 0, c->dyn, c->status);
+    auto* k = c->plain_order ? (pos ? k_rattle_rigid3<true, true> : k_rattle_rigid3<false, true>)
+                            : (pos ? k_rattle_rigid3<true, false> : k_rattle_rigid3<false, false>);
+    launch_pdl(k, blocks, 64, 0, c->st, c->pos, c->vel, pos ? c->pos_old : nullptr, c->invmass, c->r3_atoms, c->r3_d,
+               c->nr3, eps, pos ? dt : 0.0, pos && use_rv ? 1 : 0, c->dyn, c->status);
     PGK_LAUNCHED(c);
 }
 

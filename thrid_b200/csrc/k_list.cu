@@ -201,8 +201,9 @@ __device__ __forceinline__ bool is_excluded(const int* __restrict__ exs_idx, con
 // odd and of the higher one when it is even: every cluster then owns about
 // half of its neighbours.  (All pairs in the lower cluster's row made the rows
 // of the first cell layers about twice, those of the last a third of the mean,
-// and the pair kernel's blocks as uneven.)
-__device__ __forceinline__ bool owns(int I, int J) { return ((I + J) & 1) ? I < J : I > J; }
+// and the pair kernel's blocks as uneven.)  lower: all pairs in the lower
+// cluster's row (pgk_ctx::plain_order).
+__device__ __forceinline__ bool owns(int I, int J, bool lower) { return lower || ((I + J) & 1) ? I < J : I > J; }
 
 // nearest integer of a moderate x (adding 1.5 2^23 rounds to one)
 __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
@@ -210,7 +211,7 @@ __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x
 // One block of four warps per i-cluster:
 //  1. bounding boxes: the clusters J of the distinct neighbour cells that the
 //     cluster owns (owns) and whose box comes within rcut_book (a warp takes
-//     every fourth cell, a lane a cluster);
+//     a quarter of the cells, a lane a cluster);
 //  2. the eight atoms of each such J against the eight cluster atoms in FP32
 //     (two cluster atoms per packed operation); FRAME boxes (at least four
 //     cells a side) use coordinates relative to the cluster's centre, others
@@ -222,8 +223,9 @@ __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x
 //     (bins of mask_bin), each warp ranking a quarter of the candidates, and
 //     written to the row: 32 consecutive entries then mostly share their mask
 //     bits, which keeps the pair kernel's warps uniform.
-// Every step keeps the candidates' order, so a build of the same positions
-// gives the same rows.  nlistnball (the reference's row count, one sentinel
+// Every step keeps the candidates' order (cells in scan order, slots ascending),
+// so a build of the same positions gives the same rows.  A row of more than
+// CL_CCAP candidates is sorted piece by piece (k_sort_rows joins the pieces).  nlistnball (the reference's row count, one sentinel
 // per empty row) is the number of pairs plus the atoms i < n-1 without a
 // partner of higher index; hasup[slot] = 1 marks the atoms that have one.
 // Bound by issue and the latency of the candidate loads (fetched one iteration
@@ -238,6 +240,7 @@ struct ClistArgs {
     const int* cell_of; const int* cell_start; const int* cell_cnt;
     const int* exs_idx; const int* exs_list; const int2* exs_rng;
     int ncl, ccap;
+    bool lower;
     double sqcut;
     float rbox, sqlo, sqhi;
     int* clist; int* ccnt; unsigned char* hasup; unsigned long long* counters; unsigned* status;
@@ -321,21 +324,23 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
         if (tid == 0) a.ccnt[cl] = 0;
         return;
     }
-    const int batch = 4 * max(1, CL_JCAP / smaxj);       // cells of one round of step 1
+    const int bw = min(max(1, CL_JCAP / smaxj), (ncel + 3) >> 2);   // a warp's cells in one round of step 1
+    const int batch = 4 * bw;
     const float rb2 = a.rbox * a.rbox;
     int* __restrict__ row = a.clist + (size_t)cl * a.ccap;
     const float mid = 0.5f * (a.sqlo + a.sqhi), band = 0.5f * (a.sqhi - a.sqlo) * 1.0001f;
     int npair = 0;
     unsigned up = 0;
     int count = 0;                                       // row entries so far (uniform)
+    int pieces = 0;                                      // sorted pieces of the row
     for (int q0 = 0; q0 < ncel; q0 += batch) {
         // 1: owned clusters near the bounding box
         int nj = 0;
-        for (int q = q0 + w; q < min(ncel, q0 + batch); q += 4) {
+        for (int q = q0 + w * bw; q < min(ncel, q0 + (w + 1) * bw); ++q) {
             const int J1 = scell[q].y;
             for (int jb = scell[q].x; jb < J1; jb += 32) {
                 const int J = jb + lane;
-                bool ok = J < J1 && (J == cl || owns(cl, J));
+                bool ok = J < J1 && (J == cl || owns(cl, J, a.lower));
                 if (ok) {
                     const float4 c = a.cbox[2 * J], h = a.cbox[2 * J + 1];
                     float dx = c.x - ctr.x, dy = c.y - ctr.y, dz = c.z - ctr.z;
@@ -361,6 +366,7 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
         __syncthreads();
         const int ntot = 8 * soff[4];                    // candidate atoms
         for (int c0 = 0; c0 < ntot; c0 += CL_CCAP) {
+            ++pieces;
             const int nc = min(CL_CCAP, ntot - c0);
             const int part = ((nc + 127) >> 7) << 5;     // a warp's share, a multiple of 32
             const int lo = w * part, hi = min(nc, lo + part);
@@ -523,9 +529,62 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
     if (lane < 8 && ((up >> lane) & 1u)) a.hasup[s0 + lane] = 1;
     if (lane == 0 && npair) atomicAdd(&a.counters[0], (unsigned long long)npair);
     if (tid == 0) {
+        if (pieces > 1) a.counters[3] = 1ull;
         a.ccnt[cl] = min(count, a.ccap);
         if (count > a.ccap) atomicOr(a.status, ST_LIST_OVERFLOW);
         atomicMax(&a.counters[1], (unsigned long long)count);
+    }
+}
+
+// Rows that k_build_clist sorted in pieces: one stable sort over the whole row
+// (a warp per row; rows already in order are left alone).
+__global__ void __launch_bounds__(128) k_sort_rows(int* __restrict__ clist, const int* __restrict__ ccnt, int ncl, int ccap,
+                                                   const unsigned long long* __restrict__ counters) {
+    extern __shared__ int srow[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, cl = blockIdx.x * 4 + w;
+    if (cl >= ncl || counters[3] == 0ull) return;
+    int* buf = srow + (size_t)w * (ccap + 256);
+    int* bin = buf + ccap;
+    int* row = clist + (size_t)cl * ccap;
+    const int n = ccnt[cl];
+    bool ok = true;
+    for (int k = lane; k < n; k += 32) {
+        const int e = row[k];
+        buf[k] = e;
+        ok = ok && (k == 0 || mask_bin((unsigned)row[k - 1] >> 24) <= mask_bin((unsigned)e >> 24));
+    }
+    if (__all_sync(0xffffffffu, ok)) return;
+    for (int q = lane; q < 256; q += 32) bin[q] = 0;
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) atomicAdd(&bin[mask_bin((unsigned)buf[k] >> 24)], 1);
+    __syncwarp();
+    int v[8], tot = 0;                               // exclusive prefix sums of the bins, 8 a lane
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { v[q] = bin[8 * lane + q]; tot += v[q]; }
+    int run = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += y;
+    }
+    run -= tot;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { bin[8 * lane + q] = run; run += v[q]; }
+    __syncwarp();
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        const bool in = k < n;
+        const int e = in ? buf[k] : 0;
+        const unsigned kb = in ? mask_bin((unsigned)e >> 24) : 256u + lane;
+        const unsigned grp = __match_any_sync(0xffffffffu, kb);
+        const int rank = __popc(grp & ((1u << lane) - 1u));
+        const int base = in ? bin[kb] : 0;
+        __syncwarp();
+        if (in) {
+            row[base + rank] = e;
+            if (rank == 0) bin[kb] = base + __popc(grp);
+        }
+        __syncwarp();
     }
 }
 
@@ -606,6 +665,17 @@ static pgk_status ensure_sorted_capacity(pgk_ctx* c, int npad_cap) {
     return alloc_rows(c);
 }
 
+// pgk_ctx::plain_order from here on
+pgk_status keep_plain_order(pgk_ctx* c) {
+    if (!c->mixed() || c->plain_order) return PGK_OK;
+    c->plain_order = true;
+    c->pseg = 1;                            // the allocated segments of a row hold the whole of it (alloc_rows)
+    c->pcap = c->ccap;
+    if (c->prune_buffer > 0.f) PGK_CUDA(c, cudaMemsetAsync(&c->prune->force, 1, 1, c->st));   // re-prune
+    ++c->list_epoch;                        // captured steps hold the segments
+    return PGK_OK;
+}
+
 pgk_status launch_mklist(pgk_ctx* c) {
     int n = c->natom;
     // the box may have changed on the device (MTK): read it back
@@ -660,7 +730,7 @@ pgk_status launch_mklist(pgk_ctx* c) {
         a.pf = c->pf_s; a.cbox = c->cbox; a.pos_s = c->pos_s;
         a.cell_of = c->cell_of; a.cell_start = c->cell_start; a.cell_cnt = c->cell_cnt;
         a.exs_idx = c->exs_idx; a.exs_list = c->exs_list; a.exs_rng = c->exs_rng;
-        a.ncl = c->ncl; a.ccap = c->ccap;
+        a.ncl = c->ncl; a.ccap = c->ccap; a.lower = c->plain_order;
         a.sqcut = sq; a.rbox = (float)(c->prm.rcut_book + 0.05);
         a.sqlo = (float)(sq * (1.0 - 1.0e-5) - scr); a.sqhi = (float)(sq * (1.0 + 1.0e-5) + scr);
         a.clist = c->clist; a.ccnt = c->ccnt; a.hasup = c->hasup; a.counters = c->counters; a.status = c->status;
@@ -670,6 +740,12 @@ pgk_status launch_mklist(pgk_ctx* c) {
             frame = frame && nc[d] >= 4 && c->prm.rcut_book + 0.5 * h.cellsize[d] + 0.1 < 0.5 * h.box[d];
         if (frame) k_build_clist<true><<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
         else k_build_clist<false><<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
+        const size_t ssm = (size_t)4 * (c->ccap + 256) * sizeof(int);
+        if (c->plain_order && ssm <= 160 * 1024) {
+            PGK_CUDA(c, smem_limit(k_sort_rows, ssm));
+            k_sort_rows<<<(c->ncl + 3) / 4, 128, ssm, c->st>>>(c->clist, c->ccnt, c->ncl, c->ccap, c->counters);
+            PGK_LAUNCHED(c);
+        }
         if (n > 1) k_count_noup<<<(n - 1 + 255) / 256, 256, 0, c->st>>>(c->hasup, c->iperm, n - 1, c->counters);
         c->launches += 7;
         PGK_CUDA(c, cudaGetLastError());

@@ -156,6 +156,22 @@ struct pgk_ctx {
     // per cluster: the pair kernel's work units (a warp each), so that small
     // boxes fill the SMs
     int pseg = 1, pcap = 0;
+    // Mixed precision: whole rows of the lower cluster's pairs (owns) and the
+    // plain RATTLE sweeps (rattle_group_plain), which is the order that sums
+    // and roundings had before rows were shared out by parity and cut into
+    // segments.  Another order moves positions by 1e-8 A in a few steps, and
+    // where results amplify that, the order is part of the result:
+    //   heat-flux regions  the records sum a bare 1/r up to rrcut, so one pair
+    //                      on the other side of the cutoff moves a record by up
+    //                      to 1e-2 of itself (8,232 waters, 14 records: 2e-4 to
+    //                      4e-3 in one run of six);
+    //   served replicas    long runs of small systems: up to 9e-5 in the
+    //                      velocities after 300 steps (eight replicas at once
+    //                      take 106 ms in either order, one at a time 9 % more).
+    // Elsewhere the faster forms stay (49 steps of 12,000 atoms: 5.6 -> 4.4 ms,
+    // velocities to 1e-6).  Set by keep_plain_order; the rows follow from the
+    // next list build on.
+    bool plain_order = false;
     int* plist = nullptr;         // [ncl * pseg * pcap]
     int* pcnt = nullptr;          // [ncl * pseg]
     void* xq_prune = nullptr;     // xq (int4) or xq64 (double4) at the last prune
@@ -170,7 +186,7 @@ struct pgk_ctx {
     double4* xq64 = nullptr;      // fp64: x,y,z,q sorted
     int* typ_s = nullptr;
     unsigned long long* counters = nullptr;   // [0] list pairs, [1] longest cluster row, [2] rows without
-                                              //  a higher-index partner; [4..6] count_pairs scratch
+                                              //  a higher-index partner, [3] rows sorted in pieces; [4..6] count_pairs scratch
     unsigned char* hasup = nullptr;           // [npad_cap] a slot's atom has a list partner of higher index
     bool list_valid = false;
     long long list_epoch = 0;     // incremented by every list build (invalidates captured graphs)
@@ -324,6 +340,7 @@ pgk_status pgk_fail(pgk_ctx* c, pgk_status s, const std::string& msg);
 
 // ---- launchers (k_list.cu) ----
 pgk_status launch_transcor(pgk_ctx* c);
+pgk_status keep_plain_order(pgk_ctx* c);
 pgk_status launch_mklist(pgk_ctx* c);
 pgk_status export_nblist(pgk_ctx* c, int32_t* nb_index, int32_t* nb_list, int64_t cap, int64_t* nl);
 

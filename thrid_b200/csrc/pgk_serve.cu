@@ -125,6 +125,7 @@ static void run_job(pgk_server* sv, Job* j) {
     cudaSetDevice(sv->device);
     pgk_ctx* c = nullptr;
     pgk_status s = pgk_init(&j->sys->s, &j->prm, &c);
+    if (s == PGK_OK) s = keep_plain_order(c);
     if (s == PGK_OK) s = pgk_upload_state(c, j->x0.data(), j->v0.data(), j->box0);
     if (s == PGK_OK && j->has_chain) s = pgk_set_chain(c, &j->chain);
     if (s == PGK_OK && j->has_hf) {
