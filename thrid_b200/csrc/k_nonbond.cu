@@ -54,7 +54,7 @@ __device__ __forceinline__ void prune_decide(PruneDev* __restrict__ P, const Dyn
     if (!keep) {
         P->dmax = 0u;
         P->force = 0;
-        for (int d = 0; d < 3; ++d) P->box[d] = dyn->box[d];
+        for (int d = 0; d < 3; ++d) { P->box[d] = dyn->box[d]; P->binv[d] = 1.0 / dyn->box[d]; }
         P->nprune += 1ull;
     }
 }
@@ -121,11 +121,18 @@ __global__ void k_pack_fp64(const double* __restrict__ pos, const double* __rest
     if (i >= 0) v = make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], chrg[i]);
     if (s < npad) xq[s] = v;
     if (P) {
-        // displacement since the last prune (minimum image, current box), rounded up
+        // displacement since the last prune (minimum image, current box),
+        // rounded up.  In fractional coordinates, as the mixed pack's: the
+        // origin is scaled to the current box, so that a pair's distance
+        // changes by at most the box term r |L/L0 - 1| and two displacements
+        // (unscaled, the image vector of a pair across a face would change
+        // by L - L0 unseen)
         float dd = 0.f;
         if (i >= 0) {
             const double4 o = xq_prune[s];
-            double dx = v.x - o.x, dy = v.y - o.y, dz = v.z - o.z;
+            double dx = fma(-dyn->box[0] * P->binv[0], o.x, v.x);
+            double dy = fma(-dyn->box[1] * P->binv[1], o.y, v.y);
+            double dz = fma(-dyn->box[2] * P->binv[2], o.z, v.z);
             dx -= dyn->box[0] * rint(dx * dyn->boxinv[0]);
             dy -= dyn->box[1] * rint(dy * dyn->boxinv[1]);
             dz -= dyn->box[2] * rint(dz * dyn->boxinv[2]);
@@ -1133,7 +1140,9 @@ pgk_status launch_pair(pgk_ctx* c, int group, int vmode, bool finish) {
     if (c->prune_buffer > 0.f) {
         const float rp = prune_radius(c);
         a.P = c->prune; a.plist = c->plist; a.pcnt = c->pcnt;
-        a.xq_prune = c->xq_prune; a.rp2f = rp * rp; a.rp2 = (double)a.rp2f;
+        a.xq_prune = c->xq_prune; a.rp2f = rp * rp;
+        const double rpd = std::max(c->prm.rrcut, c->prm.rcut) + (double)c->prune_buffer;
+        a.rp2 = rpd * rpd;
     }
     if (c->rec_pre_pair) {
         PGK_CUDA(c, cudaEventRecord(c->ev_pre_pair, c->st));

@@ -56,10 +56,11 @@ enum AccIdx {
 #define ST_RATTLEV_NOCONV  (1u << 4)
 #define ST_UNSUPPORTED     (1u << 5)
 
-// Pruned pair list state (mixed precision): the pair kernel reads a copy of
+// Pruned pair list state (both precisions): the pair kernel reads a copy of
 // the book list whose masks keep only pairs inside rprune = cutoff + buffer
-// at the last prune.  dmax tracks the largest atom displacement since then
-// (float bits, atomicMax); the list is re-pruned before a pair evaluation
+// at the last prune.  dmax tracks the largest atom displacement since then,
+// in fractional coordinates times the current box (float bits, atomicMax);
+// the list is re-pruned before a pair evaluation
 // when 2*dmax plus the box-scaling term reaches the buffer, or when the book
 // list was rebuilt (force), so no pair of the book list that comes inside
 // the cutoff is ever missing from the pruned list.
@@ -68,7 +69,7 @@ struct PruneDev {
     int force;
     int do_prune;
     unsigned done;                // blocks of the pack finished (zero between launches)
-    double box[3];                // box at the last prune
+    double box[3], binv[3];       // box at the last prune and its inverse
     unsigned long long nprune;    // prunes done (diagnostic)
 };
 
