@@ -18,8 +18,8 @@
 // k_hf_pair walks the same 8-atom cluster rows as the pair kernel, twice: lanes
 // own entries and sum the neighbour's shares, then lanes own cluster atoms and
 // sum theirs.
-// Pair arithmetic is FP32 in mixed precision and FP64 otherwise; region
-// geometry and all sums are FP64 in global memory.
+// Pair distances and scalar factors are FP32 in mixed precision and FP64
+// otherwise; velocities, region geometry and the sums in memory are FP64.
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -95,11 +95,10 @@ __global__ void k_hf_slots(const int* __restrict__ perm, int npad, const double*
 
 // Per atom: heat-flux z, molecule tag, velocities and region bits into the
 // sorted slots (iperm; null: no pair list), kinetic transport into the sums.
-template <bool MIXED>
 __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ pos, const double* __restrict__ mass,
                                                     const int* __restrict__ iperm, FluxDev f,
                                                     const DynState* __restrict__ dyn, double* __restrict__ zs,
-                                                    int* __restrict__ ms, void* __restrict__ vs,
+                                                    int* __restrict__ ms, double4* __restrict__ vs,
                                                     uint4* __restrict__ bs) {
     pdl_enter();
     __shared__ double sk[PGK_HF_MAX_REGIONS];
@@ -121,8 +120,7 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
             ms[s] = hf_tag(f.h, i, m.w);
             bs[s] = m;
             for (int q = 0; q < FLUX_SUMS; ++q) f.sum[(size_t)FLUX_SUMS * s + q] = 0.0;
-            if (MIXED) ((float4*)vs)[s] = make_float4((float)vx, (float)vy, (float)vz, (float)pvz);
-            else ((double4*)vs)[s] = make_double4(vx, vy, vz, pvz);
+            vs[s] = make_double4(vx, vy, vz, pvz);
         }
     }
     unsigned any = __reduce_or_sync(0xffffffffu, in);
@@ -149,30 +147,48 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
 // entry, those of a pair inside one molecule at once (they are a class of
 // their own).  An atom exactly on a plane has hf_frag's own cases: the virial
 // part of its pairs goes to the regions directly.
-// Pair arithmetic is T (FP32 in mixed precision, the reciprocal root refined
-// by one Newton step), all sums over atoms and regions are FP64.
-// Bound by issue (about 70 instructions per pair) at 16 warps per SM.
-// Measured, mixed: 43,200-atom slab, 23 regions: 0.159 ms and 0.020 ms for the
-// regions (0.33 ms with the regions inside the pair loop, four a walk); 8,232-
-// atom water box, one region: 0.035 ms, unchanged.
+// A pair's distance and scalar factors are T (FP32 in mixed precision), and so
+// are a lane's partial sums of the cluster atoms' energies (at most a row's
+// entries / 32 terms; FP64 there changes no digit of the error and costs 5 %);
+// velocities, f . v, the entries' sums and all sums over lanes, rows, atoms and
+// regions are FP64.  Error of the records against FP64 as with the divided 1/r
+// and per-atom FP64 virials: 2,592 atoms of propanol, LJ virials 9e-7 and 4e-7
+// of the largest region.
+// Bound by issue at 16 warps per SM.  Measured, mixed: 43,200-atom slab, 23
+// regions: 0.177 ms and 0.012 ms for the regions (0.33 ms with the regions
+// inside the pair loop, four a walk); 8,232-atom water box, one region: 0.045
+// ms.  (Velocities and f . v in FP32: 0.165 and 0.042 ms, and 1.2 to 1.5 times
+// the error.)
 // Rows are cut into segments until 16 warps per SM have work (small boxes).
 struct FluxPairArgs {
     const int* rows; const int* cnt; int ccap; int ncl; int nseg;
     int cut;                     // rows, cnt: nseg segments of ccap entries per cluster, else whole rows
     const int* typ_s; const int* perm; int ntyp;
-    const double* zs; const int* ms; const void* vs; const uint4* bs;
+    const double* zs; const int* ms; const double4* vs; const uint4* bs;
     double rrcut, rr2, rl2, rmax2;
 };
 
-template <bool MIXED> struct FluxT { typedef float T; typedef float4 V; };
-template <> struct FluxT<false> { typedef double T; typedef double4 V; };
+template <bool MIXED> struct FluxT { typedef float T; };
+template <> struct FluxT<false> { typedef double T; };
 
-__device__ __forceinline__ float flux_rinv(float r2) {
+// 1/r and 1/r^2.  FP32: the approximate root (2^-22.9) and one Newton step
+// y (1 + e/2) with e = 1 - r^2 y^2 exact to 2^-47 (the product's rounding is
+// taken back), so 1/r is off by its last rounding, and one residual step for
+// the square: no less than a divided root and a division, in half as many
+// instructions.
+__device__ __forceinline__ void flux_rinv(float r2, float& rinv, float& rinv2) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
-    return y * fmaf(-0.5f * r2 * y, y, 1.5f);
+    const float h = r2 * y, hl = fmaf(r2, y, -h);
+    const float e = fmaf(-hl, y, fmaf(-h, y, 1.f));
+    rinv = fmaf(0.5f * y, e, y);
+    const float q = rinv * rinv;
+    rinv2 = fmaf(fmaf(-r2, q, 1.f), q, q);
 }
-__device__ __forceinline__ double flux_rinv(double r2) { return rsqrt(r2); }
+__device__ __forceinline__ void flux_rinv(double r2, double& rinv, double& rinv2) {
+    rinv = rsqrt(r2);
+    rinv2 = rinv * rinv;
+}
 
 // One pair's terms of the per-atom arrays (categories Coulomb, LJ): energies
 // and half forces; false beyond both cutoffs.
@@ -200,7 +216,8 @@ __device__ __forceinline__ bool hf_term(const int4& qi, const double4& pi, const
     }
     const T r2 = dx * dx + dy * dy + dz * dz;
     if (r2 > (T)a.rmax2) return false;
-    const T rinv = flux_rinv(r2), rinv2 = rinv * rinv;
+    T rinv, rinv2;
+    flux_rinv(r2, rinv, rinv2);
     const bool coul = MIXED ? r2 <= (T)a.rr2 : sqrt((double)r2) <= a.rrcut;
     const T phc = coul ? qq * rinv : (T)0;               // ewaldr_hf.F90:336-371, bare 1/r
     T phl = (T)0, ftl = (T)0;
@@ -233,9 +250,9 @@ __device__ __forceinline__ bool hf_term(const int4& qi, const double4& pi, const
 // Bound by issue (the pair arithmetic is done twice) and by the entries'
 // atomics.  Measured, mixed: 43,200-atom slab, 23 regions 0.79 ms (4.86 ms with
 // one lane's atomics for every pair, into shared memory for the cluster atom
-// and global memory for the entry's); 8,232-atom water box, one region 0.103 ms
+// and global memory for the entry's); 8,232-atom water box, one region 0.114 ms
 // (1.27 ms).  Three blocks per SM without spills, or six regions a walk, were
-// no faster (call of 14 steps 7.92, 8.04 ms against 7.87).
+// no faster (slab, call of 10 steps: 7.92, 8.04 ms against 7.87).
 template <bool MIXED, int KW>
 __global__ void __launch_bounds__(128, MIXED ? 4 : 3)
 k_hf_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxPairArgs a,
@@ -484,10 +501,9 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
             const DynState* __restrict__ dyn) {
     pdl_enter();
     typedef typename FluxT<MIXED>::T T;
-    typedef typename FluxT<MIXED>::V V;
     __shared__ int4 sxq[4][8];
     __shared__ double4 sx64[MIXED ? 1 : 4][8];
-    __shared__ V sv[4][8];
+    __shared__ double4 sv[4][8];
     __shared__ double szi[4][8];
     __shared__ int smi[4][8], sti[4][8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -495,7 +511,7 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
     const double B0 = 1.0 / L0, B1 = 1.0 / L1, B2 = 1.0 / Lz;
     const T sx = (T)(L0 * (1.0 / 4294967296.0)), sy = (T)(L1 * (1.0 / 4294967296.0)), sz = (T)(Lz * (1.0 / 4294967296.0));
     const T rr2 = (T)a.rr2, rl2 = (T)a.rl2, rmax2 = (T)a.rmax2;
-    const V* __restrict__ vs = (const V*)a.vs;
+    const double4* __restrict__ vs = a.vs;
     const long long nunit = (long long)a.ncl * a.nseg;
     for (long long u = blockIdx.x * 4 + w; u < nunit; u += gridDim.x * 4) {
         const int cl = (int)(u / a.nseg), seg = (int)(u - (long long)cl * a.nseg);
@@ -524,12 +540,11 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
             const unsigned m = e >> 24;
             const double zj = a.zs[j];
             const int mj = a.ms[j], tj = a.typ_s[j];
-            const V vj = vs[j];
+            const double4 vj = vs[j];
             int4 qj = make_int4(0, 0, 0, 0);
             double4 pj = make_double4(0, 0, 0, 0);
             if (MIXED) qj = xq[j]; else pj = xq64[j];
-            T pjc = (T)0, pjl = (T)0;
-            double sjc = 0.0, sjl = 0.0;
+            double pjc = 0.0, pjl = 0.0, sjc = 0.0, sjl = 0.0;
 #pragma unroll
             for (int ii = 0; ii < 8; ++ii) {
                 if (!((m >> ii) & 1u)) continue;
@@ -548,7 +563,8 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
                 }
                 const T r2 = dx * dx + dy * dy + dz * dz;
                 if (r2 > rmax2) continue;
-                const T rinv = flux_rinv(r2), rinv2 = rinv * rinv;
+                T rinv, rinv2;
+                flux_rinv(r2, rinv, rinv2);
                 const T phc = r2 <= rr2 ? qq * rinv : (T)0;              // ewaldr_hf.F90:336-371, bare 1/r
                 T phl = (T)0, ftl = (T)0;
                 if (r2 <= rl2) {                                         // ewaldr_hf.F90:376-470
@@ -559,14 +575,14 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
                     phl = E * (t12 - (T)2 * t6);
                     ftl = (T)12 * E * (t12 - t6) * rinv2;
                 }
-                const V vi = sv[w][ii];
-                const T fv = dx * (vi.x + vj.x) + dy * (vi.y + vj.y) + dz * (vi.z + vj.z);
+                const double4 vi = sv[w][ii];
+                const double fv = (double)dx * (vi.x + vj.x) + (double)dy * (vi.y + vj.y) + (double)dz * (vi.z + vj.z);
                 const int mi = smi[w][ii];
                 const bool same = !((mi ^ mj) & HF_MS_ID);
                 const double zi = szi[w][ii], az = fabs(zi - zj);
                 const bool vir = !((mi < 0) && (mj < 0) && same) && az * B2 < 0.5;
-                double sc = vir ? 0.5 * (double)(phc * rinv2 * fv) : 0.0;
-                double sl = vir ? 0.5 * (double)(ftl * fv) : 0.0;
+                double sc = vir ? 0.5 * (double)(phc * rinv2) * fv : 0.0;
+                double sl = vir ? 0.5 * (double)ftl * fv : 0.0;
                 if (same || ((mi | mj) & HF_MS_PLANE)) {
                     const int s = 8 * cl + ii;
                     if (vir && ((mi | mj) & HF_MS_PLANE)) {
@@ -597,12 +613,12 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
                         continue;
                     }
                 }
-                pic[ii] += phc; pil[ii] += phl; pjc += phc; pjl += phl;
+                pic[ii] += phc; pil[ii] += phl; pjc += (double)phc; pjl += (double)phl;
                 sic[ii] += sc; sil[ii] += sl; sjc += sc; sjl += sl;
             }
             double* sj = f.sum + (size_t)FLUX_SUMS * j + 4;
-            if (pjc != (T)0) atomicAdd(sj, (double)pjc);
-            if (pjl != (T)0) atomicAdd(sj + 1, (double)pjl);
+            if (pjc != 0.0) atomicAdd(sj, pjc);
+            if (pjl != 0.0) atomicAdd(sj + 1, pjl);
             if (sjc != 0.0) atomicAdd(sj + 2, -sjc);
             if (sjl != 0.0) atomicAdd(sj + 3, -sjl);
         }
@@ -631,13 +647,10 @@ k_flux_pair(const int4* __restrict__ xq, const double4* __restrict__ xq64, FluxP
 // region and every (32 / PR)-th slot each, PR the power of two that holds the
 // regions (C_r(z) - z1_r: the pairs' differences stay).  Each slot's 8 sums are
 // one 64-byte line.
-template <bool MIXED>
 __global__ void __launch_bounds__(256) k_flux_regions(const int* __restrict__ perm, int npad,
-                                                      const double* __restrict__ zs, const void* __restrict__ vs_,
+                                                      const double* __restrict__ zs, const double4* __restrict__ vs,
                                                       const uint4* __restrict__ bs, FluxDev f) {
     pdl_enter();
-    typedef typename FluxT<MIXED>::V V;
-    const V* __restrict__ vs = (const V*)vs_;
     __shared__ double st[8][32][FLUX_SUMS + 2];
     __shared__ unsigned si[8][32];
     __shared__ double sb[8 * PGK_HF_MAX_REGIONS];
@@ -648,7 +661,7 @@ __global__ void __launch_bounds__(256) k_flux_regions(const int* __restrict__ pe
     const bool has = s < npad && perm[s] >= 0;
     if (has) {
         st[w][lane][0] = zs[s];
-        st[w][lane][1] = 0.5 * (double)vs[s].w;
+        st[w][lane][1] = 0.5 * vs[s].w;
         si[w][lane] = bs[s].z;
 #pragma unroll
         for (int q = 0; q < FLUX_SUMS; ++q) st[w][lane][2 + q] = f.sum[(size_t)FLUX_SUMS * s + q];
@@ -939,7 +952,7 @@ static pgk_status ensure_hf_slots(pgk_ctx* c) {
     c->hf_slots_cap = 0;
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_zs, sizeof(double) * c->npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_ms, sizeof(int) * c->npad_cap));
-    const size_t vb = (c->mixed() ? sizeof(float4) : sizeof(double4)) * (size_t)c->npad_cap;
+    const size_t vb = sizeof(double4) * (size_t)c->npad_cap;
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_vs, vb));
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_bs, sizeof(uint4) * c->npad_cap));
     PGK_CUDA(c, pgk_dmalloc(c, &c->hf_sum, sizeof(double) * FLUX_SUMS * c->npad_cap));
@@ -1063,7 +1076,7 @@ template <bool MIXED>
 static void flux_pair_launch(pgk_ctx* c, const FluxPairArgs& a, const FluxDev& f) {
     launch_pdl(k_flux_pair<MIXED>, flux_pair_grid(c, a), 128, 0, c->st, c->xq, c->xq64, a, c->lj32, c->lj64, f, c->dyn);
     PGK_LAUNCHED(c);
-    launch_pdl(k_flux_regions<MIXED>, (c->npad + 255) / 256, 256, 0, c->st, c->perm, c->npad, c->hf_zs, c->hf_vs, c->hf_bs,
+    launch_pdl(k_flux_regions, (c->npad + 255) / 256, 256, 0, c->st, c->perm, c->npad, c->hf_zs, c->hf_vs, c->hf_bs,
                f);
     PGK_LAUNCHED(c);
 }
@@ -1083,7 +1096,7 @@ pgk_status launch_heatf(pgk_ctx* c, double* dst, bool pruned) {
     if (pair_on && (s = ensure_hf_slots(c))) return s;
     f.sum = c->hf_sum;
     const int* ip = pair_on ? c->iperm : nullptr;
-    launch_pdl(c->mixed() ? k_flux_atoms<true> : k_flux_atoms<false>, (n + 255) / 256, 256, 0, c->st, c->pos, c->mass, ip,
+    launch_pdl(k_flux_atoms, (n + 255) / 256, 256, 0, c->st, c->pos, c->mass, ip,
                f, c->dyn, c->hf_zs, c->hf_ms, c->hf_vs, c->hf_bs);
     PGK_LAUNCHED(c);
     if (pair_on) {

@@ -243,7 +243,7 @@ struct pgk_ctx {
     long long hf_rec_cap = 1;     // records hf_rec holds
     double* hf_zs = nullptr;      // [npad_cap] heat-flux z of each sorted slot
     int* hf_ms = nullptr;         // [npad_cap] molecule tag of each sorted slot
-    void* hf_vs = nullptr;        // [npad_cap] (v, transport v_z) of each sorted slot (float4 / double4)
+    double4* hf_vs = nullptr;     // [npad_cap] (v, transport v_z) of each sorted slot
     double* hf_sum = nullptr;     // [npad_cap][FLUX_SUMS] pair sums of each sorted slot (FluxDev.sum)
     uint4* hf_bs = nullptr;       // [npad_cap] region bits of each sorted slot (flux_bits)
     int hf_slots_cap = 0;
