@@ -165,7 +165,7 @@ struct FluxPairArgs {
     int cut;                     // rows, cnt: nseg segments of ccap entries per cluster, else whole rows
     const int* typ_s; const int* perm; int ntyp;
     const double* zs; const int* ms; const double4* vs; const uint4* bs;
-    double rrcut, rr2, rl2, rmax2;
+    double rr2, rl2, rmax2;      // rr2: sqrt_le_limit(rrcut) in FP64
 };
 
 template <bool MIXED> struct FluxT { typedef float T; };
@@ -218,8 +218,7 @@ __device__ __forceinline__ bool hf_term(const int4& qi, const double4& pi, const
     if (r2 > (T)a.rmax2) return false;
     T rinv, rinv2;
     flux_rinv(r2, rinv, rinv2);
-    const bool coul = MIXED ? r2 <= (T)a.rr2 : sqrt((double)r2) <= a.rrcut;
-    const T phc = coul ? qq * rinv : (T)0;               // ewaldr_hf.F90:336-371, bare 1/r
+    const T phc = r2 <= (T)a.rr2 ? qq * rinv : (T)0;               // ewaldr_hf.F90:336-371, bare 1/r
     T phl = (T)0, ftl = (T)0;
     if (r2 <= (T)a.rl2) {                                // ewaldr_hf.F90:376-470
         T R2, E;
@@ -1028,10 +1027,10 @@ static FluxPairArgs flux_pair_args(pgk_ctx* c, bool pruned) {
     a.ccap = pruned ? c->pcap : c->ccap; a.ncl = c->ncl;
     a.typ_s = c->typ_s; a.perm = c->perm; a.ntyp = c->ntyp;
     a.zs = c->hf_zs; a.ms = c->hf_ms; a.vs = c->hf_vs; a.bs = c->hf_bs;
-    a.rrcut = c->prm.rrcut;
-    a.rr2 = c->prm.rrcut * c->prm.rrcut;
+    const double rr2 = c->prm.rrcut * c->prm.rrcut;
+    a.rr2 = c->mixed() ? rr2 : sqrt_le_limit(c->prm.rrcut);
     a.rl2 = c->prm.rcut * c->prm.rcut;
-    a.rmax2 = std::max(a.rr2, a.rl2);
+    a.rmax2 = std::max(rr2, a.rl2);
     // about 16 warps per SM, in row segments where the clusters alone are fewer
     a.nseg = a.cut ? c->pseg : std::max(1, std::min(8, c->nsm * 16 / std::max(a.ncl, 1)));
     return a;

@@ -167,7 +167,7 @@ struct PairArgs {
     const int* clist; const int* ccnt; int ccap; int ncl;     // book rows
     const int* typ_s;
     int ntyp; int nspl; double h, inv_h;
-    double rr2, rl2, rmax2, rrcut;
+    double rr2, rl2, rmax2, rrx2;      // rrx2: sqrt_le_limit(rrcut)
     // FP32 copies for the mixed kernel, read straight from the parameter
     // bank inside the pair loop (no registers held for them)
     float rr2f, rl2f, inv_hf, hf; int nsplm1;
@@ -755,7 +755,8 @@ __global__ void __launch_bounds__(pair_threads(FRAME), pair_minb(FRAME)) k_pair_
 // the rounding as an add and a subtraction of 1.5 2^52 (the images differ
 // from the reference's dnint only at exactly half a box, beyond the cutoff).
 // 1/r comes from one reciprocal square root (rsqrt_d); the spline index is
-// floor(r/h) by a rounded-down add of 2^52.
+// floor(r/h) by a rounded-down add of 2^52.  The Coulomb cutoff is the
+// reference's dsqrt(r^2) <= rrcut whatever the rounding of r (sqrt_le_limit).
 // Bound by the FP64 pipe's dependent chains at 16 warps per SM (128 registers).  Measured, 200,004-atom butane rows with
 // tensor: 2.22 ms per evaluation on the book rows with divisions, sqrt and
 // dnint on 16 warps per SM; now 0.75 ms on the pruned rows.
@@ -857,7 +858,7 @@ __device__ __forceinline__ void pair_fp64_body(const double4* __restrict__ xq, c
                 if (r2 > a.rmax2) continue;
                 const double rinv = rsqrt_d(r2), rinv2 = rinv * rinv, r = r2 * rinv;
                 double fc = 0, fl = 0;
-                if (r <= a.rrcut) {
+                if (r2 <= a.rrx2) {
                     const double qq = pi.w * pj.w;
                     const double fb = __dadd_rd(r * a.inv_h, TWO52);
                     const int idx = (int)min((unsigned)__double2loint(fb), (unsigned)a.nsplm1);
@@ -1045,7 +1046,7 @@ static PairArgs pair_args(pgk_ctx* c, int group) {
     a.clist = c->clist; a.ccnt = c->ccnt; a.ccap = c->ccap; a.ncl = c->ncl;
     a.typ_s = c->typ_s; a.ntyp = c->ntyp; a.nspl = c->nspl;
     a.h = c->hspl; a.inv_h = 1.0 / c->hspl;
-    a.rrcut = c->prm.rrcut;
+    a.rrx2 = sqrt_le_limit(c->prm.rrcut);
     a.rr2 = c->prm.rrcut * c->prm.rrcut;
     a.rl2 = c->prm.rcut * c->prm.rcut;
     a.rmax2 = a.rr2 > a.rl2 ? a.rr2 : a.rl2;

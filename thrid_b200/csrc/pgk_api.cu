@@ -3,6 +3,7 @@
 // drivers that keep the whole XO-RESPA loop on the device.
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <cstdio>
 #include <functional>
 #include <cstdlib>
@@ -65,6 +66,14 @@ pgk_status spme_bench(pgk_ctx* c, int which);
 pgk_status pgk_fail(pgk_ctx* c, pgk_status s, const std::string& msg) {
     if (c) c->err = msg;
     return s;
+}
+
+double sqrt_le_limit(double rc) {
+    double x = rc * rc;
+    const double inf = std::numeric_limits<double>::infinity();
+    while (std::sqrt(x) > rc) x = std::nextafter(x, 0.0);
+    while (std::sqrt(std::nextafter(x, inf)) <= rc) x = std::nextafter(x, inf);
+    return x;
 }
 
 namespace {

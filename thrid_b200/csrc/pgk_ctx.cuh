@@ -328,6 +328,10 @@ inline void launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// largest double whose correctly rounded square root is at most rc: r2 <= this
+// is the reference's dsqrt(r2) <= rc, without the root
+double sqrt_le_limit(double rc);
+
 // error helpers
 pgk_status pgk_fail(pgk_ctx* c, pgk_status s, const std::string& msg);
 #define PGK_CUDA(ctx, call)                                                               \
