@@ -147,17 +147,22 @@ static float prune_radius(const pgk_ctx* c) {
     return (float)std::max(c->prm.rrcut, c->prm.rcut) + c->prune_buffer;
 }
 
-pgk_status launch_pack(pgk_ctx* c, bool pair) {
+pgk_status launch_pack(pgk_ctx* c, bool pair, bool joined) {
     int n = c->npad;
     if (n <= 0) return PGK_OK;
     PruneDev* P = c->prune_buffer > 0.f ? c->prune : nullptr;
     const float rp = prune_radius(c);
-    if (c->mixed())
-        launch_pdl(k_pack_mixed, (n + 255) / 256, 256, 0, c->st, c->pos, c->chrg, c->perm, n, c->dyn, c->xq,
-                   (const int4*)c->xq_prune, P, c->prune_buffer, rp, pair ? 1 : 0);
-    else
-        launch_pdl(k_pack_fp64, (n + 255) / 256, 256, 0, c->st, c->pos, c->chrg, c->perm, n, c->dyn, c->xq64,
-                   (const double4*)c->xq_prune, P, c->prune_buffer, rp, pair ? 1 : 0);
+    const unsigned nb = (n + 255) / 256;
+    const int dec = pair ? 1 : 0;
+    const int4* xp = (const int4*)c->xq_prune;
+    const double4* xp64 = (const double4*)c->xq_prune;
+    if (c->mixed()) {
+        if (joined) k_pack_mixed<<<nb, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq, xp, P, c->prune_buffer, rp, dec);
+        else launch_pdl(k_pack_mixed, nb, 256, 0, c->st, c->pos, c->chrg, c->perm, n, c->dyn, c->xq, xp, P, c->prune_buffer, rp, dec);
+    } else {
+        if (joined) k_pack_fp64<<<nb, 256, 0, c->st>>>(c->pos, c->chrg, c->perm, n, c->dyn, c->xq64, xp64, P, c->prune_buffer, rp, dec);
+        else launch_pdl(k_pack_fp64, nb, 256, 0, c->st, c->pos, c->chrg, c->perm, n, c->dyn, c->xq64, xp64, P, c->prune_buffer, rp, dec);
+    }
     PGK_LAUNCHED(c);
     PGK_CUDA(c, cudaGetLastError());
     return PGK_OK;

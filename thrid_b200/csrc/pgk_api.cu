@@ -174,7 +174,8 @@ pgk_status force_group(pgk_ctx* c, int flag, bool ene, bool vir, bool tensor_onl
     }
     bool bonded_after_pair = false;
     if (pairs) {
-        if ((s = launch_pack(c, true))) return s;
+        // zeroed with a short group before it: the stream may have just joined that group's other streams
+        if ((s = launch_pack(c, true, zeroed && !c->short_empty))) return s;
         const int vmode = vir ? (tensor_only ? PM_TENS : PM_FULL) : (ene ? PM_ENE : PM_FORCE);
         c->rec_pre_pair = third;
         c->rec_pre_pair_done = false;

@@ -349,8 +349,9 @@ pgk_status launch_mklist(pgk_ctx* c);
 pgk_status export_nblist(pgk_ctx* c, int32_t* nb_index, int32_t* nb_list, int64_t cap, int64_t* nl);
 
 // ---- launchers (k_nonbond.cu) ----
-// pair: a pair evaluation follows (the pack then decides whether it prunes)
-pgk_status launch_pack(pgk_ctx* c, bool pair);
+// pair: a pair evaluation follows (the pack then decides whether it prunes);
+// joined: the stream may have just joined others (no dependent launch)
+pgk_status launch_pack(pgk_ctx* c, bool pair, bool joined = false);
 #define PM_FORCE 0
 #define PM_ENE 1
 #define PM_TENS 2
