@@ -202,6 +202,25 @@ static void worker_main(pgk_server* sv) {
     }
 }
 
+// sorted slots of a system: every cell padded to a multiple of 8
+static double estimate_slots(const pgk_system* s, const pgk_params* p) {
+    const double nc = std::max(1.0, std::floor(p->xcel / p->rcut_book)) *
+                      std::max(1.0, std::floor(p->ycel / p->rcut_book)) *
+                      std::max(1.0, std::floor(p->zcel / p->rcut_book));
+    return s->natom + 7.0 * nc;
+}
+
+// what pgk_set_hf and a run of nsteps add to a context (hf_setup,
+// ensure_hf_slots, the device records), with the same margin
+static int64_t estimate_hf_bytes(const pgk_system* s, const pgk_params* p, const pgk_hfparams& h, int64_t nsteps) {
+    const double nreg = h.nhfregion, hfi = std::max(1, h.heatfinterval);
+    const double bytes = estimate_slots(s, p) * (8 + 4 + 32 + 16 + 64)     // z, tag, velocities, region bits, pair sums
+                       + s->natom * (8.0 * (8 + 24 * nreg) + 24 + 3 * 4)   // arrays, random forces, indices
+                       + s->nmole * (2 * 24.0 + 4)                         // centres, velocities, thermostat type
+                       + nreg * 8.0 * (16 * 17 + PGK_HF_NCOL * ((double)nsteps / hfi + 1));   // sums, records
+    return (int64_t)(bytes * 1.25);
+}
+
 extern "C" {
 
 int64_t pgk_estimate_bytes(const pgk_system* s, const pgk_params* p) {
@@ -209,10 +228,7 @@ int64_t pgk_estimate_bytes(const pgk_system* s, const pgk_params* p) {
     const double n = s->natom;
     const bool mixed = p->precision == PGK_PREC_MIXED;
     const double vol = p->xcel * p->ycel * p->zcel;
-    const double nc = std::max(1.0, std::floor(p->xcel / p->rcut_book)) *
-                      std::max(1.0, std::floor(p->ycel / p->rcut_book)) *
-                      std::max(1.0, std::floor(p->zcel / p->rcut_book));
-    const double npad = n + 7.0 * nc;
+    const double npad = estimate_slots(s, p);
     const double rs = p->rcut_book + 2.0;
     double cap = (n / vol * 4.0 / 3.0 * 3.14159265358979 * rs * rs * rs + 128) * 1.25;   // rows regrow with headroom
     if (p->max_nbr > 0) cap = p->max_nbr;
@@ -267,7 +283,7 @@ pgk_status pgk_server_submit(pgk_server* sv, const pgk_request* r, int64_t* id) 
         if (r->hf->lt_mole_based) j->ltmole.assign(r->hf->lt_mole_based, r->hf->lt_mole_based + r->sys->nmole);
     }
     j->bytes = pgk_estimate_bytes(r->sys, r->prm);
-    if (j->has_hf) j->bytes += (int64_t)8 * r->sys->natom * (8 + 8 * 3 * j->hf.nhfregion + 12);
+    if (j->has_hf) j->bytes += estimate_hf_bytes(r->sys, r->prm, j->hf, r->nsteps);
     {
         std::lock_guard<std::mutex> lk(sv->mu);
         j->id = sv->next_id++;
