@@ -1233,6 +1233,16 @@ struct TuneVal { int p[6]; float us[6]; };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneVal> g_tune;
 
+// start and end of a timed section; destroyed on every way out
+struct TuneEvents {
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    cudaError_t create() { const cudaError_t e = cudaEventCreate(&e0); return e != cudaSuccess ? e : cudaEventCreate(&e1); }
+    ~TuneEvents() {
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+    }
+};
+
 // x_ext: as fft_pass (the half spectrum's width for the y and z passes of the
 // real-to-complex transform)
 template <typename T, int AXIS, int SRC, bool CONV>
@@ -1240,9 +1250,8 @@ static pgk_status tune_axis(pgk_ctx* c, int slot, int& best, float& best_us, int
     typedef typename C2<T>::t T2;
     const int n = c->K[AXIS];
     const int npen = AXIS == 0 ? c->K[1] * c->K[2] : (x_ext > 0 ? x_ext : c->K[0]);
-    cudaEvent_t e0, e1;
-    PGK_CUDA(c, cudaEventCreate(&e0));
-    PGK_CUDA(c, cudaEventCreate(&e1));
+    TuneEvents ev;
+    PGK_CUDA(c, ev.create());
     ConvArgs ca{};
     ca.bsp = c->bsp; ca.alpha = c->prm.alpha; ca.netchrgsq = c->netchrgsq; ca.corr = c->prm.ifnetqcorrp;
     ca.acc = c->acc; ca.want = 0; ca.K1f = x_ext > 0 ? c->K[0] : 0;
@@ -1252,18 +1261,16 @@ static pgk_status tune_axis(pgk_ctx* c, int slot, int& best, float& best_us, int
         c->fft_p[slot] = P;
         pgk_status s = fft_pass<T, AXIS, SRC, CONV>(c, -1, CONV ? &ca : nullptr, x_ext);   // warm-up (and smem limit)
         if (s) return s;
-        PGK_CUDA(c, cudaEventRecord(e0, c->st));
+        PGK_CUDA(c, cudaEventRecord(ev.e0, c->st));
         for (int r = 0; r < 3; ++r)
             if ((s = fft_pass<T, AXIS, SRC, CONV>(c, -1, CONV ? &ca : nullptr, x_ext))) return s;
-        PGK_CUDA(c, cudaEventRecord(e1, c->st));
-        PGK_CUDA(c, cudaEventSynchronize(e1));
+        PGK_CUDA(c, cudaEventRecord(ev.e1, c->st));
+        PGK_CUDA(c, cudaEventSynchronize(ev.e1));
         float ms = 0.f;
-        PGK_CUDA(c, cudaEventElapsedTime(&ms, e0, e1));
+        PGK_CUDA(c, cudaEventElapsedTime(&ms, ev.e0, ev.e1));
         const float us = ms * 1e3f / 3.f;
         if (us < best_us) { best_us = us; best = P; }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     c->fft_p[slot] = best;
     return PGK_OK;
 }
@@ -1273,27 +1280,24 @@ template <typename T>
 static pgk_status tune_rx(pgk_ctx* c, int& best, float& best_us) {
     typedef typename C2<T>::t T2;
     const int n = c->plan_rx.n, npen = c->K[1] * c->K[2];
-    cudaEvent_t e0, e1;
-    PGK_CUDA(c, cudaEventCreate(&e0));
-    PGK_CUDA(c, cudaEventCreate(&e1));
+    TuneEvents ev;
+    PGK_CUDA(c, ev.create());
     best = 0; best_us = 1e30f;
     for (int P = 1; P <= 64 && P <= npen; P *= 2) {
         if (((size_t)2 * P * (n + 1) + 2 * n + 1) * sizeof(T2) > 160 * 1024) break;
         c->fft_p[4] = P;
         pgk_status s = sizeof(T) == 4 ? fft_rx_pass<T, 1, true>(c) : fft_rx_pass<T, 2, true>(c);
         if (s) return s;
-        PGK_CUDA(c, cudaEventRecord(e0, c->st));
+        PGK_CUDA(c, cudaEventRecord(ev.e0, c->st));
         for (int r = 0; r < 3; ++r)
             if ((s = sizeof(T) == 4 ? fft_rx_pass<T, 1, true>(c) : fft_rx_pass<T, 2, true>(c))) return s;
-        PGK_CUDA(c, cudaEventRecord(e1, c->st));
-        PGK_CUDA(c, cudaEventSynchronize(e1));
+        PGK_CUDA(c, cudaEventRecord(ev.e1, c->st));
+        PGK_CUDA(c, cudaEventSynchronize(ev.e1));
         float ms = 0.f;
-        PGK_CUDA(c, cudaEventElapsedTime(&ms, e0, e1));
+        PGK_CUDA(c, cudaEventElapsedTime(&ms, ev.e0, ev.e1));
         const float us = ms * 1e3f / 3.f;
         if (us < best_us) { best_us = us; best = P; }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     c->fft_p[4] = best;
     return PGK_OK;
 }
@@ -1304,29 +1308,26 @@ template <typename T>
 static pgk_status tune_plane(pgk_ctx* c, TuneVal& v) {
     v.p[5] = 0; v.us[5] = 0.f;
     if (!plane_fits<T>(c)) return PGK_OK;
-    cudaEvent_t e0, e1;
-    PGK_CUDA(c, cudaEventCreate(&e0));
-    PGK_CUDA(c, cudaEventCreate(&e1));
+    TuneEvents ev;
+    PGK_CUDA(c, ev.create());
     float best = v.us[4] + v.us[1];
     for (int bt = 128; bt <= PLANE_BT; bt *= 2) {
         c->fft_p[5] = bt;
         pgk_status s = PGK_OK;
         for (int r = 0; r < 4 && !s; ++r) {
-            if (r == 1) PGK_CUDA(c, cudaEventRecord(e0, c->st));          // r 0: warm-up (and smem limit)
+            if (r == 1) PGK_CUDA(c, cudaEventRecord(ev.e0, c->st));          // r 0: warm-up (and smem limit)
             s = fft_plane_pass<T, sizeof(T) == 4 ? 1 : 2, true>(c);
             if (!s) s = fft_plane_pass<T, 0, false>(c);
         }
         if (s) return s;
-        PGK_CUDA(c, cudaEventRecord(e1, c->st));
-        PGK_CUDA(c, cudaEventSynchronize(e1));
+        PGK_CUDA(c, cudaEventRecord(ev.e1, c->st));
+        PGK_CUDA(c, cudaEventSynchronize(ev.e1));
         float ms = 0.f;
-        PGK_CUDA(c, cudaEventElapsedTime(&ms, e0, e1));
+        PGK_CUDA(c, cudaEventElapsedTime(&ms, ev.e0, ev.e1));
         const float us = ms * 1e3f / 6.f;
         if (v.us[5] == 0.f || us < v.us[5]) v.us[5] = us;
         if (us < best) { best = us; v.p[5] = bt; }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     c->fft_p[5] = v.p[5];
     return PGK_OK;
 }
