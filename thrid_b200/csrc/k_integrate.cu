@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(32 * RATTLE_WARPS) k_rattle_warp(double* __res
 // The multiplier's division by R.r_old uses the reciprocal of the constraint's
 // former sweep, corrected by the geometric series 1/(1 - e) = (1 + e)(1 + e^2)
 // (1 + e^4)(1 + e^8), e = 1 - (R.r_old) y; its error is e^16, and |e| > 0.1
-// divides.
+// divides, as does an e that is no number (R perpendicular to r_old before).
 // Bound by the latency of the serial FP64 chain, which is what these forms
 // shorten (one sweep of a constraint: about 12 dependent operations instead of
 // 14 and a division).  Measured, positions + velocities: 512 waters 18.0 + 12.6
@@ -856,7 +856,7 @@ __device__ __forceinline__ void rattle_group(const int (&at)[G::NA], const doubl
                 const double rr = 2.0 * fma(r0, h0, fma(r1, h1, r2 * h2));
                 const bool done = fabs(num) * rc[q] < eps;      // |r^2 - d^2| / d^2
                 const double e = fma(-rr, y[q], 1.0);
-                if (fabs(e) > 0.1) y[q] = 1.0 / rr;
+                if (!(fabs(e) <= 0.1)) y[q] = 1.0 / rr;      // NaN: y came from R.r_old = 0
                 else {
                     const double e2 = e * e, e4 = e2 * e2, e8 = e4 * e4;
                     double p = fma(e2, 1.0 + e, 1.0 + e);
