@@ -1263,7 +1263,7 @@ __global__ void __launch_bounds__(FLUX_BT) k_bonded_flux(const double* __restric
             if (q >= na) break;
             const int i = at[q];
             z[q] = hf_z(f.h, pos, i, Lz);
-            b[q] = flux_bits(f.h, z[q], Lz);
+            b[q] = flux_bits(f.h, i, z[q], Lz);
             mol[q] = f.h.hftyp[i] == PGK_HFTYP_MOLE ? ~f.h.mol_of[i] : 0;     // negative: molecule-based
             v[3 * q] = f.vel[3 * i]; v[3 * q + 1] = f.vel[3 * i + 1]; v[3 * q + 2] = f.vel[3 * i + 2];
             const double tr = share * e * flux_vz(f, i);

@@ -80,7 +80,7 @@ __global__ void k_hf_slots(const int* __restrict__ perm, int npad, const double*
     int i = perm[s];
     if (i < 0) { zs[s] = 0.0; ms[s] = HF_MS_ID; bs[s] = make_uint4(0u, 0u, 0u, 0u); return; }
     const double z = hf_z(h, pos, i, dyn->box[2]);
-    const uint4 b = flux_bits(h, z, dyn->box[2]);
+    const uint4 b = flux_bits(h, i, z, dyn->box[2]);
     zs[s] = z;
     bs[s] = b;
     ms[s] = hf_tag(h, i, b.w);
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
     if (i < f.h.natom) {
         const double vx = f.vel[3 * i], vy = f.vel[3 * i + 1], vz = f.vel[3 * i + 2];
         const double z = hf_z(f.h, pos, i, dyn->box[2]), pvz = flux_vz(f, i);
-        const uint4 m = flux_bits(f.h, z, dyn->box[2]);
+        const uint4 m = flux_bits(f.h, i, z, dyn->box[2]);
         in = m.z;
         kz = 0.5 * mass[i] * (vx * vx + vy * vy + vz * vz) * pvz;
         if (iperm) {
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(256) k_flux_kspace(const double* __restrict__ 
     double p = 0.0, v = 0.0;
     unsigned in = 0u;
     if (i < f.h.natom) {
-        in = flux_bits(f.h, hf_z(f.h, pos, i, dyn->box[2]), dyn->box[2]).z;
+        in = flux_bits(f.h, i, hf_z(f.h, pos, i, dyn->box[2]), dyn->box[2]).z;
         p = pot[i] * flux_vz(f, i);
         const double* t = vir + (size_t)9 * i + 6;
         v = t[0] * f.vel[3 * i] + t[1] * f.vel[3 * i + 1] + t[2] * f.vel[3 * i + 2];

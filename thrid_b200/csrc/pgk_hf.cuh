@@ -87,11 +87,13 @@ struct FluxDev {
                              // Coulomb, LJ) x (pairs inside one molecule, between two)
 };
 
-// bits r of a z: below slab r, above it, inside it (transport term, z wrapped
-// once more as calheatf.F90 does), exactly on one of its planes
-__device__ __forceinline__ uint4 flux_bits(const HfDev& h, double z, double Lz) {
+// bits r of atom i's heat-flux z: below slab r, above it, inside it (transport
+// term: calheatf.F90 shifts an atom's own z once, as hf_z has, and a centre of
+// mass, which calcom has shifted already, once more; the shifts matter for
+// molecules more than a box away), exactly on one of its planes
+__device__ __forceinline__ uint4 flux_bits(const HfDev& h, int i, double z, double Lz) {
     uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    const double pz = hf_wrap1(z, Lz);
+    const double pz = h.hftyp[i] == PGK_HFTYP_MOLE ? hf_wrap1(z, Lz) : z;
     for (int r = 0; r < h.nreg; ++r) {
         const unsigned b = 1u << r;
         if (z < h.z1[r]) m.x |= b;
