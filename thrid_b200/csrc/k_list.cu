@@ -201,9 +201,10 @@ __device__ __forceinline__ bool is_excluded(const int* __restrict__ exs_idx, con
 // odd and of the higher one when it is even: every cluster then owns about
 // half of its neighbours.  (All pairs in the lower cluster's row made the rows
 // of the first cell layers about twice, those of the last a third of the mean,
-// and the pair kernel's blocks as uneven.)  lower: all pairs in the lower
+// and the pair kernel's blocks as uneven.)  LOWER: all pairs in the lower
 // cluster's row (pgk_ctx::plain_order).
-__device__ __forceinline__ bool owns(int I, int J, bool lower) { return lower || ((I + J) & 1) ? I < J : I > J; }
+template <bool LOWER>
+__device__ __forceinline__ bool owns(int I, int J) { return LOWER || ((I + J) & 1) ? I < J : I > J; }
 
 // nearest integer of a moderate x (adding 1.5 2^23 rounds to one)
 __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
@@ -223,8 +224,8 @@ __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x
 //     (bins of mask_bin), each warp ranking a quarter of the candidates, and
 //     written to the row: 32 consecutive entries then mostly share their mask
 //     bits, which keeps the pair kernel's warps uniform.
-// Every step keeps the candidates' order (cells in scan order, slots ascending),
-// so a build of the same positions gives the same rows.  A row of more than
+// Every step keeps the candidates' order (LOWER: cells in scan order, slots
+// ascending), so a build of the same positions gives the same rows.  A row of more than
 // CL_CCAP candidates is sorted piece by piece (k_sort_rows joins the pieces).  nlistnball (the reference's row count, one sentinel
 // per empty row) is the number of pairs plus the atoms i < n-1 without a
 // partner of higher index; hasup[slot] = 1 marks the atoms that have one.
@@ -240,14 +241,13 @@ struct ClistArgs {
     const int* cell_of; const int* cell_start; const int* cell_cnt;
     const int* exs_idx; const int* exs_list; const int2* exs_rng;
     int ncl, ccap;
-    bool lower;
     double sqcut;
     float rbox, sqlo, sqhi;
     int* clist; int* ccnt; unsigned char* hasup; unsigned long long* counters; unsigned* status;
 };
 
-template <bool FRAME>
-__global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState* __restrict__ dyn) {
+template <bool FRAME, bool LOWER>
+__global__ void __launch_bounds__(128, LOWER ? 6 : 0) k_build_clist(ClistArgs a, const DynState* __restrict__ dyn) {
     __shared__ int sJ[4][CL_JCAP];
     __shared__ unsigned cand[CL_CCAP];
     __shared__ int hist[4][256];
@@ -324,7 +324,8 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
         if (tid == 0) a.ccnt[cl] = 0;
         return;
     }
-    const int bw = min(max(1, CL_JCAP / smaxj), (ncel + 3) >> 2);   // a warp's cells in one round of step 1
+    int bw = max(1, CL_JCAP / smaxj);                    // a warp's cells in one round of step 1
+    if (LOWER) bw = min(bw, (ncel + 3) >> 2);
     const int batch = 4 * bw;
     const float rb2 = a.rbox * a.rbox;
     int* __restrict__ row = a.clist + (size_t)cl * a.ccap;
@@ -336,11 +337,14 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
     for (int q0 = 0; q0 < ncel; q0 += batch) {
         // 1: owned clusters near the bounding box
         int nj = 0;
-        for (int q = q0 + w * bw; q < min(ncel, q0 + (w + 1) * bw); ++q) {
+        // LOWER: a warp's cells consecutive, so that the candidates come in scan order; else every fourth cell, which
+        // spreads the near cells, and with them the entries, over the warps
+        const int qs = LOWER ? 1 : 4, qb = LOWER ? q0 + w * bw : q0 + w, qe = min(ncel, LOWER ? qb + bw : q0 + batch);
+        for (int q = qb; q < qe; q += qs) {
             const int J1 = scell[q].y;
             for (int jb = scell[q].x; jb < J1; jb += 32) {
                 const int J = jb + lane;
-                bool ok = J < J1 && (J == cl || owns(cl, J, a.lower));
+                bool ok = J < J1 && (J == cl || owns<LOWER>(cl, J));
                 if (ok) {
                     const float4 c = a.cbox[2 * J], h = a.cbox[2 * J + 1];
                     float dx = c.x - ctr.x, dy = c.y - ctr.y, dz = c.z - ctr.z;
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
         __syncthreads();
         const int ntot = 8 * soff[4];                    // candidate atoms
         for (int c0 = 0; c0 < ntot; c0 += CL_CCAP) {
-            ++pieces;
+            if (LOWER) ++pieces;
             const int nc = min(CL_CCAP, ntot - c0);
             const int part = ((nc + 127) >> 7) << 5;     // a warp's share, a multiple of 32
             const int lo = w * part, hi = min(nc, lo + part);
@@ -529,7 +533,7 @@ __global__ void __launch_bounds__(128) k_build_clist(ClistArgs a, const DynState
     if (lane < 8 && ((up >> lane) & 1u)) a.hasup[s0 + lane] = 1;
     if (lane == 0 && npair) atomicAdd(&a.counters[0], (unsigned long long)npair);
     if (tid == 0) {
-        if (pieces > 1) a.counters[3] = 1ull;
+        if (LOWER && pieces > 1) a.counters[3] = 1ull;
         a.ccnt[cl] = min(count, a.ccap);
         if (count > a.ccap) atomicOr(a.status, ST_LIST_OVERFLOW);
         atomicMax(&a.counters[1], (unsigned long long)count);
@@ -730,7 +734,7 @@ pgk_status launch_mklist(pgk_ctx* c) {
         a.pf = c->pf_s; a.cbox = c->cbox; a.pos_s = c->pos_s;
         a.cell_of = c->cell_of; a.cell_start = c->cell_start; a.cell_cnt = c->cell_cnt;
         a.exs_idx = c->exs_idx; a.exs_list = c->exs_list; a.exs_rng = c->exs_rng;
-        a.ncl = c->ncl; a.ccap = c->ccap; a.lower = c->plain_order;
+        a.ncl = c->ncl; a.ccap = c->ccap;
         a.sqcut = sq; a.rbox = (float)(c->prm.rcut_book + 0.05);
         a.sqlo = (float)(sq * (1.0 - 1.0e-5) - scr); a.sqhi = (float)(sq * (1.0 + 1.0e-5) + scr);
         a.clist = c->clist; a.ccnt = c->ccnt; a.hasup = c->hasup; a.counters = c->counters; a.status = c->status;
@@ -738,8 +742,9 @@ pgk_status launch_mklist(pgk_ctx* c) {
         bool frame = true;
         for (int d = 0; d < 3; ++d)
             frame = frame && nc[d] >= 4 && c->prm.rcut_book + 0.5 * h.cellsize[d] + 0.1 < 0.5 * h.box[d];
-        if (frame) k_build_clist<true><<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
-        else k_build_clist<false><<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
+        auto* build = c->plain_order ? (frame ? k_build_clist<true, true> : k_build_clist<false, true>)
+                                     : (frame ? k_build_clist<true, false> : k_build_clist<false, false>);
+        build<<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
         const size_t ssm = (size_t)4 * (c->ccap + 256) * sizeof(int);
         if (c->plain_order && ssm <= 160 * 1024) {
             PGK_CUDA(c, smem_limit(k_sort_rows, ssm));
