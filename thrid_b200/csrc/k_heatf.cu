@@ -154,10 +154,10 @@ __global__ void __launch_bounds__(256) k_flux_atoms(const double* __restrict__ p
 // regions are FP64.  Error of the records against FP64 as with the divided 1/r
 // and per-atom FP64 virials: 2,592 atoms of propanol, LJ virials 9e-7 and 4e-7
 // of the largest region.
-// Bound by issue at 16 warps per SM.  Measured, mixed: 43,200-atom slab, 23
-// regions: 0.177 ms and 0.012 ms for the regions (0.33 ms with the regions
-// inside the pair loop, four a walk); 8,232-atom water box, one region: 0.045
-// ms.  (Velocities and f . v in FP32: 0.165 and 0.042 ms, and 1.2 to 1.5 times
+// Bound by latency at 16 warps per SM (128 registers): issue 49 % busy, stalls on
+// the entries' records and fixed latencies.  Measured, mixed: 43,200-atom slab,
+// 23 regions: 0.177 ms and 0.012 ms for the regions (0.33 ms with the regions
+// inside the pair loop, four a walk); 8,232-atom water box, one region: 0.045 ms.  (Velocities and f . v in FP32: 0.165 and 0.042 ms, and 1.2 to 1.5 times
 // the error.)
 // Rows are cut into segments until 16 warps per SM have work (small boxes).
 struct FluxPairArgs {
@@ -246,11 +246,11 @@ __device__ __forceinline__ bool hf_term(const int4& qi, const double4& pi, const
 // atoms', added over the four lanes and flushed once.  Pairs of the class
 // (same molecule / different) that the row has fewer of, and atoms exactly on
 // a plane, add to both atoms directly.
-// Bound by issue (the pair arithmetic is done twice) and by the entries'
-// atomics.  Measured, mixed: 43,200-atom slab, 23 regions 0.79 ms (4.86 ms with
-// one lane's atomics for every pair, into shared memory for the cluster atom
-// and global memory for the entry's); 8,232-atom water box, one region 0.114 ms
-// (1.27 ms).  Three blocks per SM without spills, or six regions a walk, were
+// Bound by latency at 16 warps per SM (issue 43 % busy; the pair arithmetic is
+// done twice, and the entries' records are loaded for each window).  Measured,
+// mixed: 43,200-atom slab, 23 regions 0.79 ms (4.86 ms with one lane's atomics
+// for every pair, into shared memory for the cluster atom and global memory for
+// the entry's); 8,232-atom water box, one region 0.114 ms (1.27 ms).  Three blocks per SM without spills, or six regions a walk, were
 // no faster (slab, call of 10 steps: 7.92, 8.04 ms against 7.87).
 template <bool MIXED, int KW>
 __global__ void __launch_bounds__(128, MIXED ? 4 : 3)

@@ -5,9 +5,10 @@
 // precision modes (positions, velocities, constraints, chain variables).
 //
 // Per-atom kernels are HBM-bound (one read + one write of x/v, one read of the
-// force accumulator); the chain and box kernels run on one thread and read
-// the kinetic-energy / virial sums from the fixed-point accumulators, so a
-// whole MD step needs no host round trip and can be captured in a CUDA graph.
+// force accumulator).  The chain update is serial on one lane, the step's
+// coefficients take a lane per axis and the pressure a lane per tensor
+// component, all from the kinetic-energy / virial sums in the accumulators, so
+// a whole MD step needs no host round trip and can be captured in a CUDA graph.
 #include <cmath>
 
 #include "pgk_ctx.cuh"
@@ -189,9 +190,7 @@ __global__ void k_rattle_vel(const double* __restrict__ pos, double* __restrict_
     if (!finished) atomicOr(status, ST_RATTLEV_NOCONV);
 }
 
-// sum m v^2 and sum m v_a v_b (nhcint kint, calpress kinetic terms)
-
-// ---- chain updates (single thread) -------------------------------------------
+// ---- chain updates (one lane) -------------------------------------------
 struct ChainArgs {
     pgk_mdparams md;
     int degfree;

@@ -225,12 +225,13 @@ __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x
 //     written to the row: 32 consecutive entries then mostly share their mask
 //     bits, which keeps the pair kernel's warps uniform.
 // Every step keeps the candidates' order (LOWER: cells in scan order, slots
-// ascending), so a build of the same positions gives the same rows.  A row of more than
-// CL_CCAP candidates is sorted piece by piece (k_sort_rows joins the pieces).  nlistnball (the reference's row count, one sentinel
-// per empty row) is the number of pairs plus the atoms i < n-1 without a
-// partner of higher index; hasup[slot] = 1 marks the atoms that have one.
-// Bound by issue and the latency of the candidate loads (fetched one iteration
-// ahead).  Measured: 200,004 atoms 1.78 ms (one warp per cluster, a
+// ascending), so a build of the same positions gives the same rows.  A row of
+// more than CL_CCAP candidates is sorted piece by piece (LOWER: k_sort_rows joins
+// the pieces).  nlistnball (the reference's row count, one sentinel per empty
+// row) is the number of pairs plus the atoms i < n-1 without a partner of higher
+// index; hasup[slot] = 1 marks the atoms that have one.
+// Bound by issue (63 % busy), the barriers between the steps and the latency of
+// the candidate loads (fetched one iteration ahead).  Measured: 200,004 atoms 1.78 ms (one warp per cluster, a
 // bounding-box test per atom, FP64-to-FP32 conversions per pair) -> 0.82;
 // 12,000 atoms 0.311 -> 0.093; 1,536 atoms 0.104 -> 0.030 ms.
 #define CL_JCAP (MAX_CELL_ATOMS / 8)   // clusters that a warp can queue

@@ -762,7 +762,9 @@ __global__ void __launch_bounds__(pair_threads(FRAME), pair_minb(FRAME)) k_pair_
 // 1/r comes from one reciprocal square root (rsqrt_d); the spline index is
 // floor(r/h) by a rounded-down add of 2^52.  The Coulomb cutoff is the
 // reference's dsqrt(r^2) <= rrcut whatever the rounding of r (sqrt_le_limit).
-// Bound by the FP64 pipe's dependent chains at 16 warps per SM (128 registers).  Measured, 200,004-atom butane rows with
+// Bound by the shared-memory pipe, which the 32-byte spline rows fill with bank
+// conflicts (L1 68 % busy), and by latency at 16 warps per SM (128 registers):
+// issue 40 %, FP64 pipe 36 % busy.  Measured, 200,004-atom butane rows with
 // tensor: 2.22 ms per evaluation on the book rows with divisions, sqrt and
 // dnint on 16 warps per SM; now 0.75 ms on the pruned rows.
 // 1/sqrt(x) in double: the FP32 approximation (relative error e0 ~ 1e-7) and
