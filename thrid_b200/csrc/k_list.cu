@@ -231,17 +231,22 @@ __device__ __forceinline__ float rnd_int(float x) { return __fadd_rn(__fadd_rn(x
 // row) is the number of pairs plus the atoms i < n-1 without a partner of higher
 // index; hasup[slot] = 1 marks the atoms that have one.
 // Bound by issue (63 % busy), the barriers between the steps and the latency of
-// the candidate loads (fetched one iteration ahead).  Measured: 200,004 atoms 1.78 ms (one warp per cluster, a
-// bounding-box test per atom, FP64-to-FP32 conversions per pair) -> 0.82;
-// 12,000 atoms 0.311 -> 0.093; 1,536 atoms 0.104 -> 0.030 ms.
+// the candidate loads (fetched one iteration ahead).  Measured: 200,004 atoms
+// 1.78 ms (one warp per cluster, a bounding-box test per atom, FP64-to-FP32
+// conversions per pair) -> 0.82; 12,000 atoms 0.311 -> 0.093; 1,536 atoms 0.104
+// -> 0.030 ms.
 #define CL_JCAP (MAX_CELL_ATOMS / 8)   // clusters that a warp can queue
-#define CL_CCAP 2048         // candidates sorted at a time (multiple of 128)
+// candidates sorted at a time (multiple of 128).  LOWER: the first layers' rows are twice the mean, and 4,096 take
+// them in one piece but for a few
+#define CL_CCAP(LOWER) ((LOWER) ? 4096 : 2048)
+#define ROW_PIECES ((int)0x80000000)   // ClistArgs::mark
 #define CL_EXCAP 32          // excluded partners of an atom staged in shared memory (longer lists: global)
 struct ClistArgs {
     const float4* pf; const float4* cbox; const double* pos_s;
     const int* cell_of; const int* cell_start; const int* cell_cnt;
     const int* exs_idx; const int* exs_list; const int2* exs_rng;
     int ncl, ccap;
+    int mark;                      // bit that a row sorted in pieces sets in its count (for k_sort_rows), or 0
     double sqcut;
     float rbox, sqlo, sqhi;
     int* clist; int* ccnt; unsigned char* hasup; unsigned long long* counters; unsigned* status;
@@ -250,7 +255,8 @@ struct ClistArgs {
 template <bool FRAME, bool LOWER>
 __global__ void __launch_bounds__(128, LOWER ? 6 : 0) k_build_clist(ClistArgs a, const DynState* __restrict__ dyn) {
     __shared__ int sJ[4][CL_JCAP];
-    __shared__ unsigned cand[CL_CCAP];
+    constexpr int ccap = CL_CCAP(LOWER);
+    __shared__ unsigned cand[ccap];
     __shared__ int hist[4][256];
     __shared__ int soff[5], sne[4], swarp[4], smaxj;
     __shared__ float4 sxy[4], sz[4];               // cluster atoms 2p, 2p+1: (x0, x1, y0, y1), (z0, z1, -, -)
@@ -370,9 +376,9 @@ __global__ void __launch_bounds__(128, LOWER ? 6 : 0) k_build_clist(ClistArgs a,
         }
         __syncthreads();
         const int ntot = 8 * soff[4];                    // candidate atoms
-        for (int c0 = 0; c0 < ntot; c0 += CL_CCAP) {
+        for (int c0 = 0; c0 < ntot; c0 += ccap) {
             if (LOWER) ++pieces;
-            const int nc = min(CL_CCAP, ntot - c0);
+            const int nc = min(ccap, ntot - c0);
             const int part = ((nc + 127) >> 7) << 5;     // a warp's share, a multiple of 32
             const int lo = w * part, hi = min(nc, lo + part);
             for (int q = tid; q < 4 * 256; q += 128) (&hist[0][0])[q] = 0;
@@ -534,34 +540,30 @@ __global__ void __launch_bounds__(128, LOWER ? 6 : 0) k_build_clist(ClistArgs a,
     if (lane < 8 && ((up >> lane) & 1u)) a.hasup[s0 + lane] = 1;
     if (lane == 0 && npair) atomicAdd(&a.counters[0], (unsigned long long)npair);
     if (tid == 0) {
-        if (LOWER && pieces > 1) a.counters[3] = 1ull;
-        a.ccnt[cl] = min(count, a.ccap);
+        a.ccnt[cl] = min(count, a.ccap) | (LOWER && pieces > 1 ? a.mark : 0);
         if (count > a.ccap) atomicOr(a.status, ST_LIST_OVERFLOW);
         atomicMax(&a.counters[1], (unsigned long long)count);
     }
 }
 
 // Rows that k_build_clist sorted in pieces: one stable sort over the whole row
-// (a warp per row; rows already in order are left alone).
-__global__ void __launch_bounds__(128) k_sort_rows(int* __restrict__ clist, const int* __restrict__ ccnt, int ncl, int ccap,
-                                                   const unsigned long long* __restrict__ counters) {
+// (a warp per row; rows that are not marked are left alone).
+__global__ void __launch_bounds__(128) k_sort_rows(int* __restrict__ clist, int* __restrict__ ccnt, int ncl, int ccap) {
     extern __shared__ int srow[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, cl = blockIdx.x * 4 + w;
-    if (cl >= ncl || counters[3] == 0ull) return;
+    if (cl >= ncl || ccnt[cl] >= 0) return;
     int* buf = srow + (size_t)w * (ccap + 256);
     int* bin = buf + ccap;
     int* row = clist + (size_t)cl * ccap;
-    const int n = ccnt[cl];
-    bool ok = true;
+    const int n = ccnt[cl] & ~ROW_PIECES;
+    for (int q = lane; q < 256; q += 32) bin[q] = 0;
+    __syncwarp();
+    if (lane == 0) ccnt[cl] = n;
     for (int k = lane; k < n; k += 32) {
         const int e = row[k];
         buf[k] = e;
-        ok = ok && (k == 0 || mask_bin((unsigned)row[k - 1] >> 24) <= mask_bin((unsigned)e >> 24));
+        atomicAdd(&bin[mask_bin((unsigned)e >> 24)], 1);
     }
-    if (__all_sync(0xffffffffu, ok)) return;
-    for (int q = lane; q < 256; q += 32) bin[q] = 0;
-    __syncwarp();
-    for (int k = lane; k < n; k += 32) atomicAdd(&bin[mask_bin((unsigned)buf[k] >> 24)], 1);
     __syncwarp();
     int v[8], tot = 0;                               // exclusive prefix sums of the bins, 8 a lane
 #pragma unroll
@@ -735,7 +737,9 @@ pgk_status launch_mklist(pgk_ctx* c) {
         a.pf = c->pf_s; a.cbox = c->cbox; a.pos_s = c->pos_s;
         a.cell_of = c->cell_of; a.cell_start = c->cell_start; a.cell_cnt = c->cell_cnt;
         a.exs_idx = c->exs_idx; a.exs_list = c->exs_list; a.exs_rng = c->exs_rng;
-        a.ncl = c->ncl; a.ccap = c->ccap;
+        const size_t ssm = (size_t)4 * (c->ccap + 256) * sizeof(int);      // k_sort_rows
+        const bool sort = c->plain_order && ssm <= 160 * 1024;
+        a.ncl = c->ncl; a.ccap = c->ccap; a.mark = sort ? ROW_PIECES : 0;
         a.sqcut = sq; a.rbox = (float)(c->prm.rcut_book + 0.05);
         a.sqlo = (float)(sq * (1.0 - 1.0e-5) - scr); a.sqhi = (float)(sq * (1.0 + 1.0e-5) + scr);
         a.clist = c->clist; a.ccnt = c->ccnt; a.hasup = c->hasup; a.counters = c->counters; a.status = c->status;
@@ -746,10 +750,9 @@ pgk_status launch_mklist(pgk_ctx* c) {
         auto* build = c->plain_order ? (frame ? k_build_clist<true, true> : k_build_clist<false, true>)
                                      : (frame ? k_build_clist<true, false> : k_build_clist<false, false>);
         build<<<c->ncl, 128, 0, c->st>>>(a, c->dyn);
-        const size_t ssm = (size_t)4 * (c->ccap + 256) * sizeof(int);
-        if (c->plain_order && ssm <= 160 * 1024) {
+        if (sort) {
             PGK_CUDA(c, smem_limit(k_sort_rows, ssm));
-            k_sort_rows<<<(c->ncl + 3) / 4, 128, ssm, c->st>>>(c->clist, c->ccnt, c->ncl, c->ccap, c->counters);
+            k_sort_rows<<<(c->ncl + 3) / 4, 128, ssm, c->st>>>(c->clist, c->ccnt, c->ncl, c->ccap);
             PGK_LAUNCHED(c);
         }
         if (n > 1) k_count_noup<<<(n - 1 + 255) / 256, 256, 0, c->st>>>(c->hasup, c->iperm, n - 1, c->counters);

@@ -186,7 +186,7 @@ struct pgk_ctx {
     double4* xq64 = nullptr;      // fp64: x,y,z,q sorted
     int* typ_s = nullptr;
     unsigned long long* counters = nullptr;   // [0] list pairs, [1] longest cluster row, [2] rows without
-                                              //  a higher-index partner, [3] rows sorted in pieces; [4..6] count_pairs scratch
+                                              //  a higher-index partner; [4..6] count_pairs scratch
     unsigned char* hasup = nullptr;           // [npad_cap] a slot's atom has a list partner of higher index
     bool list_valid = false;
     long long list_epoch = 0;     // incremented by every list build (invalidates captured graphs)
